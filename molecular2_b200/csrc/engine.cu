@@ -9,6 +9,7 @@
 
 #include "engine.h"
 #include "md.cuh"
+#include "quartet.cuh"
 
 namespace m2 {
 
@@ -214,6 +215,51 @@ static std::vector<double> boys_table() {
   return t;
 }
 
+// Polynomial Boys tables: per order and interval the polynomial of degree
+// BOYSP_COEF - 1 in (T - centre) that interpolates F_m at the interval's
+// Chebyshev nodes, in extended precision.
+static std::vector<double> boys_poly_tables() {
+  constexpr int NC = BOYSP_COEF, M = BOYSP_MMAX;
+  const long double width = (long double)BOYS_TMAX / BOYSP_ROWS, pi = acosl(-1.0L);
+  std::vector<double> t((size_t)(M + 1) * BOYSP_SIZE);
+  for (int row = 0; row < BOYSP_ROWS; ++row) {
+    const long double mid = (row + 0.5L) * width;
+    long double f[M + 1][NC];  // F_m at the nodes
+    for (int j = 0; j < NC; ++j) {
+      const long double T = mid + 0.5L * width * cosl(pi * (j + 0.5L) / NC), ex = expl(-T);
+      long double term = 1.0L / (2 * M + 1), sum = term;
+      for (int i = 1; i < 2000 && term > 1e-22L * sum; ++i) {
+        term *= 2.0L * T / (2 * M + 2 * i + 1);
+        sum += term;
+      }
+      f[M][j] = ex * sum;
+      for (int m = M - 1; m >= 0; --m) f[m][j] = (2.0L * T * f[m + 1][j] + ex) / (2 * m + 1);
+    }
+    for (int m = 0; m <= M; ++m) {
+      // Chebyshev coefficients, then powers of u = (T - mid) / (width / 2)
+      long double mono[NC] = {0}, t0[NC] = {0}, t1[NC] = {0};
+      t0[0] = 1.0L;
+      t1[1] = 1.0L;
+      for (int k = 0; k < NC; ++k) {
+        long double c = 0.0L;
+        for (int j = 0; j < NC; ++j) c += f[m][j] * cosl(pi * k * (j + 0.5L) / NC);
+        c *= (k == 0 ? 1.0L : 2.0L) / NC;
+        for (int i = 0; i < NC; ++i) mono[i] += c * t0[i];
+        long double t2[NC];  // T_{k+2} = 2 u T_{k+1} - T_k
+        for (int i = 0; i < NC; ++i) t2[i] = (i > 0 ? 2.0L * t1[i - 1] : 0.0L) - t0[i];
+        for (int i = 0; i < NC; ++i) {
+          t0[i] = t1[i];
+          t1[i] = t2[i];
+        }
+      }
+      long double sc = 1.0L;
+      for (int i = 0; i < NC; ++i, sc *= 2.0L / width)
+        t[(size_t)m * BOYSP_SIZE + row * NC + i] = (double)(mono[i] * sc);
+    }
+  }
+  return t;
+}
+
 // ---------------------------------------------------------------- transforms
 // Dc[a][b] = sum T[mu][a] Df[mu][nu] T[nu][b] over the shells' pure blocks
 // (identity for Cartesian shells).  One thread per Cartesian element.
@@ -372,6 +418,10 @@ int jk_create(const jk_basis* obs, const jk_basis* aux, int natom, const double*
   rc = upload_basis(e, e->obs, e->dobs);
   if (rc == JK_OK && e->has_aux) rc = upload_basis(e, e->aux, e->daux);
   if (rc == JK_OK) rc = check_cuda(e, e->boys.upload(boys_table(), e->stream), "boys table");
+  if (rc == JK_OK) {
+    static const std::vector<double> poly = boys_poly_tables();
+    rc = check_cuda(e, e->boysp.upload(poly, e->stream), "boys polynomials");
+  }
   if (rc == JK_OK) rc = check_cuda(e, cudaStreamSynchronize(e->stream), "boys table");
   if (rc == JK_OK) rc = build_pairs(e);
   *out = e;

@@ -73,10 +73,20 @@ struct PairClassHost {
   std::vector<int> sa, sb, prim_off, nprim;
   std::vector<double> Q;
 };
+// One class's part of the engine's pooled pair arrays.
+template <class T>
+struct DevSpan {
+  T* p = nullptr;
+};
 struct PairClassDev {
   int la = 0, lb = 0, npair = 0;
-  DevBuf<int> sa, sb, prim_off, nprim;
-  DevBuf<double> Q;
+  DevSpan<int> sa, sb, prim_off, nprim;
+  DevSpan<double> Q;
+  // entries: slices of a pair's primitives (quartet.cuh)
+  int nent = 0, max_np = 0;
+  DevSpan<int> ent_pair, ent_np, ent_first;
+  DevSpan<long long> ent_goff;
+  DevSpan<double> ent_prim;
 };
 
 struct DFState {
@@ -157,16 +167,19 @@ struct jk_engine {
 
   // shell pairs (orbital basis)
   m2::PairClassDev pcls[m2::NPAIRCLASS];
+  m2::DevBuf<int> pair_ints;                         // pools behind pcls
+  m2::DevBuf<double> pair_dbls;
+  m2::DevBuf<long long> pair_offs;
   m2::DevBuf<double> pp_p, pp_x, pp_y, pp_z, pp_K, pp_a;  // primitive pairs (pp_a: exponent of shell a)
   m2::DevBuf<double> ap_p, ap_x, ap_y, ap_z, ap_K;         // fitting primitives as (P, unit) pairs
   m2::DevBuf<int> aux_prim_off;                           // per fitting shell
   m2::DevBuf<int> aux_by_l[m2::MAX_L_AUX + 1];             // fitting shells grouped by l
   int aux_by_l_count[m2::MAX_L_AUX + 1] = {0, 0, 0, 0};
   std::vector<double> schwarz_host;                  // nshell x nshell, row-major (symmetric)
-  m2::DevBuf<double> schwarz_dev;                    // nshell x nshell
   double Qmax = 0.0;
 
   m2::DevBuf<double> boys;                           // Boys table
+  m2::DevBuf<double> boysp;                          // polynomial Boys tables (quartet.cuh)
 
   // scratch for J/K builds
   m2::DevBuf<double> Dcart, Jcart, Kcart, Dnorm, Dmax, Dfinal, Jfinal, Kfinal;

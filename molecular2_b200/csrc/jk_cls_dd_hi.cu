@@ -3,13 +3,9 @@
 #include "jk_kernels.cuh"
 
 namespace m2 {
-void launch_jk_bra_dd_hi(int B, int nden, const JKParams& P, dim3 grid, cudaStream_t s) {
-  if (B == 4) { if (nden == 2) k_jk_direct<2, 2, 2, 1, 2><<<grid, 128, 0, s>>>(P); else k_jk_direct<2, 2, 2, 1><<<grid, 128, 0, s>>>(P); }
-  if (B == 5) { if (nden == 2) k_jk_direct<2, 2, 2, 2, 2><<<grid, 128, 0, s>>>(P); else k_jk_direct<2, 2, 2, 2><<<grid, 128, 0, s>>>(P); }
-}
-
-void launch_schwarz_dd(const SchwarzParams& P, dim3 grid, cudaStream_t s) {
-  k_schwarz<2, 2><<<grid, 64, 0, s>>>(P);
+void launch_jk_bra_dd_hi(int B, const JKParams& P, dim3 grid, cudaStream_t s) {
+  if (B == 4) launch_jk_class<2, 2, 2, 1>(P, grid, s);
+  if (B == 5) launch_jk_class<2, 2, 2, 2>(P, grid, s);
 }
 
 }  // namespace m2

@@ -5,19 +5,19 @@
 // six angular classes ss, ps, pp, ds, dp, dd and, inside a class, sorted by
 // their Schwarz bound Q_ab (descending).  A unique shell quartet is a pair of
 // pairs {ab, cd}: class(ab) > class(cd), or the same class with index(cd) <=
-// index(ab).  One kernel instantiation per class pair (21 for l <= 2), the 21
-// launches of a build spread longest first over the engine's side streams so
-// that they run concurrently; a block owns one bra pair and a chunk of kets,
-// one thread one quartet.  Because kets
-// are Q-sorted, the kets that can pass Q_ab Q_cd Dmax >= precision form a
-// prefix found by binary search; each quartet then applies molecular2's
-// screen max6(|D| shell blocks) Q_ab Q_cd >= precision (:111-115).
+// index(ab).  Pairs are cut into entries of at most ENTRY_PRIMS primitive pairs
+// (quartet.cuh) and the kernels work on entry pairs.  One kernel instantiation
+// per class pair (21 for l <= 2), the 21 launches of a build spread longest
+// first over the engine's side streams so that they run concurrently.  Because
+// kets are Q-sorted, the kets that can pass Q_ab Q_cd Dmax >= precision form a
+// prefix found by binary search; each ket then goes through molecular2's
+// screen max6(|D| shell blocks) Q_ab Q_cd >= precision (:111-115) before a
+// thread takes it.
 //
 // Digestion follows :121-153 (6 updates with the permutational degeneracy
 // factor, symmetrised at the end with the 1/4 of :161-162).  J_ab is shared by
-// the whole block and is reduced with warp shuffles before one atomic per
-// element per warp; the other five blocks are accumulated per quartet and
-// added with FP64 atomics.  Everything runs in the Cartesian representation:
+// the whole block and reduced in it before one atomic per element; the other
+// five blocks are added per entry pair with FP64 atomics.  Everything runs in the Cartesian representation:
 // D is transformed to Cartesian functions first and J, K back afterwards.
 #include <algorithm>
 #include <cmath>
@@ -33,20 +33,71 @@ namespace m2 {
 
 PairView view(const PairClassDev& c) { return PairView{c.sa.p, c.sb.p, c.prim_off.p, c.nprim.p, c.Q.p, c.npair}; }
 
+EntryView entry_view(const PairClassDev& c) {
+  return EntryView{c.ent_pair.p, c.ent_np.p, c.ent_first.p, c.ent_goff.p, c.ent_prim.p, c.nent};
+}
+
 PrimView prim_view(const jk_engine* e) { return PrimView{e->pp_p.p, e->pp_x.p, e->pp_y.p, e->pp_z.p, e->pp_K.p}; }
 
 ShellView shell_view(const jk_engine* e) {
   return ShellView{e->dobs.x.p, e->dobs.y.p, e->dobs.z.p, e->dobs.cart_off.p};
 }
 
-static void launch_schwarz(int la, int lb, const SchwarzParams& P, int npair, cudaStream_t s) {
-  dim3 grid((npair + 63) / 64);
-  if (la == 0 && lb == 0) k_schwarz<0, 0><<<grid, 64, 0, s>>>(P);
-  if (la == 1 && lb == 0) k_schwarz<1, 0><<<grid, 64, 0, s>>>(P);
-  if (la == 1 && lb == 1) k_schwarz<1, 1><<<grid, 64, 0, s>>>(P);
-  if (la == 2 && lb == 0) k_schwarz<2, 0><<<grid, 64, 0, s>>>(P);
-  if (la == 2 && lb == 1) k_schwarz<2, 1><<<grid, 64, 0, s>>>(P);
-  if (la == 2 && lb == 2) launch_schwarz_dd(P, grid, s);
+// Entries of one sorted class (quartet.cuh): each pair's primitives, largest
+// prefactor first, in slices of nearly equal length.
+struct HostEntries {
+  std::vector<int> pair, np, first;
+  std::vector<long long> goff;
+  std::vector<double> prim;
+};
+static void build_entries(const PairClassHost& c, const std::vector<double>* pp, HostEntries& E) {
+  const std::vector<double>&p = pp[0], &x = pp[1], &y = pp[2], &z = pp[3], &K = pp[4], &al = pp[5];
+  const int np = (int)c.sa.size();
+  std::vector<int> order, prims;  // prims: primitive of each (entry, slot), entry by entry
+  E.first.resize(np + 1);
+  for (int i = 0; i < np; ++i) {
+    E.first[i] = (int)E.pair.size();
+    const int n = c.nprim[i], ne = (n + ENTRY_PRIMS - 1) / ENTRY_PRIMS;
+    order.resize(n);
+    std::iota(order.begin(), order.end(), c.prim_off[i]);
+    if (n > 1)
+      std::stable_sort(order.begin(), order.end(),
+                       [&](int u, int v) { return std::fabs(K[u]) * p[v] > std::fabs(K[v]) * p[u]; });
+    for (int k = 0, o = 0; k < ne; ++k) {
+      const int m = (n - o + (ne - k) - 1) / (ne - k);
+      E.pair.push_back(i);
+      E.np.push_back(m);
+      prims.insert(prims.end(), order.begin() + o, order.begin() + o + m);
+      o += m;
+    }
+  }
+  const int nent = (int)E.pair.size();
+  E.first[np] = nent;
+  E.goff.resize((nent + 31) / 32);
+  long long tot = 0;
+  for (int g = 0; g < (int)E.goff.size(); ++g) {
+    E.goff[g] = tot;
+    int mx = 0;
+    for (int e = 32 * g; e < std::min(nent, 32 * g + 32); ++e) mx = std::max(mx, E.np[e]);
+    tot += (long long)mx * ENTRY_FIELDS * 32;
+  }
+  E.prim.assign(tot, 0.0);
+  const double c2pi = std::sqrt(PI25X2());
+  for (int e = 0, o = 0; e < nent; ++e)
+    for (int k = 0; k < E.np[e]; ++k, ++o) {
+      const int i = prims[o];
+      const double f[ENTRY_FIELDS] = {p[i], x[i], y[i], z[i], K[i] * c2pi / p[i], 0.5 / p[i], al[i]};
+      double* q = E.prim.data() + E.goff[e / 32] + (long long)k * ENTRY_FIELDS * 32 + e % 32;
+      for (int j = 0; j < ENTRY_FIELDS; ++j) q[j * 32] = f[j];
+    }
+}
+
+// Appends v to a pool and returns its position there.
+template <class T>
+static size_t append(std::vector<T>& pool, const std::vector<T>& v) {
+  const size_t o = pool.size();
+  pool.insert(pool.end(), v.begin(), v.end());
+  return o;
 }
 
 int build_pairs(jk_engine* e) {
@@ -57,7 +108,8 @@ int build_pairs(jk_engine* e) {
       cls[pair_class(la, lb)].la = la;
       cls[pair_class(la, lb)].lb = lb;
     }
-  std::vector<double> pp_p, pp_x, pp_y, pp_z, pp_K, pp_a;
+  std::vector<double> pp[6];
+  std::vector<double>&pp_p = pp[0], &pp_x = pp[1], &pp_y = pp[2], &pp_z = pp[3], &pp_K = pp[4], &pp_a = pp[5];
   for (int i = 0; i < hb.nshell; ++i)
     for (int j = 0; j < hb.nshell; ++j) {
       const int li = hb.l[i], lj = hb.l[j];
@@ -97,30 +149,56 @@ int build_pairs(jk_engine* e) {
   if (st == cudaSuccess) st = e->pp_a.upload(pp_a, s);
   if (st != cudaSuccess) return check_cuda(e, st, "upload primitive pairs");
 
-  // Schwarz bounds on the GPU, class by class
+  // Schwarz bounds on the GPU, all classes from one upload
   const int ns = hb.nshell;
   e->schwarz_host.assign((size_t)ns * ns, 0.0);
   e->Qmax = 0.0;
+  size_t ntot = 0;
+  std::vector<int> ints;
+  size_t io[NPAIRCLASS][4], qo[NPAIRCLASS];
   for (int k = 0; k < NPAIRCLASS; ++k) {
     PairClassHost& c = cls[k];
     PairClassDev& d = e->pcls[k];
     d.la = c.la;
     d.lb = c.lb;
     d.npair = (int)c.sa.size();
-    if (d.npair == 0) continue;
-    st = d.sa.upload(c.sa, s);
-    if (st == cudaSuccess) st = d.sb.upload(c.sb, s);
-    if (st == cudaSuccess) st = d.prim_off.upload(c.prim_off, s);
-    if (st == cudaSuccess) st = d.nprim.upload(c.nprim, s);
-    if (st == cudaSuccess) st = d.Q.alloc(d.npair);
+    io[k][0] = append(ints, c.sa);
+    io[k][1] = append(ints, c.sb);
+    io[k][2] = append(ints, c.prim_off);
+    io[k][3] = append(ints, c.nprim);
+    qo[k] = ntot;
+    ntot += c.sa.size();
+  }
+  std::vector<double> Q(ntot);
+  if (ntot > 0) {
+    DevBuf<int> di;
+    DevBuf<double> dq;
+    st = di.upload(ints, s);
+    if (st == cudaSuccess) st = dq.alloc(ntot);
     if (st != cudaSuccess) return check_cuda(e, st, "upload pairs");
-    SchwarzParams P{view(d), prim_view(e), shell_view(e), e->dobs.l.p, e->dobs.pure.p, e->dobs.sph.p,
-                    e->boys.p, d.Q.p};
-    launch_schwarz(c.la, c.lb, P, d.npair, s);
-    c.Q.resize(d.npair);
-    st = cudaMemcpyAsync(c.Q.data(), d.Q.p, d.npair * sizeof(double), cudaMemcpyDeviceToHost, s);
+    for (int k = 0; k < NPAIRCLASS; ++k) {
+      if (e->pcls[k].npair == 0) continue;
+      const PairView v{di.p + io[k][0], di.p + io[k][1], di.p + io[k][2], di.p + io[k][3], nullptr, e->pcls[k].npair};
+      SchwarzParams P{v, prim_view(e), shell_view(e), e->dobs.l.p, e->dobs.pure.p, e->dobs.sph.p, e->boys.p,
+                      dq.p + qo[k]};
+      launch_schwarz(cls[k].la, cls[k].lb, P, e->pcls[k].npair, s);
+    }
+    st = cudaMemcpyAsync(Q.data(), dq.p, ntot * sizeof(double), cudaMemcpyDeviceToHost, s);
     if (st == cudaSuccess) st = cudaStreamSynchronize(s);
     if (st != cudaSuccess) return check_cuda(e, st, "schwarz kernel");
+  }
+
+  // sort each class, cut it into entries, and upload everything from one pool per type
+  struct Pos {
+    size_t sa, sb, off, np, Q, epair, enp, efirst, goff, prim;
+  } pos[NPAIRCLASS];
+  ints.clear();
+  std::vector<double> dbls;
+  std::vector<long long> offs;
+  for (int k = 0; k < NPAIRCLASS; ++k) {
+    PairClassHost& c = cls[k];
+    PairClassDev& d = e->pcls[k];
+    c.Q.assign(Q.begin() + qo[k], Q.begin() + qo[k] + d.npair);
     // sort the class by Q descending
     std::vector<int> order(d.npair);
     std::iota(order.begin(), order.end(), 0);
@@ -143,26 +221,45 @@ int build_pairs(jk_engine* e) {
       e->schwarz_host[(size_t)c.sb[o] * ns + c.sa[o]] = c.Q[o];
       e->Qmax = std::max(e->Qmax, c.Q[o]);
     }
-    st = d.sa.upload(sorted.sa, s);
-    if (st == cudaSuccess) st = d.sb.upload(sorted.sb, s);
-    if (st == cudaSuccess) st = d.prim_off.upload(sorted.prim_off, s);
-    if (st == cudaSuccess) st = d.nprim.upload(sorted.nprim, s);
-    if (st == cudaSuccess) st = d.Q.upload(sorted.Q, s);
-    if (st == cudaSuccess) st = cudaStreamSynchronize(s);
-    if (st != cudaSuccess) return check_cuda(e, st, "upload sorted pairs");
+    HostEntries E;
+    build_entries(sorted, pp, E);
+    d.nent = (int)E.pair.size();
+    d.max_np = E.np.empty() ? 0 : *std::max_element(E.np.begin(), E.np.end());
+    pos[k] = Pos{append(ints, sorted.sa), append(ints, sorted.sb), append(ints, sorted.prim_off),
+                 append(ints, sorted.nprim), append(dbls, sorted.Q), append(ints, E.pair), append(ints, E.np),
+                 append(ints, E.first), append(offs, E.goff), 0};
+    dbls.resize((dbls.size() + 31) / 32 * 32);  // a warp's 32 doubles start on a 256-byte boundary
+    pos[k].prim = append(dbls, E.prim);
   }
-  st = e->schwarz_dev.upload(e->schwarz_host, s);
-  if (st == cudaSuccess) st = cudaStreamSynchronize(s);
-  return check_cuda(e, st, "schwarz matrix");
+  st = e->pair_ints.upload(ints, s);
+  if (st == cudaSuccess) st = e->pair_dbls.upload(dbls, s);
+  if (st == cudaSuccess) st = e->pair_offs.upload(offs, s);
+  if (st == cudaSuccess) st = cudaStreamSynchronize(s);  // host vectors die on return
+  if (st != cudaSuccess) return check_cuda(e, st, "upload sorted pairs");
+  for (int k = 0; k < NPAIRCLASS; ++k) {
+    PairClassDev& d = e->pcls[k];
+    const Pos& o = pos[k];
+    int* pi = e->pair_ints.p;
+    d.sa.p = pi + o.sa;
+    d.sb.p = pi + o.sb;
+    d.prim_off.p = pi + o.off;
+    d.nprim.p = pi + o.np;
+    d.Q.p = e->pair_dbls.p + o.Q;
+    d.ent_pair.p = pi + o.epair;
+    d.ent_np.p = pi + o.enp;
+    d.ent_first.p = pi + o.efirst;
+    d.ent_goff.p = e->pair_offs.p + o.goff;
+    d.ent_prim.p = e->pair_dbls.p + o.prim;
+  }
+  return JK_OK;
 }
 
-// Kets per block: one per thread (128) when the class has enough (bra, chunk)
-// blocks to fill the GPU; classes with few bra pairs take smaller chunks so
-// their work still spreads over about 4 blocks per SM (idle threads of a
-// block only cost its residency).
-static int ket_chunk(int nbra, int nket_max) {
-  int k = 128;
-  while (k > 32 && (long long)nbra * ((nket_max + k - 1) / k) < 4 * 148) k /= 2;
+// Ket entries per block: many, so that the bra set-up (Boys table, term
+// products) is shared, but fewer for classes whose blocks would not fill the
+// GPU otherwise.
+static int ket_chunk(long long nbra, long long nket, int layers) {
+  int k = JK_LIST;
+  while (k > 32 && nbra * ((nket + k - 1) / k) * layers < (k > JK_THREADS ? 32 : 8) * 148) k /= 2;
   return k;
 }
 
@@ -195,24 +292,29 @@ static void launch_classes(jk_engine* e, cudaStream_t s, Launch&& launch) {
   cs.join();
 }
 
-static void launch_jk(const jk_engine* e, int A, int B, const JKParams& Pin, int nbra, int nket_max, cudaStream_t s,
-                      int nden = 1) {
+static void launch_jk(const jk_engine* e, int A, int B, const JKParams& Pin, cudaStream_t s) {
   JKParams P = Pin;
+  const PairClassDev &ca = e->pcls[A], &cb = e->pcls[B];
   int nb = 0;
-  bra_share(e, nbra, P.bra0, P.bra_step, nb);
+  bra_share(e, ca.npair, P.bra0, P.bra_step, nb);
   if (nb == 0) return;
-  P.kchunk = ket_chunk(nb, nket_max);
-  dim3 grid(nb, (nket_max + P.kchunk - 1) / P.kchunk);
+  P.bra = view(ca);
+  P.ket = view(cb);
+  P.bra_ent = entry_view(ca);
+  P.ket_ent = entry_view(cb);
+  P.same_class = (A == B);
+  P.kchunk = ket_chunk((long long)ca.nent / P.bra_step, cb.nent, jk_layers(ca.la, ca.lb, cb.la, cb.lb));
+  dim3 grid(ca.nent, (cb.nent + P.kchunk - 1) / P.kchunk);
   if (A <= 2)
-    launch_jk_bra_s(A, B, nden, P, grid, s);
+    launch_jk_bra_s(A, B, P, grid, s);
   else if (A == 3)
-    launch_jk_bra_ds(B, nden, P, grid, s);
+    launch_jk_bra_ds(B, P, grid, s);
   else if (A == 4)
-    launch_jk_bra_dp(B, nden, P, grid, s);
+    launch_jk_bra_dp(B, P, grid, s);
   else if (B < 4)
-    launch_jk_bra_dd_lo(B, nden, P, grid, s);
+    launch_jk_bra_dd_lo(B, P, grid, s);
   else
-    launch_jk_bra_dd_hi(B, nden, P, grid, s);
+    launch_jk_bra_dd_hi(B, P, grid, s);
 }
 
 int direct_jk_device(jk_engine* e, const double* dD, double precision, double mult, double* dJ, double* dK,
@@ -237,27 +339,23 @@ int direct_jk_device(jk_engine* e, const double* dD, double precision, double mu
   cudaMemsetAsync(e->class_work.p, 0, sizeof(unsigned long long) * 3 * NPAIRCLASS * NPAIRCLASS, s);
   e->class_work_valid = true;
   JKParams P{};
-  P.pp = prim_view(e);
   P.sh = shell_view(e);
   P.Dnorm = e->Dnorm.p;
   P.nshell = ns;
   P.Dmax = e->Dmax.p;
+  P.nden = 1;
   P.Dc = e->Dcart.p;
   P.nc = nc;
   P.Jc = e->Jcart.p;
   P.Kc = e->Kcart.p;
   P.dstride = (size_t)nc * nc;
   P.precision = precision;
-  P.boys = e->boys.p;
+  P.boysp = e->boysp.p;
   P.counter = counter;
-  P.kchunk = 128;  // one ket per thread: small classes still spread over the SMs
   launch_classes(e, s, [&](int A, int B, cudaStream_t cs) {
     JKParams Q = P;
-    Q.bra = view(e->pcls[A]);
-    Q.ket = view(e->pcls[B]);
-    Q.same_class = (A == B);
     Q.work = e->class_work.p + 3 * (A * NPAIRCLASS + B);
-    launch_jk(e, A, B, Q, e->pcls[A].npair, e->pcls[B].npair, cs);
+    launch_jk(e, A, B, Q, cs);
   });
   // J = 1/4 (J + J^T) mult, K = 1/2 * 1/4 (K + K^T) mult  (src/fockbuild.cpp:146-149, 161-162)
   launch_cart_to_final_sym(e, e->Jcart.p, 0.25 * mult, dJ, s);
@@ -291,18 +389,18 @@ int direct_jk_uhf_device(jk_engine* e, const double* dDa, const double* dDb, dou
   e->last_counter = counter;
   cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s);
   JKParams P{};
-  P.pp = prim_view(e);
   P.sh = shell_view(e);
   P.Dnorm = e->Dnorm.p;
   P.nshell = ns;
   P.Dmax = e->Dmax.p;
+  P.nden = 2;
   P.Dc = Dc2.p;
   P.nc = nc;
   P.Jc = Jc2.p;
   P.Kc = Kc2.p;
   P.dstride = ncc;
   P.precision = precision;
-  P.boys = e->boys.p;
+  P.boysp = e->boysp.p;
   P.counter = counter;
   if ((st = e->class_work.alloc(3 * NPAIRCLASS * NPAIRCLASS)) != cudaSuccess)
     return check_cuda(e, st, "jk_direct_uhf work counters");
@@ -310,11 +408,8 @@ int direct_jk_uhf_device(jk_engine* e, const double* dDa, const double* dDb, dou
   e->class_work_valid = true;
   launch_classes(e, s, [&](int A, int B, cudaStream_t cs) {
     JKParams Q = P;
-    Q.bra = view(e->pcls[A]);
-    Q.ket = view(e->pcls[B]);
-    Q.same_class = (A == B);
     Q.work = e->class_work.p + 3 * (A * NPAIRCLASS + B);
-    launch_jk(e, A, B, Q, e->pcls[A].npair, e->pcls[B].npair, cs, 2);
+    launch_jk(e, A, B, Q, cs);
   });
   launch_cart_to_final_sym(e, Jc2.p, 0.25 * mult, dJa, s);
   launch_cart_to_final_sym(e, Jc2.p + ncc, 0.25 * mult, dJb, s);
@@ -394,26 +489,21 @@ int direct_jk_noalloc(jk_engine* e, const double* dD, double precision, double m
   cudaMemsetAsync(Kc, 0, sizeof(double) * nc * nc, s);
   cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s);
   JKParams P{};
-  P.pp = prim_view(e);
   P.sh = shell_view(e);
   P.Dnorm = Dn;
   P.nshell = ns;
   P.Dmax = Dmax;
+  P.nden = 1;
   P.Dc = Dc;
   P.nc = nc;
   P.Jc = Jc;
   P.Kc = Kc;
   P.precision = precision;
-  P.boys = e->boys.p;
+  P.boysp = e->boysp.p;
   P.counter = counter;
   P.dstride = NOALLOC_CC;
-  P.kchunk = 128;  // one ket per thread: small classes still spread over the SMs
   launch_classes(e, s, [&](int A, int B, cudaStream_t cs) {
-    JKParams Q = P;
-    Q.bra = view(e->pcls[A]);
-    Q.ket = view(e->pcls[B]);
-    Q.same_class = (A == B);
-    launch_jk(e, A, B, Q, e->pcls[A].npair, e->pcls[B].npair, cs);
+    launch_jk(e, A, B, P, cs);
   });
   launch_cart_to_final_sym(e, Jc, 0.25 * mult, dJ, s);
   launch_cart_to_final_sym(e, Kc, 0.125 * mult, dK, s);

@@ -2,6 +2,7 @@
 // Included by the per-class translation units jk_cls_*.cu and jk_direct.cu.
 #pragma once
 #include "md.cuh"
+#include "quartet.cuh"
 
 namespace m2 {
 
@@ -171,23 +172,24 @@ __device__ __forceinline__ void quartet_cart(const PrimView& pp, int b0, int nb,
 
 struct JKParams {
   PairView bra, ket;
+  EntryView bra_ent, ket_ent;
   int same_class;
-  PrimView pp;
   ShellView sh;
   const double* Dnorm;  // nshell x nshell (final-basis shell-block max norms)
   int nshell;
   const double* Dmax;   // device scalar
-  const double* Dc;     // Cartesian density, nc x nc (NDEN of them, dstride apart)
+  int nden;             // densities digested per quartet: 1 (RHF), or the two spins of UHF (1 or 2)
+  const double* Dc;     // Cartesian density, nc x nc (nden of them, dstride apart)
   int nc;
-  double* Jc;           // raw accumulators (NDEN of each, dstride apart)
+  double* Jc;           // raw accumulators (nden of each, dstride apart)
   double* Kc;
   size_t dstride;       // elements between consecutive densities / accumulators
   double precision;
-  const double* boys;
+  const double* boysp;  // polynomial Boys tables, BOYSP_SIZE doubles per order
   unsigned long long* counter;
   unsigned long long* work;  // NULL or this class pair's [quartets, sum bra primitive pairs, sum primitive quartets]
-  int kchunk;
-  int bra0, bra_step;        // block x handles bra pair bra0 + x * bra_step (a rank's share of the class)
+  int kchunk;                // ket entries per block, at most JK_LIST
+  int bra0, bra_step;        // this rank's bra pairs: bra0, bra0 + bra_step, ...
 };
 
 // Pairs of a class are sorted by Schwarz bound Q descending and then, inside
@@ -219,142 +221,312 @@ __device__ __forceinline__ void atomic_add_f64(double* a, double v) {
   if (v != 0.0) atomicAdd(a, v);
 }
 
-// NDEN densities (1: RHF; 2: the alpha and beta densities of UHF,
-// UnrestrictedFock::formJKdirect, src/fockbuild.cpp:266-362) are digested from
-// the same integrals; the screen uses the norms of their sum.
-template <int LA, int LB, int LC, int LD, int NDEN = 1>
-__global__ void __launch_bounds__(128) k_jk_direct(const JKParams P) {
-  constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
-  constexpr bool BIG = NA * NB * NC * ND > UNROLL_LIMIT;
-  const int bra = P.bra0 + blockIdx.x * P.bra_step;
+// How a thread works on its quartet.  JK_FULL: all ket components at once, the
+// ket s or p shell with an s shell.  JK_PP: one first-shell component of a pp
+// ket per block layer (blockIdx.z), its three partners together.  JK_ONE: one
+// ket component per layer.  The layers recompute the Hermite integrals R
+// (nherm(L) of them, ~2 flops each) but leave the Hermite-space sums W and R in
+// registers; a thread that holds a whole p or d quartet spills them.
+enum { JK_FULL = 0, JK_PP = 1, JK_ONE = 2 };
+__host__ __device__ constexpr int jk_mode(int la, int lb, int lc, int ld) {
+  if (lc == 0) return JK_FULL;
+  if (lc == 1 && ld == 0) return ncart(la) * ncart(lb) <= 9 ? JK_FULL : JK_ONE;
+  if (lc == 1 && ld == 1 && ncart(la) * ncart(lb) <= 9) return JK_PP;
+  return JK_ONE;
+}
+__host__ __device__ constexpr int jk_layers(int la, int lb, int lc, int ld) {
+  return jk_mode(la, lb, lc, ld) == JK_FULL ? 1
+         : jk_mode(la, lb, lc, ld) == JK_PP ? ncart(lc)
+                                            : ncart(lc) * ncart(ld);
+}
+constexpr int JK_THREADS = 128;
+constexpr int JK_LIST = 1024;      // most ket entries of one block
+// primitive quartets whose prefactor is below this in every lane are skipped
+// (their integrals are below 1e-18, like the primitive pairs never listed)
+constexpr double JK_PRIM_EPS = 1e-21;
+
+template <int LA, int LB>
+struct JKShared {
+  double boys[BOYSP_SIZE];
+  BraShared<LA, LB> bra;
+  double Dab[2][ncart(LA) * ncart(LB)];
+  int list[JK_LIST];
+  int n;
+};
+template <int LA, int LB>
+constexpr size_t jk_smem(int nden) {
+  return sizeof(JKShared<LA, LB>) + sizeof(double) * (size_t)nden * ncart(LA) * ncart(LB) * JK_THREADS + 16;
+}
+
+// Direct J/K of one class pair.  Block (x, y, z): bra entry x, ket entries
+// [y kchunk, (y + 1) kchunk), component layer z.  The block first screens its
+// kets and packs the survivors (density screening leaves 60 % of the lanes of
+// a fixed ket-to-lane map busy on C20H42), then a thread takes one survivor at
+// a time: Hermite sums W over the ket primitives for each bra primitive, bra
+// transform from the tables in shared memory, digestion with FP64 atomics.
+// J_ab is kept per thread in shared memory and reduced once per block.
+// Two densities (UHF, UnrestrictedFock::formJKdirect,
+// src/fockbuild.cpp:266-362) are digested from the same integrals; the screen
+// uses the norms of their sum.
+// Measured (one thread per contracted quartet with its 6 to 81 integrals in
+// local memory -> this kernel): H2O/cc-pVDZ 18.0 -> 0.29 ms, (H2O)8/cc-pVDZ
+// 44.3 -> 5.0 ms, C20H42/6-311G** 262 -> 52 ms.  What bounds it now, on C20H42:
+// the L1 data path (40 to 73 % of its wavefronts, nine Boys coefficients and
+// five fields per primitive quartet, scattered density reads) and 5.6e9 FP64
+// atomics (107 of the 185 G/s that random addresses allow); the FP64 pipe is
+// at 20 to 33 %.  Entries of 16 primitives were slower (56 ms, and 0.66 ms on
+// H2O, whose longest chain they double).
+template <int LA, int LB, int LC, int LD>
+__global__ void __launch_bounds__(JK_THREADS) k_jk_direct(const JKParams P) {
+  constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD), NAB = NA * NB;
+  constexpr int LAB = LA + LB, LCD = LC + LD, L = LAB + LCD, HAB = nherm(LAB);
+  constexpr int MODE = jk_mode(LA, LB, LC, LD);
+  constexpr int GC = MODE == JK_FULL ? NC : 1, GD = MODE == JK_ONE ? 1 : ND, G = GC * GD;
+  extern __shared__ __align__(16) unsigned char jk_sm[];
+  JKShared<LA, LB>& S = *reinterpret_cast<JKShared<LA, LB>*>(jk_sm);
+  double* s_jab = reinterpret_cast<double*>(jk_sm + ((sizeof(JKShared<LA, LB>) + 15) & ~(size_t)15));
+
+  const int eb = blockIdx.x;
+  const int bra = P.bra_ent.pair[eb];
+  if (bra % P.bra_step != P.bra0) return;
   const int a = P.bra.sa[bra], b = P.bra.sb[bra];
   const double Qab = P.bra.Q[bra];
   const double Dmax = *P.Dmax;
   if (!(Qab * Dmax > 0.0)) return;
-  int nket = window_up(q_prefix(P.ket.Q, P.ket.npair, P.precision / (Qab * Dmax)), P.ket.npair);
-  if (P.same_class) nket = min(nket, bra + 1);
+  int npk = window_up(q_prefix(P.ket.Q, P.ket.npair, P.precision / (Qab * Dmax)), P.ket.npair);
+  if (P.same_class) npk = min(npk, bra + 1);
+  const int nent = P.ket_ent.first[npk];
   const int start = blockIdx.y * P.kchunk;
-  if (start >= nket) return;
-  const int end = min(start + P.kchunk, nket);
+  if (start >= nent) return;
+  const int end = min(start + P.kchunk, nent);
+  const int tid = threadIdx.x, lane = tid & 31;
 
-  const double Ax = P.sh.x[a], Ay = P.sh.y[a], Az = P.sh.z[a];
-  const double Bx = P.sh.x[b], By = P.sh.y[b], Bz = P.sh.z[b];
-  const int a0 = P.sh.coff[a], b0 = P.sh.coff[b];
-  const int bp0 = P.bra.prim_off[bra], bnp = P.bra.nprim[bra];
-  const int nc = P.nc;
-
-  double jab[NDEN][NA * NB];
-#pragma unroll
-  for (int dd = 0; dd < NDEN; ++dd)
-#pragma unroll
-    for (int i = 0; i < NA * NB; ++i) jab[dd][i] = 0.0;
+  // screen: max6(|D| blocks) Q_ab Q_cd >= precision
+  if (tid == 0) S.n = 0;
+  __syncthreads();
   unsigned long long cnt = 0, wb = 0, wq = 0;
-
-  for (int kl = start + threadIdx.x; kl < end; kl += blockDim.x) {
-    const int c = P.ket.sa[kl], d = P.ket.sb[kl];
-    const double Qcd = P.ket.Q[kl];
+  {
     const double* Dn = P.Dnorm;
     const int ns = P.nshell;
-    double dn = fmax(fmax(Dn[a * ns + b], Dn[c * ns + d]), fmax(Dn[a * ns + c], Dn[a * ns + d]));
-    dn = fmax(dn, fmax(Dn[b * ns + c], Dn[b * ns + d]));
-    if (dn * Qab * Qcd < P.precision) continue;
-    ++cnt;
-    wb += bnp;
-    wq += (unsigned long long)bnp * P.ket.nprim[kl];
-    double eri[NA * NB * NC * ND];
-    quartet_cart<LA, LB, LC, LD>(P.pp, bp0, bnp, Ax, Ay, Az, Bx, By, Bz, P.pp, P.ket.prim_off[kl], P.ket.nprim[kl],
-                                 P.sh.x[c], P.sh.y[c], P.sh.z[c], P.sh.x[d], P.sh.y[d], P.sh.z[d], P.boys, eri);
-    const double deg = ((a == b) ? 1.0 : 2.0) * ((c == d) ? 1.0 : 2.0) * ((P.same_class && kl == bra) ? 1.0 : 2.0);
-    const int c0 = P.sh.coff[c], d0 = P.sh.coff[d];
-#pragma unroll
-    for (int dd = 0; dd < NDEN; ++dd) {
-    const double* __restrict__ Dc = P.Dc + dd * P.dstride;
-    double* __restrict__ Jd = P.Jc + dd * P.dstride;
-    double* __restrict__ Kd = P.Kc + dd * P.dstride;
-    double jcd[NC * ND], kac[NA * NC], kbd[NB * ND], kad[NA * ND], kbc[NB * NC];
-#pragma unroll
-    for (int i = 0; i < NC * ND; ++i) jcd[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < NA * NC; ++i) kac[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < NB * ND; ++i) kbd[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < NA * ND; ++i) kad[i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < NB * NC; ++i) kbc[i] = 0.0;
-    if constexpr (!BIG) {
-#pragma unroll
-      for (int ia = 0; ia < NA; ++ia)
-#pragma unroll
-        for (int ib = 0; ib < NB; ++ib) {
-          const double dab = Dc[(size_t)(a0 + ia) * nc + b0 + ib];
-#pragma unroll
-          for (int ic = 0; ic < NC; ++ic) {
-            const double dac = Dc[(size_t)(a0 + ia) * nc + c0 + ic];
-            const double dbc = Dc[(size_t)(b0 + ib) * nc + c0 + ic];
-#pragma unroll
-            for (int id = 0; id < ND; ++id) {
-              const double v = eri[((ia * NB + ib) * NC + ic) * ND + id] * deg;
-              jab[dd][ia * NB + ib] += Dc[(size_t)(c0 + ic) * nc + d0 + id] * v;
-              jcd[ic * ND + id] += dab * v;
-              kac[ia * NC + ic] += Dc[(size_t)(b0 + ib) * nc + d0 + id] * v;
-              kbd[ib * ND + id] += dac * v;
-              kad[ia * ND + id] += dbc * v;
-              kbc[ib * NC + ic] += Dc[(size_t)(a0 + ia) * nc + d0 + id] * v;
-            }
-          }
+    const double dab = Dn[a * ns + b];
+    const bool count = blockIdx.z == 0 && P.bra_ent.first[bra] == eb;
+    const int bnp = P.bra.nprim[bra];
+    for (int e0 = start; e0 < end; e0 += JK_THREADS) {
+      const int e = e0 + tid;
+      bool pass = false;
+      if (e < end) {
+        const int kl = P.ket_ent.pair[e];
+        const int c = P.ket.sa[kl], d = P.ket.sb[kl];
+        double dn = fmax(fmax(dab, Dn[c * ns + d]), fmax(Dn[a * ns + c], Dn[a * ns + d]));
+        dn = fmax(dn, fmax(Dn[b * ns + c], Dn[b * ns + d]));
+        pass = !(dn * Qab * P.ket.Q[kl] < P.precision);
+        if (pass && count && P.ket_ent.first[kl] == e) {
+          ++cnt;
+          wb += bnp;
+          wq += (unsigned long long)bnp * P.ket.nprim[kl];
         }
-    } else {
-#pragma unroll 1
-      for (int ia = 0; ia < NA; ++ia)
-#pragma unroll 1
-        for (int ib = 0; ib < NB; ++ib) {
-          const double dab = Dc[(size_t)(a0 + ia) * nc + b0 + ib];
-          double jsum = 0.0;
-#pragma unroll 1
-          for (int ic = 0; ic < NC; ++ic) {
-            const double dac = Dc[(size_t)(a0 + ia) * nc + c0 + ic];
-            const double dbc = Dc[(size_t)(b0 + ib) * nc + c0 + ic];
-            double kacs = 0.0, kbcs = 0.0;
-#pragma unroll
-            for (int id = 0; id < ND; ++id) {
-              const double v = eri[((ia * NB + ib) * NC + ic) * ND + id] * deg;
-              jsum += Dc[(size_t)(c0 + ic) * nc + d0 + id] * v;
-              jcd[ic * ND + id] += dab * v;
-              kacs += Dc[(size_t)(b0 + ib) * nc + d0 + id] * v;
-              kbd[ib * ND + id] += dac * v;
-              kad[ia * ND + id] += dbc * v;
-              kbcs += Dc[(size_t)(a0 + ia) * nc + d0 + id] * v;
-            }
-            kac[ia * NC + ic] += kacs;
-            kbc[ib * NC + ic] += kbcs;
-          }
-          jab[dd][ia * NB + ib] += jsum;
-        }
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, pass);
+      int pos = 0;
+      if (lane == 0 && m) pos = atomicAdd(&S.n, __popc(m));
+      pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(m & ((1u << lane) - 1));
+      if (pass) S.list[pos] = e;
     }
-#pragma unroll
-    for (int i = 0; i < NC * ND; ++i) atomic_add_f64(Jd + (size_t)(c0 + i / ND) * nc + d0 + i % ND, jcd[i]);
-#pragma unroll
-    for (int i = 0; i < NA * NC; ++i) atomic_add_f64(Kd + (size_t)(a0 + i / NC) * nc + c0 + i % NC, kac[i]);
-#pragma unroll
-    for (int i = 0; i < NB * ND; ++i) atomic_add_f64(Kd + (size_t)(b0 + i / ND) * nc + d0 + i % ND, kbd[i]);
-#pragma unroll
-    for (int i = 0; i < NA * ND; ++i) atomic_add_f64(Kd + (size_t)(a0 + i / ND) * nc + d0 + i % ND, kad[i]);
-#pragma unroll
-    for (int i = 0; i < NB * NC; ++i) atomic_add_f64(Kd + (size_t)(b0 + i / NC) * nc + c0 + i % NC, kbc[i]);
-    }  // densities
   }
-  // J_ab: the whole block shares the bra pair
-  const unsigned lane = threadIdx.x & 31;
-#pragma unroll
-  for (int dd = 0; dd < NDEN; ++dd)
-#pragma unroll
-    for (int i = 0; i < NA * NB; ++i) {
-      double v = jab[dd][i];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-      if (lane == 0) atomic_add_f64(P.Jc + dd * P.dstride + (size_t)(a0 + i / NB) * nc + b0 + i % NB, v);
+  __syncthreads();
+  const int n = S.n;
+  if (n == 0) return;
+
+  const int a0 = P.sh.coff[a], b0 = P.sh.coff[b], nc = P.nc;
+  const int nb = P.bra_ent.np[eb];
+  for (int i = tid; i < BOYSP_SIZE; i += JK_THREADS) S.boys[i] = __ldg(P.boysp + (size_t)L * BOYSP_SIZE + i);
+  for (int i = tid; i < P.nden * NAB; i += JK_THREADS)
+    S.Dab[i / NAB][i % NAB] =
+        P.Dc[(i / NAB) * P.dstride + (size_t)(a0 + (i % NAB) / NB) * nc + b0 + (i % NAB) % NB];
+  for (int i = 0; i < P.nden * NAB; ++i) s_jab[i * JK_THREADS + tid] = 0.0;
+  load_bra<LA, LB>(S.bra, entry_prims(P.bra_ent, eb), nb, P.sh.x[a], P.sh.y[a], P.sh.z[a], P.sh.x[b], P.sh.y[b],
+                   P.sh.z[b]);
+
+  // this layer's ket component (block-uniform)
+  int ic0 = 0, id0 = 0, cx = 0, cy = 0, cz = 0, dx = 0, dy = 0, dz = 0;
+  if constexpr (MODE == JK_PP) ic0 = blockIdx.z;
+  if constexpr (MODE == JK_ONE) {
+    ic0 = blockIdx.z / ND;
+    id0 = blockIdx.z % ND;
+    if constexpr (LD > 0) {
+      dx = c_herm.t[nherm(LD - 1) + id0];
+      dy = c_herm.u[nherm(LD - 1) + id0];
+      dz = c_herm.v[nherm(LD - 1) + id0];
     }
+  }
+  if constexpr (MODE != JK_FULL && LC > 0) {
+    cx = c_herm.t[nherm(LC - 1) + ic0];
+    cy = c_herm.u[nherm(LC - 1) + ic0];
+    cz = c_herm.v[nherm(LC - 1) + ic0];
+  }
+
+  for (int t0 = (tid >> 5) * 32; t0 < n; t0 += JK_THREADS) {
+    const bool active = t0 + lane < n;
+    const int e = S.list[active ? t0 + lane : n - 1];
+    const int kl = P.ket_ent.pair[e];
+    const int c = P.ket.sa[kl], d = P.ket.sb[kl];
+    const double* kp = entry_prims(P.ket_ent, e);
+    const int nk = P.ket_ent.np[e];
+    const int nkm = __reduce_max_sync(0xffffffffu, nk);
+    const double deg = !active ? 0.0
+                               : ((a == b) ? 1.0 : 2.0) * ((c == d) ? 1.0 : 2.0) *
+                                     ((P.same_class && kl == bra) ? 1.0 : 2.0);
+    double Cx = 0, Cy = 0, Cz = 0, Ex = 0, Ey = 0, Ez = 0;
+    if constexpr (LC > 0) {
+      Cx = P.sh.x[c];
+      Cy = P.sh.y[c];
+      Cz = P.sh.z[c];
+    }
+    if constexpr (LD > 0) {
+      Ex = P.sh.x[d];
+      Ey = P.sh.y[d];
+      Ez = P.sh.z[d];
+    }
+    double v[NAB * G];  // [ab][c][d]
+#pragma unroll
+    for (int i = 0; i < NAB * G; ++i) v[i] = 0.0;
+    for (int ib = 0; ib < nb; ++ib) {
+      const double p = S.bra.prim[ib][0], Px = S.bra.prim[ib][1], Py = S.bra.prim[ib][2], Pz = S.bra.prim[ib][3];
+      const double Kb = S.bra.prim[ib][4] * deg;
+      double W[G][HAB];
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+#pragma unroll
+        for (int h = 0; h < HAB; ++h) W[g][h] = 0.0;
+      for (int k = 0; k < nkm; ++k) {
+        const int kk = min(k, nk - 1);
+        const double KK = k < nk ? Kb * entry_field(kp, kk, 4) : 0.0;
+        if (!__any_sync(0xffffffffu, fabs(KK) > JK_PRIM_EPS)) break;  // largest first: the rest is smaller
+        const double q = entry_field(kp, kk, 0);
+        const double Qx = entry_field(kp, kk, 1), Qy = entry_field(kp, kk, 2), Qz = entry_field(kp, kk, 3);
+        double R[nherm(L)];
+        quartet_R<L>(p, q, KK, Px - Qx, Py - Qy, Pz - Qz, S.boys, R);
+        if constexpr (LCD == 0) {
+#pragma unroll
+          for (int h = 0; h < HAB; ++h) W[0][h] += R[h];
+        } else if constexpr (MODE == JK_FULL) {  // ps
+          const double h2 = entry_field(kp, kk, 5);
+          const double QC[3] = {Qx - Cx, Qy - Cy, Qz - Cz};
+          static_for<3 * HAB>([&](auto gh) {
+            constexpr int g = decltype(gh)::value / HAB, h = decltype(gh)::value % HAB;
+            W[g][h] += QC[g] * R[h] - h2 * R[hidx(herm_t(h) + (g == 0), herm_u(h) + (g == 1), herm_v(h) + (g == 2))];
+          });
+        } else {
+          const double h2 = entry_field(kp, kk, 5);
+          double e1[3][LCD + 1];
+          const double QC[3] = {Qx - Cx, Qy - Cy, Qz - Cz}, QD[3] = {Qx - Ex, Qy - Ey, Qz - Ez};
+          const int ce[3] = {cx, cy, cz}, de[3] = {dx, dy, dz};
+#pragma unroll
+          for (int x = 0; x < 3; ++x) {
+            e1[x][0] = 1.0;
+#pragma unroll
+            for (int t = 1; t <= LCD; ++t) e1[x][t] = 0.0;
+#pragma unroll
+            for (int s = 0; s < LC; ++s)
+              if (s < ce[x]) e1_raise<LCD>(e1[x], QC[x], h2);
+            if constexpr (MODE == JK_ONE)
+#pragma unroll
+              for (int s = 0; s < LD; ++s)
+                if (s < de[x]) e1_raise<LCD>(e1[x], QD[x], h2);
+          }
+          if constexpr (MODE == JK_ONE) {
+            ket_accumulate<LAB, LCD>(W[0], R, e1[0], e1[1], e1[2], cx + dx, cy + dy, cz + dz);
+          } else {
+#pragma unroll
+            for (int g = 0; g < GD; ++g) {
+              double r[LCD + 1];
+#pragma unroll
+              for (int t = 0; t <= LCD; ++t) r[t] = e1[g][t];
+              e1_raise<LCD>(r, QD[g], h2);
+              ket_accumulate<LAB, LCD>(W[g], R, g == 0 ? r : e1[0], g == 1 ? r : e1[1], g == 2 ? r : e1[2],
+                                       cx + (g == 0), cy + (g == 1), cz + (g == 2));
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int g = 0; g < G; ++g) bra_transform<LA, LB, G>(S.bra.M[LAB > 0 ? ib : 0], W[g], v + g);
+    }
+    // digestion: 6 updates per integral (src/fockbuild.cpp:121-153)
+    const int c0 = P.sh.coff[c] + ic0, d0 = P.sh.coff[d] + id0;
+#pragma unroll 1
+    for (int dd = 0; dd < P.nden; ++dd) {
+      const double* __restrict__ Dc = P.Dc + dd * P.dstride;
+      double* __restrict__ Jd = P.Jc + dd * P.dstride;
+      double* __restrict__ Kd = P.Kc + dd * P.dstride;
+      double* jab = s_jab + (size_t)dd * NAB * JK_THREADS + tid;
+      const double* Dab = S.Dab[dd];
+      double Dcd[G];
+#pragma unroll
+      for (int g = 0; g < G; ++g) Dcd[g] = Dc[(size_t)(c0 + g / GD) * nc + d0 + g % GD];
+#pragma unroll
+      for (int i = 0; i < NAB; ++i) {
+        double s = 0.0;
+#pragma unroll
+        for (int g = 0; g < G; ++g) s += Dcd[g] * v[i * G + g];
+        jab[i * JK_THREADS] += s;
+      }
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        double s = 0.0;
+#pragma unroll
+        for (int i = 0; i < NAB; ++i) s += Dab[i] * v[i * G + g];
+        atomic_add_f64(Jd + (size_t)(c0 + g / GD) * nc + d0 + g % GD, s);
+      }
+      // K_ac, K_bc from D_bd, D_ad; K_ad, K_bd from D_bc, D_ac
+#pragma unroll
+      for (int side = 0; side < 2; ++side) {
+        const int r0 = side ? d0 : c0, q0 = side ? c0 : d0;
+        constexpr int GX[2] = {GC, GD};
+        const int nr = GX[side], nq = GX[1 - side];
+#pragma unroll
+        for (int r = 0; r < nr; ++r) {
+          double ka[NA], kb[NB];
+#pragma unroll
+          for (int i = 0; i < NA; ++i) ka[i] = 0.0;
+#pragma unroll
+          for (int j = 0; j < NB; ++j) kb[j] = 0.0;
+#pragma unroll
+          for (int q = 0; q < nq; ++q) {
+            const int g = side ? q * GD + r : r * GD + q;
+            double Da[NA], Db[NB];
+#pragma unroll
+            for (int i = 0; i < NA; ++i) Da[i] = Dc[(size_t)(a0 + i) * nc + q0 + q];
+#pragma unroll
+            for (int j = 0; j < NB; ++j) Db[j] = Dc[(size_t)(b0 + j) * nc + q0 + q];
+#pragma unroll
+            for (int i = 0; i < NA; ++i)
+#pragma unroll
+              for (int j = 0; j < NB; ++j) {
+                ka[i] += Db[j] * v[(i * NB + j) * G + g];
+                kb[j] += Da[i] * v[(i * NB + j) * G + g];
+              }
+          }
+#pragma unroll
+          for (int i = 0; i < NA; ++i) atomic_add_f64(Kd + (size_t)(a0 + i) * nc + r0 + r, ka[i]);
+#pragma unroll
+          for (int j = 0; j < NB; ++j) atomic_add_f64(Kd + (size_t)(b0 + j) * nc + r0 + r, kb[j]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // J_ab: one warp per component
+  for (int i = tid >> 5; i < P.nden * NAB; i += JK_THREADS / 32) {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < JK_THREADS / 32; ++w) s += s_jab[i * JK_THREADS + w * 32 + lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0)
+      atomic_add_f64(P.Jc + (i / NAB) * P.dstride + (size_t)(a0 + (i % NAB) / NB) * nc + b0 + (i % NAB) % NB, s);
+  }
+  if (blockIdx.z != 0) return;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     cnt += __shfl_down_sync(0xffffffffu, cnt, o);
@@ -369,6 +541,14 @@ __global__ void __launch_bounds__(128) k_jk_direct(const JKParams P) {
       atomicAdd(P.work + 2, wq);
     }
   }
+}
+
+template <int LA, int LB, int LC, int LD>
+inline void launch_jk_class(const JKParams& P, dim3 grid, cudaStream_t s) {
+  const size_t sm = jk_smem<LA, LB>(P.nden);
+  cudaFuncSetAttribute(k_jk_direct<LA, LB, LC, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  grid.z = jk_layers(LA, LB, LC, LD);
+  k_jk_direct<LA, LB, LC, LD><<<grid, JK_THREADS, sm, s>>>(P);
 }
 
 // Schwarz bound of each pair of one class: sqrt(max diag (ab|ab)) over the
@@ -432,13 +612,14 @@ __global__ void __launch_bounds__(64) k_schwarz(const SchwarzParams P) {
 struct PairClassDev;
 PairView view(const PairClassDev& c);
 
+EntryView entry_view(const PairClassDev& c);
+
 // per-translation-unit launchers (jk_cls_*.cu); A, B are pair-class ids
-// nden: densities digested per quartet (1 or 2)
-void launch_jk_bra_s(int A, int B, int nden, const JKParams& P, dim3 grid, cudaStream_t s);   // A in {0,1,2}
-void launch_jk_bra_ds(int B, int nden, const JKParams& P, dim3 grid, cudaStream_t s);         // A = 3
-void launch_jk_bra_dp(int B, int nden, const JKParams& P, dim3 grid, cudaStream_t s);         // A = 4
-void launch_jk_bra_dd_lo(int B, int nden, const JKParams& P, dim3 grid, cudaStream_t s);      // A = 5, B < 4
-void launch_jk_bra_dd_hi(int B, int nden, const JKParams& P, dim3 grid, cudaStream_t s);      // A = 5, B >= 4
-void launch_schwarz_dd(const SchwarzParams& P, dim3 grid, cudaStream_t s);
+void launch_jk_bra_s(int A, int B, const JKParams& P, dim3 grid, cudaStream_t s);   // A in {0,1,2}
+void launch_jk_bra_ds(int B, const JKParams& P, dim3 grid, cudaStream_t s);         // A = 3
+void launch_jk_bra_dp(int B, const JKParams& P, dim3 grid, cudaStream_t s);         // A = 4
+void launch_jk_bra_dd_lo(int B, const JKParams& P, dim3 grid, cudaStream_t s);      // A = 5, B < 4
+void launch_jk_bra_dd_hi(int B, const JKParams& P, dim3 grid, cudaStream_t s);      // A = 5, B >= 4
+void launch_schwarz(int la, int lb, const SchwarzParams& P, int npair, cudaStream_t s);  // schwarz.cu
 
 }  // namespace m2
