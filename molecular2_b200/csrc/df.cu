@@ -17,12 +17,14 @@
 // (dense.cu).
 #include <algorithm>
 #include <cmath>
+#include <functional>
 #include <string>
 #include <vector>
 
 #include "dense.cuh"
 #include "df_kernels.cuh"
 #include "engine.h"
+#include "onebody.cuh"
 
 namespace m2 {
 
@@ -33,7 +35,7 @@ int prepare_aux(jk_engine* e) {
   if (!e->has_aux) return set_error(e, JK_ERR_STATE, "no fitting basis was given to jk_create");
   if (e->ap_p.p) return JK_OK;
   const HostBasis& a = e->aux;
-  std::vector<double> p, x, y, z, K;
+  std::vector<double> p, x, y, z, K, Kp, h;
   std::vector<int> off;
   for (int s = 0; s < a.nshell; ++s) {
     off.push_back((int)p.size());
@@ -43,6 +45,8 @@ int prepare_aux(jk_engine* e) {
       y.push_back(a.xyz[3 * s + 1]);
       z.push_back(a.xyz[3 * s + 2]);
       K.push_back(a.coefs[a.prim_off[s] + k]);
+      Kp.push_back(K.back() * SQRT_PI25X2() / p.back());
+      h.push_back(0.5 / p.back());
     }
   }
   cudaStream_t st = e->stream;
@@ -51,6 +55,8 @@ int prepare_aux(jk_engine* e) {
   if (r == cudaSuccess) r = e->ap_y.upload(y, st);
   if (r == cudaSuccess) r = e->ap_z.upload(z, st);
   if (r == cudaSuccess) r = e->ap_K.upload(K, st);
+  if (r == cudaSuccess) r = e->ap_Kp.upload(Kp, st);
+  if (r == cudaSuccess) r = e->ap_h.upload(h, st);
   if (r == cudaSuccess) r = e->aux_prim_off.upload(off, st);
   for (int l = 0; l <= MAX_L_AUX && r == cudaSuccess; ++l) {
     std::vector<int> sh;
@@ -58,6 +64,12 @@ int prepare_aux(jk_engine* e) {
       if (a.l[s] == l) sh.push_back(s);
     e->aux_by_l_count[l] = (int)sh.size();
     r = e->aux_by_l[l].upload(sh, st);
+  }
+  std::vector<int> groups[jk_engine::NAUXGROUP];
+  for (int s = 0; s < a.nshell; ++s) groups[a.l[s] <= 1 ? a.l[s] : 2 * a.l[s] - (a.pure[s] ? 2 : 1)].push_back(s);
+  for (int g = 0; g < jk_engine::NAUXGROUP && r == cudaSuccess; ++g) {
+    e->aux_group_count[g] = (int)groups[g].size();
+    r = e->aux_group[g].upload(groups[g], st);
   }
   if (r == cudaSuccess) r = cudaStreamSynchronize(st);
   return check_cuda(e, r, "prepare fitting basis");
@@ -67,51 +79,96 @@ static PrimView aux_view(const jk_engine* e) {
   return PrimView{e->ap_p.p, e->ap_x.p, e->ap_y.p, e->ap_z.p, e->ap_K.p};
 }
 
-// Launch parameters of the three-index kernels for fitting shells of angular
-// momentum l and orbital pair class pc.
-Eri3Params eri3_params(const jk_engine* e, int l, int pc) {
+// Launch parameters of the three-index kernels for fitting group g and orbital
+// pair class pc.
+static Eri3Params eri3_params(const jk_engine* e, int g, int pc) {
   Eri3Params P{};
-  P.ap = aux_view(e);
-  P.aux_shells = e->aux_by_l[l].p;
-  P.naux_shells = e->aux_by_l_count[l];
-  P.aux_prim_off = e->aux_prim_off.p;
-  P.aux_nprim = e->daux.nprim.p;
-  P.ax = e->daux.x.p;
-  P.ay = e->daux.y.p;
-  P.az = e->daux.z.p;
-  P.aux_foff = e->daux.final_off.p;
-  P.aux_pure = e->daux.pure.p;
+  P.aux = AuxView{e->aux_group[g].p, e->aux_group_count[g], e->aux_prim_off.p, e->daux.nprim.p,
+                  e->ap_p.p,         e->ap_x.p,             e->ap_y.p,         e->ap_z.p,
+                  e->ap_Kp.p,        e->ap_h.p,             e->daux.final_off.p};
+  P.ent = entry_view(e->pcls[pc]);
   P.pairs = view(e->pcls[pc]);
-  P.pp = prim_view(e);
   P.ox = e->dobs.x.p;
   P.oy = e->dobs.y.p;
   P.oz = e->dobs.z.p;
   P.obs_foff = e->dobs.final_off.p;
   P.obs_pure = e->dobs.pure.p;
   P.sph = e->dobs.sph.p;
-  P.boys = e->boys.p;
-  P.n = e->obs.n_final;
+  P.boysp = e->boysp.p;
   P.naux = e->aux.n_final;
+  P.nlist = e->pcls[pc].npair;
+  P.n = e->obs.n_final;
   return P;
 }
 
-// T3[x][P][y] = (P|xy), full n x naux x n.
+// Every (fitting group, pair class) launch, longest first on the side streams
+// (cost: pairs x fitting shells x Cartesian sizes), so that the small ones fill
+// the tails of the large ones; they write disjoint parts of T, or add to J.
+// set(P, pc) completes the parameters and says whether the class has work.
+int eri3_all(jk_engine* e, bool j, cudaStream_t s, const std::function<bool(Eri3Params&, int)>& set) {
+  static const double ncp[NPAIRCLASS] = {1, 3, 9, 6, 18, 36};
+  static const int gl[jk_engine::NAUXGROUP] = {0, 1, 2, 2, 3, 3};
+  struct Item {
+    int g, pc;
+    double cost;
+    Eri3Params P;
+  };
+  std::vector<Item> items;
+  for (int g = 0; g < jk_engine::NAUXGROUP; ++g)
+    for (int pc = 0; pc < NPAIRCLASS; ++pc) {
+      if (!e->aux_group_count[g] || !e->pcls[pc].npair) continue;
+      Item it{g, pc, 0.0, eri3_params(e, g, pc)};
+      if (!set(it.P, pc)) continue;
+      it.cost = (double)it.P.nlist * e->aux_group_count[g] * ncp[pc] * (gl[g] + 1) * (gl[g] + 2);
+      items.push_back(it);
+    }
+  std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.cost > b.cost; });
+  static decltype(&launch_eri3_s) const launch[jk_engine::NAUXGROUP] = {
+      launch_eri3_s, launch_eri3_p, launch_eri3_d_pure, launch_eri3_d_cart, launch_eri3_f_pure, launch_eri3_f_cart};
+  ClassStreams cs(e, s);
+  for (const Item& it : items) launch[it.g](it.pc, it.P, j, cs.next(it.cost));
+  cs.join();
+  return check_cuda(e, cudaGetLastError(), "three-index launch");
+}
+
+// T3[x][y][P] = (P|xy), full n x n x naux.
 static int compute_T3(jk_engine* e, double* T3, cudaStream_t s) {
   const int n = e->obs.n_final, naux = e->aux.n_final;
   cudaMemsetAsync(T3, 0, sizeof(double) * (size_t)n * naux * n, s);
-  for (int l = 0; l <= MAX_L_AUX; ++l) {
-    if (!e->aux_by_l_count[l]) continue;
-    for (int pc = 0; pc < NPAIRCLASS; ++pc) {
-      if (!e->pcls[pc].npair) continue;
-      Eri3Params P = eri3_params(e, l, pc);
-      P.T3 = T3;
-      if (l == 0) launch_eri3_l0(pc, P, s);
-      if (l == 1) launch_eri3_l1(pc, P, s);
-      if (l == 2) launch_eri3_l2(pc, P, s);
-      if (l == 3) launch_eri3_l3(pc, P, s);
-    }
-  }
-  return check_cuda(e, cudaGetLastError(), "eri3 launch");
+  return eri3_all(e, false, s, [&](Eri3Params& P, int) {
+    P.nrow = P.ncol = n;
+    P.T = T3;
+    return true;
+  });
+}
+
+// cc[a] = coefficients c of the final fitting functions on their Cartesian components
+__global__ void k_aux_cart(int nc, const int* __restrict__ cshell, const int* __restrict__ ccomp,
+                           const int* __restrict__ l, const int* __restrict__ pure, const int* __restrict__ foff,
+                           const double* __restrict__ sph, const double* __restrict__ c, double* __restrict__ cc) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nc) return;
+  const int sh = cshell[i], ic = ccomp[i], ls = l[sh], f0 = foff[sh];
+  double v = 0.0;
+  if (pure[sh])
+    for (int m = 0; m < 2 * ls + 1; ++m) v += sph[sph_off(ls) + m * ncart(ls) + ic] * c[f0 + m];
+  else
+    v = c[f0 + ic];
+  cc[i] = v;
+}
+
+// J (n x n, lower triangle) += sum_P c_P (P|xy), integrals recomputed; cc is
+// scratch of n_cart fitting components.
+int eri3_J(jk_engine* e, const double* c, double* cc, double* J, cudaStream_t s) {
+  const int nc = e->aux.n_cart;
+  k_aux_cart<<<(nc + 127) / 128, 128, 0, s>>>(nc, e->daux.cart_shell.p, e->daux.cart_comp.p, e->daux.l.p,
+                                              e->daux.pure.p, e->daux.final_off.p, e->daux.sph.p, c, cc);
+  return eri3_all(e, true, s, [&](Eri3Params& P, int) {
+    P.cc = cc;
+    P.aux_coff = e->daux.cart_off.p;
+    P.J = J;
+    return true;
+  });
 }
 
 int compute_V(jk_engine* e, double* V, cudaStream_t s) {
@@ -141,18 +198,25 @@ int compute_V(jk_engine* e, double* V, cudaStream_t s) {
   return check_cuda(e, cudaGetLastError(), "eri2 launch");
 }
 
-// packed reference layout: Tp[(x(x+1)/2 + y) + P*npair], x >= y
-__global__ void k_pack_T3(int n, int naux, const double* __restrict__ T3, double* __restrict__ Tp) {
-  const size_t npair = (size_t)n * (n + 1) / 2;
-  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= npair * naux) return;
-  const int P = (int)(idx / npair);
-  const size_t xy = idx % npair;
-  int x = (int)floor((sqrt(8.0 * (double)xy + 1.0) - 1.0) * 0.5);
-  while ((size_t)x * (x + 1) / 2 > xy) --x;
-  while ((size_t)(x + 1) * (x + 2) / 2 <= xy) ++x;
-  const int y = (int)(xy - (size_t)x * (x + 1) / 2);
-  Tp[idx] = T3[((size_t)x * naux + P) * n + y];
+// packed reference layout: Tp[(x(x+1)/2 + y) + P*npair], x >= y, from T3[x][y][P]:
+// 32 x 32 tiles of (pair, P) through shared memory
+__global__ void __launch_bounds__(256) k_pack_T3(int n, int naux, const double* __restrict__ T3,
+                                                 double* __restrict__ Tp) {
+  __shared__ double tile[32][33];
+  const size_t npair = (size_t)n * (n + 1) / 2, q0 = (size_t)blockIdx.x * 32;
+  const int P0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int r = ty; r < 32; r += 8) {
+    const size_t xy = q0 + r;
+    if (xy >= npair || P0 + tx >= naux) continue;
+    int x = (int)floor((sqrt(8.0 * (double)xy + 1.0) - 1.0) * 0.5);
+    while ((size_t)x * (x + 1) / 2 > xy) --x;
+    while ((size_t)(x + 1) * (x + 2) / 2 <= xy) ++x;
+    const int y = (int)(xy - (size_t)x * (x + 1) / 2);
+    tile[r][tx] = T3[((size_t)x * n + y) * naux + P0 + tx];
+  }
+  __syncthreads();
+  for (int r = ty; r < 32; r += 8)
+    if (q0 + tx < npair && P0 + r < naux) Tp[(size_t)(P0 + r) * npair + q0 + tx] = tile[tx][r];
 }
 
 // gamma_K = sum_{x,i} X[x][K][i] C[x][i]   (C column-major n x o)
@@ -309,8 +373,8 @@ int df_setup(jk_engine* e) {
   g.sak = naux;
   g.a_lower = (k0 == 0);
   g.B = T3.p;
-  g.sbk = n;
-  g.sbn = 1;
+  g.sbk = 1;
+  g.sbn = naux;
   g.bsb = (long long)naux * n;
   g.C = d.B64.p;
   g.scm = n;
@@ -381,6 +445,7 @@ int df_jk_device(jk_engine* e, const double* dC, int nocc, int mode, double* dJ,
   return check_cuda(e, cudaGetLastError(), "jk_df launch");
 }
 
+// S, and T and V unless both are NULL.
 int one_body_device(jk_engine* e, double* S, double* T, double* V, cudaStream_t s) {
   const int n = e->obs.n_final;
   DevBuf<double> Z, C;
@@ -389,20 +454,20 @@ int one_body_device(jk_engine* e, double* S, double* T, double* V, cudaStream_t 
   if (st != cudaSuccess) return check_cuda(e, st, "one_body upload");
   // shell pairs whose primitive products all vanish are not in the pair
   // lists; their blocks are zero, not whatever the buffers held before
-  for (double* M : {S, T, V}) cudaMemsetAsync(M, 0, sizeof(double) * (size_t)n * n, s);
+  for (double* M : {S, T, V})
+    if (M) cudaMemsetAsync(M, 0, sizeof(double) * (size_t)n * n, s);
   for (int pc = 0; pc < NPAIRCLASS; ++pc) {
     if (!e->pcls[pc].npair) continue;
     OneBodyParams P{};
     P.pairs = view(e->pcls[pc]);
-    P.pp = prim_view(e);
-    P.pa = e->pp_a.p;
+    P.ent = entry_view(e->pcls[pc]);
     P.ox = e->dobs.x.p;
     P.oy = e->dobs.y.p;
     P.oz = e->dobs.z.p;
     P.foff = e->dobs.final_off.p;
     P.pure = e->dobs.pure.p;
     P.sph = e->dobs.sph.p;
-    P.boys = e->boys.p;
+    P.boysp = e->boysp.p;
     P.natom = e->natom;
     P.Z = Z.p;
     P.cxyz = C.p;
@@ -435,7 +500,7 @@ int jk_eri3(jk_engine* e, double* Tpacked) {
   if (st != cudaSuccess) return check_cuda(e, st, "jk_eri3 allocation");
   if ((rc = compute_T3(e, T3.p, e->stream))) return rc;
   const size_t tot = npair * naux;
-  k_pack_T3<<<(unsigned)((tot + 255) / 256), 256, 0, e->stream>>>(n, naux, T3.p, Tp.p);
+  k_pack_T3<<<dim3((unsigned)((npair + 31) / 32), (naux + 31) / 32), 256, 0, e->stream>>>(n, naux, T3.p, Tp.p);
   st = cudaMemcpyAsync(Tpacked, Tp.p, tot * sizeof(double), cudaMemcpyDeviceToHost, e->stream);
   if (st == cudaSuccess) st = cudaStreamSynchronize(e->stream);
   return check_cuda(e, st, "jk_eri3");

@@ -1,0 +1,9 @@
+// Three-index (P|mn) kernel instantiations for pure f fitting shells.
+// Split across translation units only so that nvcc compiles them in parallel.
+#include "df_kernels.cuh"
+
+namespace m2 {
+
+void launch_eri3_f_pure(int pc, const Eri3Params& P, bool j, cudaStream_t s) { launch_eri3_l<3, true>(pc, P, j, s); }
+
+}  // namespace m2

@@ -1,6 +1,5 @@
 // Device side of the density-fitting integrals: three-index (P|mn) and
-// two-index (P|Q) Coulomb integrals over the fitting basis, and the one-body
-// S, T, V integrals.  McMurchie-Davidson through quartet_cart with a unit
+// two-index (P|Q) Coulomb integrals over the fitting basis.  McMurchie-Davidson through quartet_cart with a unit
 // s function as the partner of each fitting function (libint2 BraKet::xs_xx
 // and xs_xs in molecular2, src/eris.cpp:89-156, 304-356).
 #pragma once
@@ -27,114 +26,338 @@ __device__ __forceinline__ void sph_index(const double* in, double* out, int k, 
       }
 }
 
+// Fitting shells of one angular momentum, all pure or all Cartesian.
+struct AuxView {
+  const int* shells;
+  int count;
+  const int* prim_off;
+  const int* nprim;
+  const double *p, *x, *y, *z;  // primitives
+  const double* Kp;             // coefficient sqrt(2 pi^(5/2)) / p
+  const double* h;              // 1 / (2p)
+  const int* foff;              // final function offsets
+};
+
 struct Eri3Params {
-  PrimView ap;            // fitting primitives as (P, unit) pairs
-  const int* aux_shells;  // fitting shells of this class (angular momentum LP)
-  int naux_shells;
-  const int* aux_prim_off;
-  const int* aux_nprim;
-  const double *ax, *ay, *az;
-  const int* aux_foff;    // final function offsets
-  const int* aux_pure;
-  PairView pairs;         // orbital pairs of one class
-  PrimView pp;
+  AuxView aux;
+  EntryView ent;          // orbital pairs of one class
+  PairView pairs;
   const double *ox, *oy, *oz;
   const int* obs_foff;
   const int* obs_pure;
   const double* sph;
-  const double* boys;
-  int n, naux;
-  double* T3;             // [x][P][y]
-};
-
-// Final-basis block (P|mn) of fitting shell sP and orbital shell pair ip of
-// the class: out[(a * dims[1] + x) * dims[2] + y]; c and t are scratch of
-// NP*NM*NN doubles each, the result is one of them.
-template <int LP, int LM, int LN>
-__device__ __forceinline__ const double* eri3_block(const Eri3Params& P, int sP, int ip, double* c, double* t,
-                                                    int* dims) {
-  const int m = P.pairs.sa[ip], n = P.pairs.sb[ip];
-  const double Ax = P.ax[sP], Ay = P.ay[sP], Az = P.az[sP];
-  quartet_cart<LP, 0, LM, LN>(P.ap, P.aux_prim_off[sP], P.aux_nprim[sP], Ax, Ay, Az, Ax, Ay, Az, P.pp,
-                              P.pairs.prim_off[ip], P.pairs.nprim[ip], P.ox[m], P.oy[m], P.oz[m], P.ox[n], P.oy[n],
-                              P.oz[n], P.boys, c);
-  dims[0] = ncart(LP);
-  dims[1] = ncart(LM);
-  dims[2] = ncart(LN);
-  double* cur = c;
-  double* nxt = t;
-  const int pure[3] = {P.aux_pure[sP], P.obs_pure[m], P.obs_pure[n]};
-  const int ls[3] = {LP, LM, LN};
-  for (int k = 0; k < 3; ++k)
-    if (pure[k]) {
-      sph_index(cur, nxt, k, dims, ls[k], P.sph);
-      dims[k] = 2 * ls[k] + 1;
-      double* sw = cur;
-      cur = nxt;
-      nxt = sw;
-    }
-  return cur;
-}
-
-template <int LP, int LM, int LN>
-__global__ void __launch_bounds__(64) k_eri3(const Eri3Params P) {
-  constexpr int N3 = ncart(LP) * ncart(LM) * ncart(LN);
-  const int ip = blockIdx.x * blockDim.x + threadIdx.x;
-  const int is = blockIdx.y;
-  if (ip >= P.pairs.npair || is >= P.naux_shells) return;
-  const int sP = P.aux_shells[is];
-  const int m = P.pairs.sa[ip], n = P.pairs.sb[ip];
-  double c[N3], t[N3];
-  int dims[3];
-  const double* cur = eri3_block<LP, LM, LN>(P, sP, ip, c, t, dims);
-  const int f0 = P.aux_foff[sP], m0 = P.obs_foff[m], n0 = P.obs_foff[n];
-  const size_t nQ = (size_t)P.naux * P.n;
-  for (int a = 0; a < dims[0]; ++a)
-    for (int x = 0; x < dims[1]; ++x)
-      for (int y = 0; y < dims[2]; ++y) {
-        const double v = cur[(a * dims[1] + x) * dims[2] + y];
-        P.T3[(size_t)(m0 + x) * nQ + (size_t)(f0 + a) * P.n + n0 + y] = v;
-        P.T3[(size_t)(n0 + y) * nQ + (size_t)(f0 + a) * P.n + m0 + x] = v;
-      }
-}
-
-// One tile pair of the tiled three-index tensor: T[r][P][c] = (P | x y) for
-// x = x0 + r and y = y0 + c inside the TB x TB tile (TB = 128), over the
-// shell pairs `plist` of the class that touch the tile pair (either
-// orientation).  Entries of the block outside the tile are not written.
-struct Eri3TileArgs {
-  const int* plist;  // indices into the class's pair list
+  const double* boysp;
+  const int* plist;       // the pairs to do (indices into the class list), or NULL for all
   int nlist;
-  int x0, y0;        // first function of the row tile and of the column tile
+  // T[(r ncol + c) naux + P] = (P | x y) for x = x0 + r < x0 + nrow and
+  // y = y0 + c < y0 + ncol, both orientations of a pair
+  int x0, y0, nrow, ncol;
   int naux;
-  double* T;         // [r][P][c], TB * naux * TB doubles
+  double* T;
+  // k_eri3_J: J[x][y] (x >= y) += sum over this view's P of cc_P (P | x y)
+  const double* cc;       // coefficients of the Cartesian fitting components
+  const int* aux_coff;    // Cartesian function offsets of the fitting shells
+  int n;
+  double* J;              // n x n column-major
 };
-constexpr int DF_TILE = 128;
 
-template <int LP, int LM, int LN>
-__global__ void __launch_bounds__(64) k_eri3_tile(const Eri3Params P, const Eri3TileArgs A) {
-  constexpr int N3 = ncart(LP) * ncart(LM) * ncart(LN);
-  const int il = blockIdx.x * blockDim.x + threadIdx.x;
-  const int is = blockIdx.y;
-  if (il >= A.nlist || is >= P.naux_shells) return;
-  const int ip = A.plist[il];
-  const int sP = P.aux_shells[is];
-  const int m = P.pairs.sa[ip], n = P.pairs.sb[ip];
-  double c[N3], t[N3];
-  int dims[3];
-  const double* cur = eri3_block<LP, LM, LN>(P, sP, ip, c, t, dims);
-  const int f0 = P.aux_foff[sP], m0 = P.obs_foff[m], n0 = P.obs_foff[n];
-  const size_t rs = (size_t)A.naux * DF_TILE;  // stride of r
-  for (int a = 0; a < dims[0]; ++a)
-    for (int x = 0; x < dims[1]; ++x)
-      for (int y = 0; y < dims[2]; ++y) {
-        const double v = cur[(a * dims[1] + x) * dims[2] + y];
-        const int X = m0 + x, Y = n0 + y;
-        const unsigned r1 = (unsigned)(X - A.x0), c1 = (unsigned)(Y - A.y0);
-        if (r1 < DF_TILE && c1 < DF_TILE) A.T[r1 * rs + (size_t)(f0 + a) * DF_TILE + c1] = v;
-        const unsigned r2 = (unsigned)(Y - A.x0), c2 = (unsigned)(X - A.y0);
-        if (r2 < DF_TILE && c2 < DF_TILE) A.T[r2 * rs + (size_t)(f0 + a) * DF_TILE + c2] = v;
+constexpr int DF_TILE = 128;
+constexpr int E3_THREADS = 128;  // most threads of a block
+
+// Whether a thread keeps all functions of its fitting shell at once (their
+// Hermite sums and Cartesian blocks beside R in registers), or the block does
+// one function per layer.
+__host__ __device__ constexpr int e3_nfun(int lp, bool pure) { return pure ? 2 * lp + 1 : ncart(lp); }
+__host__ __device__ constexpr bool e3_full(int la, int lb, int lp, bool pure) {
+  return e3_nfun(lp, pure) * (ncart(la) * ncart(lb) + nherm(la + lb)) + nherm(la + lb + lp) <= 90 &&
+         (lp <= 1 || pure);
+}
+
+template <int LA, int LB, int LP>
+struct Eri3Shared {
+  double boys[BOYSP_SIZE];
+  BraShared<LA, LB> bra;
+  double sphP[(2 * LP + 1) * ncart(LP)];
+  double red[E3_THREADS / 32][nherm(LA + LB)];
+};
+
+// W[h] += f R[h + a] for the Hermite index a of degree LP
+template <int HL, int LP, int A>
+__device__ __forceinline__ void shift_accumulate(double* W, const double* R, double f) {
+  constexpr int a = LP > 0 ? nherm(LP - 1) + A : 0;
+  static_for<nherm(HL)>([&](auto hh) {
+    constexpr int h = decltype(hh)::value;
+    W[h] += f * R[hidx(herm_t(h) + herm_t(a), herm_u(h) + herm_u(a), herm_v(h) + herm_v(a))];
+  });
+}
+
+// d index of a Cartesian block [6][REST] or [REST][6] (STRIDE) to the pure d
+// functions, in place of the first five: xy, yz, z^2, xz, x^2 - y^2.
+template <int N, int STRIDE>
+__device__ __forceinline__ void pure_d(const double* in, double* out, const double* T) {
+  // rows of the solid-harmonic block and their non-zero components
+  out[0 * STRIDE] = __ldg(T + 0 * 6 + 1) * in[1 * STRIDE];
+  out[1 * STRIDE] = __ldg(T + 1 * 6 + 4) * in[4 * STRIDE];
+  out[2 * STRIDE] = __ldg(T + 2 * 6 + 0) * in[0 * STRIDE] + __ldg(T + 2 * 6 + 3) * in[3 * STRIDE] +
+                    __ldg(T + 2 * 6 + 5) * in[5 * STRIDE];
+  out[3 * STRIDE] = __ldg(T + 3 * 6 + 2) * in[2 * STRIDE];
+  out[4 * STRIDE] = __ldg(T + 4 * 6 + 0) * in[0 * STRIDE] + __ldg(T + 4 * 6 + 3) * in[3 * STRIDE];
+}
+
+// (P|mn).  Block = (orbital pair, function layer, slice of the fitting
+// shells); the lanes hold fitting shells and T keeps P fastest, so a warp
+// writes neighbouring words (a lane per orbital pair scattered 8-byte words
+// over rows naux apart).  A pure or s, p fitting function centred on its own
+// primitive has only Hermite terms of its top degree (solid harmonics are
+// harmonic), (1/2q)^l of its Cartesian coefficients.  Measured through the FP64
+// build on tiled storage, (H2O)16/aug-cc-pVDZ (n 656, naux 2400), which takes
+// one pass of T and one of J: 340 -> 79 ms (a thread per contracted (pair,
+// shell) before, T re-made for J).
+template <int LA, int LB, int LP, bool PURE>
+__global__ void __launch_bounds__(E3_THREADS, 2) k_eri3(const Eri3Params P) {
+  constexpr int NA = ncart(LA), NB = ncart(LB), NAB = NA * NB, LAB = LA + LB, H = nherm(LAB), L = LAB + LP;
+  constexpr int NP = ncart(LP), NF = e3_nfun(LP, PURE);
+  constexpr bool FULL = e3_full(LA, LB, LP, PURE), TOP = LP <= 1 || PURE;
+  constexpr int G = FULL ? NF : 1;
+  extern __shared__ __align__(16) unsigned char e3_sm[];
+  Eri3Shared<LA, LB, LP>& S = *reinterpret_cast<Eri3Shared<LA, LB, LP>*>(e3_sm);
+  const int tid = threadIdx.x;
+  const int ip = P.plist ? P.plist[blockIdx.x] : (int)blockIdx.x;
+  const int a = P.pairs.sa[ip], b = P.pairs.sb[ip];
+  const int e0 = P.ent.first[ip], e1 = P.ent.first[ip + 1];
+  const int f0 = blockIdx.y;  // the layer's function
+  for (int i = tid; i < BOYSP_SIZE; i += blockDim.x) S.boys[i] = __ldg(P.boysp + (size_t)L * BOYSP_SIZE + i);
+  if constexpr (PURE && LP > 1)
+    for (int i = tid; i < NF * NP; i += blockDim.x) S.sphP[i] = P.sph[sph_off(LP) + i];
+  const double A[3] = {P.ox[a], P.oy[a], P.oz[a]}, B[3] = {P.ox[b], P.oy[b], P.oz[b]};
+  if (e1 - e0 == 1) load_bra<LA, LB>(S.bra, entry_prims(P.ent, e0), P.ent.np[e0], A[0], A[1], A[2], B[0], B[1], B[2]);
+
+  for (int s0 = blockIdx.z * blockDim.x; s0 < P.aux.count; s0 += gridDim.z * blockDim.x) {
+    const bool active = s0 + tid < P.aux.count;
+    const int sh = P.aux.shells[active ? s0 + tid : P.aux.count - 1];
+    const int j0 = P.aux.prim_off[sh], nj = P.aux.nprim[sh];
+    const int njm = __reduce_max_sync(0xffffffffu, nj);
+    double out[G][NAB];
+#pragma unroll
+    for (int g = 0; g < G; ++g)
+#pragma unroll
+      for (int i = 0; i < NAB; ++i) out[g][i] = 0.0;
+    for (int e = e0; e < e1; ++e) {
+      const int nb = P.ent.np[e];
+      if (e1 - e0 > 1) {
+        __syncthreads();
+        load_bra<LA, LB>(S.bra, entry_prims(P.ent, e), nb, A[0], A[1], A[2], B[0], B[1], B[2]);
       }
+      for (int ib = 0; ib < nb; ++ib) {
+        const double* q = S.bra.prim[ib];
+        double W[G][H];
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+          for (int h = 0; h < H; ++h) W[g][h] = 0.0;
+        for (int j = 0; j < njm; ++j) {
+          const int k = j0 + min(j, nj - 1);
+          const double KK = j < nj ? q[4] * __ldg(P.aux.Kp + k) : 0.0;
+          double R[nherm(L)];
+          quartet_R<L>(q[0], __ldg(P.aux.p + k), KK, q[1] - __ldg(P.aux.x + k), q[2] - __ldg(P.aux.y + k),
+                       q[3] - __ldg(P.aux.z + k), S.boys, R);
+          if constexpr (LP == 0) {
+#pragma unroll
+            for (int h = 0; h < H; ++h) W[0][h] += R[h];
+          } else if constexpr (TOP) {
+            const double h1 = -__ldg(P.aux.h + k);
+            const double hl = LP == 1 ? h1 : (LP == 2 ? h1 * h1 : h1 * h1 * h1);
+            static_for<G>([&](auto gg) {
+              constexpr int g = decltype(gg)::value;
+              static_for<NP>([&](auto aa) {
+                constexpr int ca = decltype(aa)::value;
+                if constexpr (LP == 1) {
+                  if (FULL ? g == ca : f0 == ca) shift_accumulate<LAB, LP, ca>(W[g], R, hl);
+                } else {
+                  const double c = S.sphP[(FULL ? g : f0) * NP + ca];
+                  if (c != 0.0) shift_accumulate<LAB, LP, ca>(W[g], R, hl * c);
+                }
+              });
+            });
+          } else {
+            const double h1 = __ldg(P.aux.h + k);
+            const int ce[3] = {c_herm.t[nherm(LP - 1) + f0], c_herm.u[nherm(LP - 1) + f0], c_herm.v[nherm(LP - 1) + f0]};
+            double ex[3][LP + 1];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+#pragma unroll
+              for (int t = 0; t <= LP; ++t) ex[x][t] = t == 0 ? 1.0 : 0.0;
+#pragma unroll
+              for (int t = 0; t < LP; ++t)
+                if (t < ce[x]) e1_raise<LP>(ex[x], 0.0, h1);
+            }
+            ket_accumulate<LAB, LP>(W[0], R, ex[0], ex[1], ex[2], ce[0], ce[1], ce[2]);
+          }
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) bra_transform<LA, LB, 1>(S.bra.M[LAB > 0 ? ib : 0], W[g], out[g]);
+      }
+    }
+    if (!active) continue;
+    // final orbital functions, both orientations
+    const bool pa = LA == 2 && P.obs_pure[a], pb = LB == 2 && P.obs_pure[b];
+    const int fa = pa ? 5 : NA, fb = pb ? 5 : NB;
+    const int m0 = P.obs_foff[a], n0 = P.obs_foff[b];
+    double* T = P.T + P.aux.foff[sh] + (FULL ? 0 : f0);
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      if constexpr (LA == 2) {
+        if (pa) {
+          double t[5 * NB];
+#pragma unroll
+          for (int j = 0; j < NB; ++j) pure_d<NB, NB>(out[g] + j, t + j, P.sph + sph_off(2));
+#pragma unroll
+          for (int i = 0; i < 5 * NB; ++i) out[g][i] = t[i];
+        }
+      }
+      if constexpr (LB == 2) {
+        if (pb) {
+#pragma unroll
+          for (int i = 0; i < NA; ++i) {
+            double t[5];
+            pure_d<1, 1>(out[g] + i * 6, t, P.sph + sph_off(2));
+#pragma unroll
+            for (int j = 0; j < 5; ++j) out[g][i * 6 + j] = t[j];
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < NA; ++i)
+#pragma unroll
+        for (int j = 0; j < NB; ++j)
+          if (i < fa && j < fb) {
+            const int X = m0 + i, Y = n0 + j;
+            const unsigned r1 = (unsigned)(X - P.x0), c1 = (unsigned)(Y - P.y0);
+            if (r1 < (unsigned)P.nrow && c1 < (unsigned)P.ncol) T[((size_t)r1 * P.ncol + c1) * P.naux + g] = out[g][i * NB + j];
+            const unsigned r2 = (unsigned)(Y - P.x0), c2 = (unsigned)(X - P.y0);
+            if (r2 < (unsigned)P.nrow && c2 < (unsigned)P.ncol) T[((size_t)r2 * P.ncol + c2) * P.naux + g] = out[g][i * NB + j];
+          }
+    }
+  }
+}
+
+// J_mn = sum_P c_P (P|mn) without storing an integral: the coefficients are
+// folded into the fitting functions' Hermite expansions, the block sums the
+// bra's Hermite potential W over its lanes' shells and transforms it once.
+template <int LA, int LB, int LP, bool PURE>
+__global__ void __launch_bounds__(E3_THREADS, 2) k_eri3_J(const Eri3Params P) {
+  constexpr int NA = ncart(LA), NB = ncart(LB), NAB = NA * NB, LAB = LA + LB, H = nherm(LAB), L = LAB + LP;
+  constexpr int NP = ncart(LP);
+  constexpr bool TOP = LP <= 1 || PURE;
+  extern __shared__ __align__(16) unsigned char e3_sm[];
+  Eri3Shared<LA, LB, LP>& S = *reinterpret_cast<Eri3Shared<LA, LB, LP>*>(e3_sm);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int ip = blockIdx.x;
+  const int a = P.pairs.sa[ip], b = P.pairs.sb[ip];
+  for (int i = tid; i < BOYSP_SIZE; i += blockDim.x) S.boys[i] = __ldg(P.boysp + (size_t)L * BOYSP_SIZE + i);
+  const double A[3] = {P.ox[a], P.oy[a], P.oz[a]}, B[3] = {P.ox[b], P.oy[b], P.oz[b]};
+  __shared__ double cart[NAB];
+  for (int i = tid; i < NAB; i += blockDim.x) cart[i] = 0.0;
+  for (int e = P.ent.first[ip]; e < P.ent.first[ip + 1]; ++e) {
+    const int nb = P.ent.np[e];
+    __syncthreads();
+    load_bra<LA, LB>(S.bra, entry_prims(P.ent, e), nb, A[0], A[1], A[2], B[0], B[1], B[2]);
+    for (int ib = 0; ib < nb; ++ib) {
+      const double* q = S.bra.prim[ib];
+      double W[H];
+#pragma unroll
+      for (int h = 0; h < H; ++h) W[h] = 0.0;
+      for (int s = tid; s < P.aux.count; s += blockDim.x) {
+        const int sh = P.aux.shells[s];
+        const int j0 = P.aux.prim_off[sh], nj = P.aux.nprim[sh];
+        const double* cc = P.cc + P.aux_coff[sh];
+        for (int k = j0; k < j0 + nj; ++k) {
+          double R[nherm(L)];
+          quartet_R<L>(q[0], __ldg(P.aux.p + k), q[4] * __ldg(P.aux.Kp + k), q[1] - __ldg(P.aux.x + k),
+                       q[2] - __ldg(P.aux.y + k), q[3] - __ldg(P.aux.z + k), S.boys, R);
+          const double h1 = -__ldg(P.aux.h + k);
+          if constexpr (TOP) {
+            const double hl = LP == 0 ? 1.0 : (LP == 1 ? h1 : (LP == 2 ? h1 * h1 : h1 * h1 * h1));
+            static_for<NP>([&](auto aa) { shift_accumulate<LAB, LP, decltype(aa)::value>(W, R, hl * cc[decltype(aa)::value]); });
+          } else {
+#pragma unroll 1
+            for (int c = 0; c < NP; ++c) {
+              const int ce[3] = {c_herm.t[nherm(LP - 1) + c], c_herm.u[nherm(LP - 1) + c], c_herm.v[nherm(LP - 1) + c]};
+              double ex[3][LP + 1];
+#pragma unroll
+              for (int x = 0; x < 3; ++x) {
+#pragma unroll
+                for (int t = 0; t <= LP; ++t) ex[x][t] = t == 0 ? (x == 0 ? cc[c] : 1.0) : 0.0;
+#pragma unroll
+                for (int t = 0; t < LP; ++t)
+                  if (t < ce[x]) e1_raise<LP>(ex[x], 0.0, -h1);
+              }
+              ket_accumulate<LAB, LP>(W, R, ex[0], ex[1], ex[2], ce[0], ce[1], ce[2]);
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < H; ++h) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) W[h] += __shfl_down_sync(0xffffffffu, W[h], o);
+        if (lane == 0) S.red[tid >> 5][h] = W[h];
+      }
+      __syncthreads();
+      for (int h = tid; h < H; h += blockDim.x) {
+        double v = 0.0;
+        for (int w = 0; w < (int)blockDim.x / 32; ++w) v += S.red[w][h];
+        S.red[0][h] = v;
+      }
+      __syncthreads();
+      for (int i = tid; i < NAB; i += blockDim.x)
+        cart[i] += bra_component<LA, LB>(S.bra.M[LAB > 0 ? ib : 0], S.red[0], i);
+      __syncthreads();
+    }
+  }
+  // final functions, lower triangle
+  const bool pa = LA >= 2 && P.obs_pure[a], pb = LB >= 2 && P.obs_pure[b];
+  const int fa = pa ? 2 * LA + 1 : NA, fb = pb ? 2 * LB + 1 : NB;
+  const int m0 = P.obs_foff[a], n0 = P.obs_foff[b];
+  for (int i = tid; i < fa * fb; i += blockDim.x) {
+    const int m = i / fb, q = i % fb;
+    double v = 0.0;
+    for (int i1 = pa ? 0 : m; i1 < (pa ? NA : m + 1); ++i1) {
+      const double ta = pa ? P.sph[sph_off(LA) + m * NA + i1] : 1.0;
+      for (int j1 = pb ? 0 : q; j1 < (pb ? NB : q + 1); ++j1)
+        v += ta * (pb ? P.sph[sph_off(LB) + q * NB + j1] : 1.0) * cart[i1 * NB + j1];
+    }
+    const int X = m0 + m, Y = n0 + q;
+    if (a == b && X < Y) continue;  // the same block holds its mirror image
+    atomicAdd(P.J + (size_t)(X < Y ? X : Y) * P.n + (X < Y ? Y : X), v);
+  }
+}
+
+template <int LA, int LB, int LP, bool PURE>
+inline void launch_eri3_class(const Eri3Params& P, bool j, cudaStream_t s) {
+  const size_t sm = sizeof(Eri3Shared<LA, LB, LP>);
+  const int iters = (P.aux.count + E3_THREADS - 1) / E3_THREADS;
+  const int threads = ((P.aux.count + iters - 1) / iters + 31) / 32 * 32;
+  if (j) {
+    cudaFuncSetAttribute(k_eri3_J<LA, LB, LP, PURE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k_eri3_J<LA, LB, LP, PURE><<<P.pairs.npair, threads, sm, s>>>(P);
+    return;
+  }
+  cudaFuncSetAttribute(k_eri3<LA, LB, LP, PURE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  const int layers = e3_full(LA, LB, LP, PURE) ? 1 : e3_nfun(LP, PURE);
+  // one block walks over all fitting shells of a pair unless that leaves the GPU short of blocks
+  int z = 1;
+  while (z < iters && (long long)P.nlist * layers * z < 8 * 148) ++z;
+  k_eri3<LA, LB, LP, PURE><<<dim3(P.nlist, layers, z), threads, sm, s>>>(P);
+}
+template <int LP, bool PURE>
+inline void launch_eri3_l(int pc, const Eri3Params& P, bool j, cudaStream_t s) {
+  if (pc == 0) launch_eri3_class<0, 0, LP, PURE>(P, j, s);
+  if (pc == 1) launch_eri3_class<1, 0, LP, PURE>(P, j, s);
+  if (pc == 2) launch_eri3_class<1, 1, LP, PURE>(P, j, s);
+  if (pc == 3) launch_eri3_class<2, 0, LP, PURE>(P, j, s);
+  if (pc == 4) launch_eri3_class<2, 1, LP, PURE>(P, j, s);
+  if (pc == 5) launch_eri3_class<2, 2, LP, PURE>(P, j, s);
 }
 
 struct Eri2Params {
@@ -192,112 +415,13 @@ __global__ void __launch_bounds__(64) k_eri2(const Eri2Params P) {
     }
 }
 
-// ---------------------------------------------------------------- one-body
-struct OneBodyParams {
-  PairView pairs;
-  PrimView pp;
-  const double* pa;  // exponent of shell a per primitive pair
-  const double *ox, *oy, *oz;
-  const int* foff;
-  const int* pure;
-  const double* sph;
-  const double* boys;
-  int natom;
-  const double* Z;
-  const double* cxyz;  // 3*natom
-  int n;
-  double *S, *T, *V;   // n x n final basis
-};
-
-template <int LA, int LB>
-__global__ void __launch_bounds__(64) k_onebody(const OneBodyParams P) {
-  constexpr int NA = ncart(LA), NB = ncart(LB), L = LA + LB;
-  const int ip = blockIdx.x * blockDim.x + threadIdx.x;
-  if (ip >= P.pairs.npair) return;
-  const int a = P.pairs.sa[ip], b = P.pairs.sb[ip];
-  const double Ax = P.ox[a], Ay = P.oy[a], Az = P.oz[a], Bx = P.ox[b], By = P.oy[b], Bz = P.oz[b];
-  double s[NA * NB], t[NA * NB], v[NA * NB];
-  for (int i = 0; i < NA * NB; ++i) s[i] = t[i] = v[i] = 0.0;
-  const int p0 = P.pairs.prim_off[ip], np = P.pairs.nprim[ip];
-  for (int k = p0; k < p0 + np; ++k) {
-    const double p = P.pp.p[k], Px = P.pp.x[k], Py = P.pp.y[k], Pz = P.pp.z[k], K = P.pp.K[k];
-    const double al = P.pa[k], be = p - al;
-    E1<LA, LB + 2> ex, ey, ez;
-    const double oo2p = 0.5 / p;
-    md_E1<LA, LB + 2>(Px - Ax, Px - Bx, oo2p, ex);
-    md_E1<LA, LB + 2>(Py - Ay, Py - By, oo2p, ey);
-    md_E1<LA, LB + 2>(Pz - Az, Pz - Bz, oo2p, ez);
-    const double ov = K * pow(M_PI / p, 1.5);
-    // nuclear attraction: sum_C -Z_C 2 pi/p K sum_tuv E_t E_u E_v R_tuv(p, P-C)
-    double Rsum[nherm(L)];
-    for (int h = 0; h < nherm(L); ++h) Rsum[h] = 0.0;
-    for (int c = 0; c < P.natom; ++c) {
-      const double X = Px - P.cxyz[3 * c], Y = Py - P.cxyz[3 * c + 1], Zc = Pz - P.cxyz[3 * c + 2];
-      double F[L + 1], R[nherm(L)];
-      boys<L>(p * (X * X + Y * Y + Zc * Zc), P.boys, F);
-      md_R<L>(p, X, Y, Zc, F, R);
-      const double z = P.Z[c];
-      for (int h = 0; h < nherm(L); ++h) Rsum[h] -= z * R[h];
-    }
-    const double vp = 2.0 * M_PI / p * K;
-#pragma unroll
-    for (int ia = 0; ia < NA; ++ia) {
-      const int ax = cart_a(LA, ia), ay = cart_b(LA, ia), az = cart_c(LA, ia);
-#pragma unroll
-      for (int ib = 0; ib < NB; ++ib) {
-        const int bx = cart_a(LB, ib), by = cart_b(LB, ib), bz = cart_c(LB, ib);
-        const double sx = ex.e[ax][bx][0], sy = ey.e[ay][by][0], sz = ez.e[az][bz][0];
-        s[ia * NB + ib] += ov * sx * sy * sz;
-        auto kin = [&](const E1<LA, LB + 2>& e, int i, int j) {
-          double r = -2.0 * be * be * e.e[i][j + 2][0] + be * (2 * j + 1) * e.e[i][j][0];
-          if (j > 1) r -= 0.5 * j * (j - 1) * e.e[i][j - 2][0];
-          return r;
-        };
-        t[ia * NB + ib] += ov * (kin(ex, ax, bx) * sy * sz + sx * kin(ey, ay, by) * sz + sx * sy * kin(ez, az, bz));
-        double acc = 0.0;
-        for (int tt = 0; tt <= ax + bx; ++tt)
-          for (int u = 0; u <= ay + by; ++u)
-            for (int w = 0; w <= az + bz; ++w)
-              acc += ex.e[ax][bx][tt] * ey.e[ay][by][u] * ez.e[az][bz][w] * Rsum[hidx(tt, u, w)];
-        v[ia * NB + ib] += vp * acc;
-      }
-    }
-  }
-  // final basis and store both orientations
-  double* blocks[3] = {s, t, v};
-  double* outs[3] = {P.S, P.T, P.V};
-  const int pa = P.pure[a], pb = P.pure[b];
-  const int fa = pa ? 2 * LA + 1 : NA, fb = pb ? 2 * LB + 1 : NB;
-  const int a0 = P.foff[a], b0 = P.foff[b];
-  for (int k = 0; k < 3; ++k) {
-    const double* c = blocks[k];
-    for (int m = 0; m < fa; ++m)
-      for (int q = 0; q < fb; ++q) {
-        double val = 0.0;
-        for (int i = 0; i < NA; ++i) {
-          const double ta = pa ? P.sph[sph_off(LA) + m * NA + i] : (i == m ? 1.0 : 0.0);
-          if (ta == 0.0) continue;
-          for (int j = 0; j < NB; ++j) {
-            const double tb = pb ? P.sph[sph_off(LB) + q * NB + j] : (j == q ? 1.0 : 0.0);
-            val += ta * tb * c[i * NB + j];
-          }
-        }
-        outs[k][(size_t)(b0 + q) * P.n + a0 + m] = val;
-        outs[k][(size_t)(a0 + m) * P.n + b0 + q] = val;
-      }
-  }
-}
-
-// launchers in df_cls_*.cu
-void launch_eri3_l0(int pair_class_id, const Eri3Params& P, cudaStream_t s);
-void launch_eri3_l1(int pair_class_id, const Eri3Params& P, cudaStream_t s);
-void launch_eri3_l2(int pair_class_id, const Eri3Params& P, cudaStream_t s);
-void launch_eri3_l3(int pair_class_id, const Eri3Params& P, cudaStream_t s);
-void launch_eri3_tile_l0(int pair_class_id, const Eri3Params& P, const Eri3TileArgs& A, cudaStream_t s);
-void launch_eri3_tile_l1(int pair_class_id, const Eri3Params& P, const Eri3TileArgs& A, cudaStream_t s);
-void launch_eri3_tile_l2(int pair_class_id, const Eri3Params& P, const Eri3TileArgs& A, cudaStream_t s);
-void launch_eri3_tile_l3(int pair_class_id, const Eri3Params& P, const Eri3TileArgs& A, cudaStream_t s);
+// launchers in df_cls_*.cu: pair class id, T (j false) or J (j true)
+void launch_eri3_s(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
+void launch_eri3_p(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
+void launch_eri3_d_pure(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
+void launch_eri3_d_cart(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
+void launch_eri3_f_pure(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
+void launch_eri3_f_cart(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
 void launch_eri2(int LP, int LQ, const Eri2Params& P, cudaStream_t s);
-void launch_onebody(int pair_class_id, const OneBodyParams& P, cudaStream_t s);
 
 }  // namespace m2

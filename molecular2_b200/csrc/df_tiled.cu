@@ -45,7 +45,8 @@ namespace m2 {
 using namespace tc;
 
 PrimView prim_view(const jk_engine* e);
-Eri3Params eri3_params(const jk_engine* e, int l, int pc);
+int eri3_all(jk_engine* e, bool j, cudaStream_t s, const std::function<bool(Eri3Params&, int)>& set);
+int eri3_J(jk_engine* e, const double* c, double* cc, double* J, cudaStream_t s);
 void stage_mark(jk_engine* e, int k, cudaStream_t s);
 
 namespace {
@@ -388,34 +389,17 @@ __global__ void k_store_tile(int t, int npt, int naux, const double* __restrict_
 }
 
 // ---------------------------------------------------------------- FP64-build helpers
-// d_P += w * sum_{r,c} T[r][P][c] D[x][y], x = x0 + r, y = y0 + c (D column-major n x n)
+// d_P += w * sum_{r,c} T[r][c][P] D[x][y], x = x0 + r, y = y0 + c (D column-major n x n)
 __global__ void __launch_bounds__(256) k_tile_d(int naux, int n, int x0, int y0, double w, const double* __restrict__ T,
                                                 const double* __restrict__ D, double* __restrict__ d) {
-  const int r = blockIdx.y, x = x0 + r;
-  const int P = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int r = blockIdx.y, x = x0 + r, P = blockIdx.x * 256 + threadIdx.x;
   if (P >= naux || x >= n) return;
-  const double* tr = T + ((size_t)r * naux + P) * TB;
+  const double* tr = T + (size_t)r * TB * naux + P;
+  const int nc = min(TB, n - y0);
   double acc = 0.0;
-#pragma unroll
-  for (int k = 0; k < TB / 32; ++k) {
-    const int c = lane + 32 * k, y = y0 + c;
-    if (y < n) acc += tr[c] * D[(size_t)y * n + x];
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if (lane == 0) atomicAdd(d + P, w * acc);
-}
-
-// J[x][y] (lower triangle) += sum_P T[r][P][c] cv_P over a range of P
-__global__ void __launch_bounds__(TB) k_tile_J(int naux, int n, int x0, int y0, int pchunk, const double* __restrict__ T,
-                                              const double* __restrict__ cv, double* __restrict__ J) {
-  const int r = blockIdx.y, c = threadIdx.x, x = x0 + r, y = y0 + c;
-  const int P0 = blockIdx.x * pchunk, P1 = min(naux, P0 + pchunk);
-  if (x >= n || y >= n || y > x) return;
-  const double* tr = T + (size_t)r * naux * TB + c;
-  double acc = 0.0;
-  for (int P = P0; P < P1; ++P) acc += tr[(size_t)P * TB] * __ldg(cv + P);
-  atomicAdd(J + (size_t)y * n + x, acc);
+#pragma unroll 8
+  for (int c = 0; c < nc; ++c) acc += tr[(size_t)c * naux] * __ldg(D + (size_t)(y0 + c) * n + x);
+  atomicAdd(d + P, w * acc);
 }
 
 // Cpad (npad x nocc column-major, zero rows beyond n) from C (n x nocc)
@@ -478,51 +462,22 @@ static int build_tile_lists(jk_engine* e) {
   return check_cuda(e, st, "tiled DF: tile lists");
 }
 
-// T[r][P][c] = (P | x y) for tile pair t (zeroed first)
+// T[r][c][P] = (P | x y) for tile pair t (zeroed first)
 static int tile_integrals(jk_engine* e, int t, double* T, cudaStream_t s) {
   TiledDF& D = e->tiled;
-  const int naux = e->aux.n_final;
   int I, J;
   tile_of(t, I, J);
-  cudaMemsetAsync(T, 0, sizeof(double) * TB * (size_t)naux * TB, s);
-  // the (fitting l, pair class) launches write disjoint parts of T: they run
-  // longest first on the side streams (cost: pairs x fitting functions x
-  // Cartesian sizes), so that the small ones fill the tails of the large ones
-  static const double ncp[NPAIRCLASS] = {1, 3, 9, 6, 18, 36};
-  struct Item {
-    int l, pc;
-    double cost;
-  };
-  Item items[(MAX_L_AUX + 1) * NPAIRCLASS];
-  int nitems = 0;
-  for (int l = 0; l <= MAX_L_AUX; ++l) {
-    if (!e->aux_by_l_count[l]) continue;
-    for (int pc = 0; pc < NPAIRCLASS; ++pc) {
-      const long long o0 = D.list_off[(size_t)t * NPAIRCLASS + pc], o1 = D.list_off[(size_t)t * NPAIRCLASS + pc + 1];
-      if (o1 > o0) items[nitems++] = {l, pc, (double)(o1 - o0) * e->aux_by_l_count[l] * ncp[pc] * (l + 1) * (l + 2)};
-    }
-  }
-  std::sort(items, items + nitems, [](const Item& a, const Item& b) { return a.cost > b.cost; });
-  ClassStreams cs(e, s);
-  for (int k = 0; k < nitems; ++k) {
-    const int l = items[k].l, pc = items[k].pc;
-    const long long o0 = D.list_off[(size_t)t * NPAIRCLASS + pc];
-    const Eri3Params P = eri3_params(e, l, pc);
-    Eri3TileArgs A{};
-    A.plist = D.plist.p + o0;
-    A.nlist = (int)(D.list_off[(size_t)t * NPAIRCLASS + pc + 1] - o0);
-    A.x0 = TB * I;
-    A.y0 = TB * J;
-    A.naux = naux;
-    A.T = T;
-    cudaStream_t q = cs.next(items[k].cost);
-    if (l == 0) launch_eri3_tile_l0(pc, P, A, q);
-    if (l == 1) launch_eri3_tile_l1(pc, P, A, q);
-    if (l == 2) launch_eri3_tile_l2(pc, P, A, q);
-    if (l == 3) launch_eri3_tile_l3(pc, P, A, q);
-  }
-  cs.join();
-  return check_cuda(e, cudaGetLastError(), "tile integrals");
+  cudaMemsetAsync(T, 0, sizeof(double) * TB * (size_t)e->aux.n_final * TB, s);
+  return eri3_all(e, false, s, [&](Eri3Params& P, int pc) {
+    const long long o0 = D.list_off[(size_t)t * NPAIRCLASS + pc], o1 = D.list_off[(size_t)t * NPAIRCLASS + pc + 1];
+    P.plist = D.plist.p + o0;
+    P.nlist = (int)(o1 - o0);
+    P.x0 = TB * I;
+    P.y0 = TB * J;
+    P.nrow = P.ncol = TB;
+    P.T = T;
+    return o1 > o0;
+  });
 }
 
 // Metric, its Cholesky factor and inverse, and the tile-pair lists: all the
@@ -591,7 +546,7 @@ int df_tiled_setup(jk_engine* e) {
   const size_t tot = (size_t)TB * naux * TB;
   for (int t = 0; t < T.npt; ++t) {
     if ((rc = tile_integrals(e, t, Tt.p, s))) return rc;
-    // Bt[r][K][c] = sum_P Linv[K][P] T[r][P][c]
+    // Bt[r][K][c] = sum_P Linv[K][P] T[r][c][P]
     DGemm g;
     g.M = naux;
     g.N = TB;
@@ -602,8 +557,8 @@ int df_tiled_setup(jk_engine* e) {
     g.sak = naux;
     g.a_lower = true;
     g.B = Tt.p;
-    g.sbk = TB;
-    g.sbn = 1;
+    g.sbk = 1;
+    g.sbn = naux;
     g.bsb = (long long)naux * TB;
     g.C = Bt.p;
     g.scm = TB;
@@ -792,40 +747,31 @@ int tiled_xprime_pass(jk_engine* e, const double* Cp, int i0, int ocur, double* 
     tile_of(t, I, J);
     if ((rc = tile_integrals(e, t, Tt, s))) return rc;
     if (hook && (rc = hook(t, I, J))) return rc;
-    // X'[x in I][P][i] += sum_c T[r][P][c] C[128J + c][i]: rows (r, P) in one GEMM
+    // X'[x in I][P][i] += sum_c T[r][c][P] C[128J + c][i], one GEMM per row r
     DGemm a;
-    a.M = TB * naux;
+    a.M = naux;
     a.N = ocur;
     a.K = TB;
+    a.batch = TB;
     a.A = Tt;
-    a.sam = TB;
-    a.sak = 1;
+    a.sam = 1;
+    a.sak = naux;
+    a.bsa = (long long)TB * naux;
     a.B = Cp + (size_t)TB * J + (size_t)i0 * npad;
     a.sbk = 1;
     a.sbn = npad;
     a.C = X + (size_t)TB * I * naux * ocur;
     a.scm = ocur;
     a.scn = 1;
+    a.bsc = (long long)naux * ocur;
     a.beta = 1.0;
     if ((st = dgemm(a, s)) != cudaSuccess) return check_cuda(e, st, "X' (rows)");
-    if (I != J) {  // X'[y in J][P][i] += sum_r T[r][P][c] C[128I + r][i], one GEMM per P
-      DGemm b;
-      b.M = TB;
-      b.N = ocur;
-      b.K = TB;
-      b.batch = naux;
-      b.A = Tt;
-      b.sam = 1;
-      b.sak = (long long)naux * TB;
-      b.bsa = TB;
+    if (I != J) {  // X'[y in J][P][i] += sum_r T[r][c][P] C[128I + r][i], one GEMM per column c
+      DGemm b = a;
+      b.sak = (long long)TB * naux;
+      b.bsa = naux;
       b.B = Cp + (size_t)TB * I + (size_t)i0 * npad;
-      b.sbk = 1;
-      b.sbn = npad;
       b.C = X + (size_t)TB * J * naux * ocur;
-      b.scm = (long long)naux * ocur;
-      b.scn = 1;
-      b.bsc = ocur;
-      b.beta = 1.0;
       if ((st = dgemm(b, s)) != cudaSuccess) return check_cuda(e, st, "X' (columns)");
     }
   }
@@ -843,13 +789,14 @@ static int tiled_fp64(jk_engine* e, const double* dC, int nocc, double* dJ, doub
   const int n = e->obs.n_final, naux = e->aux.n_final, npad = T.npad;
   const size_t tbytes = sizeof(double) * (size_t)TB * naux * TB;
   // scratch that does not depend on the slice
-  DevBuf<double> Tt, Cp, Dm, dv, cv, tv;
+  DevBuf<double> Tt, Cp, Dm, dv, cv, tv, cc;
   cudaError_t st = Tt.alloc(tbytes / sizeof(double));
   if (st == cudaSuccess) st = Cp.alloc((size_t)npad * nocc);
   if (st == cudaSuccess) st = Dm.alloc((size_t)n * n);
   if (st == cudaSuccess) st = dv.alloc(naux);
   if (st == cudaSuccess) st = cv.alloc(naux);
   if (st == cudaSuccess) st = tv.alloc(naux);
+  if (st == cudaSuccess) st = cc.alloc(e->aux.n_cart);
   if (st != cudaSuccess) return check_cuda(e, st, "tiled FP64 scratch");
   // the mixed build's X block is released (its next call allocates it again)
   // so that the occupied slices, each one more integral pass, are as wide as
@@ -895,19 +842,14 @@ static int tiled_fp64(jk_engine* e, const double* dC, int nocc, double* dJ, doub
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->device);
   int rc;
-  auto j_pass_tile = [&](int t, int I, int J) {
-    const int pchunk = (naux + 15) / 16;
-    k_tile_J<<<dim3((naux + pchunk - 1) / pchunk, TB), TB, 0, s>>>(naux, n, TB * I, TB * J, pchunk, Tt.p, cv.p, dJ);
-    (void)t;
-  };
   stage_mark(e, 0, s);
   for (int ch = 0; ch < nch; ++ch) {
     const int i0 = ch * oc, ocur = std::min(oc, nocc - i0);
     rc = tiled_xprime_pass(e, Cp.p, i0, ocur, X.p, Tt.p, s, [&](int t, int I, int J) {
       (void)t;
       if (ch == 0)
-        k_tile_d<<<dim3((naux + 7) / 8, TB), 256, 0, s>>>(naux, n, TB * I, TB * J, I == J ? 1.0 : 2.0, Tt.p, Dm.p, dv.p);
-      if (ch == 1) j_pass_tile(t, I, J);
+        k_tile_d<<<dim3((naux + 255) / 256, TB), 256, 0, s>>>(naux, n, TB * I, TB * J, I == J ? 1.0 : 2.0, Tt.p, Dm.p,
+                                                              dv.p);
       return JK_OK;
     });
     if (rc) return rc;
@@ -933,6 +875,7 @@ static int tiled_fp64(jk_engine* e, const double* dC, int nocc, double* dJ, doub
       g.B = tv.p;
       g.C = cv.p;
       if ((st = dgemm(g, s)) != cudaSuccess) return check_cuda(e, st, "L^-T (L^-1 d)");
+      if ((rc = eri3_J(e, cv.p, cc.p, dJ, s))) return rc;
     }
     // Y = L^-1 X' for every row x, XB rows at a time
     for (int x0 = 0; x0 < n; x0 += XB) {
@@ -984,13 +927,6 @@ static int tiled_fp64(jk_engine* e, const double* dC, int nocc, double* dJ, doub
     }
     if (ch == 0) stage_mark(e, 3, s);  // profiling: K of the first slice
   }
-  if (nch == 1)  // J needs V^-1 d, known only after the first pass
-    for (int t = 0; t < T.npt; ++t) {
-      int I, J;
-      tile_of(t, I, J);
-      if ((rc = tile_integrals(e, t, Tt.p, s))) return rc;
-      j_pass_tile(t, I, J);
-    }
   mirror_lower(dJ, n, s);
   mirror_lower(dK, n, s);
   stage_mark(e, 4, s);

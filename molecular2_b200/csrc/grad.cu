@@ -14,6 +14,7 @@
 
 #include "engine.h"
 #include "grad_kernels.cuh"
+#include "onebody.cuh"
 
 namespace m2 {
 
@@ -42,25 +43,35 @@ __global__ void k_scale_K(int n, const double* __restrict__ K, const double* __r
   K2b[i] = 2.0 * (p[i] - alpha[i]) * K[i];
 }
 
-// kets per 64-thread block: one per thread, halved for classes with few bra
-// pairs so that their blocks still spread over the SMs
-static void launch_grad2e(const jk_engine* e, int A, int B, const Grad2eParams& Pin, int nbra, int nket,
-                          cudaStream_t s) {
+static void launch_grad2e(const jk_engine* e, int A, int B, const Grad2eParams& Pin, cudaStream_t s) {
   Grad2eParams P = Pin;
+  const PairClassDev &ca = e->pcls[A], &cb = e->pcls[B];
   int nb = 0;
-  bra_share(e, nbra, P.bra0, P.bra_step, nb);
+  bra_share(e, ca.npair, P.bra0, P.bra_step, nb);
   if (nb == 0) return;
-  P.kchunk = 64;
-  if ((long long)nb * ((nket + 63) / 64) < 4 * 148) P.kchunk = 32;
-  dim3 grid(nb, (nket + P.kchunk - 1) / P.kchunk, 6);  // z: the six shifted classes
+  P.bra = view(ca);
+  P.ket = view(cb);
+  P.bra_ent = entry_view(ca);
+  P.ket_ent = entry_view(cb);
+  P.same_class = (A == B);
+  // ket entries per block: many share the bra set-up, fewer where the blocks
+  // would not fill the GPU
+  const long long layers = ncart(cb.la) * ncart(cb.lb), nbra = ca.nent / P.bra_step, nket = cb.nent;
+  P.kchunk = GRAD_LIST;
+  while (P.kchunk > 32 &&
+         nbra * ((nket + P.kchunk - 1) / P.kchunk) * layers < (P.kchunk > GRAD_THREADS ? 32 : 8) * 148)
+    P.kchunk /= 2;
+  dim3 grid(ca.nent, (unsigned)((nket + P.kchunk - 1) / P.kchunk), (unsigned)layers);
   if (A <= 2)
     launch_grad2e_bra_s(A, B, P, grid, s);
   else if (A == 3)
     launch_grad2e_bra_ds(B, P, grid, s);
   else if (A == 4)
     launch_grad2e_bra_dp(B, P, grid, s);
-  else
+  else if (B < 4)
     launch_grad2e_bra_dd(B, P, grid, s);
+  else
+    launch_grad2e_bra_dd_hi(B, P, grid, s);
 }
 
 void launch_scale_K(int n, const double* K, const double* p, const double* alpha, double* K2a, double* K2b,
@@ -96,43 +107,33 @@ int grad_rhf_device(jk_engine* e, const double* dD, const double* dW, double pre
   for (int k = 0; k < ns; ++k)
     if (e->obs.atom[k] < 0 || e->obs.atom[k] >= na)
       return set_error(e, JK_ERR_ARG, "gradient: every shell needs an owning atom (jk_basis.atom)");
-  const size_t npp = e->pp_p.n;
-  DevBuf<double> S, T, V, Dc, Wc, Dn, Dmax, K2a, K2b, Z, C;
+  DevBuf<double> S, Dc, Wc, Dn, Dmax, Z, C;
   DevBuf<int> atom;
   DevBuf<unsigned char> sig[NPAIRCLASS];
   cudaError_t st = cudaSuccess;
-  for (auto* b : {&S, &T, &V})
-    if (st == cudaSuccess) st = b->alloc((size_t)n * n);
+  if (st == cudaSuccess) st = S.alloc((size_t)n * n);
   if (st == cudaSuccess) st = Dc.alloc((size_t)nc * nc);
   if (st == cudaSuccess) st = Wc.alloc((size_t)nc * nc);
   if (st == cudaSuccess) st = Dn.alloc((size_t)ns * ns);
   if (st == cudaSuccess) st = Dmax.alloc(2);
-  if (st == cudaSuccess) st = K2a.alloc(npp);
-  if (st == cudaSuccess) st = K2b.alloc(npp);
   if (st == cudaSuccess) st = atom.upload(e->obs.atom, s);
   if (st == cudaSuccess) st = Z.upload(e->Z, s);
   if (st == cudaSuccess) st = C.upload(e->atom_xyz, s);
   for (int k = 0; k < NPAIRCLASS && st == cudaSuccess; ++k)
     if (e->pcls[k].npair) st = sig[k].alloc(e->pcls[k].npair);
   if (st != cudaSuccess) return check_cuda(e, st, "gradient allocation");
-  int rc = one_body_device(e, S.p, T.p, V.p, s);
+  int rc = one_body_device(e, S.p, nullptr, nullptr, s);
   if (rc) return rc;
   for (int k = 0; k < NPAIRCLASS; ++k)
     if (e->pcls[k].npair)
       k_pair_sig<<<(e->pcls[k].npair + 127) / 128, 128, 0, s>>>(view(e->pcls[k]), e->dobs.final_off.p, e->dobs.x.p,
                                                                e->dobs.y.p, e->dobs.z.p, S.p, n, sig[k].p);
-  k_scale_K<<<(unsigned)((npp + 255) / 256), 256, 0, s>>>((int)npp, e->pp_K.p, e->pp_p.p, e->pp_a.p, K2a.p, K2b.p);
   launch_shell_norms(e, dD, Dn.p, Dmax.p, s);
   launch_final_to_cart(e, dD, Dc.p, s);
   launch_final_to_cart(e, dW, Wc.p, s);
   if (with_2e) cudaMemsetAsync(g2e, 0, sizeof(double) * 3 * na, s);
   cudaMemsetAsync(g1e, 0, sizeof(double) * 3 * na, s);
   Grad2eParams P{};
-  P.pp = prim_view(e);
-  P.pp2a = P.pp;
-  P.pp2a.K = K2a.p;
-  P.pp2b = P.pp;
-  P.pp2b.K = K2b.p;
   P.sh = shell_view(e);
   P.atom = atom.p;
   P.Dnorm = Dn.p;
@@ -141,9 +142,9 @@ int grad_rhf_device(jk_engine* e, const double* dD, const double* dW, double pre
   P.Dc = Dc.p;
   P.nc = nc;
   P.precision = precision;
-  P.boys = e->boys.p;
+  P.boysp = e->boysp.p;
   P.grad = g2e;
-  P.kchunk = 64;  // one ket per thread (64-thread blocks)
+  P.natom = na;
   // the class launches run on the engine's side streams, longest first (the
   // gradient is accumulated with atomics, so they commute)
   static const double ncp[6] = {1, 3, 9, 6, 18, 36};
@@ -160,12 +161,9 @@ int grad_rhf_device(jk_engine* e, const double* dD, const double* dW, double pre
   ClassStreams cs(e, s);
   for (const Item& it : items) {
     Grad2eParams Q = P;
-    Q.bra = view(e->pcls[it.A]);
-    Q.ket = view(e->pcls[it.B]);
     Q.bra_sig = sig[it.A].p;
     Q.ket_sig = sig[it.B].p;
-    Q.same_class = (it.A == it.B);
-    launch_grad2e(e, it.A, it.B, Q, e->pcls[it.A].npair, e->pcls[it.B].npair, cs.next(it.cost));
+    launch_grad2e(e, it.A, it.B, Q, cs.next(it.cost));
   }
   cs.join();
   // one-body terms: whole on the first rank of a partition, none on the others
@@ -174,8 +172,7 @@ int grad_rhf_device(jk_engine* e, const double* dD, const double* dW, double pre
     if (!e->pcls[k].npair) continue;
     Grad1eParams Q{};
     Q.pairs = view(e->pcls[k]);
-    Q.pp = prim_view(e);
-    Q.pa = e->pp_a.p;
+    Q.ent = entry_view(e->pcls[k]);
     Q.ox = e->dobs.x.p;
     Q.oy = e->dobs.y.p;
     Q.oz = e->dobs.z.p;
@@ -185,7 +182,7 @@ int grad_rhf_device(jk_engine* e, const double* dD, const double* dW, double pre
     Q.Dc = Dc.p;
     Q.Wc = Wc.p;
     Q.nc = nc;
-    Q.boys = e->boys.p;
+    Q.boysp = e->boysp.p;
     Q.natom = na;
     Q.Z = Z.p;
     Q.cxyz = C.p;

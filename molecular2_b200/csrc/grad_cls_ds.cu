@@ -1,13 +1,13 @@
-// Kernel instantiations of the RHF gradient adjoint, bra class ds.
+// Kernel instantiations of the RHF gradient, bra class ds.
 // Split across translation units only so that nvcc compiles them in parallel.
 #include "grad_kernels.cuh"
 
 namespace m2 {
 void launch_grad2e_bra_ds(int B, const Grad2eParams& P, dim3 grid, cudaStream_t s) {
-  if (B == 0) k_grad2e<2, 0, 0, 0><<<grid, 64, 0, s>>>(P);
-  if (B == 1) k_grad2e<2, 0, 1, 0><<<grid, 64, 0, s>>>(P);
-  if (B == 2) k_grad2e<2, 0, 1, 1><<<grid, 64, 0, s>>>(P);
-  if (B == 3) k_grad2e<2, 0, 2, 0><<<grid, 64, 0, s>>>(P);
+  if (B == 0) launch_grad2e_class<2, 0, 0, 0>(P, grid, s);
+  if (B == 1) launch_grad2e_class<2, 0, 1, 0>(P, grid, s);
+  if (B == 2) launch_grad2e_class<2, 0, 1, 1>(P, grid, s);
+  if (B == 3) launch_grad2e_class<2, 0, 2, 0>(P, grid, s);
 }
 
 }  // namespace m2

@@ -179,9 +179,9 @@ int build_pairs(jk_engine* e) {
     for (int k = 0; k < NPAIRCLASS; ++k) {
       if (e->pcls[k].npair == 0) continue;
       const PairView v{di.p + io[k][0], di.p + io[k][1], di.p + io[k][2], di.p + io[k][3], nullptr, e->pcls[k].npair};
-      SchwarzParams P{v, prim_view(e), shell_view(e), e->dobs.l.p, e->dobs.pure.p, e->dobs.sph.p, e->boys.p,
+      SchwarzParams P{v, prim_view(e), shell_view(e), e->dobs.l.p, e->dobs.pure.p, e->dobs.sph.p, e->boysp.p,
                       dq.p + qo[k]};
-      launch_schwarz(cls[k].la, cls[k].lb, P, e->pcls[k].npair, s);
+      launch_schwarz(cls[k].la, cls[k].lb, P, s);
     }
     st = cudaMemcpyAsync(Q.data(), dq.p, ntot * sizeof(double), cudaMemcpyDeviceToHost, s);
     if (st == cudaSuccess) st = cudaStreamSynchronize(s);

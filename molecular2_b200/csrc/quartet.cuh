@@ -41,6 +41,8 @@ __host__ __device__ constexpr int herm_v(int h) { return cart_c(herm_k(h), h - n
 
 constexpr int ENTRY_PRIMS = 8;   // primitive pairs per entry
 constexpr int ENTRY_FIELDS = 7;  // p, Px, Py, Pz, K sqrt(2 pi^(5/2)) / p, 1/(2p), exponent of the first shell
+__host__ __device__ constexpr double PI25X2() { return 34.986836655249725; }          // 2 pi^(5/2)
+__host__ __device__ constexpr double SQRT_PI25X2() { return 5.914967172795612; }      // its square root
 
 struct EntryView {
   const int* pair;        // pair index in the class list (Schwarz-sorted)
@@ -55,6 +57,26 @@ __device__ __forceinline__ const double* entry_prims(const EntryView& v, int e) 
 }
 __device__ __forceinline__ double entry_field(const double* base, int k, int f) {
   return __ldg(base + (k * ENTRY_FIELDS + f) * 32);
+}
+
+// Ket entries e in [start, end) with pass(e), packed into list; returns their
+// number.  All threads of the block call this (n_shared: a shared counter).
+template <class Pass>
+__device__ __forceinline__ int pack_kets(int start, int end, int* list, int* n_shared, Pass&& pass) {
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) *n_shared = 0;
+  __syncthreads();
+  for (int e0 = start; e0 < end; e0 += blockDim.x) {
+    const int e = e0 + threadIdx.x;
+    const bool ok = e < end && pass(e);
+    const unsigned m = __ballot_sync(0xffffffffu, ok);
+    int pos = 0;
+    if (lane == 0 && m) pos = atomicAdd(n_shared, __popc(m));
+    pos = __shfl_sync(0xffffffffu, pos, 0) + __popc(m & ((1u << lane) - 1));
+    if (ok) list[pos] = e;
+  }
+  __syncthreads();
+  return *n_shared;
 }
 
 // ---------------------------------------------------------------- Boys
@@ -95,18 +117,14 @@ __device__ __forceinline__ void boys_poly(double T, const double* tab, double* F
   }
 }
 
-// R_tuv (t + u + v <= L) times `scale` of a primitive quartet with exponents
-// p, q and distance (X, Y, Z): prefactor and reduced exponent from one
-// reciprocal square root.
+// scale R_tuv (t + u + v <= L) for the reduced exponent a and distance (X, Y, Z).
 template <int L>
-__device__ __forceinline__ void quartet_R(double p, double q, double KK, double X, double Y, double Z,
-                                          const double* tab, double* R) {
-  const double r = rsqrt(p + q);
-  const double a = p * q * r * r;
+__device__ __forceinline__ void hermite_R(double a, double scale, double X, double Y, double Z, const double* tab,
+                                          double* R) {
   double F[L + 1];
   boys_poly<L>(a * (X * X + Y * Y + Z * Z), tab, F);
   const double m2a = -2.0 * a;
-  double pw = KK * r;
+  double pw = scale;
 #pragma unroll
   for (int n = 0; n <= L; ++n) {
     F[n] *= pw;
@@ -134,6 +152,14 @@ __device__ __forceinline__ void quartet_R(double p, double q, double KK, double 
     R[0] = F[n];
   });
 }
+// The same for a primitive quartet with exponents p, q and prefactors KK =
+// K'_ab K'_cd: prefactor and reduced exponent from one reciprocal square root.
+template <int L>
+__device__ __forceinline__ void quartet_R(double p, double q, double KK, double X, double Y, double Z,
+                                          const double* tab, double* R) {
+  const double r = rsqrt(p + q);
+  hermite_R<L>(p * q * r * r, KK * r, X, Y, Z, tab, R);
+}
 
 // ---------------------------------------------------------------- bra tables
 // Hermite expansion of the Cartesian products of one primitive pair as a list
@@ -154,7 +180,8 @@ __host__ __device__ constexpr int e1_size(int la, int lb) { return (la + 1) * (l
 
 template <int LA, int LB>
 struct TermTab {
-  unsigned char x[nterms(LA, LB)], y[nterms(LA, LB)], z[nterms(LA, LB)];
+  unsigned char x[nterms(LA, LB)], y[nterms(LA, LB)], z[nterms(LA, LB)];  // e1_pos of the three factors
+  short first[ncart(LA) * ncart(LB) + 1];                                 // first term of each component
 };
 template <int LA, int LB>
 __host__ __device__ constexpr TermTab<LA, LB> make_terms() {
@@ -164,6 +191,7 @@ __host__ __device__ constexpr TermTab<LA, LB> make_terms() {
     for (int j = 0; j < ncart(LB); ++j) {
       const int ax = cart_a(LA, i), ay = cart_b(LA, i), az = cart_c(LA, i);
       const int bx = cart_a(LB, j), by = cart_b(LB, j), bz = cart_c(LB, j);
+      T.first[i * ncart(LB) + j] = (short)n;
       for (int t = 0; t <= ax + bx; ++t)
         for (int u = 0; u <= ay + by; ++u)
           for (int v = 0; v <= az + bz; ++v, ++n) {
@@ -172,6 +200,7 @@ __host__ __device__ constexpr TermTab<LA, LB> make_terms() {
             T.z[n] = (unsigned char)e1_pos(LA, LB, az, bz, v);
           }
     }
+  T.first[ncart(LA) * ncart(LB)] = (short)n;
   return T;
 }
 __constant__ constexpr TermTab<0, 0> c_terms00 = make_terms<0, 0>();
@@ -258,6 +287,22 @@ __device__ __forceinline__ void bra_transform(const double* M, const double* W, 
   }
 }
 
+// One component of the bra transform, by a run-time index: sum of M W.
+template <int LA, int LB>
+__device__ __forceinline__ double bra_component(const double* M, const double* W, int ij) {
+  if constexpr (LA + LB == 0) {
+    return W[0];
+  } else {
+    const TermTab<LA, LB>& T = term_tab<LA, LB>();
+    constexpr int N = LA + LB + 1;
+    int k = T.first[ij];
+    const int k1 = T.first[ij + 1];
+    double acc = 0.0;
+    for (; k < k1; ++k) acc += M[k] * W[hidx(T.x[k] % N, T.y[k] % N, T.z[k] % N)];
+    return acc;
+  }
+}
+
 // ---------------------------------------------------------------- ket expansion
 // One application of (x - centre) to a one-direction Hermite expansion.
 template <int N>
@@ -290,6 +335,160 @@ __device__ __forceinline__ void ket_accumulate(double* W, const double* R, const
       });
     }
   });
+}
+
+// ---------------------------------------------------------------- derivatives
+// With P = (alpha A + beta B)/p and R = A - B, d/dA = (alpha/p) d/dP + d/dR: the
+// first part shifts a Hermite index, the second differentiates the expansion
+// coefficients (and the prefactor exp(-mu R^2), whose factor belongs to them),
+// which leaves their order unchanged.  One table of R integrals of order L + 1
+// therefore gives the derivatives with respect to all centres.
+
+// (x - centre) applied to an expansion e and to its R derivative r; Xr = d(X)/dR.
+template <int N>
+__device__ __forceinline__ void e1_raise_dual(double* e, double* r, double X, double Xr, double h) {
+  double n[N + 1];
+#pragma unroll
+  for (int t = 0; t <= N; ++t) n[t] = Xr * e[t];
+  e1_raise<N>(e, X, h);
+  e1_raise<N>(r, X, h);
+#pragma unroll
+  for (int t = 0; t <= N; ++t) r[t] += n[t];
+}
+
+// Term products of the bra entry and their derivatives d/dR_x, x = 0, 1, 2.
+template <int LA, int LB>
+struct BraGradShared {
+  double prim[ENTRY_PRIMS][6];  // p, Px, Py, Pz, K', alpha/p
+  double E[ENTRY_PRIMS][2][3][e1_size(LA, LB)];
+  double M[ENTRY_PRIMS][4][nterms(LA, LB)];
+};
+template <int LA, int LB>
+__device__ __forceinline__ void load_bra_grad(BraGradShared<LA, LB>& S, const double* base, int nb, double Ax,
+                                              double Ay, double Az, double Bx, double By, double Bz) {
+  const int tid = threadIdx.x;
+  for (int i = tid; i < nb * 6; i += blockDim.x) {
+    const int ib = i / 6, f = i % 6;
+    S.prim[ib][f] = f < 5 ? entry_field(base, ib, f) : entry_field(base, ib, 6) * 2.0 * entry_field(base, ib, 5);
+  }
+  for (int i = tid; i < nb * 3; i += blockDim.x) {
+    const int ib = i / 3, dir = i % 3;
+    const double A = dir == 0 ? Ax : (dir == 1 ? Ay : Az), B = dir == 0 ? Bx : (dir == 1 ? By : Bz);
+    const double P = entry_field(base, ib, 1 + dir), h = entry_field(base, ib, 5);
+    const double al = entry_field(base, ib, 6), fa = 2.0 * h * al, fb = 1.0 - fa;  // alpha/p, beta/p
+    constexpr int N = LA + LB;
+    double ea[N + 1], ra[N + 1];
+#pragma unroll
+    for (int t = 0; t <= N; ++t) ea[t] = ra[t] = 0.0;
+    ea[0] = 1.0;
+    ra[0] = -2.0 * al * fb * (A - B);
+#pragma unroll
+    for (int a = 0; a <= LA; ++a) {
+      if (a > 0) e1_raise_dual<N>(ea, ra, P - A, -fb, h);
+      double eb[N + 1], rb[N + 1];
+#pragma unroll
+      for (int t = 0; t <= N; ++t) {
+        eb[t] = ea[t];
+        rb[t] = ra[t];
+      }
+#pragma unroll
+      for (int b = 0; b <= LB; ++b) {
+        if (b > 0) e1_raise_dual<N>(eb, rb, P - B, fa, h);
+#pragma unroll
+        for (int t = 0; t <= N; ++t) {
+          S.E[ib][0][dir][e1_pos(LA, LB, a, b, t)] = eb[t];
+          S.E[ib][1][dir][e1_pos(LA, LB, a, b, t)] = rb[t];
+        }
+      }
+    }
+  }
+  __syncthreads();
+  constexpr int NT = nterms(LA, LB);
+  const TermTab<LA, LB>& T = term_tab<LA, LB>();
+  for (int i = tid; i < nb * 4 * NT; i += blockDim.x) {
+    const int ib = i / (4 * NT), w = (i / NT) % 4, k = i % NT;  // w = 0: value, 1 + x: d/dR_x
+    S.M[ib][w][k] = S.E[ib][w == 1][0][T.x[k]] * S.E[ib][w == 2][1][T.y[k]] * S.E[ib][w == 3][2][T.z[k]];
+  }
+  __syncthreads();
+}
+
+// f(component, term, Hermite index), all constants, over the terms of (LA, LB)
+template <int LA, int LB, class F>
+__device__ __forceinline__ void for_terms(F&& f) {
+  static_for<ncart(LA) * ncart(LB)>([&](auto ij) {
+    constexpr int c = decltype(ij)::value, i = c / ncart(LB), j = c % ncart(LB);
+    constexpr int nu = cart_b(LA, i) + cart_b(LB, j) + 1, nv = cart_c(LA, i) + cart_c(LB, j) + 1;
+    constexpr int nt = (cart_a(LA, i) + cart_a(LB, j) + 1) * nu * nv;
+    constexpr int k0 = term_off(LA, LB, c);
+    static_for<nt>([&](auto q) {
+      constexpr int k = decltype(q)::value;
+      f(std::integral_constant<int, c>{}, std::integral_constant<int, k0 + k>{},
+        std::integral_constant<int, hidx(k / (nu * nv), (k / nv) % nu, k % nv)>{});
+    });
+  });
+}
+
+// One primitive quartet's derivatives for bra weights G (Hermite orders <= HL)
+// and one ket component with expansions e, their R derivatives r and bounds
+// (tx, ty, tz): gP[x] += d/dP_x, gR[x] += the ket's d/dR_x part.  R holds orders
+// up to HL + LK + 1.  V is the bra's potential at one ket Hermite index.
+template <int HL, int LK>
+__device__ __forceinline__ void ket_gradient(const double* G, const double* R, const double (*e)[LK + 1],
+                                             const double (*r)[LK + 1], int tx, int ty, int tz, double* gP,
+                                             double* gR) {
+  static_for<nherm(LK + 1)>([&](auto gg) {
+    constexpr int a = herm_t(decltype(gg)::value), b = herm_u(decltype(gg)::value), c = herm_v(decltype(gg)::value);
+    const bool box = a <= tx && b <= ty && c <= tz;
+    const bool sx = a > 0 && a - 1 <= tx && b <= ty && c <= tz;
+    const bool sy = b > 0 && a <= tx && b - 1 <= ty && c <= tz;
+    const bool sz = c > 0 && a <= tx && b <= ty && c - 1 <= tz;
+    if (box || sx || sy || sz) {
+      double v0 = 0.0, v1 = 0.0;
+      static_for<nherm(HL)>([&](auto hh) {
+        constexpr int h = decltype(hh)::value;
+        if constexpr (h & 1)
+          v1 += G[h] * R[hidx(herm_t(h) + a, herm_u(h) + b, herm_v(h) + c)];
+        else
+          v0 += G[h] * R[hidx(herm_t(h) + a, herm_u(h) + b, herm_v(h) + c)];
+      });
+      const double V = ((a + b + c) & 1) ? -(v0 + v1) : v0 + v1;
+      if constexpr (a + b + c <= LK) {
+        if (box) {
+          gR[0] += r[0][a] * e[1][b] * e[2][c] * V;
+          gR[1] += e[0][a] * r[1][b] * e[2][c] * V;
+          gR[2] += e[0][a] * e[1][b] * r[2][c] * V;
+        }
+      }
+      if constexpr (a > 0)
+        if (sx) gP[0] -= e[0][a - 1] * e[1][b] * e[2][c] * V;
+      if constexpr (b > 0)
+        if (sy) gP[1] -= e[0][a] * e[1][b - 1] * e[2][c] * V;
+      if constexpr (c > 0)
+        if (sz) gP[2] -= e[0][a] * e[1][b] * e[2][c - 1] * V;
+    }
+  });
+}
+// One-direction expansions of the ket component (i, j) in each direction and
+// their R derivatives.
+template <int LC, int LD>
+__device__ __forceinline__ void ket_expansions(double (*e)[LC + LD + 1], double (*r)[LC + LD + 1], const double* Q,
+                                               const double* C, const double* D, double ga, double h, const int* ce,
+                                               const int* de) {
+  constexpr int N = LC + LD;
+  const double fc = 2.0 * h * ga, fd = 1.0 - fc;  // gamma/q, delta/q
+#pragma unroll
+  for (int x = 0; x < 3; ++x) {
+#pragma unroll
+    for (int t = 0; t <= N; ++t) e[x][t] = r[x][t] = 0.0;
+    e[x][0] = 1.0;
+    r[x][0] = -2.0 * ga * fd * (C[x] - D[x]);
+#pragma unroll
+    for (int s = 0; s < LC; ++s)
+      if (s < ce[x]) e1_raise_dual<N>(e[x], r[x], Q[x] - C[x], -fd, h);
+#pragma unroll
+    for (int s = 0; s < LD; ++s)
+      if (s < de[x]) e1_raise_dual<N>(e[x], r[x], Q[x] - D[x], fc, h);
+  }
 }
 
 }  // namespace m2

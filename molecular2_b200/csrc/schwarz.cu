@@ -4,14 +4,13 @@
 
 namespace m2 {
 
-void launch_schwarz(int la, int lb, const SchwarzParams& P, int npair, cudaStream_t s) {
-  dim3 grid((npair + 63) / 64);
-  if (la == 0 && lb == 0) k_schwarz<0, 0><<<grid, 64, 0, s>>>(P);
-  if (la == 1 && lb == 0) k_schwarz<1, 0><<<grid, 64, 0, s>>>(P);
-  if (la == 1 && lb == 1) k_schwarz<1, 1><<<grid, 64, 0, s>>>(P);
-  if (la == 2 && lb == 0) k_schwarz<2, 0><<<grid, 64, 0, s>>>(P);
-  if (la == 2 && lb == 1) k_schwarz<2, 1><<<grid, 64, 0, s>>>(P);
-  if (la == 2 && lb == 2) k_schwarz<2, 2><<<grid, 64, 0, s>>>(P);
+void launch_schwarz(int la, int lb, const SchwarzParams& P, cudaStream_t s) {
+  if (la == 0 && lb == 0) launch_schwarz_class<0, 0>(P, s);
+  if (la == 1 && lb == 0) launch_schwarz_class<1, 0>(P, s);
+  if (la == 1 && lb == 1) launch_schwarz_class<1, 1>(P, s);
+  if (la == 2 && lb == 0) launch_schwarz_class<2, 0>(P, s);
+  if (la == 2 && lb == 1) launch_schwarz_class<2, 1>(P, s);
+  if (la == 2 && lb == 2) launch_schwarz_class<2, 2>(P, s);
 }
 
 }  // namespace m2

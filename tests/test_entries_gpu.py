@@ -51,3 +51,34 @@ def test_direct_contraction_lengths(lens, spherical):
     *refs, nq = oracle.jk_direct_uhf(obs, Da, Db, Q, 1e-14)
     for got, ref in zip(eng.jk_direct_uhf(Da, Db, 1e-14), refs):
         assert np.abs(got - ref).max() < TOL
+
+
+@pytest.mark.parametrize("lens", CASES)
+def test_schwarz_and_one_body_contraction_lengths(lens):
+    """Schwarz bounds (square roots of one integral, |Q| <= 2) and S, T, V (|V| <= 60; sums over up to 289
+    primitives and 3 nuclei, 60 * 300 * 1.1e-16 = 2e-12; 5e-12 leaves a factor two)."""
+    obs = basis(lens)
+    eng = IntegralEngine(obs)
+    assert np.abs(eng.getPrescreen() - oracle.schwarz(obs)).max() < 1e-13
+    for got, ref in zip(eng.one_body(), oracle.one_body(obs)):
+        assert np.abs(ref).max() < 60.0
+        assert np.abs(got - ref).max() < 5e-12
+
+
+@pytest.mark.parametrize("lens", CASES)
+@pytest.mark.parametrize("spherical", [True, False])
+def test_gradient_contraction_lengths(lens, spherical):
+    """Terms are integrals times 2 alpha (alpha <= 40, |g| <= 100 a term), at most 324 x 289 of them:
+    the sum's rounding is below 100 * sqrt(94,000) * 1.1e-16 = 3e-12; 2e-11 leaves a factor six."""
+    obs = basis(lens, spherical)
+    rng = np.random.default_rng(4)
+    C = rng.normal(size=(obs.nbf, 3)) * 0.3
+    D, W = 2.0 * C @ C.T, (C * np.array([-1.0, -0.7, -0.4])) @ C.T
+    g, g2 = IntegralEngine(obs).compute_forces(D, W, 1e-14)
+    ref2 = oracle.grad2e(obs, D, oracle.schwarz(obs), 1e-14)
+    S1, T1, V1 = oracle.one_body_deriv(obs)
+    na = obs.mol.natom
+    ref = ref2 + obs.mol.enuc_grad() + np.array(
+        [np.sum((T1[i] + V1[i]) * D) - 2.0 * np.sum(S1[i] * W) for i in range(3 * na)]).reshape(na, 3)
+    assert max(np.abs(ref).max(), np.abs(ref2).max()) < 100.0
+    assert max(np.abs(g - ref).max(), np.abs(g2 - ref2).max()) < 2e-11
