@@ -28,14 +28,12 @@
 
 namespace m2 {
 
-PrimView prim_view(const jk_engine* e);
-ShellView shell_view(const jk_engine* e);
 
 int prepare_aux(jk_engine* e) {
   if (!e->has_aux) return set_error(e, JK_ERR_STATE, "no fitting basis was given to jk_create");
   if (e->ap_p.p) return JK_OK;
   const HostBasis& a = e->aux;
-  std::vector<double> p, x, y, z, K, Kp, h;
+  std::vector<double> p, x, y, z, Kp, h;
   std::vector<int> off;
   for (int s = 0; s < a.nshell; ++s) {
     off.push_back((int)p.size());
@@ -44,8 +42,7 @@ int prepare_aux(jk_engine* e) {
       x.push_back(a.xyz[3 * s]);
       y.push_back(a.xyz[3 * s + 1]);
       z.push_back(a.xyz[3 * s + 2]);
-      K.push_back(a.coefs[a.prim_off[s] + k]);
-      Kp.push_back(K.back() * SQRT_PI25X2() / p.back());
+      Kp.push_back(a.coefs[a.prim_off[s] + k] * SQRT_PI25X2() / p.back());
       h.push_back(0.5 / p.back());
     }
   }
@@ -54,19 +51,11 @@ int prepare_aux(jk_engine* e) {
   if (r == cudaSuccess) r = e->ap_x.upload(x, st);
   if (r == cudaSuccess) r = e->ap_y.upload(y, st);
   if (r == cudaSuccess) r = e->ap_z.upload(z, st);
-  if (r == cudaSuccess) r = e->ap_K.upload(K, st);
   if (r == cudaSuccess) r = e->ap_Kp.upload(Kp, st);
   if (r == cudaSuccess) r = e->ap_h.upload(h, st);
   if (r == cudaSuccess) r = e->aux_prim_off.upload(off, st);
-  for (int l = 0; l <= MAX_L_AUX && r == cudaSuccess; ++l) {
-    std::vector<int> sh;
-    for (int s = 0; s < a.nshell; ++s)
-      if (a.l[s] == l) sh.push_back(s);
-    e->aux_by_l_count[l] = (int)sh.size();
-    r = e->aux_by_l[l].upload(sh, st);
-  }
   std::vector<int> groups[jk_engine::NAUXGROUP];
-  for (int s = 0; s < a.nshell; ++s) groups[a.l[s] <= 1 ? a.l[s] : 2 * a.l[s] - (a.pure[s] ? 2 : 1)].push_back(s);
+  for (int s = 0; s < a.nshell; ++s) groups[aux_group_of(a.l[s], a.pure[s])].push_back(s);
   for (int g = 0; g < jk_engine::NAUXGROUP && r == cudaSuccess; ++g) {
     e->aux_group_count[g] = (int)groups[g].size();
     r = e->aux_group[g].upload(groups[g], st);
@@ -75,17 +64,17 @@ int prepare_aux(jk_engine* e) {
   return check_cuda(e, r, "prepare fitting basis");
 }
 
-static PrimView aux_view(const jk_engine* e) {
-  return PrimView{e->ap_p.p, e->ap_x.p, e->ap_y.p, e->ap_z.p, e->ap_K.p};
+AuxView aux_group_view(const jk_engine* e, const int* shells, int count) {
+  return AuxView{shells,    count,     e->aux_prim_off.p, e->daux.nprim.p, e->ap_p.p,
+                 e->ap_x.p, e->ap_y.p, e->ap_z.p,         e->ap_Kp.p,      e->ap_h.p,
+                 e->daux.final_off.p};
 }
 
 // Launch parameters of the three-index kernels for fitting group g and orbital
 // pair class pc.
 static Eri3Params eri3_params(const jk_engine* e, int g, int pc) {
   Eri3Params P{};
-  P.aux = AuxView{e->aux_group[g].p, e->aux_group_count[g], e->aux_prim_off.p, e->daux.nprim.p,
-                  e->ap_p.p,         e->ap_x.p,             e->ap_y.p,         e->ap_z.p,
-                  e->ap_Kp.p,        e->ap_h.p,             e->daux.final_off.p};
+  P.aux = aux_group_view(e, e->aux_group[g].p, e->aux_group_count[g]);
   P.ent = entry_view(e->pcls[pc]);
   P.pairs = view(e->pcls[pc]);
   P.ox = e->dobs.x.p;
@@ -172,29 +161,21 @@ int eri3_J(jk_engine* e, const double* c, double* cc, double* J, cudaStream_t s)
 }
 
 int compute_V(jk_engine* e, double* V, cudaStream_t s) {
-  const int naux = e->aux.n_final;
-  for (int lp = 0; lp <= MAX_L_AUX; ++lp)
-    for (int lq = 0; lq <= lp; ++lq) {
-      if (!e->aux_by_l_count[lp] || !e->aux_by_l_count[lq]) continue;
+  ClassStreams cs(e, s);
+  for (int gP = jk_engine::NAUXGROUP - 1; gP >= 0; --gP)
+    for (int gQ = gP; gQ >= 0; --gQ) {
+      if (!e->aux_group_count[gP] || !e->aux_group_count[gQ]) continue;
       Eri2Params P{};
-      P.ap = aux_view(e);
-      P.shells_p = e->aux_by_l[lp].p;
-      P.np = e->aux_by_l_count[lp];
-      P.shells_q = e->aux_by_l[lq].p;
-      P.nq = e->aux_by_l_count[lq];
-      P.aux_prim_off = e->aux_prim_off.p;
-      P.aux_nprim = e->daux.nprim.p;
-      P.ax = e->daux.x.p;
-      P.ay = e->daux.y.p;
-      P.az = e->daux.z.p;
-      P.aux_foff = e->daux.final_off.p;
-      P.aux_pure = e->daux.pure.p;
+      P.P = aux_group_view(e, e->aux_group[gP].p, e->aux_group_count[gP]);
+      P.Q = aux_group_view(e, e->aux_group[gQ].p, e->aux_group_count[gQ]);
       P.sph = e->dobs.sph.p;
-      P.boys = e->boys.p;
-      P.naux = naux;
+      P.boysp = e->boysp.p;
+      P.naux = e->aux.n_final;
+      P.same = gP == gQ;
       P.V = V;
-      launch_eri2(lp, lq, P, s);
+      launch_eri2(gP, gQ, P, cs.next((double)P.P.count * P.Q.count));
     }
+  cs.join();
   return check_cuda(e, cudaGetLastError(), "eri2 launch");
 }
 

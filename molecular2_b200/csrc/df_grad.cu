@@ -13,6 +13,7 @@
 //   d           = bt L^-1  over K (d^P_ij = sum_Q V^-1_PQ (Q|ij))   (TRSM)
 //   W2          = d^T d - 1/2 c c^T                            (DGEMM + DGER)
 //   Z^P         = C d^P C^T,  W3^P = c_P D - 2 Z^P              (batched DGEMM)
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -24,10 +25,7 @@ namespace m2 {
 
 int grad_rhf_device(jk_engine* e, const double* dD, const double* dW, double precision, double* g2e, double* g1e,
                     cudaStream_t s, bool with_2e);
-void launch_scale_K(int n, const double* K, const double* p, const double* alpha, double* K2a, double* K2b,
-                    cudaStream_t s);
 void nuclear_repulsion_grad(const jk_engine* e, std::vector<double>& gn);
-PrimView prim_view(const jk_engine* e);
 
 // gt_K = 2 sum_i bt[K](i,i)
 __global__ void k_trace_bt(int naux, int o, const double* __restrict__ bt, double* __restrict__ g) {
@@ -48,13 +46,6 @@ __global__ void k_w3(size_t nn, int naux, const double* __restrict__ c, const do
   Z[i] = c[P] * D[i % nn] - 2.0 * Z[i];
 }
 
-// 2 alpha K for the (P, unit) fitting primitives (alpha = p)
-__global__ void k_scale_aux(int n, const double* __restrict__ K, const double* __restrict__ p,
-                            double* __restrict__ K2) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) K2[i] = 2.0 * p[i] * K[i];
-}
-
 // Ce = C diag(eps), C column-major n x o
 __global__ void k_scale_cols(int n, int o, const double* __restrict__ C, const double* __restrict__ eps,
                              double* __restrict__ Ce) {
@@ -64,83 +55,91 @@ __global__ void k_scale_cols(int n, int o, const double* __restrict__ C, const d
 
 int grad_df_2e_tiled(jk_engine* e, const double* dC, int nocc, const double* dD, double* g2e, cudaStream_t s);
 
-// k_grad3 over every orbital pair class for the fitting shells `shells` (all
-// of angular momentum l) with W3 holding fitting functions from w3_f0 on.
-static void launch_grad3_all(jk_engine* e, int l, const int* shells, int nshells, const double* W3, int w3_f0,
-                             const double* K2a, const double* K2b, double* g2e, cudaStream_t s) {
-  const PrimView ap{e->ap_p.p, e->ap_x.p, e->ap_y.p, e->ap_z.p, e->ap_K.p};
-  for (int pc = 0; pc < NPAIRCLASS; ++pc) {
-    if (!e->pcls[pc].npair) continue;
+// Cc (nc x o) = coefficients of the Cartesian functions for C (n x o), column-major
+__global__ void k_cart_rows(int nc, int n, int o, const int* __restrict__ cshell, const int* __restrict__ ccomp,
+                            const int* __restrict__ l, const int* __restrict__ pure, const int* __restrict__ foff,
+                            const double* __restrict__ sph, const double* __restrict__ C, double* __restrict__ Cc) {
+  const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (size_t)nc * o) return;
+  const int a = (int)(idx % nc), i = (int)(idx / nc), sh = cshell[a], ic = ccomp[a], ls = l[sh], f0 = foff[sh];
+  const double* c = C + (size_t)i * n + f0;
+  double v = 0.0;
+  if (pure[sh])
+    for (int m = 0; m < 2 * ls + 1; ++m) v += sph[sph_off(ls) + m * ncart(ls) + ic] * c[m];
+  else
+    v = c[ic];
+  Cc[idx] = v;
+}
+static void launch_cart_rows(const jk_engine* e, int o, const double* C, double* Cc, cudaStream_t s) {
+  const int nc = e->obs.n_cart;
+  k_cart_rows<<<(unsigned)(((size_t)nc * o + 255) / 256), 256, 0, s>>>(
+      nc, e->obs.n_final, o, e->dobs.cart_shell.p, e->dobs.cart_comp.p, e->dobs.l.p, e->dobs.pure.p,
+      e->dobs.final_off.p, e->dobs.sph.p, C, Cc);
+}
+
+// k_grad3 over every orbital pair class and the given fitting shells of each
+// group, with W3 (Cartesian orbital functions) holding fitting functions from
+// w3_f0 on; the launches add to the gradient and run on the side streams,
+// longest first.
+static void launch_grad3_all(jk_engine* e, const int* const* shells, const int* counts, const double* W3, int w3_f0,
+                             double* g2e, cudaStream_t s) {
+  static decltype(&launch_grad3_s) const launch[jk_engine::NAUXGROUP] = {
+      launch_grad3_s, launch_grad3_p, launch_grad3_d_pure, launch_grad3_d_cart, launch_grad3_f_pure, launch_grad3_f_cart};
+  static const double ncp[NPAIRCLASS] = {1, 3, 9, 6, 18, 36};
+  static const int gl[jk_engine::NAUXGROUP] = {0, 1, 2, 2, 3, 3};
+  struct Item {
+    int g, pc;
+    double cost;
+  };
+  std::vector<Item> items;
+  for (int g = 0; g < jk_engine::NAUXGROUP; ++g)
+    for (int pc = 0; pc < NPAIRCLASS; ++pc)
+      if (counts[g] && e->pcls[pc].npair)
+        items.push_back({g, pc, (double)e->pcls[pc].nent * counts[g] * ncp[pc] * (gl[g] + 1) * (gl[g] + 2)});
+  std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.cost > b.cost; });
+  ClassStreams cs(e, s);
+  for (const Item& it : items) {
     Grad3Params P{};
-    P.ap = ap;
-    P.aux_shells = shells;
-    P.naux_shells = nshells;
-    P.aux_prim_off = e->aux_prim_off.p;
-    P.aux_nprim = e->daux.nprim.p;
-    P.ax = e->daux.x.p;
-    P.ay = e->daux.y.p;
-    P.az = e->daux.z.p;
-    P.aux_foff = e->daux.final_off.p;
-    P.aux_pure = e->daux.pure.p;
+    P.aux = aux_group_view(e, shells[it.g], counts[it.g]);
     P.aux_atom = e->daux.atom.p;
-    P.pairs = view(e->pcls[pc]);
-    P.pp = prim_view(e);
-    P.pp2a = P.pp;
-    P.pp2a.K = K2a;
-    P.pp2b = P.pp;
-    P.pp2b.K = K2b;
+    P.atom = e->dobs.atom.p;
+    P.ent = entry_view(e->pcls[it.pc]);
+    P.pairs = view(e->pcls[it.pc]);
     P.ox = e->dobs.x.p;
     P.oy = e->dobs.y.p;
     P.oz = e->dobs.z.p;
-    P.obs_foff = e->dobs.final_off.p;
-    P.obs_pure = e->dobs.pure.p;
-    P.obs_atom = e->dobs.atom.p;
-    P.sph_obs = e->dobs.sph.p;
-    P.sph_aux = e->dobs.sph.p;
-    P.boys = e->boys.p;
-    P.n = e->obs.n_final;
+    P.coff = e->dobs.cart_off.p;
+    P.sph = e->dobs.sph.p;
+    P.boysp = e->boysp.p;
+    P.nc = e->obs.n_cart;
     P.W3 = W3;
     P.w3_f0 = w3_f0;
+    P.natom = e->natom;
     P.grad = g2e;
-    if (l == 0) launch_grad3_l0(pc, P, s);
-    if (l == 1) launch_grad3_l1(pc, P, s);
-    if (l == 2) launch_grad3_l2(pc, P, s);
-    if (l == 3) launch_grad3_l3(pc, P, s);
+    launch[it.g](it.pc, P, cs.next(it.cost));
   }
+  cs.join();
 }
 
-// k_grad2 over every pair of fitting angular momenta with the weights W2.
-static void launch_grad2_all(jk_engine* e, const double* ap2K, const double* W2, double* g2e, cudaStream_t s) {
-  const PrimView ap{e->ap_p.p, e->ap_x.p, e->ap_y.p, e->ap_z.p, e->ap_K.p};
-  PrimView aps = ap;
-  aps.K = ap2K;
-  for (int lp = 0; lp <= MAX_L_AUX; ++lp)
-    for (int lq = 0; lq <= MAX_L_AUX; ++lq) {
-      if (!e->aux_by_l_count[lp] || !e->aux_by_l_count[lq]) continue;
+// k_grad2 over every ordered pair of fitting groups with the weights W2.
+static void launch_grad2_all(jk_engine* e, const double* W2, double* g2e, cudaStream_t s) {
+  ClassStreams cs(e, s);
+  for (int gP = jk_engine::NAUXGROUP - 1; gP >= 0; --gP)
+    for (int gQ = jk_engine::NAUXGROUP - 1; gQ >= 0; --gQ) {
+      if (!e->aux_group_count[gP] || !e->aux_group_count[gQ]) continue;
       Grad2Params P{};
-      P.ap = ap;
-      P.ap2 = aps;
-      P.shells_p = e->aux_by_l[lp].p;
-      P.np = e->aux_by_l_count[lp];
-      P.shells_q = e->aux_by_l[lq].p;
-      P.nq = e->aux_by_l_count[lq];
-      P.aux_prim_off = e->aux_prim_off.p;
-      P.aux_nprim = e->daux.nprim.p;
-      P.ax = e->daux.x.p;
-      P.ay = e->daux.y.p;
-      P.az = e->daux.z.p;
-      P.aux_foff = e->daux.final_off.p;
-      P.aux_pure = e->daux.pure.p;
+      P.P = aux_group_view(e, e->aux_group[gP].p, e->aux_group_count[gP]);
+      P.Q = aux_group_view(e, e->aux_group[gQ].p, e->aux_group_count[gQ]);
       P.aux_atom = e->daux.atom.p;
       P.sph = e->dobs.sph.p;
-      P.boys = e->boys.p;
+      P.boysp = e->boysp.p;
       P.naux = e->aux.n_final;
       P.W2 = W2;
       P.grad = g2e;
-      launch_grad2(lp, lq, P, s);
+      launch_grad2(gP, gQ, P, cs.next((double)P.P.count * P.Q.count));
     }
+  cs.join();
 }
-
 
 // dC: n x nocc column-major occupied orbitals; dD = 2 C C^T; g2e receives
 // the two-electron DF gradient (zeroed here).  Synchronises the stream.
@@ -148,19 +147,19 @@ int grad_df_2e_device(jk_engine* e, const double* dC, int nocc, const double* dD
   DFState& d = e->df;
   if (e->tiled.metric_ready || (!d.ready && df_use_tiled(e))) return grad_df_2e_tiled(e, dC, nocc, dD, g2e, s);
   const int n = e->obs.n_final, naux = d.naux, o = nocc, na = e->natom;
-  const size_t nn = (size_t)n * n;
   for (int k = 0; k < e->aux.nshell; ++k)
     if (e->aux.atom[k] < 0 || e->aux.atom[k] >= na)
       return set_error(e, JK_ERR_ARG, "DF gradient: every fitting shell needs an owning atom (jk_basis.atom)");
-  DevBuf<double> X, bt, c, W2, Z, K2a, K2b, ap2;
-  cudaError_t st = X.alloc((size_t)n * naux * o);
+  const int nc = e->obs.n_cart;
+  const size_t ncc = (size_t)nc * nc;
+  DevBuf<double> X, bt, c, W2, Z, Cc, Dc;
+  cudaError_t st = X.alloc((size_t)nc * naux * o);
   if (st == cudaSuccess) st = bt.alloc((size_t)o * o * naux);
   if (st == cudaSuccess) st = c.alloc(naux);
   if (st == cudaSuccess) st = W2.alloc((size_t)naux * naux);
-  if (st == cudaSuccess) st = Z.alloc(nn * naux);
-  if (st == cudaSuccess) st = K2a.alloc(e->pp_p.n);
-  if (st == cudaSuccess) st = K2b.alloc(e->pp_p.n);
-  if (st == cudaSuccess) st = ap2.alloc(e->ap_p.n);
+  if (st == cudaSuccess) st = Z.alloc(ncc * naux);
+  if (st == cudaSuccess) st = Cc.alloc((size_t)nc * o);
+  if (st == cudaSuccess) st = Dc.alloc(ncc);
   if (st != cudaSuccess) return check_cuda(e, st, "DF gradient allocation");
   if (!d.Linv.p) return set_error(e, JK_ERR_STATE, "DF gradient: L^-1 missing (run jk_df_setup)");
   DevBuf<double> dd, gt;
@@ -225,31 +224,33 @@ int grad_df_2e_device(jk_engine* e, const double* dC, int nocc, const double* dD
     r.alpha = -0.5; r.beta = 1.0;
     if ((rc = gemm(r, "DF gradient: W2"))) return rc;
   }
-  // Y[P] = C d^P (n x o, reusing X), Z[P] = Y[P] C^T (n x n)
+  // W3 over Cartesian orbital functions: Y[P] = Cc d^P (nc x o, reusing X), Z[P] = Y[P] Cc^T
+  launch_cart_rows(e, o, dC, Cc.p, s);
+  launch_final_to_cart(e, dD, Dc.p, s);
   {
     DGemm g;
-    g.M = n; g.N = o; g.K = o; g.batch = naux;
-    g.A = dC; g.sam = 1; g.sak = n;
+    g.M = nc; g.N = o; g.K = o; g.batch = naux;
+    g.A = Cc.p; g.sam = 1; g.sak = nc;
     g.B = dd.p; g.sbk = 1; g.sbn = o; g.bsb = (long long)o * o;
-    g.C = X.p; g.scm = 1; g.scn = n; g.bsc = (long long)n * o;
+    g.C = X.p; g.scm = 1; g.scn = nc; g.bsc = (long long)nc * o;
     if ((rc = gemm(g, "DF gradient: Y = C d"))) return rc;
     DGemm z;
-    z.M = n; z.N = n; z.K = o; z.batch = naux;
-    z.A = X.p; z.sam = 1; z.sak = n; z.bsa = (long long)n * o;
-    z.B = dC; z.sbk = n; z.sbn = 1;
-    z.C = Z.p; z.scm = 1; z.scn = n; z.bsc = (long long)nn;
+    z.M = nc; z.N = nc; z.K = o; z.batch = naux;
+    z.A = X.p; z.sam = 1; z.sak = nc; z.bsa = (long long)nc * o;
+    z.B = Cc.p; z.sbk = nc; z.sbn = 1;
+    z.C = Z.p; z.scm = 1; z.scn = nc; z.bsc = (long long)ncc;
     if ((rc = gemm(z, "DF gradient: Z = Y C^T"))) return rc;
   }
-  k_w3<<<(unsigned)((nn * naux + 255) / 256), 256, 0, s>>>(nn, naux, c.p, dD, Z.p);
-  // primitive weights of the shifted classes
-  launch_scale_K((int)e->pp_p.n, e->pp_K.p, e->pp_p.p, e->pp_a.p, K2a.p, K2b.p, s);
-  k_scale_aux<<<(unsigned)((e->ap_p.n + 255) / 256), 256, 0, s>>>((int)e->ap_p.n, e->ap_K.p, e->ap_p.p, ap2.p);
+  k_w3<<<(unsigned)((ncc * naux + 255) / 256), 256, 0, s>>>(ncc, naux, c.p, Dc.p, Z.p);
   cudaMemsetAsync(g2e, 0, sizeof(double) * 3 * na, s);
   // three-index derivatives
-  for (int l = 0; l <= MAX_L_AUX; ++l)
-    if (e->aux_by_l_count[l]) launch_grad3_all(e, l, e->aux_by_l[l].p, e->aux_by_l_count[l], Z.p, 0, K2a.p, K2b.p, g2e, s);
+  {
+    const int* shells[jk_engine::NAUXGROUP];
+    for (int g = 0; g < jk_engine::NAUXGROUP; ++g) shells[g] = e->aux_group[g].p;
+    launch_grad3_all(e, shells, e->aux_group_count, Z.p, 0, g2e, s);
+  }
   // metric derivatives
-  launch_grad2_all(e, ap2.p, W2.p, g2e, s);
+  launch_grad2_all(e, W2.p, g2e, s);
   st = cudaGetLastError();
   if (st == cudaSuccess) st = cudaStreamSynchronize(s);  // scratch dies on return
   return check_cuda(e, st, "DF gradient kernels");
@@ -328,11 +329,12 @@ int grad_df_2e_tiled(jk_engine* e, const double* dC, int nocc, const double* dD,
   DFState& d = e->df;
   TiledDF& T = e->tiled;
   const int n = e->obs.n_final, naux = e->aux.n_final, o = nocc, na = e->natom, npad = T.npad;
-  const size_t nn = (size_t)n * n, oo = (size_t)o * o;
+  const int nc = e->obs.n_cart;
+  const size_t ncc = (size_t)nc * nc, oo = (size_t)o * o;
   for (int k = 0; k < e->aux.nshell; ++k)
     if (e->aux.atom[k] < 0 || e->aux.atom[k] >= na)
       return set_error(e, JK_ERR_ARG, "DF gradient: every fitting shell needs an owning atom (jk_basis.atom)");
-  DevBuf<double> btp, bt, dd, gt, c, W2, Cp, Tt, K2a, K2b, ap2;
+  DevBuf<double> btp, bt, dd, gt, c, W2, Cp, Tt, Cc, Dc;
   cudaError_t st = btp.alloc(oo * naux);
   if (st == cudaSuccess) st = dd.alloc(oo * naux);
   if (st == cudaSuccess) st = gt.alloc(naux);
@@ -340,9 +342,8 @@ int grad_df_2e_tiled(jk_engine* e, const double* dC, int nocc, const double* dD,
   if (st == cudaSuccess) st = W2.alloc((size_t)naux * naux);
   if (st == cudaSuccess) st = Cp.alloc((size_t)npad * o);
   if (st == cudaSuccess) st = Tt.alloc((size_t)DF_TILE * naux * DF_TILE);
-  if (st == cudaSuccess) st = K2a.alloc(e->pp_p.n);
-  if (st == cudaSuccess) st = K2b.alloc(e->pp_p.n);
-  if (st == cudaSuccess) st = ap2.alloc(e->ap_p.n);
+  if (st == cudaSuccess) st = Cc.alloc((size_t)nc * o);
+  if (st == cudaSuccess) st = Dc.alloc(ncc);
   if (st != cudaSuccess) return check_cuda(e, st, "tiled DF gradient allocation");
   auto gemm = [&](const DGemm& g, const char* what) {
     const cudaError_t r = dgemm(g, s);
@@ -411,52 +412,54 @@ int grad_df_2e_tiled(jk_engine* e, const double* dC, int nocc, const double* dD,
     r.alpha = -0.5; r.beta = 1.0;
     if ((rc = gemm(r, "tiled DF gradient: W2"))) return rc;
   }
-  launch_scale_K((int)e->pp_p.n, e->pp_K.p, e->pp_p.p, e->pp_a.p, K2a.p, K2b.p, s);
-  k_scale_aux<<<(unsigned)((e->ap_p.n + 255) / 256), 256, 0, s>>>((int)e->ap_p.n, e->ap_K.p, e->ap_p.p, ap2.p);
+  launch_cart_rows(e, o, dC, Cc.p, s);
+  launch_final_to_cart(e, dD, Dc.p, s);
   cudaMemsetAsync(g2e, 0, sizeof(double) * 3 * na, s);
   // W3 = c_P D - 2 C d^P C^T and its contraction, one block of fitting shells at a time
   {
     size_t fr = 0, tot = 0;
     cudaMemGetInfo(&fr, &tot);
-    const double per_f = 8.0 * ((double)nn + (double)n * o);
+    const double per_f = 8.0 * ((double)ncc + (double)nc * o);
     const int wmax = (int)std::max(16.0, std::min<double>(naux, 0.6 * (double)fr / per_f));
     DevBuf<double> Y, Z;
-    if ((st = Y.alloc((size_t)n * o * wmax)) == cudaSuccess) st = Z.alloc(nn * wmax);
+    if ((st = Y.alloc((size_t)nc * o * wmax)) == cudaSuccess) st = Z.alloc(ncc * wmax);
     if (st != cudaSuccess) return check_cuda(e, st, "tiled DF gradient W3 block");
     const HostBasis& ab = e->aux;
-    DevBuf<int> lists[MAX_L_AUX + 1];
+    DevBuf<int> lists[jk_engine::NAUXGROUP];
     for (int s0 = 0; s0 < ab.nshell;) {
       int s1 = s0;
       while (s1 < ab.nshell && ab.off_final[s1 + 1] - ab.off_final[s0] <= wmax) ++s1;
       if (s1 == s0) return set_error(e, JK_ERR_ARG, "tiled DF gradient: fitting shell wider than the block");
       const int f0 = ab.off_final[s0], w = ab.off_final[s1] - f0;
-      DGemm y;  // Y[P] = C d^P (n x o)
-      y.M = n; y.N = o; y.K = o; y.batch = w;
-      y.A = dC; y.sam = 1; y.sak = n;
+      DGemm y;  // Y[P] = Cc d^P (nc x o)
+      y.M = nc; y.N = o; y.K = o; y.batch = w;
+      y.A = Cc.p; y.sam = 1; y.sak = nc;
       y.B = dd.p + (size_t)f0 * oo; y.sbk = 1; y.sbn = o; y.bsb = (long long)oo;
-      y.C = Y.p; y.scm = 1; y.scn = n; y.bsc = (long long)n * o;
+      y.C = Y.p; y.scm = 1; y.scn = nc; y.bsc = (long long)nc * o;
       if ((rc = gemm(y, "tiled DF gradient: Y = C d"))) return rc;
-      DGemm z;  // Z[P] = Y[P] C^T (n x n)
-      z.M = n; z.N = n; z.K = o; z.batch = w;
-      z.A = Y.p; z.sam = 1; z.sak = n; z.bsa = (long long)n * o;
-      z.B = dC; z.sbk = n; z.sbn = 1;
-      z.C = Z.p; z.scm = 1; z.scn = n; z.bsc = (long long)nn;
+      DGemm z;  // Z[P] = Y[P] Cc^T (nc x nc)
+      z.M = nc; z.N = nc; z.K = o; z.batch = w;
+      z.A = Y.p; z.sam = 1; z.sak = nc; z.bsa = (long long)nc * o;
+      z.B = Cc.p; z.sbk = nc; z.sbn = 1;
+      z.C = Z.p; z.scm = 1; z.scn = nc; z.bsc = (long long)ncc;
       if ((rc = gemm(z, "tiled DF gradient: Z = Y C^T"))) return rc;
-      k_w3<<<(unsigned)((nn * w + 255) / 256), 256, 0, s>>>(nn, w, c.p + f0, dD, Z.p);
-      for (int l = 0; l <= MAX_L_AUX; ++l) {
-        std::vector<int> sh;
-        for (int k = s0; k < s1; ++k)
-          if (ab.l[k] == l) sh.push_back(k);
-        if (sh.empty()) continue;
-        if ((st = lists[l].upload(sh, s)) != cudaSuccess) return check_cuda(e, st, "tiled DF gradient shells");
-        launch_grad3_all(e, l, lists[l].p, (int)sh.size(), Z.p, f0, K2a.p, K2b.p, g2e, s);
+      k_w3<<<(unsigned)((ncc * w + 255) / 256), 256, 0, s>>>(ncc, w, c.p + f0, Dc.p, Z.p);
+      std::vector<int> sh[jk_engine::NAUXGROUP];
+      for (int k = s0; k < s1; ++k) sh[aux_group_of(ab.l[k], ab.pure[k])].push_back(k);
+      const int* shells[jk_engine::NAUXGROUP];
+      int counts[jk_engine::NAUXGROUP];
+      for (int g = 0; g < jk_engine::NAUXGROUP; ++g) {
+        if ((st = lists[g].upload(sh[g], s)) != cudaSuccess) return check_cuda(e, st, "tiled DF gradient shells");
+        shells[g] = lists[g].p;
+        counts[g] = (int)sh[g].size();
       }
+      launch_grad3_all(e, shells, counts, Z.p, f0, g2e, s);
       st = cudaStreamSynchronize(s);  // Y, Z and the shell lists are reused by the next block
       if (st != cudaSuccess) return check_cuda(e, st, "tiled DF gradient block");
       s0 = s1;
     }
   }
-  launch_grad2_all(e, ap2.p, W2.p, g2e, s);
+  launch_grad2_all(e, W2.p, g2e, s);
   st = cudaGetLastError();
   if (st == cudaSuccess) st = cudaStreamSynchronize(s);
   return check_cuda(e, st, "tiled DF gradient kernels");

@@ -1,26 +1,31 @@
-// Kernel instantiations of the density-fitted gradient, two-index (metric)
-// derivatives for every ordered pair of fitting angular momenta.
+// Two-index (metric) derivatives of the density-fitted gradient for every
+// ordered pair of fitting groups (s, p, pure d, Cartesian d, pure f, Cartesian f).
 #include "df_grad_kernels.cuh"
 
 namespace m2 {
-void launch_grad2(int LP, int LQ, const Grad2Params& P, cudaStream_t s) {
-  dim3 grid((P.nq + 63) / 64, P.np);
-  if (LP == 0 && LQ == 0) k_grad2<0, 0><<<grid, 64, 0, s>>>(P);
-  if (LP == 0 && LQ == 1) k_grad2<0, 1><<<grid, 64, 0, s>>>(P);
-  if (LP == 0 && LQ == 2) k_grad2<0, 2><<<grid, 64, 0, s>>>(P);
-  if (LP == 0 && LQ == 3) k_grad2<0, 3><<<grid, 64, 0, s>>>(P);
-  if (LP == 1 && LQ == 0) k_grad2<1, 0><<<grid, 64, 0, s>>>(P);
-  if (LP == 1 && LQ == 1) k_grad2<1, 1><<<grid, 64, 0, s>>>(P);
-  if (LP == 1 && LQ == 2) k_grad2<1, 2><<<grid, 64, 0, s>>>(P);
-  if (LP == 1 && LQ == 3) k_grad2<1, 3><<<grid, 64, 0, s>>>(P);
-  if (LP == 2 && LQ == 0) k_grad2<2, 0><<<grid, 64, 0, s>>>(P);
-  if (LP == 2 && LQ == 1) k_grad2<2, 1><<<grid, 64, 0, s>>>(P);
-  if (LP == 2 && LQ == 2) k_grad2<2, 2><<<grid, 64, 0, s>>>(P);
-  if (LP == 2 && LQ == 3) k_grad2<2, 3><<<grid, 64, 0, s>>>(P);
-  if (LP == 3 && LQ == 0) k_grad2<3, 0><<<grid, 64, 0, s>>>(P);
-  if (LP == 3 && LQ == 1) k_grad2<3, 1><<<grid, 64, 0, s>>>(P);
-  if (LP == 3 && LQ == 2) k_grad2<3, 2><<<grid, 64, 0, s>>>(P);
-  if (LP == 3 && LQ == 3) k_grad2<3, 3><<<grid, 64, 0, s>>>(P);
+
+template <int LP, bool PP, int LQ, bool PQ>
+static void go(const Grad2Params& P, cudaStream_t s) {
+  const int chunks = (P.Q.count + G2_THREADS - 1) / G2_THREADS;
+  k_grad2<LP, PP, LQ, PQ><<<dim3(P.P.count, chunks), G2_THREADS, 0, s>>>(P);
+}
+template <int LP, bool PP>
+static void go_q(int gQ, const Grad2Params& P, cudaStream_t s) {
+  if (gQ == 0) go<LP, PP, 0, true>(P, s);
+  if (gQ == 1) go<LP, PP, 1, true>(P, s);
+  if (gQ == 2) go<LP, PP, 2, true>(P, s);
+  if (gQ == 3) go<LP, PP, 2, false>(P, s);
+  if (gQ == 4) go<LP, PP, 3, true>(P, s);
+  if (gQ == 5) go<LP, PP, 3, false>(P, s);
+}
+
+void launch_grad2(int gP, int gQ, const Grad2Params& P, cudaStream_t s) {
+  if (gP == 0) go_q<0, true>(gQ, P, s);
+  if (gP == 1) go_q<1, true>(gQ, P, s);
+  if (gP == 2) go_q<2, true>(gQ, P, s);
+  if (gP == 3) go_q<2, false>(gQ, P, s);
+  if (gP == 4) go_q<3, true>(gQ, P, s);
+  if (gP == 5) go_q<3, false>(gQ, P, s);
 }
 
 }  // namespace m2

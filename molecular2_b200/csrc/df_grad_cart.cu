@@ -1,0 +1,11 @@
+// Three-index derivative kernels of the density-fitted gradient for Cartesian d and f
+// fitting shells.  Split across translation units only so that nvcc compiles
+// them in parallel.
+#include "df_grad_kernels.cuh"
+
+namespace m2 {
+
+void launch_grad3_d_cart(int pc, const Grad3Params& P, cudaStream_t s) { launch_grad3_l<2, false>(pc, P, s); }
+void launch_grad3_f_cart(int pc, const Grad3Params& P, cudaStream_t s) { launch_grad3_l<3, false>(pc, P, s); }
+
+}  // namespace m2

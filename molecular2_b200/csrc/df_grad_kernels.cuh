@@ -9,231 +9,330 @@
 //   dE2 = sum_{P,mn} (mn|P)^x W3_{mn,P} + sum_{PQ} (P|Q)^x W2_{PQ},
 //   W3_{mn,P} = c_P D_mn - 2 sum_ij C_mi C_nj d^P_ij,
 //   W2_{PQ}   = -1/2 c_P c_Q + sum_ij d^P_ij d^Q_ij.
-// Derivatives of the orbital centres are taken as in grad_kernels.cuh (shifted
-// classes weighted by 2 alpha); the fitting centre of (mn|P) follows from
-// translational invariance, and for (P|Q) d/dQ = -d/dP.
+// The orbital centres' derivatives come from one Hermite table per primitive
+// quartet as in grad_kernels.cuh; with the fitting function as the bra, d/dP is
+// its shift and d/dn = -d/dP - d/dm.  For (P|Q) d/dQ = -d/dP.
 #pragma once
 #include "df_kernels.cuh"
 #include "grad_kernels.cuh"
 
 namespace m2 {
 
-// Adjoint of sph_index: index k of a 3-index block goes from the final (pure)
-// functions of shell l back to its Cartesian components.
-__device__ __forceinline__ void sph_index_adj(const double* in, double* out, int k, const int* n, int l,
-                                              const double* sph) {
-  const int nf = 2 * l + 1, ncl = ncart(l);
-  int pre = 1, post = 1;
-  for (int j = 0; j < k; ++j) pre *= n[j];
-  for (int j = k + 1; j < 3; ++j) post *= n[j];
-  const double* T = sph + sph_off(l);
-  for (int a = 0; a < pre; ++a)
-    for (int i = 0; i < ncl; ++i)
-      for (int c = 0; c < post; ++c) {
-        double v = 0.0;
-        for (int m = 0; m < nf; ++m) v += T[m * ncl + i] * in[(a * nf + m) * post + c];
-        out[(a * ncl + i) * post + c] = v;
-      }
-}
-
-// quartet_cart kept out of line for the derivative classes: inlined into
-// k_grad3, the CUDA 12.9 build (with ptxas -O3 and with -O0 alike) gave wrong
-// contributions for the fitting classes d and f with p-p orbital pairs, while
-// a host build of the same source and this out-of-line form both agree with
-// finite differences of the integrals.
-template <int LA, int LB, int LC, int LD>
-__device__ __noinline__ void quartet_cart_ool(const PrimView& pp, int b0, int nb, double Ax, double Ay, double Az,
-                                              double Bx, double By, double Bz, const PrimView& kp, int k0, int nk,
-                                              double Cx, double Cy, double Cz, double Dx, double Dy, double Dz,
-                                              const double* __restrict__ boys_tab, double* out) {
-  quartet_cart<LA, LB, LC, LD>(pp, b0, nb, Ax, Ay, Az, Bx, By, Bz, kp, k0, nk, Cx, Cy, Cz, Dx, Dy, Dz, boys_tab, out);
-}
-
 struct Grad3Params {
-  PrimView ap;            // fitting primitives as (P, unit) pairs
-  const int* aux_shells;  // fitting shells of this angular momentum
-  int naux_shells;
-  const int* aux_prim_off;
-  const int* aux_nprim;
-  const double *ax, *ay, *az;
-  const int* aux_foff;
-  const int* aux_pure;
+  AuxView aux;            // fitting shells of one group
   const int* aux_atom;
-  PairView pairs;         // orbital pairs of one class
-  PrimView pp, pp2a, pp2b;
+  const int* atom;        // orbital shell -> atom
+  EntryView ent;          // orbital pairs of one class
+  PairView pairs;
   const double *ox, *oy, *oz;
-  const int* obs_foff;
-  const int* obs_pure;
-  const int* obs_atom;
-  const double* sph_obs;
-  const double* sph_aux;
-  const double* boys;
-  int n;
-  const double* W3;       // [P - w3_f0][n][m] final basis: W3[((P - w3_f0) * n + y) * n + x]
+  const int* coff;        // Cartesian function offsets of the orbital shells
+  const double* sph;
+  const double* boysp;
+  int nc;
+  const double* W3;       // [P - w3_f0][y][x] over Cartesian orbital functions: W3[((P - w3_f0) * nc + y) * nc + x]
   int w3_f0;              // first fitting function held in W3
+  int natom;
   double* grad;           // 3 * natom
 };
 
-// One shifted class per block layer: blockIdx.z = 0, 1 (orbital centre m
-// raised, lowered), 2, 3 (n); the fitting centre's derivative is minus their
-// sum (translational invariance).  All threads of a block share the fitting
-// shell, so its atom's term is reduced over the warp first.
-template <int LP, int LM, int LN>
-__global__ void __launch_bounds__(64) k_grad3(const Grad3Params P) {
-  constexpr int NP = ncart(LP), NM = ncart(LM), NN = ncart(LN);
-  constexpr int N3 = NP * NM * NN;
-  const int sh = blockIdx.z;
-  if ((sh == 1 && LM == 0) || (sh == 3 && LN == 0)) return;
-  const int is = blockIdx.y;
-  if (is >= P.naux_shells) return;
-  const int ip = blockIdx.x * blockDim.x + threadIdx.x;
-  const int sP = P.aux_shells[is];
-  double g[3] = {0, 0, 0};
-  if (ip < P.pairs.npair) {
-    const int m = P.pairs.sa[ip], n = P.pairs.sb[ip];
-    // weights of this block, final basis -> Cartesian
-    const int pure[3] = {P.aux_pure[sP], P.obs_pure[m], P.obs_pure[n]};
-    const int ls[3] = {LP, LM, LN};
-    int dims[3] = {pure[0] ? 2 * LP + 1 : NP, pure[1] ? 2 * LM + 1 : NM, pure[2] ? 2 * LN + 1 : NN};
-    double w0[N3], w1[N3];
-    const int f0 = P.aux_foff[sP], m0 = P.obs_foff[m], n0 = P.obs_foff[n];
-    for (int a = 0; a < dims[0]; ++a)
-      for (int x = 0; x < dims[1]; ++x)
-        for (int y = 0; y < dims[2]; ++y)
-          w0[(a * dims[1] + x) * dims[2] + y] = P.W3[((size_t)(f0 - P.w3_f0 + a) * P.n + n0 + y) * P.n + m0 + x];
-    double* cur = w0;
-    double* nxt = w1;
-    for (int k = 0; k < 3; ++k)
-      if (pure[k]) {
-        sph_index_adj(cur, nxt, k, dims, ls[k], k == 0 ? P.sph_aux : P.sph_obs);
-        dims[k] = ncart(ls[k]);
-        double* sw = cur;
-        cur = nxt;
-        nxt = sw;
-      }
-    const double* Wt = cur;  // [a][x][y] Cartesian, as a (LP, 0 | LM, LN) block
-    const double Px = P.ax[sP], Py = P.ay[sP], Pz = P.az[sP];
-    const double Ax = P.ox[m], Ay = P.oy[m], Az = P.oz[m], Bx = P.ox[n], By = P.oy[n], Bz = P.oz[n];
-    const int ap0 = P.aux_prim_off[sP], anp = P.aux_nprim[sP];
-    const int kp0 = P.pairs.prim_off[ip], knp = P.pairs.nprim[ip];
-    if (sh == 0) {
-      double I[NP * ncart(LM + 1) * NN];
-      quartet_cart_ool<LP, 0, LM + 1, LN>(P.ap, ap0, anp, Px, Py, Pz, Px, Py, Pz, P.pp2a, kp0, knp, Ax, Ay, Az, Bx,
-                                          By, Bz, P.boys, I);
-      contract_shift<LP, 0, LM, LN, 2, 1>(I, Wt, g);
-    } else if (sh == 1) {
-      if constexpr (LM > 0) {
-        double I[NP * ncart(LM - 1) * NN];
-        quartet_cart_ool<LP, 0, LM - 1, LN>(P.ap, ap0, anp, Px, Py, Pz, Px, Py, Pz, P.pp, kp0, knp, Ax, Ay, Az, Bx,
-                                            By, Bz, P.boys, I);
-        contract_shift<LP, 0, LM, LN, 2, -1>(I, Wt, g);
-      }
-    } else if (sh == 2) {
-      double I[NP * NM * ncart(LN + 1)];
-      quartet_cart_ool<LP, 0, LM, LN + 1>(P.ap, ap0, anp, Px, Py, Pz, Px, Py, Pz, P.pp2b, kp0, knp, Ax, Ay, Az, Bx,
-                                          By, Bz, P.boys, I);
-      contract_shift<LP, 0, LM, LN, 3, 1>(I, Wt, g);
-    } else {
-      if constexpr (LN > 0) {
-        double I[NP * NM * ncart(LN - 1)];
-        quartet_cart_ool<LP, 0, LM, LN - 1>(P.ap, ap0, anp, Px, Py, Pz, Px, Py, Pz, P.pp, kp0, knp, Ax, Ay, Az, Bx,
-                                            By, Bz, P.boys, I);
-        contract_shift<LP, 0, LM, LN, 3, -1>(I, Wt, g);
+template <int LP>
+struct Grad3Shared {
+  double boys[BOYSP_SIZE];
+  double sphP[(2 * LP + 1) * ncart(LP)];
+  double red[GRAD_THREADS / 32][3];
+};
+
+// Block = (fitting shell, kets by blocks, ket component).  The weights of a ket
+// entry are folded into the fitting shell's Hermite expansion G, of which a
+// pure, s or p shell has only the top degree.  (H2O)8/cc-pVDZ: the whole
+// gradient call 86 -> 8.8 ms (44 ms of it four shifted evaluations a pair with
+// their integral blocks in local memory).
+template <int LP, bool PURE, int LC, int LD>
+__global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad3(const Grad3Params P) {
+  constexpr int NP = ncart(LP), NF = e3_nfun(LP, PURE), ND = ncart(LD), LCD = LC + LD, L = LP + LCD;
+  constexpr bool TOP = LP <= 1 || PURE;
+  constexpr int NG = TOP ? NP : nherm(LP);
+  extern __shared__ __align__(16) unsigned char g3_sm[];
+  Grad3Shared<LP>& S = *reinterpret_cast<Grad3Shared<LP>*>(g3_sm);
+  double* s_g = reinterpret_cast<double*>(g3_sm + ((sizeof(Grad3Shared<LP>) + 15) & ~(size_t)15));
+  const int tid = threadIdx.x, lane = tid & 31;
+  const bool local = P.natom <= GRAD_ATOMS;
+  double* g_atom = local ? s_g : P.grad;
+  for (int i = tid; i < BOYSP_SIZE; i += GRAD_THREADS) S.boys[i] = __ldg(P.boysp + (size_t)(L + 1) * BOYSP_SIZE + i);
+  if constexpr (PURE && LP > 1)
+    for (int i = tid; i < NF * NP; i += GRAD_THREADS) S.sphP[i] = P.sph[sph_off(LP) + i];
+  if (local)
+    for (int i = tid; i < 3 * P.natom; i += GRAD_THREADS) s_g[i] = 0.0;
+  __syncthreads();
+  const int sh = P.aux.shells[blockIdx.x];
+  const int j0 = P.aux.prim_off[sh], nj = P.aux.nprim[sh];
+  const double* W3 = P.W3 + (size_t)(P.aux.foff[sh] - P.w3_f0) * P.nc * P.nc;
+  const int ic = blockIdx.z / ND, id = blockIdx.z % ND;
+  int ce[3], de[3];
+  ce[0] = LC > 0 ? c_herm.t[nherm(LC - 1) + ic] : 0;
+  ce[1] = LC > 0 ? c_herm.u[nherm(LC - 1) + ic] : 0;
+  ce[2] = LC > 0 ? c_herm.v[nherm(LC - 1) + ic] : 0;
+  de[0] = LD > 0 ? c_herm.t[nherm(LD - 1) + id] : 0;
+  de[1] = LD > 0 ? c_herm.u[nherm(LD - 1) + id] : 0;
+  de[2] = LD > 0 ? c_herm.v[nherm(LD - 1) + id] : 0;
+  const int tx = ce[0] + de[0], ty = ce[1] + de[1], tz = ce[2] + de[2];
+  double sP[3] = {0, 0, 0};
+  for (int e0 = blockIdx.y * GRAD_THREADS; e0 < P.ent.nent; e0 += gridDim.y * GRAD_THREADS) {
+    const bool active = e0 + tid < P.ent.nent;
+    const int e = active ? e0 + tid : P.ent.nent - 1;
+    const int kl = P.ent.pair[e], c = P.pairs.sa[kl], d = P.pairs.sb[kl];
+    const double* kp = entry_prims(P.ent, e);
+    const int nk = P.ent.np[e];
+    const int nkm = __reduce_max_sync(0xffffffffu, nk);
+    // the sum over ordered (m, n) counts an off-diagonal canonical pair twice
+    const double deg = !active ? 0.0 : (c == d ? 1.0 : 2.0);
+    const double Cc[3] = {P.ox[c], P.oy[c], P.oz[c]}, Dd[3] = {P.ox[d], P.oy[d], P.oz[d]};
+    double w[NP];  // weights of the Cartesian fitting components
+    {
+      const double* q = W3 + (size_t)(P.coff[d] + id) * P.nc + P.coff[c] + ic;
+      double f[NF];
+#pragma unroll
+      for (int i = 0; i < NF; ++i) f[i] = deg * __ldg(q + (size_t)i * P.nc * P.nc);
+      if constexpr (PURE && LP > 1) {
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+          w[i] = 0.0;
+#pragma unroll
+          for (int m = 0; m < NF; ++m) w[i] += S.sphP[m * NP + i] * f[m];
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < NP; ++i) w[i] = f[i];
       }
     }
-    // the sum over ordered (m, n) counts an off-diagonal canonical pair twice
-    const double deg = (m == n) ? 1.0 : 2.0;
-    const int at = P.obs_atom[sh < 2 ? m : n];
+    double gP[3] = {0, 0, 0}, gC[3] = {0, 0, 0};
+    for (int j = j0; j < j0 + nj; ++j) {
+      const double p = __ldg(P.aux.p + j), Px = __ldg(P.aux.x + j), Py = __ldg(P.aux.y + j), Pz = __ldg(P.aux.z + j);
+      const double Kb = __ldg(P.aux.Kp + j), h1 = __ldg(P.aux.h + j);
+      double G[NG];
+      if constexpr (TOP) {
+        const double hl = LP == 0 ? 1.0 : (LP == 1 ? h1 : (LP == 2 ? h1 * h1 : h1 * h1 * h1));
+#pragma unroll
+        for (int i = 0; i < NP; ++i) G[i] = hl * w[i];
+      } else {
+        static_for<NG>([&](auto hh) {
+          constexpr int h = decltype(hh)::value;
+          double g = 0.0;
+          static_for<NP>([&](auto ii) {
+            constexpr int i = decltype(ii)::value;
+            g += w[i] * centred_coef(cart_a(LP, i), herm_t(h), h1) * centred_coef(cart_b(LP, i), herm_u(h), h1) *
+                 centred_coef(cart_c(LP, i), herm_v(h), h1);
+          });
+          G[h] = g;
+        });
+      }
+      for (int k = 0; k < nkm; ++k) {
+        const int kk = min(k, nk - 1);
+        const double KK = k < nk ? Kb * entry_field(kp, kk, 4) : 0.0;
+        const double q = entry_field(kp, kk, 0);
+        const double Q[3] = {entry_field(kp, kk, 1), entry_field(kp, kk, 2), entry_field(kp, kk, 3)};
+        const double h2 = entry_field(kp, kk, 5), ga = entry_field(kp, kk, 6);
+        double R[nherm(L + 1)];
+        quartet_R<L + 1>(p, q, KK, Px - Q[0], Py - Q[1], Pz - Q[2], S.boys, R);
+        double ex[3][LCD + 1], er[3][LCD + 1];
+        ket_expansions<LC, LD>(ex, er, Q, Cc, Dd, ga, h2, ce, de);
+        double gp[3] = {0, 0, 0};
+        ket_gradient<LP, LCD, TOP ? LP : 0>(G, R, ex, er, tx, ty, tz, gp, gC);
+        const double fc = 2.0 * h2 * ga;
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+          gP[x] += gp[x];
+          gC[x] -= fc * gp[x];
+        }
+      }
+    }
+    const int atc = 3 * P.atom[c], atd = 3 * P.atom[d];
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
-      g[x] *= deg;
-      if (g[x] != 0.0) atomicAdd(P.grad + 3 * at + x, g[x]);
+      sP[x] += gP[x];
+      if (active) {
+        atomicAdd(g_atom + atc + x, gC[x]);
+        atomicAdd(g_atom + atd + x, -gP[x] - gC[x]);
+      }
     }
   }
-  // the fitting centre: minus the orbital centres' terms, one atomic per warp
-  const int aP = P.aux_atom[sP];
+  // the fitting centre: one sum per block
 #pragma unroll
   for (int x = 0; x < 3; ++x) {
-    double v = g[x];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(P.grad + 3 * aP + x, -v);
+    for (int o = 16; o > 0; o >>= 1) sP[x] += __shfl_down_sync(0xffffffffu, sP[x], o);
+    if (lane == 0) S.red[tid >> 5][x] = sP[x];
   }
+  __syncthreads();
+  if (tid < 3) {
+    double v = 0.0;
+    for (int k = 0; k < GRAD_THREADS / 32; ++k) v += S.red[k][tid];
+    atomicAdd(P.grad + 3 * P.aux_atom[sh] + tid, v);
+  }
+  if (local)
+    for (int i = tid; i < 3 * P.natom; i += GRAD_THREADS)
+      if (s_g[i] != 0.0) atomicAdd(P.grad + i, s_g[i]);
+}
+
+template <int LP, bool PURE, int LC, int LD>
+inline void launch_grad3_class(const Grad3Params& P, cudaStream_t s) {
+  const size_t sm = sizeof(Grad3Shared<LP>) + 16 + (P.natom <= GRAD_ATOMS ? 24 * (size_t)P.natom : 0);
+  cudaFuncSetAttribute(k_grad3<LP, PURE, LC, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  const int layers = ncart(LC) * ncart(LD), chunks = (P.ent.nent + GRAD_THREADS - 1) / GRAD_THREADS;
+  // blocks walk over several ket chunks where there are enough of them to fill the GPU
+  int y = 1;
+  while (y < chunks && (long long)P.aux.count * layers * y < 16 * 148) ++y;
+  k_grad3<LP, PURE, LC, LD><<<dim3(P.aux.count, y, layers), GRAD_THREADS, sm, s>>>(P);
+}
+template <int LP, bool PURE>
+inline void launch_grad3_l(int pc, const Grad3Params& P, cudaStream_t s) {
+  if (pc == 0) launch_grad3_class<LP, PURE, 0, 0>(P, s);
+  if (pc == 1) launch_grad3_class<LP, PURE, 1, 0>(P, s);
+  if (pc == 2) launch_grad3_class<LP, PURE, 1, 1>(P, s);
+  if (pc == 3) launch_grad3_class<LP, PURE, 2, 0>(P, s);
+  if (pc == 4) launch_grad3_class<LP, PURE, 2, 1>(P, s);
+  if (pc == 5) launch_grad3_class<LP, PURE, 2, 2>(P, s);
 }
 
 struct Grad2Params {
-  PrimView ap, ap2;       // fitting primitives; ap2 has K * 2 alpha
-  const int* shells_p;
-  int np;
-  const int* shells_q;
-  int nq;
-  const int* aux_prim_off;
-  const int* aux_nprim;
-  const double *ax, *ay, *az;
-  const int* aux_foff;
-  const int* aux_pure;
+  AuxView P, Q;           // two groups of fitting shells
   const int* aux_atom;
   const double* sph;
-  const double* boys;
+  const double* boysp;
   int naux;
   const double* W2;       // naux x naux, symmetric
   double* grad;
 };
 
-// one thread per ordered pair (P, Q) of fitting shells: W2 . d/dP (P|Q)
-// goes to P's atom and its negative to Q's atom
-template <int LP, int LQ>
-__global__ void __launch_bounds__(64) k_grad2(const Grad2Params P) {
-  constexpr int NP = ncart(LP), NQ = ncart(LQ);
-  const int iq = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ip = blockIdx.y;
-  if (iq >= P.nq || ip >= P.np) return;
-  const int sP = P.shells_p[ip], sQ = P.shells_q[iq];
-  const int aP = P.aux_atom[sP], aQ = P.aux_atom[sQ];
-  if (aP == aQ) return;  // one-centre: d/dP + d/dQ = 0 on the same atom
-  const int pure[3] = {P.aux_pure[sP], P.aux_pure[sQ], 0};
-  const int ls[3] = {LP, LQ, 0};
-  int dims[3] = {pure[0] ? 2 * LP + 1 : NP, pure[1] ? 2 * LQ + 1 : NQ, 1};
-  double w0[NP * NQ], w1[NP * NQ];
-  const int p0 = P.aux_foff[sP], q0 = P.aux_foff[sQ];
-  for (int a = 0; a < dims[0]; ++a)
-    for (int b = 0; b < dims[1]; ++b) w0[a * dims[1] + b] = P.W2[(size_t)(q0 + b) * P.naux + p0 + a];
-  double* cur = w0;
-  double* nxt = w1;
-  for (int k = 0; k < 2; ++k)
-    if (pure[k]) {
-      sph_index_adj(cur, nxt, k, dims, ls[k], P.sph);
-      dims[k] = ncart(ls[k]);
-      double* sw = cur;
-      cur = nxt;
-      nxt = sw;
-    }
-  const double Ax = P.ax[sP], Ay = P.ay[sP], Az = P.az[sP];
-  const double Cx = P.ax[sQ], Cy = P.ay[sQ], Cz = P.az[sQ];
-  double g[3] = {0, 0, 0};
-  {
-    double I[ncart(LP + 1) * NQ];
-    quartet_cart<LP + 1, 0, LQ, 0>(P.ap2, P.aux_prim_off[sP], P.aux_nprim[sP], Ax, Ay, Az, Ax, Ay, Az, P.ap,
-                                   P.aux_prim_off[sQ], P.aux_nprim[sQ], Cx, Cy, Cz, Cx, Cy, Cz, P.boys, I);
-    contract_shift<LP, 0, LQ, 0, 0, 1>(I, cur, g);
-  }
-  if constexpr (LP > 0) {
-    double I[ncart(LP - 1) * NQ];
-    quartet_cart<LP - 1, 0, LQ, 0>(P.ap, P.aux_prim_off[sP], P.aux_nprim[sP], Ax, Ay, Az, Ax, Ay, Az, P.ap,
-                                   P.aux_prim_off[sQ], P.aux_nprim[sQ], Cx, Cy, Cz, Cx, Cy, Cz, P.boys, I);
-    contract_shift<LP, 0, LQ, 0, 0, -1>(I, cur, g);
-  }
+// Hermite coefficients of one fitting shell's functions from weights of its
+// final functions: the top degree only (TOP), or all degrees.
+template <int LP, bool PURE>
+__device__ __forceinline__ void aux_cart_weights(const double* f, const double* sph, double* w) {
+  constexpr int NP = ncart(LP), NF = e3_nfun(LP, PURE);
 #pragma unroll
-  for (int x = 0; x < 3; ++x) {
-    atomicAdd(P.grad + 3 * aP + x, g[x]);
-    atomicAdd(P.grad + 3 * aQ + x, -g[x]);
+  for (int i = 0; i < NP; ++i) {
+    if constexpr (PURE && LP > 1) {
+      w[i] = 0.0;
+#pragma unroll
+      for (int m = 0; m < NF; ++m) w[i] += sph[m * NP + i] * f[m];
+    } else {
+      w[i] = f[i];
+    }
   }
 }
 
-// launchers (df_grad_l*.cu, df_grad2.cu)
-void launch_grad3_l0(int pair_class_id, const Grad3Params& P, cudaStream_t s);
-void launch_grad3_l1(int pair_class_id, const Grad3Params& P, cudaStream_t s);
-void launch_grad3_l2(int pair_class_id, const Grad3Params& P, cudaStream_t s);
-void launch_grad3_l3(int pair_class_id, const Grad3Params& P, cudaStream_t s);
-void launch_grad2(int LP, int LQ, const Grad2Params& P, cudaStream_t s);
+// W2 . d/dP (P|Q) over the pairs of two groups: block = shell P, lanes = shells
+// Q; it goes to P's atom and its negative to Q's atom.
+constexpr int G2_THREADS = 64;
+template <int LP, bool PP, int LQ, bool PQ>
+__global__ void __launch_bounds__(G2_THREADS) k_grad2(const Grad2Params P) {
+  constexpr int NP = ncart(LP), NQ = ncart(LQ), FP = e3_nfun(LP, PP), FQ = e3_nfun(LQ, PQ), L = LP + LQ + 1;
+  constexpr bool TOP = (LP <= 1 || PP) && (LQ <= 1 || PQ);
+  __shared__ double boys[BOYSP_SIZE];
+  __shared__ double sphP[FP * NP], sphQ[FQ * NQ];
+  const int tid = threadIdx.x, lane = tid & 31;
+  for (int i = tid; i < BOYSP_SIZE; i += G2_THREADS) boys[i] = __ldg(P.boysp + (size_t)L * BOYSP_SIZE + i);
+  if (PP && LP > 1)
+    for (int i = tid; i < FP * NP; i += G2_THREADS) sphP[i] = P.sph[sph_off(LP) + i];
+  if (PQ && LQ > 1)
+    for (int i = tid; i < FQ * NQ; i += G2_THREADS) sphQ[i] = P.sph[sph_off(LQ) + i];
+  __syncthreads();
+  const int sP = P.P.shells[blockIdx.x], aP = P.aux_atom[sP];
+  const int p0 = P.P.foff[sP];
+  double tot[3] = {0, 0, 0};
+  for (int s = blockIdx.y * G2_THREADS + tid; s < P.Q.count; s += gridDim.y * G2_THREADS) {
+    const int sQ = P.Q.shells[s], aQ = P.aux_atom[sQ];
+    if (aP == aQ) continue;  // one-centre: d/dP + d/dQ = 0 on the same atom
+    const int q0 = P.Q.foff[sQ];
+    double w[NQ][NP];  // [Cartesian Q][Cartesian P]
+    {
+      double t[FQ][NP];
+#pragma unroll
+      for (int b = 0; b < FQ; ++b) {
+        double f[FP];
+#pragma unroll
+        for (int a = 0; a < FP; ++a) f[a] = P.W2[(size_t)(q0 + b) * P.naux + p0 + a];
+        aux_cart_weights<LP, PP>(f, sphP, t[b]);
+      }
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        double f[FQ], o[NQ];
+#pragma unroll
+        for (int b = 0; b < FQ; ++b) f[b] = t[b][i];
+        aux_cart_weights<LQ, PQ>(f, sphQ, o);
+#pragma unroll
+        for (int b = 0; b < NQ; ++b) w[b][i] = o[b];
+      }
+    }
+    double g[3] = {0, 0, 0};
+    for (int j = P.P.prim_off[sP]; j < P.P.prim_off[sP] + P.P.nprim[sP]; ++j)
+      for (int k = P.Q.prim_off[sQ]; k < P.Q.prim_off[sQ] + P.Q.nprim[sQ]; ++k) {
+        const double hp = __ldg(P.P.h + j), hq = -__ldg(P.Q.h + k);
+        double R[nherm(L)];
+        quartet_R<L>(__ldg(P.P.p + j), __ldg(P.Q.p + k), __ldg(P.P.Kp + j) * __ldg(P.Q.Kp + k),
+                     __ldg(P.P.x + j) - __ldg(P.Q.x + k), __ldg(P.P.y + j) - __ldg(P.Q.y + k),
+                     __ldg(P.P.z + j) - __ldg(P.Q.z + k), boys, R);
+        if constexpr (TOP) {
+          double hl = 1.0;
+#pragma unroll
+          for (int i = 0; i < LP; ++i) hl *= hp;
+#pragma unroll
+          for (int i = 0; i < LQ; ++i) hl *= hq;
+          double v[3] = {0, 0, 0};
+          static_for<NP * NQ>([&](auto ab) {
+            constexpr int i = decltype(ab)::value % NP, b = decltype(ab)::value / NP;
+            constexpr int t = cart_a(LP, i) + cart_a(LQ, b), u = cart_b(LP, i) + cart_b(LQ, b),
+                          z = cart_c(LP, i) + cart_c(LQ, b);
+            v[0] += w[b][i] * R[hidx(t + 1, u, z)];
+            v[1] += w[b][i] * R[hidx(t, u + 1, z)];
+            v[2] += w[b][i] * R[hidx(t, u, z + 1)];
+          });
+#pragma unroll
+          for (int x = 0; x < 3; ++x) g[x] += hl * v[x];
+        } else {  // every degree of a Cartesian d or f shell; the sign of Q's odd degrees is in -h
+          for (int i = 0; i < NP; ++i)
+            for (int b = 0; b < NQ; ++b) {
+              int pe[3] = {0, 0, 0}, qe[3] = {0, 0, 0};
+              if (LP > 0) pe[0] = c_herm.t[nherm(LP - 1) + i], pe[1] = c_herm.u[nherm(LP - 1) + i], pe[2] = c_herm.v[nherm(LP - 1) + i];
+              if (LQ > 0) qe[0] = c_herm.t[nherm(LQ - 1) + b], qe[1] = c_herm.u[nherm(LQ - 1) + b], qe[2] = c_herm.v[nherm(LQ - 1) + b];
+              for (int m = 0; m < nherm(LP); ++m) {
+                const double cp = centred_coef(pe[0], c_herm.t[m], hp) * centred_coef(pe[1], c_herm.u[m], hp) *
+                                  centred_coef(pe[2], c_herm.v[m], hp) * w[b][i];
+                if (cp == 0.0) continue;
+                for (int n = 0; n < nherm(LQ); ++n) {
+                  const int t = c_herm.t[n], u = c_herm.u[n], z = c_herm.v[n];
+                  const double c0 = cp * centred_coef(qe[0], t, -hq) * centred_coef(qe[1], u, -hq) * centred_coef(qe[2], z, -hq);
+                  const double c = ((t + u + z) & 1) ? -c0 : c0;
+                  if (c == 0.0) continue;
+                  const int T = t + c_herm.t[m], U = u + c_herm.u[m], Z = z + c_herm.v[m];
+                  g[0] += c * R[hidx(T + 1, U, Z)];
+                  g[1] += c * R[hidx(T, U + 1, Z)];
+                  g[2] += c * R[hidx(T, U, Z + 1)];
+                }
+              }
+            }
+        }
+      }
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+      tot[x] += g[x];
+      atomicAdd(P.grad + 3 * aQ + x, -g[x]);
+    }
+  }
+#pragma unroll
+  for (int x = 0; x < 3; ++x) {
+    double v = tot[x];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0 && v != 0.0) atomicAdd(P.grad + 3 * aP + x, v);
+  }
+}
+
+// launchers (df_grad_*.cu): orbital pair class id; fitting groups gP, gQ
+void launch_grad3_s(int pair_class_id, const Grad3Params& P, cudaStream_t s);
+void launch_grad3_p(int pair_class_id, const Grad3Params& P, cudaStream_t s);
+void launch_grad3_d_pure(int pair_class_id, const Grad3Params& P, cudaStream_t s);
+void launch_grad3_d_cart(int pair_class_id, const Grad3Params& P, cudaStream_t s);
+void launch_grad3_f_pure(int pair_class_id, const Grad3Params& P, cudaStream_t s);
+void launch_grad3_f_cart(int pair_class_id, const Grad3Params& P, cudaStream_t s);
+void launch_grad2(int gP, int gQ, const Grad2Params& P, cudaStream_t s);
 
 }  // namespace m2

@@ -1,30 +1,13 @@
 // Device side of the density-fitting integrals: three-index (P|mn) and
-// two-index (P|Q) Coulomb integrals over the fitting basis.  McMurchie-Davidson through quartet_cart with a unit
-// s function as the partner of each fitting function (libint2 BraKet::xs_xx
+// two-index (P|Q) Coulomb integrals over the fitting basis, McMurchie-Davidson
+// with a unit s function as the partner of each fitting function (libint2 BraKet::xs_xx
 // and xs_xs in molecular2, src/eris.cpp:89-156, 304-356).
 #pragma once
 #include "jk_kernels.cuh"
 
-namespace m2 {
+struct jk_engine;
 
-// Transform index k (0..2) of a 3-index Cartesian block (dims n[0..2]) to the
-// final basis of its shell (pure block of sph when p != 0).  Rolled loops:
-// these kernels run once per geometry.
-__device__ __forceinline__ void sph_index(const double* in, double* out, int k, const int* n, int l,
-                                          const double* sph) {
-  const int nf = 2 * l + 1, ncl = ncart(l);
-  int pre = 1, post = 1;
-  for (int j = 0; j < k; ++j) pre *= n[j];
-  for (int j = k + 1; j < 3; ++j) post *= n[j];
-  const double* T = sph + sph_off(l);
-  for (int a = 0; a < pre; ++a)
-    for (int m = 0; m < nf; ++m)
-      for (int c = 0; c < post; ++c) {
-        double v = 0.0;
-        for (int i = 0; i < ncl; ++i) v += T[m * ncl + i] * in[(a * ncl + i) * post + c];
-        out[(a * nf + m) * post + c] = v;
-      }
-}
+namespace m2 {
 
 // Fitting shells of one angular momentum, all pure or all Cartesian.
 struct AuxView {
@@ -37,6 +20,8 @@ struct AuxView {
   const double* h;              // 1 / (2p)
   const int* foff;              // final function offsets
 };
+
+AuxView aux_group_view(const jk_engine* e, const int* shells, int count);  // df.cu
 
 struct Eri3Params {
   AuxView aux;
@@ -360,58 +345,109 @@ inline void launch_eri3_l(int pc, const Eri3Params& P, bool j, cudaStream_t s) {
   if (pc == 5) launch_eri3_class<2, 2, LP, PURE>(P, j, s);
 }
 
+// Group number of a fitting shell: s, p, pure d, Cartesian d, pure f, Cartesian f.
+inline int aux_group_of(int l, int pure) { return l <= 1 ? l : 2 * l - (pure ? 2 : 1); }
+
+// Coefficient of Hermite order t in x^i exp(-q x^2), h = 1/(2q), i <= 3.
+__device__ __forceinline__ double centred_coef(int i, int t, double h) {
+  if (t > i || ((i - t) & 1)) return 0.0;
+  double v = (i == 3 && t == 1) ? 3.0 * h * h : (i == 2 && t == 0) ? h : 1.0;
+  if (t == i)
+    for (int k = 0; k < i; ++k) v *= h;
+  return v;
+}
+
 struct Eri2Params {
-  PrimView ap;
-  const int* shells_p;
-  int np;
-  const int* shells_q;
-  int nq;
-  const int* aux_prim_off;
-  const int* aux_nprim;
-  const double *ax, *ay, *az;
-  const int* aux_foff;
-  const int* aux_pure;
+  AuxView P, Q;     // two groups of fitting shells
   const double* sph;
-  const double* boys;
+  const double* boysp;
   int naux;
-  double* V;  // naux x naux
+  int same;         // P and Q are one group: each unordered pair once
+  double* V;        // naux x naux
 };
 
-template <int LP, int LQ>
-__global__ void __launch_bounds__(64) k_eri2(const Eri2Params P) {
-  constexpr int NP = ncart(LP), NQ = ncart(LQ);
-  const int iq = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ip = blockIdx.y;
-  if (iq >= P.nq || ip >= P.np) return;
-  const int sP = P.shells_p[ip], sQ = P.shells_q[iq];
-  const double Ax = P.ax[sP], Ay = P.ay[sP], Az = P.az[sP];
-  const double Cx = P.ax[sQ], Cy = P.ay[sQ], Cz = P.az[sQ];
-  double c[NP * NQ], t[NP * NQ];
-  quartet_cart<LP, 0, LQ, 0>(P.ap, P.aux_prim_off[sP], P.aux_nprim[sP], Ax, Ay, Az, Ax, Ay, Az, P.ap,
-                             P.aux_prim_off[sQ], P.aux_nprim[sQ], Cx, Cy, Cz, Cx, Cy, Cz, P.boys, c);
-  int dims[3] = {NP, NQ, 1};
-  double* cur = c;
-  double* nxt = t;
-  if (P.aux_pure[sP]) {
-    sph_index(cur, nxt, 0, dims, LP, P.sph);
-    dims[0] = 2 * LP + 1;
-    double* sw = cur;
-    cur = nxt;
-    nxt = sw;
-  }
-  if (P.aux_pure[sQ]) {
-    sph_index(cur, nxt, 1, dims, LQ, P.sph);
-    dims[1] = 2 * LQ + 1;
-    double* sw = cur;
-    cur = nxt;
-    nxt = sw;
-  }
-  const int p0 = P.aux_foff[sP], q0 = P.aux_foff[sQ];
-  for (int a = 0; a < dims[0]; ++a)
-    for (int b = 0; b < dims[1]; ++b) {
-      const double v = cur[a * dims[1] + b];
-      P.V[(size_t)(q0 + b) * P.naux + p0 + a] = v;
-      P.V[(size_t)(p0 + a) * P.naux + q0 + b] = v;
+// (P|Q) of two groups: block = shell P, lanes = shells Q.  A pair of pure, s or
+// p shells needs only the Hermite integrals of the two top degrees.
+constexpr int E2_THREADS = 64;
+template <int LP, bool PP, int LQ, bool PQ>
+__global__ void __launch_bounds__(E2_THREADS) k_eri2(const Eri2Params P) {
+  constexpr int NP = ncart(LP), NQ = ncart(LQ), FP = e3_nfun(LP, PP), FQ = e3_nfun(LQ, PQ), L = LP + LQ;
+  constexpr bool TOP = (LP <= 1 || PP) && (LQ <= 1 || PQ);
+  __shared__ double boys[BOYSP_SIZE];
+  __shared__ double sphP[FP * NP], sphQ[FQ * NQ];
+  const int tid = threadIdx.x;
+  for (int i = tid; i < BOYSP_SIZE; i += E2_THREADS) boys[i] = __ldg(P.boysp + (size_t)L * BOYSP_SIZE + i);
+  for (int i = tid; i < FP * NP; i += E2_THREADS)
+    sphP[i] = PP && LP > 1 ? P.sph[sph_off(LP) + i] : (i / NP == i % NP ? 1.0 : 0.0);
+  for (int i = tid; i < FQ * NQ; i += E2_THREADS)
+    sphQ[i] = PQ && LQ > 1 ? P.sph[sph_off(LQ) + i] : (i / NQ == i % NQ ? 1.0 : 0.0);
+  __syncthreads();
+  const int s = blockIdx.y * E2_THREADS + tid;
+  if (s >= P.Q.count || (P.same && s > (int)blockIdx.x)) return;
+  const int sP = P.P.shells[blockIdx.x], sQ = P.Q.shells[s];
+  double A[NP][NQ];  // Cartesian block (its top-degree part)
+#pragma unroll
+  for (int i = 0; i < NP; ++i)
+#pragma unroll
+    for (int j = 0; j < NQ; ++j) A[i][j] = 0.0;
+  for (int j = P.P.prim_off[sP]; j < P.P.prim_off[sP] + P.P.nprim[sP]; ++j)
+    for (int k = P.Q.prim_off[sQ]; k < P.Q.prim_off[sQ] + P.Q.nprim[sQ]; ++k) {
+      const double hp = __ldg(P.P.h + j), hq = __ldg(P.Q.h + k);
+      double R[nherm(L)];
+      quartet_R<L>(__ldg(P.P.p + j), __ldg(P.Q.p + k), __ldg(P.P.Kp + j) * __ldg(P.Q.Kp + k),
+                   __ldg(P.P.x + j) - __ldg(P.Q.x + k), __ldg(P.P.y + j) - __ldg(P.Q.y + k),
+                   __ldg(P.P.z + j) - __ldg(P.Q.z + k), boys, R);
+      if constexpr (TOP) {
+        double hl = (LQ & 1) ? -1.0 : 1.0;
+#pragma unroll
+        for (int i = 0; i < LP; ++i) hl *= hp;
+#pragma unroll
+        for (int i = 0; i < LQ; ++i) hl *= hq;
+        static_for<NP * NQ>([&](auto ab) {
+          constexpr int i = decltype(ab)::value / NQ, b = decltype(ab)::value % NQ;
+          A[i][b] += hl * R[hidx(cart_a(LP, i) + cart_a(LQ, b), cart_b(LP, i) + cart_b(LQ, b),
+                                 cart_c(LP, i) + cart_c(LQ, b))];
+        });
+      } else {
+        for (int m = 0; m < nherm(LP); ++m)
+          for (int n = 0; n < nherm(LQ); ++n) {
+            const int t = c_herm.t[n], u = c_herm.u[n], z = c_herm.v[n];
+            const double r0 = R[hidx(t + c_herm.t[m], u + c_herm.u[m], z + c_herm.v[m])];
+            const double r = ((t + u + z) & 1) ? -r0 : r0;
+            for (int i = 0; i < NP; ++i) {
+              int e[3] = {0, 0, 0};
+              if (LP > 0) e[0] = c_herm.t[nherm(LP - 1) + i], e[1] = c_herm.u[nherm(LP - 1) + i], e[2] = c_herm.v[nherm(LP - 1) + i];
+              const double cp = r * centred_coef(e[0], c_herm.t[m], hp) * centred_coef(e[1], c_herm.u[m], hp) *
+                                centred_coef(e[2], c_herm.v[m], hp);
+              if (cp == 0.0) continue;
+              for (int b = 0; b < NQ; ++b) {
+                int f[3] = {0, 0, 0};
+                if (LQ > 0) f[0] = c_herm.t[nherm(LQ - 1) + b], f[1] = c_herm.u[nherm(LQ - 1) + b], f[2] = c_herm.v[nherm(LQ - 1) + b];
+                A[i][b] += cp * centred_coef(f[0], t, hq) * centred_coef(f[1], u, hq) * centred_coef(f[2], z, hq);
+              }
+            }
+          }
+      }
+    }
+  const int p0 = P.P.foff[sP], q0 = P.Q.foff[sQ];
+  double t[FP][NQ];
+#pragma unroll
+  for (int m = 0; m < FP; ++m)
+#pragma unroll
+    for (int b = 0; b < NQ; ++b) {
+      t[m][b] = 0.0;
+#pragma unroll
+      for (int i = 0; i < NP; ++i) t[m][b] += sphP[m * NP + i] * A[i][b];
+    }
+#pragma unroll
+  for (int m = 0; m < FP; ++m)
+#pragma unroll
+    for (int f = 0; f < FQ; ++f) {
+      double v = 0.0;
+#pragma unroll
+      for (int b = 0; b < NQ; ++b) v += sphQ[f * NQ + b] * t[m][b];
+      P.V[(size_t)(q0 + f) * P.naux + p0 + m] = v;
+      P.V[(size_t)(p0 + m) * P.naux + q0 + f] = v;
     }
 }
 
@@ -422,6 +458,6 @@ void launch_eri3_d_pure(int pair_class_id, const Eri3Params& P, bool j, cudaStre
 void launch_eri3_d_cart(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
 void launch_eri3_f_pure(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
 void launch_eri3_f_cart(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
-void launch_eri2(int LP, int LQ, const Eri2Params& P, cudaStream_t s);
+void launch_eri2(int gP, int gQ, const Eri2Params& P, cudaStream_t s);  // groups gP >= gQ
 
 }  // namespace m2

@@ -44,7 +44,6 @@
 namespace m2 {
 using namespace tc;
 
-PrimView prim_view(const jk_engine* e);
 int eri3_all(jk_engine* e, bool j, cudaStream_t s, const std::function<bool(Eri3Params&, int)>& set);
 int eri3_J(jk_engine* e, const double* c, double* cc, double* J, cudaStream_t s);
 void stage_mark(jk_engine* e, int k, cudaStream_t s);

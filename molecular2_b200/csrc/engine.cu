@@ -194,27 +194,6 @@ int upload_basis(jk_engine* e, const HostBasis& hb, DevBasis& db) {
   return check_cuda(e, st, "upload basis");
 }
 
-// Boys table: F_m(k h), m < BOYS_NCOL, by the convergent series at the top
-// order and downward recursion.
-static std::vector<double> boys_table() {
-  std::vector<double> t(BOYS_NGRID * BOYS_NCOL);
-  const int M = BOYS_NCOL - 1;
-  for (int k = 0; k < BOYS_NGRID; ++k) {
-    double T = k * BOYS_STEP;
-    double term = 1.0 / (2 * M + 1), sum = term;
-    for (int j = 1; j < 2000; ++j) {
-      term *= 2.0 * T / (2 * M + 2 * j + 1);
-      sum += term;
-      if (term < 1e-18 * sum) break;
-    }
-    double ex = std::exp(-T);
-    double* row = &t[k * BOYS_NCOL];
-    row[M] = ex * sum;
-    for (int m = M - 1; m >= 0; --m) row[m] = (2.0 * T * row[m + 1] + ex) / (2 * m + 1);
-  }
-  return t;
-}
-
 // Polynomial Boys tables: per order and interval the polynomial of degree
 // BOYSP_COEF - 1 in (T - centre) that interpolates F_m at the interval's
 // Chebyshev nodes, in extended precision.
@@ -417,12 +396,11 @@ int jk_create(const jk_basis* obs, const jk_basis* aux, int natom, const double*
   }
   rc = upload_basis(e, e->obs, e->dobs);
   if (rc == JK_OK && e->has_aux) rc = upload_basis(e, e->aux, e->daux);
-  if (rc == JK_OK) rc = check_cuda(e, e->boys.upload(boys_table(), e->stream), "boys table");
   if (rc == JK_OK) {
     static const std::vector<double> poly = boys_poly_tables();
     rc = check_cuda(e, e->boysp.upload(poly, e->stream), "boys polynomials");
   }
-  if (rc == JK_OK) rc = check_cuda(e, cudaStreamSynchronize(e->stream), "boys table");
+  if (rc == JK_OK) rc = check_cuda(e, cudaStreamSynchronize(e->stream), "boys polynomials");
   if (rc == JK_OK) rc = build_pairs(e);
   *out = e;
   return rc;

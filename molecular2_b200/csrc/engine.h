@@ -171,11 +171,9 @@ struct jk_engine {
   m2::DevBuf<double> pair_dbls;
   m2::DevBuf<long long> pair_offs;
   m2::DevBuf<double> pp_p, pp_x, pp_y, pp_z, pp_K, pp_a;  // primitive pairs (pp_a: exponent of shell a)
-  m2::DevBuf<double> ap_p, ap_x, ap_y, ap_z, ap_K;         // fitting primitives as (P, unit) pairs
+  m2::DevBuf<double> ap_p, ap_x, ap_y, ap_z;               // fitting primitives
   m2::DevBuf<double> ap_Kp, ap_h;                          // K sqrt(2 pi^(5/2)) / p and 1/(2p)
   m2::DevBuf<int> aux_prim_off;                           // per fitting shell
-  m2::DevBuf<int> aux_by_l[m2::MAX_L_AUX + 1];             // fitting shells grouped by l
-  int aux_by_l_count[m2::MAX_L_AUX + 1] = {0, 0, 0, 0};
   // fitting shells by (l, pure): s, p, pure d, Cartesian d, pure f, Cartesian f
   static constexpr int NAUXGROUP = 6;
   m2::DevBuf<int> aux_group[NAUXGROUP];
@@ -183,7 +181,6 @@ struct jk_engine {
   std::vector<double> schwarz_host;                  // nshell x nshell, row-major (symmetric)
   double Qmax = 0.0;
 
-  m2::DevBuf<double> boys;                           // Boys table
   m2::DevBuf<double> boysp;                          // polynomial Boys tables (quartet.cuh)
 
   // scratch for J/K builds

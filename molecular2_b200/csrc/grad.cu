@@ -18,7 +18,6 @@
 
 namespace m2 {
 
-PrimView prim_view(const jk_engine* e);
 ShellView shell_view(const jk_engine* e);
 
 // significance of each pair of one class from the final-basis overlap matrix
@@ -33,14 +32,6 @@ __global__ void k_pair_sig(PairView pairs, const int* __restrict__ foff, const d
   for (int p = foff[a]; p < foff[a + 1]; ++p)
     for (int q = foff[b]; q < foff[b + 1]; ++q) s2 += S[(size_t)q * n + p] * S[(size_t)q * n + p];
   sig[i] = (same || sqrt(s2) >= 1e-12) ? 1 : 0;
-}
-
-__global__ void k_scale_K(int n, const double* __restrict__ K, const double* __restrict__ p,
-                          const double* __restrict__ alpha, double* __restrict__ K2a, double* __restrict__ K2b) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  K2a[i] = 2.0 * alpha[i] * K[i];
-  K2b[i] = 2.0 * (p[i] - alpha[i]) * K[i];
 }
 
 static void launch_grad2e(const jk_engine* e, int A, int B, const Grad2eParams& Pin, cudaStream_t s) {
@@ -72,11 +63,6 @@ static void launch_grad2e(const jk_engine* e, int A, int B, const Grad2eParams& 
     launch_grad2e_bra_dd(B, P, grid, s);
   else
     launch_grad2e_bra_dd_hi(B, P, grid, s);
-}
-
-void launch_scale_K(int n, const double* K, const double* p, const double* alpha, double* K2a, double* K2b,
-                    cudaStream_t s) {
-  k_scale_K<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, K, p, alpha, K2a, K2b);
 }
 
 // dE_nuc/dx, natom x 3 (src/rhfgrad.cpp:59-86)

@@ -14,42 +14,6 @@
 
 namespace m2 {
 
-// Contract a Cartesian block of class (.., L+SHIFT on centre WHICH, ..) with
-// the weights Wt(a,b,c,d) of class (LA,LB,LC,LD), for the three directions:
-// g[x] += sum Wt * I(component shifted by +-1 along x), times a_x for SHIFT < 0.
-template <int LA, int LB, int LC, int LD, int WHICH, int SHIFT>
-__device__ __forceinline__ void contract_shift(const double* I, const double* Wt, double* g) {
-  constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
-  constexpr int LW = WHICH == 0 ? LA : (WHICH == 1 ? LB : (WHICH == 2 ? LC : LD));
-  constexpr int NSH = ncart(LW + SHIFT);
-  constexpr int NS1 = WHICH == 1 ? NSH : NB, NS2 = WHICH == 2 ? NSH : NC, NS3 = WHICH == 3 ? NSH : ND;
-#pragma unroll 1
-  for (int ia = 0; ia < NA; ++ia)
-#pragma unroll 1
-    for (int ib = 0; ib < NB; ++ib)
-#pragma unroll 1
-      for (int ic = 0; ic < NC; ++ic)
-#pragma unroll 1
-        for (int id = 0; id < ND; ++id) {
-          const double w = Wt[((ia * NB + ib) * NC + ic) * ND + id];
-          if (w == 0.0) continue;
-          int idx[4] = {ia, ib, ic, id};
-          const int i0 = idx[WHICH];
-          const int base = nherm(LW - 1);
-          const int ex[3] = {c_herm.t[base + i0], c_herm.u[base + i0], c_herm.v[base + i0]};
-#pragma unroll
-          for (int x = 0; x < 3; ++x) {
-            int e2[3] = {ex[0], ex[1], ex[2]};
-            e2[x] += SHIFT;
-            if (e2[x] < 0) continue;
-            const double f = SHIFT > 0 ? 1.0 : -(double)ex[x];
-            idx[WHICH] = cidx(e2[0], e2[1], e2[2]);
-            g[x] += f * w * I[((idx[0] * NS1 + idx[1]) * NS2 + idx[2]) * NS3 + idx[3]];
-            idx[WHICH] = i0;
-          }
-        }
-}
-
 struct Grad2eParams {
   PairView bra, ket;
   EntryView bra_ent, ket_ent;

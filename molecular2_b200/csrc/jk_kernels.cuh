@@ -22,9 +22,8 @@ struct ShellView {
   const int* coff;  // Cartesian function offset
 };
 
-
-// Hermite triples and Cartesian exponents by index, for the classes whose
-// loops stay rolled (tables cover totals up to 9).
+// Hermite triples and Cartesian exponents by index, for run-time indices
+// (tables cover totals up to 9).
 struct HermTab {
   unsigned char t[nherm(9)], u[nherm(9)], v[nherm(9)];
 };
@@ -40,134 +39,6 @@ __host__ __device__ constexpr HermTab make_herm_tab() {
   return h;
 }
 __constant__ constexpr HermTab c_herm = make_herm_tab();
-
-// Classes with more than this many Cartesian integrals keep their component
-// loops rolled (small code, arrays in local memory); the rest unroll fully.
-constexpr int UNROLL_LIMIT = 100;
-
-// Contracted Cartesian (ab|cd) for one quartet of shell pairs, accumulated
-// over primitive pairs.  out[((ia*NB+ib)*NC+ic)*ND+id].
-template <int LA, int LB, int LC, int LD>
-__device__ __forceinline__ void quartet_cart(const PrimView& pp, int b0, int nb, double Ax, double Ay, double Az,
-                                             double Bx, double By, double Bz, const PrimView& kp, int k0, int nk,
-                                             double Cx, double Cy, double Cz, double Dx, double Dy, double Dz,
-                                             const double* __restrict__ boys_tab, double* out) {
-  constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
-  constexpr int LAB = LA + LB, LCD = LC + LD, L = LAB + LCD;
-  constexpr int NAB = NA * NB, NCD = NC * ND;
-  constexpr bool BIG = NAB * NCD > UNROLL_LIMIT;
-#pragma unroll
-  for (int i = 0; i < NAB * NCD; ++i) out[i] = 0.0;
-  for (int ib = b0; ib < b0 + nb; ++ib) {
-    const double p = __ldg(pp.p + ib), Px = __ldg(pp.x + ib), Py = __ldg(pp.y + ib), Pz = __ldg(pp.z + ib);
-    const double Kab = __ldg(pp.K + ib);
-    E1<LA, LB> ex, ey, ez;
-    const double oo2p = 0.5 / p;
-    md_E1<LA, LB>(Px - Ax, Px - Bx, oo2p, ex);
-    md_E1<LA, LB>(Py - Ay, Py - By, oo2p, ey);
-    md_E1<LA, LB>(Pz - Az, Pz - Bz, oo2p, ez);
-    for (int ik = k0; ik < k0 + nk; ++ik) {
-      const double q = __ldg(kp.p + ik), Qx = __ldg(kp.x + ik), Qy = __ldg(kp.y + ik), Qz = __ldg(kp.z + ik);
-      const double Kcd = __ldg(kp.K + ik);
-      E1<LC, LD> fx, fy, fz;
-      const double oo2q = 0.5 / q;
-      md_E1<LC, LD>(Qx - Cx, Qx - Dx, oo2q, fx);
-      md_E1<LC, LD>(Qy - Cy, Qy - Dy, oo2q, fy);
-      md_E1<LC, LD>(Qz - Cz, Qz - Dz, oo2q, fz);
-      const double pq = p + q;
-      const double alpha = p * q / pq;
-      const double pref = PI25X2() / (p * q * sqrt(pq)) * Kab * Kcd;
-      const double X = Px - Qx, Y = Py - Qy, Z = Pz - Qz;
-      double F[L + 1];
-      boys<L>(alpha * (X * X + Y * Y + Z * Z), boys_tab, F);
-      double R[nherm(L)];
-      md_R<L>(alpha, X, Y, Z, F, R);
-      if constexpr (!BIG) {
-#pragma unroll
-        for (int icd = 0; icd < NCD; ++icd) {
-          const int ic = icd / ND, id = icd % ND;
-          const int cx = cart_a(LC, ic), cy = cart_b(LC, ic), cz = cart_c(LC, ic);
-          const int dx = cart_a(LD, id), dy = cart_b(LD, id), dz = cart_c(LD, id);
-          double W[nherm(LAB)];
-#pragma unroll
-          for (int h = 0; h < nherm(LAB); ++h) {
-            int k = 0;
-            while (nherm(k) <= h) ++k;
-            const int i = h - (k > 0 ? nherm(k - 1) : 0);
-            const int t = cart_a(k, i), u = cart_b(k, i), v = cart_c(k, i);
-            double s = 0.0;
-#pragma unroll
-            for (int tau = 0; tau <= cx + dx; ++tau)
-#pragma unroll
-              for (int nu = 0; nu <= cy + dy; ++nu)
-#pragma unroll
-                for (int phi = 0; phi <= cz + dz; ++phi) {
-                  const double e = fx.e[cx][dx][tau] * fy.e[cy][dy][nu] * fz.e[cz][dz][phi];
-                  const double r = R[hidx(t + tau, u + nu, v + phi)];
-                  s += ((tau + nu + phi) & 1) ? -e * r : e * r;
-                }
-            W[h] = s;
-          }
-#pragma unroll
-          for (int iab = 0; iab < NAB; ++iab) {
-            const int ia = iab / NB, ibb = iab % NB;
-            const int ax = cart_a(LA, ia), ay = cart_b(LA, ia), az = cart_c(LA, ia);
-            const int bx = cart_a(LB, ibb), by = cart_b(LB, ibb), bz = cart_c(LB, ibb);
-            double acc = 0.0;
-#pragma unroll
-            for (int t = 0; t <= ax + bx; ++t)
-#pragma unroll
-              for (int u = 0; u <= ay + by; ++u)
-#pragma unroll
-                for (int v = 0; v <= az + bz; ++v)
-                  acc += ex.e[ax][bx][t] * ey.e[ay][by][u] * ez.e[az][bz][v] * W[hidx(t, u, v)];
-            out[iab * NCD + icd] += pref * acc;
-          }
-        }
-      } else {
-        const int cbase = nherm(LC - 1 < 0 ? -1 : LC - 1) * (LC > 0);
-        const int dbase = nherm(LD - 1 < 0 ? -1 : LD - 1) * (LD > 0);
-        const int abase = nherm(LA - 1 < 0 ? -1 : LA - 1) * (LA > 0);
-        const int bbase = nherm(LB - 1 < 0 ? -1 : LB - 1) * (LB > 0);
-#pragma unroll 1
-        for (int icd = 0; icd < NCD; ++icd) {
-          const int ic = icd / ND, id = icd % ND;
-          const int cx = c_herm.t[cbase + ic], cy = c_herm.u[cbase + ic], cz = c_herm.v[cbase + ic];
-          const int dx = c_herm.t[dbase + id], dy = c_herm.u[dbase + id], dz = c_herm.v[dbase + id];
-          double W[nherm(LAB)];
-#pragma unroll 1
-          for (int h = 0; h < nherm(LAB); ++h) {
-            const int t = c_herm.t[h], u = c_herm.u[h], v = c_herm.v[h];
-            double s = 0.0;
-            for (int tau = 0; tau <= cx + dx; ++tau)
-              for (int nu = 0; nu <= cy + dy; ++nu) {
-                const double exy = fx.e[cx][dx][tau] * fy.e[cy][dy][nu];
-                for (int phi = 0; phi <= cz + dz; ++phi) {
-                  const double e = exy * fz.e[cz][dz][phi];
-                  const double r = R[hidx(t + tau, u + nu, v + phi)];
-                  s += ((tau + nu + phi) & 1) ? -e * r : e * r;
-                }
-              }
-            W[h] = s;
-          }
-#pragma unroll 1
-          for (int iab = 0; iab < NAB; ++iab) {
-            const int ia = iab / NB, ibb = iab % NB;
-            const int ax = c_herm.t[abase + ia], ay = c_herm.u[abase + ia], az = c_herm.v[abase + ia];
-            const int bx = c_herm.t[bbase + ibb], by = c_herm.u[bbase + ibb], bz = c_herm.v[bbase + ibb];
-            double acc = 0.0;
-            for (int t = 0; t <= ax + bx; ++t)
-              for (int u = 0; u <= ay + by; ++u) {
-                const double exy = ex.e[ax][bx][t] * ey.e[ay][by][u];
-                for (int v = 0; v <= az + bz; ++v) acc += exy * ez.e[az][bz][v] * W[hidx(t, u, v)];
-              }
-            out[iab * NCD + icd] += pref * acc;
-          }
-        }
-      }
-    }
-  }
-}
 
 struct JKParams {
   PairView bra, ket;

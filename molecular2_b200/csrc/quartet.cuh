@@ -431,8 +431,9 @@ __device__ __forceinline__ void for_terms(F&& f) {
 // One primitive quartet's derivatives for bra weights G (Hermite orders <= HL)
 // and one ket component with expansions e, their R derivatives r and bounds
 // (tx, ty, tz): gP[x] += d/dP_x, gR[x] += the ket's d/dR_x part.  R holds orders
-// up to HL + LK + 1.  V is the bra's potential at one ket Hermite index.
-template <int HL, int LK>
+// up to HL + LK + 1.  V is the bra's potential at one ket Hermite index.  G holds
+// the bra's degrees LO .. HL only.
+template <int HL, int LK, int LO = 0>
 __device__ __forceinline__ void ket_gradient(const double* G, const double* R, const double (*e)[LK + 1],
                                              const double (*r)[LK + 1], int tx, int ty, int tz, double* gP,
                                              double* gR) {
@@ -444,12 +445,13 @@ __device__ __forceinline__ void ket_gradient(const double* G, const double* R, c
     const bool sz = c > 0 && a <= tx && b <= ty && c - 1 <= tz;
     if (box || sx || sy || sz) {
       double v0 = 0.0, v1 = 0.0;
-      static_for<nherm(HL)>([&](auto hh) {
-        constexpr int h = decltype(hh)::value;
+      constexpr int h0 = LO > 0 ? nherm(LO - 1) : 0;
+      static_for<nherm(HL) - h0>([&](auto hh) {
+        constexpr int i = decltype(hh)::value, h = h0 + i;
         if constexpr (h & 1)
-          v1 += G[h] * R[hidx(herm_t(h) + a, herm_u(h) + b, herm_v(h) + c)];
+          v1 += G[i] * R[hidx(herm_t(h) + a, herm_u(h) + b, herm_v(h) + c)];
         else
-          v0 += G[h] * R[hidx(herm_t(h) + a, herm_u(h) + b, herm_v(h) + c)];
+          v0 += G[i] * R[hidx(herm_t(h) + a, herm_u(h) + b, herm_v(h) + c)];
       });
       const double V = ((a + b + c) & 1) ? -(v0 + v1) : v0 + v1;
       if constexpr (a + b + c <= LK) {
