@@ -1,30 +1,37 @@
 // FP64 GEMM, blocked Cholesky and triangular inverse (dense.cuh).
 //
-// GEMM: 128 x 128 output tiles, 256 threads = 8 warps in a 2 x 4 grid, each
-// warp a 64 x 32 block of 8 x 4 FP64 tensor-core tiles (mma.sync m8n8k4,
-// the DMMA path), k tiles of 16 staged through a two-buffer shared-memory
-// ring by cp.async (8-byte copies, so any stride works; the thread-to-element
-// map follows whichever operand dimension is contiguous so the copies
-// coalesce).  Out-of-range elements are copied as zeros (cp.async with
-// source size 0).  The shared-memory pitches (136 doubles for [k][m], 20 for
-// [m][k] tiles) put the 32 lanes of a fragment load (4 k x 8 consecutive m)
-// and of a copy into the fewest bank wavefronts.
+// GEMM: 128 x BN output tiles, 256 threads = 8 warps of FP64 tensor-core tiles
+// (mma.sync m8n8k4, the DMMA path, measured 37.1 TFLOP/s on its own, the same as
+// every larger DMMA shape), k tiles of 16 in a three-stage shared-memory ring
+// filled by cp.async (out-of-range elements are copied as zeros).  The copies
+// are 16 bytes wide along an operand's contiguous dimension when its base and
+// strides allow it, 8 bytes otherwise.  The shared-memory pitches (4 modulo 16
+// doubles) spread the 4 x 8 elements of a fragment over the banks evenly.
+// BN follows N: with the one 128-wide tile that was here before, N = 80 spent
+// 37 % of its work on padding (see pick_bn).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <string>
+#include <type_traits>
 
 #include "dense.cuh"
 
 namespace m2 {
 namespace {
 
-constexpr int GBM = 128, GBN = 128, GBK = 16, GT = 256;
-constexpr int LDS = GBM + 8;   // [k][m] rows (doubles): 1088 B, 16-byte aligned, conflict-free fragments
-constexpr int LDK = GBK + 4;   // [m][k] rows (doubles): 160 B, so 4 rows of 4 k fill the 32 banks once
-constexpr int OPER = (GBK * LDS > GBM * LDK) ? GBK * LDS : GBM * LDK;  // doubles per operand buffer
-constexpr int GSMEM = 4 * OPER * (int)sizeof(double);                  // A and B, two buffers each
+constexpr int GBM = 128, GBK = 16, GT = 256, GST = 3;
+constexpr int LDK = GBK + 4;                                    // pitch of [m][k] and [n][k] tiles
+constexpr int lds(int n) { return n + (20 - n % 16) % 16; }     // pitch of [k][m] and [k][n] tiles: 4 modulo 16
+constexpr int oper(int n) { return GBK * lds(n) > n * LDK ? GBK * lds(n) : n * LDK; }  // doubles per operand stage
+constexpr int gsmem(int bn) { return GST * (oper(GBM) + oper(bn)) * (int)sizeof(double); }
+// warps along N: as square a warp tile as BN allows in multiples of 8
+constexpr int warps_n(int bn) { return bn >= 96 ? 4 : (bn % 16 == 0 ? 2 : 1); }
 
+__device__ __forceinline__ void cp16(double* dst, const double* src, int bytes) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void cp8(double* dst, const double* src, bool ok) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
@@ -37,7 +44,10 @@ __device__ __forceinline__ void dmma(double* d, double a, double b) {
                : "d"(a), "d"(b));
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_wait1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
 
 __device__ __forceinline__ void tri_tile(int t, int& tm, int& tn) {
   int m = (int)((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
@@ -47,17 +57,54 @@ __device__ __forceinline__ void tri_tile(int t, int& tm, int& tn) {
   tn = t - m * (m + 1) / 2;
 }
 
-// Operand tiles in shared memory follow the operand's contiguous dimension in
-// global memory: an operand whose k is contiguous (AK1 for A, !BN1 for B) is
-// kept as [m][k] (pitch LDK), the other as [k][m] (pitch LDS), so that the
-// 8-byte copies of a warp land in distinct banks.
-template <bool AK1, bool BN1>
-__global__ void __launch_bounds__(GT) k_dgemm(const DGemm g, int tiles_n) {
+// One stage of an operand: ROWS rows (m or n) by 16 k.  K1: k contiguous in
+// global memory, kept as [row][k]; otherwise [k][row].  Elements beyond nrow or
+// k_end are zero.
+template <int ROWS, bool K1>
+__device__ __forceinline__ void load_stage(double* sm, const double* g, long long sr, long long sk, int r0, int nrow,
+                                           int k0, int k_end, bool vec) {
+  const int t = threadIdx.x;
+  if (vec) {
+    constexpr int NV = ROWS * GBK / 2;
+#pragma unroll
+    for (int i0 = 0; i0 < NV; i0 += GT) {
+      const int i = i0 + t;
+      if (NV % GT != 0 && i >= NV) break;
+      int r, k, left;
+      if (K1) {
+        k = 2 * (i % (GBK / 2));
+        r = i / (GBK / 2);
+        left = r0 + r < nrow ? k_end - k0 - k : 0;
+      } else {
+        r = 2 * (i % (ROWS / 2));
+        k = i / (ROWS / 2);
+        left = k0 + k < k_end ? nrow - r0 - r : 0;
+      }
+      const int bytes = left >= 2 ? 16 : (left == 1 ? 8 : 0);
+      const double* src = g + (long long)(r0 + r) * sr + (long long)(k0 + k) * sk;
+      cp16(sm + (K1 ? r * LDK + k : k * lds(ROWS) + r), bytes ? src : g, bytes);
+    }
+  } else {
+    constexpr int NE = ROWS * GBK;
+#pragma unroll 4
+    for (int i = t; i < NE; i += GT) {
+      const int r = K1 ? i / GBK : i % ROWS, k = K1 ? i % GBK : i / ROWS;
+      const bool ok = r0 + r < nrow && k0 + k < k_end;
+      cp8(sm + (K1 ? r * LDK + k : k * lds(ROWS) + r),
+          ok ? g + (long long)(r0 + r) * sr + (long long)(k0 + k) * sk : g, ok);
+    }
+  }
+}
+
+template <bool AK1, bool BN1, int BN>
+__global__ void __launch_bounds__(GT) k_dgemm(const DGemm g, int tiles_n, bool vec_a, bool vec_b) {
+  constexpr int WNW = warps_n(BN), WMW = 8 / WNW, WM = GBM / WMW, WN = BN / WNW, TM = WM / 8, TN = WN / 8;
+  static_assert(TM * 8 * WMW == GBM && TN * 8 * WNW == BN, "warp tiles must cover the block tile");
   extern __shared__ __align__(16) double gsm[];
-  double* As = gsm;             // two buffers of OPER doubles
-  double* Bs = gsm + 2 * OPER;
-  auto aidx = [](int buf, int k, int m) { return buf * OPER + (AK1 ? m * LDK + k : k * LDS + m); };
-  auto bidx = [](int buf, int k, int n) { return buf * OPER + (BN1 ? k * LDS + n : n * LDK + k); };
+  double* As = gsm;
+  double* Bs = gsm + GST * oper(GBM);
+  auto aidx = [](int k, int m) { return AK1 ? m * LDK + k : k * lds(GBM) + m; };
+  auto bidx = [](int k, int n) { return BN1 ? k * lds(BN) + n : n * LDK + k; };
   int tm, tn;
   if (g.c_lower)
     tri_tile(blockIdx.x, tm, tn);
@@ -65,7 +112,7 @@ __global__ void __launch_bounds__(GT) k_dgemm(const DGemm g, int tiles_n) {
     tm = blockIdx.x / tiles_n;
     tn = blockIdx.x % tiles_n;
   }
-  const int m0 = tm * GBM, n0 = tn * GBN;
+  const int m0 = tm * GBM, n0 = tn * BN;
   const long long bz = blockIdx.z;
   const double* A = g.A + bz * g.bsa;
   const double* B = g.B + bz * g.bsb;
@@ -83,78 +130,59 @@ __global__ void __launch_bounds__(GT) k_dgemm(const DGemm g, int tiles_n) {
     kb = s0;
     ke = s1;
   }
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, wm = warp >> 2, wn = warp & 3;
-
-  auto load = [&](int buf, int k0) {
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      int m, k;
-      if (AK1) {
-        k = t & 15;
-        m = (t >> 4) + 16 * r;
-      } else {
-        m = t & 127;
-        k = (t >> 7) + 2 * r;
-      }
-      const int gm = m0 + m, gk = k0 + k;
-      const bool ok = gm < g.M && gk < ke;
-      cp8(As + aidx(buf, k, m), ok ? A + (long long)gm * g.sam + (long long)gk * g.sak : A, ok);
-    }
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      int n, k;
-      if (BN1) {
-        n = t & 127;
-        k = (t >> 7) + 2 * r;
-      } else {
-        k = t & 15;
-        n = (t >> 4) + 16 * r;
-      }
-      const int gn = n0 + n, gk = k0 + k;
-      const bool ok = gn < g.N && gk < ke;
-      cp8(Bs + bidx(buf, k, n), ok ? B + (long long)gk * g.sbk + (long long)gn * g.sbn : B, ok);
-    }
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, wm = warp / WNW, wn = warp % WNW;
+  auto load = [&](int it) {
+    const int st = it % GST, k0 = kb + it * GBK;
+    load_stage<GBM, AK1>(As + st * oper(GBM), A, g.sam, g.sak, m0, g.M, k0, ke, vec_a);
+    load_stage<BN, !BN1>(Bs + st * oper(BN), B, g.sbn, g.sbk, n0, g.N, k0, ke, vec_b);
   };
 
-  double acc[8][4][2];
+  double acc[TM][TN][2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < TN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
   const int nk = ke > kb ? (ke - kb + GBK - 1) / GBK : 0;
-  if (nk > 0) load(0, kb);
-  cp_commit();
-  const int fk = lane & 3, fr = lane >> 2;
-  for (int it = 0; it < nk; ++it) {
-    if (it + 1 < nk) load((it + 1) & 1, kb + (it + 1) * GBK);
+#pragma unroll
+  for (int it = 0; it < GST - 1; ++it) {
+    if (it < nk) load(it);
     cp_commit();
-    cp_wait1();
+  }
+  const int fk = lane & 3, fr = lane >> 2;
+  // a warp above the diagonal of a lower-triangle tile only helps to load
+  const bool above = g.c_lower && tm == tn && wm * WM + WM <= wn * WN;
+  for (int it = 0; it < nk; ++it) {
+    cp_wait<GST - 2>();
     __syncthreads();
-    const int buf = it & 1;
+    if (it + GST - 1 < nk) load(it + GST - 1);
+    cp_commit();
+    if (above) continue;
+    const double* a_s = As + (it % GST) * oper(GBM);
+    const double* b_s = Bs + (it % GST) * oper(BN);
 #pragma unroll
     for (int k4 = 0; k4 < GBK; k4 += 4) {
-      double a[8], b[4];
+      double a[TM], b[TN];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) a[i] = As[aidx(buf, k4 + fk, wm * 64 + i * 8 + fr)];
+      for (int i = 0; i < TM; ++i) a[i] = a_s[aidx(k4 + fk, wm * WM + i * 8 + fr)];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[bidx(buf, k4 + fk, wn * 32 + j * 8 + fr)];
+      for (int j = 0; j < TN; ++j) b[j] = b_s[bidx(k4 + fk, wn * WN + j * 8 + fr)];
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
+      for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[i][j], a[i], b[j]);
+        for (int j = 0; j < TN; ++j) dmma(acc[i][j], a[i], b[j]);
     }
-    __syncthreads();
   }
+  if (above) return;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int gm = m0 + wm * 64 + i * 8 + fr;
+  for (int i = 0; i < TM; ++i) {
+    const int gm = m0 + wm * WM + i * 8 + fr;
     if (gm >= g.M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < TN; ++j)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int gn = n0 + wn * 32 + j * 8 + 2 * fk + h;
+        const int gn = n0 + wn * WN + j * 8 + 2 * fk + h;
         if (gn >= g.N) continue;
         double* c = C + (long long)gm * g.scm + (long long)gn * g.scn;
         if (g.ksplit > 1)
@@ -270,6 +298,25 @@ __global__ void __launch_bounds__(CNB) k_trinv_diag(const double* L, double* Lin
 
 }  // namespace
 
+// Tile width for N columns: the least padded columns, weighted with the work a
+// narrower tile adds per column (fragment loads per DMMA).
+static int pick_bn(int N) {
+  static const struct {
+    int bn;
+    double w;
+  } opt[] = {{128, 1.0}, {96, 1.0}, {80, 1.0}, {64, 1.03}, {48, 1.06}, {40, 1.1}, {32, 1.1}, {16, 1.3}};
+  int best = 128;
+  double cost = 1e300;
+  for (const auto& o : opt) {
+    const double c = (double)((N + o.bn - 1) / o.bn) * o.bn * o.w;
+    if (c < cost) {
+      cost = c;
+      best = o.bn;
+    }
+  }
+  return best;
+}
+
 cudaError_t dgemm(const DGemm& g, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0 || g.batch <= 0) return cudaSuccess;
   if (g.c_lower && g.M != g.N) return cudaErrorInvalidValue;
@@ -281,20 +328,58 @@ cudaError_t dgemm(const DGemm& g, cudaStream_t s) {
                                                                            h.beta);
     h.beta = 1.0;
   }
-  const int tm = (h.M + GBM - 1) / GBM, tn = (h.N + GBN - 1) / GBN;
+  const int bn = h.c_lower ? 128 : pick_bn(h.N);
+  const int tm = (h.M + GBM - 1) / GBM, tn = (h.N + bn - 1) / bn;
   const long long tiles = h.c_lower ? (long long)tm * (tm + 1) / 2 : (long long)tm * tn;
   dim3 grid((unsigned)tiles, h.ksplit, h.batch);
   const bool ak1 = h.sak == 1, bn1 = h.sbn == 1;
-  auto launch = [&](auto kern) {
-    cudaError_t st = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GSMEM);
+  auto aligned = [](const double* p, long long s1, long long s2) {
+    return ((uintptr_t)p & 15) == 0 && s1 % 2 == 0 && s2 % 2 == 0;
+  };
+  const bool va = (ak1 ? aligned(h.A, h.sam, h.bsa) : h.sam == 1 && aligned(h.A, h.sak, h.bsa));
+  const bool vb = (bn1 ? aligned(h.B, h.sbk, h.bsb) : h.sbk == 1 && aligned(h.B, h.sbn, h.bsb));
+  auto launch = [&](auto kern, int smem) {
+    cudaError_t st = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (st != cudaSuccess) return st;
-    kern<<<grid, GT, GSMEM, s>>>(h, tn);
+    kern<<<grid, GT, smem, s>>>(h, tn, va, vb);
     return cudaGetLastError();
   };
-  if (ak1 && bn1) return launch(k_dgemm<true, true>);
-  if (ak1) return launch(k_dgemm<true, false>);
-  if (bn1) return launch(k_dgemm<false, true>);
-  return launch(k_dgemm<false, false>);
+  auto pick = [&](auto width) {
+    constexpr int W = decltype(width)::value;
+    if (ak1 && bn1) return launch(k_dgemm<true, true, W>, gsmem(W));
+    if (ak1) return launch(k_dgemm<true, false, W>, gsmem(W));
+    if (bn1) return launch(k_dgemm<false, true, W>, gsmem(W));
+    return launch(k_dgemm<false, false, W>, gsmem(W));
+  };
+  switch (bn) {
+    case 16: return pick(std::integral_constant<int, 16>{});
+    case 32: return pick(std::integral_constant<int, 32>{});
+    case 40: return pick(std::integral_constant<int, 40>{});
+    case 48: return pick(std::integral_constant<int, 48>{});
+    case 64: return pick(std::integral_constant<int, 64>{});
+    case 80: return pick(std::integral_constant<int, 80>{});
+    case 96: return pick(std::integral_constant<int, 96>{});
+    default: return pick(std::integral_constant<int, 128>{});
+  }
+}
+
+// Blocks of a split-k GEMM over `tiles` output tiles: the split that leaves the
+// last wave of one block per SM fullest, with at least 128 k per block.
+int split_k(long long tiles, long long K, int nsm) {
+  const long long most = std::max(1LL, std::min(65535LL, K / 128));
+  int best = 1;
+  double eff = 0.0;
+  for (int waves = 1; waves <= 8; ++waves) {
+    const long long ks = std::min(most, waves * (long long)nsm / tiles);
+    if (ks < 1) continue;
+    const long long blocks = tiles * ks, w = (blocks + nsm - 1) / nsm;
+    const double e = (double)blocks / (double)(w * nsm);
+    if (e > eff + 0.02) {
+      eff = e;
+      best = (int)ks;
+    }
+  }
+  return best;
 }
 
 void mirror_lower(double* C, int n, cudaStream_t s) {
@@ -312,7 +397,8 @@ int cholesky(jk_engine* e, double* A, int n, double* work, int* info, cudaStream
     k_potrf_diag<<<1, 256, PSMEM, s>>>(A, n, j, work, info);
     const int R = n - j - b;
     if (R <= 0) break;
-    // L21 = A21 L11^-T, in place (each output tile reads only its own rows)
+    // L21 = A21 L11^-T, in place: at most 64 columns are one tile wide
+    // (pick_bn), so each block reads only the rows it writes
     DGemm p;
     p.M = R;
     p.N = b;

@@ -26,9 +26,12 @@ struct DGemm {
   double alpha = 1.0, beta = 0.0;
   bool a_lower = false;  // A(m, k) = 0 for k > m: the k loop of a row tile stops at its last row
   bool b_lower = false;  // B(k, n) = 0 for k < n: the k loop of a column tile starts at its first column
-  bool c_lower = false;  // only tiles on or below the diagonal (tile_n <= tile_m) are computed
+  bool c_lower = false;  // only C(m, n) with n <= m is wanted; elements above it may or may not be written
   int ksplit = 1;        // > 1: the k range is split over blocks whose sums are added atomically
 };
+
+// k split for `tiles` output tiles and K terms on nsm SMs.
+int split_k(long long tiles, long long K, int nsm);
 
 // Launch on stream s.  Returns the launch status.
 cudaError_t dgemm(const DGemm& g, cudaStream_t s);

@@ -290,7 +290,6 @@ cudaError_t df_syrk_X(jk_engine* e, const double* X, int n, long long len, doubl
   int nsm = 148;
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->device);
   const int tiles = ((n + 127) / 128) * ((n + 127) / 128 + 1) / 2;
-  const long long kt = (len + 15) / 16;
   DGemm g;
   g.M = n;
   g.N = n;
@@ -305,7 +304,7 @@ cudaError_t df_syrk_X(jk_engine* e, const double* X, int n, long long len, doubl
   g.scm = 1;
   g.scn = n;
   g.c_lower = true;
-  g.ksplit = (int)std::max(1LL, std::min<long long>((2LL * nsm + tiles - 1) / tiles, kt / 8));
+  g.ksplit = split_k(tiles, len, nsm);
   cudaError_t st = dgemm(g, s);
   if (st == cudaSuccess) mirror_lower(K, n, s);
   return st == cudaSuccess ? cudaGetLastError() : st;

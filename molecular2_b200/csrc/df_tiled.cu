@@ -921,7 +921,7 @@ static int tiled_fp64(jk_engine* e, const double* dC, int nocc, double* dJ, doub
       k.scn = n;
       k.beta = 1.0;
       k.c_lower = true;
-      k.ksplit = (int)std::max(1LL, std::min<long long>((2LL * nsm + tiles - 1) / tiles, len / 128));
+      k.ksplit = split_k(tiles, len, nsm);
       if ((st = dgemm(k, s)) != cudaSuccess) return check_cuda(e, st, "K += Y Y^T");
     }
     if (ch == 0) stage_mark(e, 3, s);  // profiling: K of the first slice
