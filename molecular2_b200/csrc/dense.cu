@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(GT) k_dgemm(const DGemm g, int tiles_n, bool v
   else {
     tm = blockIdx.x / tiles_n;
     tn = blockIdx.x % tiles_n;
+    if (g.a_lower) tm = (gridDim.x / tiles_n) - 1 - tm;  // longest k ranges first
   }
   const int m0 = tm * GBM, n0 = tn * BN;
   const long long bz = blockIdx.z;
@@ -137,12 +138,6 @@ __global__ void __launch_bounds__(GT) k_dgemm(const DGemm g, int tiles_n, bool v
     load_stage<BN, !BN1>(Bs + st * oper(BN), B, g.sbn, g.sbk, n0, g.N, k0, ke, vec_b);
   };
 
-  double acc[TM][TN][2];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
-
   const int nk = ke > kb ? (ke - kb + GBK - 1) / GBK : 0;
 #pragma unroll
   for (int it = 0; it < GST - 1; ++it) {
@@ -150,6 +145,24 @@ __global__ void __launch_bounds__(GT) k_dgemm(const DGemm g, int tiles_n, bool v
     cp_commit();
   }
   const int fk = lane & 3, fr = lane >> 2;
+  // the sums start from beta / alpha C, read while the first stages arrive (read
+  // at the end, every element would wait for its own round trip behind the
+  // stores before it)
+  double acc[TM][TN][2];
+  const double c_in = g.ksplit > 1 ? 0.0 : g.beta / g.alpha;
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int gm = m0 + wm * WM + i * 8 + fr;
+#pragma unroll
+    for (int j = 0; j < TN; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int gn = n0 + wn * WN + j * 8 + 2 * fk + h;
+        acc[i][j][h] = 0.0;
+        if (c_in != 0.0 && gm < g.M && gn < g.N)
+          acc[i][j][h] = c_in * C[(long long)gm * g.scm + (long long)gn * g.scn];
+      }
+  }
   // a warp above the diagonal of a lower-triangle tile only helps to load
   const bool above = g.c_lower && tm == tn && wm * WM + WM <= wn * WN;
   for (int it = 0; it < nk; ++it) {
@@ -188,7 +201,7 @@ __global__ void __launch_bounds__(GT) k_dgemm(const DGemm g, int tiles_n, bool v
         if (g.ksplit > 1)
           atomicAdd(c, g.alpha * acc[i][j][h]);
         else
-          *c = g.beta == 0.0 ? g.alpha * acc[i][j][h] : g.alpha * acc[i][j][h] + g.beta * *c;
+          *c = g.alpha * acc[i][j][h];
       }
   }
 }

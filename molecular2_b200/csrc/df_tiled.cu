@@ -814,9 +814,13 @@ static int tiled_fp64(jk_engine* e, const double* dC, int nocc, double* dJ, doub
   if (oc < 1) return set_error(e, JK_ERR_NOMEM, "tiled FP64 DF: no room for one occupied orbital's X'");
   const int nch = (nocc + oc - 1) / oc;
   oc = (nocc + nch - 1) / nch;
+  // where a second array of X's size fits easily, Y is formed at once and K reads
+  // it there; otherwise XB rows at a time, copied back over X'
+  const bool whole = 8.0 * (double)(npad + n) * naux * oc < 0.5 * (double)fr;
+  const int yrows = whole ? n : XB;
   DevBuf<double> X, Yb;
   st = X.alloc((size_t)npad * naux * oc);
-  if (st == cudaSuccess) st = Yb.alloc((size_t)XB * naux * oc);
+  if (st == cudaSuccess) st = Yb.alloc((size_t)yrows * naux * oc);
   if (st != cudaSuccess) return check_cuda(e, st, "tiled FP64 X'");
   k_pad_rows<<<(unsigned)(((size_t)npad * nocc + 255) / 256), 256, 0, s>>>(n, npad, nocc, dC, Cp.p);
   {
@@ -876,9 +880,9 @@ static int tiled_fp64(jk_engine* e, const double* dC, int nocc, double* dJ, doub
       if ((st = dgemm(g, s)) != cudaSuccess) return check_cuda(e, st, "L^-T (L^-1 d)");
       if ((rc = eri3_J(e, cv.p, cc.p, dJ, s))) return rc;
     }
-    // Y = L^-1 X' for every row x, XB rows at a time
-    for (int x0 = 0; x0 < n; x0 += XB) {
-      const int xb = std::min(XB, n - x0);
+    // Y = L^-1 X' for every row x, yrows rows at a time
+    for (int x0 = 0; x0 < n; x0 += yrows) {
+      const int xb = std::min(yrows, n - x0);
       DGemm y;
       y.M = naux;
       y.N = ocur;
@@ -897,8 +901,9 @@ static int tiled_fp64(jk_engine* e, const double* dC, int nocc, double* dJ, doub
       y.scn = 1;
       y.bsc = (long long)naux * ocur;
       if ((st = dgemm(y, s)) != cudaSuccess) return check_cuda(e, st, "Y = L^-1 X'");
-      st = cudaMemcpyAsync(X.p + (size_t)x0 * naux * ocur, Yb.p, sizeof(double) * (size_t)xb * naux * ocur,
-                           cudaMemcpyDeviceToDevice, s);
+      if (!whole)
+        st = cudaMemcpyAsync(X.p + (size_t)x0 * naux * ocur, Yb.p, sizeof(double) * (size_t)xb * naux * ocur,
+                             cudaMemcpyDeviceToDevice, s);
       if (st != cudaSuccess) return check_cuda(e, st, "Y copy");
     }
     if (ch == 0) stage_mark(e, 2, s);  // profiling: Y = L^-1 X' of the first slice
@@ -910,10 +915,10 @@ static int tiled_fp64(jk_engine* e, const double* dC, int nocc, double* dJ, doub
       k.M = n;
       k.N = n;
       k.K = (int)len;
-      k.A = X.p;
+      k.A = whole ? Yb.p : X.p;
       k.sam = len;
       k.sak = 1;
-      k.B = X.p;
+      k.B = k.A;
       k.sbk = 1;
       k.sbn = len;
       k.C = dK;
