@@ -300,6 +300,11 @@ typedef struct jk_scf_result {
   int lindep_dropped;      /* directions removed by jk_scf_options.lindep */
 } jk_scf_result;
 
+/* Device blocks that finished calls and destroyed engines left in the library's
+ * cache (at most 4 GiB per device, reused by later calls; emptied by itself when
+ * an allocation fails) go back to the driver. */
+int jk_release_cached(int device);
+
 int jk_scf_rhf(jk_engine* e, const jk_scf_options* opt, jk_scf_result* res);
 
 /* RHF nuclear gradient dE/dx (natom x 3, atom-major) for the full density D

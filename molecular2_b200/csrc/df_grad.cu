@@ -352,7 +352,7 @@ int grad_df_2e_tiled(jk_engine* e, const double* dC, int nocc, const double* dD,
   launch_pad_rows(n, npad, o, dC, Cp.p, s);
   {
     size_t fr = 0, tot = 0;
-    cudaMemGetInfo(&fr, &tot);
+    dev_mem_info(&fr, &tot);
     int oc = (int)std::min<double>(o, std::floor(0.8 * (double)fr / (8.0 * npad * naux)));
     if (oc < 1) return set_error(e, JK_ERR_NOMEM, "tiled DF gradient: no room for X'");
     const int nch = (o + oc - 1) / oc;
@@ -418,7 +418,7 @@ int grad_df_2e_tiled(jk_engine* e, const double* dC, int nocc, const double* dD,
   // W3 = c_P D - 2 C d^P C^T and its contraction, one block of fitting shells at a time
   {
     size_t fr = 0, tot = 0;
-    cudaMemGetInfo(&fr, &tot);
+    dev_mem_info(&fr, &tot);
     const double per_f = 8.0 * ((double)ncc + (double)nc * o);
     const int wmax = (int)std::max(16.0, std::min<double>(naux, 0.6 * (double)fr / per_f));
     DevBuf<double> Y, Z;

@@ -97,7 +97,7 @@ static int df_mp2(jk_engine* e, const double* hC, const double* heps, int nmo, i
   X.reset();
   // blocks of i with V_i (nv x act*nv) resident, within a quarter of the free memory
   size_t fr = 0, tt = 0;
-  cudaMemGetInfo(&fr, &tt);
+  dev_mem_info(&fr, &tt);
   const double per_i = 8.0 * (double)nv * act * nv;
   const int ib = (int)std::max(1.0, std::min<double>(std::min(act, 64), 0.25 * (double)fr / per_i));
   if ((st = V.alloc((size_t)ib * act * nv * nv)) != cudaSuccess) return check_cuda(e, st, "jk_df_mp2 V block");

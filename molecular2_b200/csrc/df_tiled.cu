@@ -416,7 +416,7 @@ bool df_use_tiled(jk_engine* e) {
   if (e->df_storage == 2) return true;
   if (e->df_storage == 1) return false;
   size_t fr = 0, tot = 0;
-  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return false;
+  if (dev_mem_info(&fr, &tot) != cudaSuccess) return false;
   const double n = e->obs.n_final, q = e->aux.n_final;
   // the unpacked path holds T3 and B64 (FP64) at set-up, then B64 and its split copy
   return 16.0 * n * n * q > 0.8 * (double)fr;
@@ -599,7 +599,7 @@ static int tiled_mixed_prepare(jk_engine* e, int nocc) {
     if (st != cudaSuccess) return check_cuda(e, st, "tiled mixed scratch");
     // X block: as many fitted functions as fit in a quarter of the free memory (at most all)
     size_t fr = 0, tt = 0;
-    cudaMemGetInfo(&fr, &tt);
+    dev_mem_info(&fr, &tt);
     const double per_k = 4.0 * T.npad * NPX;  // hi + lo BF16
     int w = (int)std::min<double>(naux, std::max(64.0, 0.25 * fr / per_k));
     if (T.waux_max > 0) w = std::min(w, T.waux_max);
@@ -807,7 +807,7 @@ static int tiled_fp64(jk_engine* e, const double* dC, int nocc, double* dJ, doub
   // occupied slice: X' (npad x naux x oc) and a Y batch of XB rows must fit
   constexpr int XB = 64;
   size_t fr = 0, tt = 0;
-  cudaMemGetInfo(&fr, &tt);
+  dev_mem_info(&fr, &tt);
   const double per_o = 8.0 * (double)(npad + XB) * naux;
   int oc = (int)std::min<double>(nocc, std::floor(0.94 * (double)fr / per_o));
   if (T.oc_max > 0) oc = std::min(oc, T.oc_max);

@@ -24,6 +24,18 @@ int check_cuda(jk_engine* e, cudaError_t st, const char* what) {
   return set_error(e, code, std::string(what) + ": " + cudaGetErrorString(st));
 }
 
+// Only the SCF driver needs the libraries; making and destroying the two handles
+// costs 5 ms, as much as everything else of a small engine.
+int library_handles(jk_engine* e) {
+  if (!e->cublas && (cublasCreate(&e->cublas) != CUBLAS_STATUS_SUCCESS ||
+                     cublasSetStream(e->cublas, e->stream) != CUBLAS_STATUS_SUCCESS))
+    return set_error(e, JK_ERR_CUDA, "cublasCreate failed");
+  if (!e->cusolver && (cusolverDnCreate(&e->cusolver) != CUSOLVER_STATUS_SUCCESS ||
+                       cusolverDnSetStream(e->cusolver, e->stream) != CUSOLVER_STATUS_SUCCESS))
+    return set_error(e, JK_ERR_CUDA, "cusolverDnCreate failed");
+  return JK_OK;
+}
+
 static double dfact(int n) {
   double r = 1.0;
   for (int k = n; k > 1; k -= 2) r *= k;
@@ -383,16 +395,6 @@ int jk_create(const jk_basis* obs, const jk_basis* aux, int natom, const double*
     rc = check_cuda(e, st, "jk_create: device/stream");
     *out = e;
     return rc;
-  }
-  if (cublasCreate(&e->cublas) != CUBLAS_STATUS_SUCCESS ||
-      cublasSetStream(e->cublas, e->stream) != CUBLAS_STATUS_SUCCESS) {
-    *out = e;
-    return set_error(e, JK_ERR_CUDA, "jk_create: cublasCreate failed");
-  }
-  if (cusolverDnCreate(&e->cusolver) != CUSOLVER_STATUS_SUCCESS ||
-      cusolverDnSetStream(e->cusolver, e->stream) != CUSOLVER_STATUS_SUCCESS) {
-    *out = e;
-    return set_error(e, JK_ERR_CUDA, "jk_create: cusolverDnCreate failed");
   }
   rc = upload_basis(e, e->obs, e->dobs);
   if (rc == JK_OK && e->has_aux) rc = upload_basis(e, e->aux, e->daux);

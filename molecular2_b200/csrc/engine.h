@@ -30,6 +30,12 @@ struct HostBasis {
   int max_l = 0;
 };
 
+// Device memory through the cache of pool.cu: dev_free waits for the device, as
+// cudaFree does; dev_mem_info counts cached blocks as free.
+cudaError_t dev_alloc(void** p, size_t bytes);
+void dev_free(void* p);
+cudaError_t dev_mem_info(size_t* free_bytes, size_t* total);
+
 // Device array with RAII.
 template <class T>
 struct DevBuf {
@@ -40,7 +46,7 @@ struct DevBuf {
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { reset(); }
   void reset() {
-    if (p) cudaFree(p);
+    dev_free(p);
     p = nullptr;
     n = 0;
   }
@@ -48,7 +54,7 @@ struct DevBuf {
     if (count == n && p) return cudaSuccess;
     reset();
     if (count == 0) return cudaSuccess;
-    cudaError_t e = cudaMalloc(&p, count * sizeof(T));
+    cudaError_t e = dev_alloc((void**)&p, count * sizeof(T));
     if (e == cudaSuccess) n = count;
     return e;
   }
@@ -210,6 +216,7 @@ struct jk_engine {
 namespace m2 {
 // engine.cu
 int set_error(jk_engine* e, int code, const std::string& msg);
+int library_handles(jk_engine* e);  // cuBLAS and cuSOLVER, created by their first user
 int check_cuda(jk_engine* e, cudaError_t st, const char* what);
 int build_basis(const jk_basis* b, bool allow_pure, int lmax, HostBasis& out, std::string& err);
 int upload_basis(jk_engine* e, const HostBasis& hb, DevBasis& db);

@@ -122,7 +122,7 @@ void full_piv_solve(std::vector<double> A, int N, std::vector<double> b, std::ve
 }
 
 // FIFO of at most `cap` device vectors backed by buffers allocated once, so
-// the SCF loop never allocates (cudaFree would synchronise the device).
+// the SCF loop never allocates (freeing waits for the device).
 struct Ring {
   std::vector<std::unique_ptr<DevBuf<double>>> pool;
   std::vector<double*> order;  // oldest first
@@ -244,6 +244,7 @@ int scf_rhf(jk_engine* e, const jk_scf_options* o, jk_scf_result* r) {
     if (rc) return rc;
   }
   cudaStream_t s = e->stream;
+  if (int rc = library_handles(e)) return rc;
   cublasSetStream(e->cublas, s);
   Gpu g{e, s, n};
   DevBuf<double> S, T, V, H, X, F, Fm, Finc, D, Dd, Dold, C, W, Wt, eps, J, K, t1, t2, err, work, Delta;

@@ -51,6 +51,7 @@ SIGNATURES = {
     "jk_df_set_storage": (_I, [_P, _I]),
     "jk_df_mp2": (_I, [_P, _P, _P, _I, _I, _I, _P]),
     "jk_wait_selftest": (_I, [_P, ctypes.c_uint, ctypes.POINTER(_I), ctypes.POINTER(_I)]),
+    "jk_release_cached": (_I, [_I]),
     "jk_df_storage": (_I, [_P]),
     "jk_df_tensor_bytes": (ctypes.c_longlong, [_P]),
     "jk_df_set_tiled_blocks": (_I, [_P, _I, _I]),
@@ -124,6 +125,13 @@ def fock_general(obs: BasisSet, dbs: BasisSet, D, shelldiag=True, precision=1e-1
     if rc:
         raise JKError(rc, "jk_fock_general failed")
     return G
+
+
+def release_cached(device=0):
+    """Returns the device memory that the library keeps for reuse (at most 4 GiB) to the driver."""
+    rc = load_library().jk_release_cached(device)
+    if rc:
+        raise JKError(rc, "jk_release_cached failed")
 
 
 class IntegralEngine:
