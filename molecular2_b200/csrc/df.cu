@@ -330,7 +330,7 @@ int df_setup(jk_engine* e) {
   // V = L L^T (own blocked Cholesky), then L^-1
   DevBuf<double> work;
   DevBuf<int> info;
-  st = work.alloc((size_t)naux * naux);
+  st = work.alloc((size_t)naux * std::max(naux, 64));
   if (st == cudaSuccess) st = info.alloc(1);
   if (st != cudaSuccess) return check_cuda(e, st, "Cholesky workspace");
   if ((rc = cholesky(e, d.L.p, naux, work.p, info.p, s))) return rc;

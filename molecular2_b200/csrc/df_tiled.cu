@@ -501,7 +501,7 @@ int df_tiled_metric(jk_engine* e) {
   {
     DevBuf<double> work;
     DevBuf<int> info;
-    st = work.alloc((size_t)naux * naux);
+    st = work.alloc((size_t)naux * std::max(naux, 64));
     if (st == cudaSuccess) st = info.alloc(1);
     if (st != cudaSuccess) return check_cuda(e, st, "Cholesky workspace");
     if ((rc = cholesky(e, d.L.p, naux, work.p, info.p, s))) return rc;
