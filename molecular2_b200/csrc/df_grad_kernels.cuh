@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad3(const Grad3Params P) 
   const int tid = threadIdx.x, lane = tid & 31;
   const bool local = P.natom <= GRAD_ATOMS;
   double* g_atom = local ? s_g : P.grad;
-  for (int i = tid; i < BOYSP_SIZE; i += GRAD_THREADS) S.boys[i] = __ldg(P.boysp + (size_t)(L + 1) * BOYSP_SIZE + i);
+  load_boys<L + 1>(S.boys, P.boysp);
   if constexpr (PURE && LP > 1)
     for (int i = tid; i < NF * NP; i += GRAD_THREADS) S.sphP[i] = P.sph[sph_off(LP) + i];
   if (local)
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(G2_THREADS) k_grad2(const Grad2Params P) {
   __shared__ double boys[BOYSP_SIZE];
   __shared__ double sphP[FP * NP], sphQ[FQ * NQ];
   const int tid = threadIdx.x, lane = tid & 31;
-  for (int i = tid; i < BOYSP_SIZE; i += G2_THREADS) boys[i] = __ldg(P.boysp + (size_t)L * BOYSP_SIZE + i);
+  load_boys<L>(boys, P.boysp);
   if (PP && LP > 1)
     for (int i = tid; i < FP * NP; i += G2_THREADS) sphP[i] = P.sph[sph_off(LP) + i];
   if (PQ && LQ > 1)

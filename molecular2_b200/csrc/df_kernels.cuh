@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(E3_THREADS, 2) k_eri3(const Eri3Params P) {
   const int a = P.pairs.sa[ip], b = P.pairs.sb[ip];
   const int e0 = P.ent.first[ip], e1 = P.ent.first[ip + 1];
   const int f0 = blockIdx.y;  // the layer's function
-  for (int i = tid; i < BOYSP_SIZE; i += blockDim.x) S.boys[i] = __ldg(P.boysp + (size_t)L * BOYSP_SIZE + i);
+  load_boys<L>(S.boys, P.boysp);
   if constexpr (PURE && LP > 1)
     for (int i = tid; i < NF * NP; i += blockDim.x) S.sphP[i] = P.sph[sph_off(LP) + i];
   const double A[3] = {P.ox[a], P.oy[a], P.oz[a]}, B[3] = {P.ox[b], P.oy[b], P.oz[b]};
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(E3_THREADS, 2) k_eri3_J(const Eri3Params P) {
   const int tid = threadIdx.x, lane = tid & 31;
   const int ip = blockIdx.x;
   const int a = P.pairs.sa[ip], b = P.pairs.sb[ip];
-  for (int i = tid; i < BOYSP_SIZE; i += blockDim.x) S.boys[i] = __ldg(P.boysp + (size_t)L * BOYSP_SIZE + i);
+  load_boys<L>(S.boys, P.boysp);
   const double A[3] = {P.ox[a], P.oy[a], P.oz[a]}, B[3] = {P.ox[b], P.oy[b], P.oz[b]};
   __shared__ double cart[NAB];
   for (int i = tid; i < NAB; i += blockDim.x) cart[i] = 0.0;
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(E2_THREADS) k_eri2(const Eri2Params P) {
   __shared__ double boys[BOYSP_SIZE];
   __shared__ double sphP[FP * NP], sphQ[FQ * NQ];
   const int tid = threadIdx.x;
-  for (int i = tid; i < BOYSP_SIZE; i += E2_THREADS) boys[i] = __ldg(P.boysp + (size_t)L * BOYSP_SIZE + i);
+  load_boys<L>(boys, P.boysp);
   for (int i = tid; i < FP * NP; i += E2_THREADS)
     sphP[i] = PP && LP > 1 ? P.sph[sph_off(LP) + i] : (i / NP == i % NP ? 1.0 : 0.0);
   for (int i = tid; i < FQ * NQ; i += E2_THREADS)

@@ -206,20 +206,20 @@ int upload_basis(jk_engine* e, const HostBasis& hb, DevBasis& db) {
   return check_cuda(e, st, "upload basis");
 }
 
-// Polynomial Boys tables: per order and interval the polynomial of degree
-// BOYSP_COEF - 1 in (T - centre) that interpolates F_m at the interval's
-// Chebyshev nodes, in extended precision.
+// Polynomial Boys tables (quartet.cuh): per order and interval the polynomial of
+// degree BOYSP_COEF - 1 in (T - centre) that interpolates F_m at the interval's
+// Chebyshev nodes, in extended precision; then e^{-centre}.
 static std::vector<double> boys_poly_tables() {
   constexpr int NC = BOYSP_COEF, M = BOYSP_MMAX;
-  const long double width = (long double)BOYS_TMAX / BOYSP_ROWS, pi = acosl(-1.0L);
+  const long double width = BOYSP_WIDTH, pi = acosl(-1.0L);
   std::vector<double> t((size_t)(M + 1) * BOYSP_SIZE);
   for (int row = 0; row < BOYSP_ROWS; ++row) {
-    const long double mid = (row + 0.5L) * width;
-    long double f[M + 1][NC];  // F_m at the nodes
+    const long double mid = row * width;
+    long double f[M + 1][NC];  // F_m at the nodes (the first interval reaches below T = 0, where the series still holds)
     for (int j = 0; j < NC; ++j) {
       const long double T = mid + 0.5L * width * cosl(pi * (j + 0.5L) / NC), ex = expl(-T);
       long double term = 1.0L / (2 * M + 1), sum = term;
-      for (int i = 1; i < 2000 && term > 1e-22L * sum; ++i) {
+      for (int i = 1; i < 2000 && fabsl(term) > 1e-22L * fabsl(sum); ++i) {
         term *= 2.0L * T / (2 * M + 2 * i + 1);
         sum += term;
       }
@@ -246,6 +246,7 @@ static std::vector<double> boys_poly_tables() {
       long double sc = 1.0L;
       for (int i = 0; i < NC; ++i, sc *= 2.0L / width)
         t[(size_t)m * BOYSP_SIZE + row * NC + i] = (double)(mono[i] * sc);
+      t[(size_t)m * BOYSP_SIZE + BOYSP_ROWS * NC + row] = (double)expl(-mid);
     }
   }
   return t;

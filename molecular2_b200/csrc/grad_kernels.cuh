@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad2e(const Grad2eParams P
   const int ns = P.nshell;
   const double* Dn = P.Dnorm;
   const double dab = Dn[a * ns + b];
-  const int n = pack_kets(start, end, S.list, &S.n, [&](int e) {
+  const int n = pack_kets(start, end, 0, S.list, &S.n, [&](int e) {
     const int kl = P.ket_ent.pair[e];
     if (!P.ket_sig[kl]) return false;
     const int c = P.ket.sa[kl], d = P.ket.sb[kl];
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad2e(const Grad2eParams P
   const int nb = P.bra_ent.np[eb];
   const double* __restrict__ Dc = P.Dc;
   const bool local = P.natom <= GRAD_ATOMS;
-  for (int i = tid; i < BOYSP_SIZE; i += GRAD_THREADS) S.boys[i] = __ldg(P.boysp + (size_t)(L + 1) * BOYSP_SIZE + i);
+  load_boys<L + 1>(S.boys, P.boysp);
   for (int i = tid; i < NAB; i += GRAD_THREADS) S.Dab[i] = Dc[(size_t)(a0 + i / NB) * nc + b0 + i % NB];
   if (local)
     for (int i = tid; i < 3 * P.natom; i += GRAD_THREADS) s_g[i] = 0.0;
@@ -164,13 +164,15 @@ __global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad2e(const Grad2eParams P
       for_terms<LA, LB>([&](auto ab, auto k, auto h) {
         G[decltype(h)::value] += w[decltype(ab)::value] * M[decltype(k)::value];
       });
+      KetPrim next = load_ket<true>(kp, 0);
       for (int k = 0; k < nkm; ++k) {
-        const int kk = min(k, nk - 1);
-        const double KK = k < nk && active ? Kb * entry_field(kp, kk, 4) : 0.0;
+        const KetPrim kq = next;  // the next primitive's loads run behind this one's arithmetic
+        const double ga = entry_field(kp, min(k, nk - 1), 6);
+        next = load_ket<true>(kp, min(k + 1, nk - 1));
+        const double KK = k < nk && active ? Kb * kq.K : 0.0;
         if (!__any_sync(0xffffffffu, fabs(KK) > JK_PRIM_EPS)) break;  // largest first: the rest is smaller
-        const double q = entry_field(kp, kk, 0);
-        const double Q[3] = {entry_field(kp, kk, 1), entry_field(kp, kk, 2), entry_field(kp, kk, 3)};
-        const double h2 = entry_field(kp, kk, 5), ga = entry_field(kp, kk, 6);
+        const double q = kq.q, h2 = kq.h;
+        const double Q[3] = {kq.x, kq.y, kq.z};
         double R[nherm(L + 1)];
         quartet_R<L + 1>(p, q, KK, Px - Q[0], Py - Q[1], Pz - Q[2], S.boys, R);
         double ex[3][LCD + 1], er[3][LCD + 1];

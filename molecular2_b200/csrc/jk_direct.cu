@@ -258,7 +258,7 @@ int build_pairs(jk_engine* e) {
 // products) is shared, but fewer for classes whose blocks would not fill the
 // GPU otherwise.
 static int ket_chunk(long long nbra, long long nket, int layers) {
-  int k = JK_LIST;
+  int k = 4 * JK_LIST;
   while (k > 32 && nbra * ((nket + k - 1) / k) * layers < (k > JK_THREADS ? 32 : 8) * 148) k /= 2;
   return k;
 }

@@ -58,7 +58,7 @@ struct JKParams {
   const double* boysp;  // polynomial Boys tables, BOYSP_SIZE doubles per order
   unsigned long long* counter;
   unsigned long long* work;  // NULL or this class pair's [quartets, sum bra primitive pairs, sum primitive quartets]
-  int kchunk;                // ket entries per block, at most JK_LIST
+  int kchunk;                // ket entries per block
   int bra0, bra_step;        // this rank's bra pairs: bra0, bra0 + bra_step, ...
 };
 
@@ -110,7 +110,7 @@ __host__ __device__ constexpr int jk_layers(int la, int lb, int lc, int ld) {
                                             : ncart(lc) * ncart(ld);
 }
 constexpr int JK_THREADS = 128;
-constexpr int JK_LIST = 1024;      // most ket entries of one block
+constexpr int JK_LIST = 1024;      // ket entries screened and packed at a time
 // primitive quartets whose prefactor is below this in every lane are skipped
 // (their integrals are below 1e-18, like the primitive pairs never listed)
 constexpr double JK_PRIM_EPS = 1e-21;
@@ -120,7 +120,7 @@ struct JKShared {
   double boys[BOYSP_SIZE];
   BraShared<LA, LB> bra;
   double Dab[2][ncart(LA) * ncart(LB)];
-  int list[JK_LIST];
+  int list[JK_LIST + JK_THREADS];
   int n;
 };
 template <int LA, int LB>
@@ -139,13 +139,13 @@ constexpr size_t jk_smem(int nden) {
 // src/fockbuild.cpp:266-362) are digested from the same integrals; the screen
 // uses the norms of their sum.
 // Measured (one thread per contracted quartet with its 6 to 81 integrals in
-// local memory -> this kernel): H2O/cc-pVDZ 18.0 -> 0.29 ms, (H2O)8/cc-pVDZ
-// 44.3 -> 5.0 ms, C20H42/6-311G** 262 -> 52 ms.  What bounds it now, on C20H42:
-// the L1 data path (40 to 73 % of its wavefronts, nine Boys coefficients and
-// five fields per primitive quartet, scattered density reads) and 5.6e9 FP64
-// atomics (107 of the 185 G/s that random addresses allow); the FP64 pipe is
-// at 20 to 33 %.  Entries of 16 primitives were slower (56 ms, and 0.66 ms on
-// H2O, whose longest chain they double).
+// local memory -> this kernel): H2O/cc-pVDZ 18.0 -> 0.26 ms, (H2O)8/cc-pVDZ
+// 44.3 -> 4.4 ms, C20H42/6-311G** 262 -> 44 ms.  Of that, 52 -> 44 ms came from
+// fewer instructions per primitive (Boys function, reciprocal square root), the
+// next primitive's loads issued ahead, and rounds of whole warps over the packed
+// list.  Tried and slower on C20H42: entries of 16 primitives (56 for 52 ms),
+// the bra's K rows summed in shared memory instead of by global atomics (54 for
+// 44 ms), one block per bra over all kets (55 for 50 ms).
 template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(JK_THREADS) k_jk_direct(const JKParams P) {
   constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD), NAB = NA * NB;
@@ -171,37 +171,14 @@ __global__ void __launch_bounds__(JK_THREADS) k_jk_direct(const JKParams P) {
   const int end = min(start + P.kchunk, nent);
   const int tid = threadIdx.x, lane = tid & 31;
 
-  // screen: max6(|D| blocks) Q_ab Q_cd >= precision
   unsigned long long cnt = 0, wb = 0, wq = 0;
   const int ns = P.nshell;
   const double* Dn = P.Dnorm;
   const double dab = Dn[a * ns + b];
   const bool count = blockIdx.z == 0 && P.bra_ent.first[bra] == eb;
-  const int n = pack_kets(start, end, S.list, &S.n, [&](int e) {
-    const int kl = P.ket_ent.pair[e];
-    const int c = P.ket.sa[kl], d = P.ket.sb[kl];
-    double dn = fmax(fmax(dab, Dn[c * ns + d]), fmax(Dn[a * ns + c], Dn[a * ns + d]));
-    dn = fmax(dn, fmax(Dn[b * ns + c], Dn[b * ns + d]));
-    const bool pass = !(dn * Qab * P.ket.Q[kl] < P.precision);
-    if (pass && count && P.ket_ent.first[kl] == e) {
-      const int bnp = P.bra.nprim[bra];
-      ++cnt;
-      wb += bnp;
-      wq += (unsigned long long)bnp * P.ket.nprim[kl];
-    }
-    return pass;
-  });
-  if (n == 0) return;
-
   const int a0 = P.sh.coff[a], b0 = P.sh.coff[b], nc = P.nc;
   const int nb = P.bra_ent.np[eb];
-  for (int i = tid; i < BOYSP_SIZE; i += JK_THREADS) S.boys[i] = __ldg(P.boysp + (size_t)L * BOYSP_SIZE + i);
-  for (int i = tid; i < P.nden * NAB; i += JK_THREADS)
-    S.Dab[i / NAB][i % NAB] =
-        P.Dc[(i / NAB) * P.dstride + (size_t)(a0 + (i % NAB) / NB) * nc + b0 + (i % NAB) % NB];
-  for (int i = 0; i < P.nden * NAB; ++i) s_jab[i * JK_THREADS + tid] = 0.0;
-  load_bra<LA, LB>(S.bra, entry_prims(P.bra_ent, eb), nb, P.sh.x[a], P.sh.y[a], P.sh.z[a], P.sh.x[b], P.sh.y[b],
-                   P.sh.z[b]);
+  bool ready = false;
 
   // this layer's ket component (block-uniform)
   int ic0 = 0, id0 = 0, cx = 0, cy = 0, cz = 0, dx = 0, dy = 0, dz = 0;
@@ -221,6 +198,40 @@ __global__ void __launch_bounds__(JK_THREADS) k_jk_direct(const JKParams P) {
     cz = c_herm.v[nherm(LC - 1) + ic0];
   }
 
+  int have = 0;  // survivors left over from the stretch before
+  for (int l0 = start; l0 < end; l0 += JK_LIST) {
+    // screen: max6(|D| blocks) Q_ab Q_cd >= precision
+    const int got = pack_kets(l0, min(l0 + JK_LIST, end), have, S.list, &S.n, [&](int e) {
+      const int kl = P.ket_ent.pair[e];
+      const int c = P.ket.sa[kl], d = P.ket.sb[kl];
+      double dn = fmax(fmax(dab, Dn[c * ns + d]), fmax(Dn[a * ns + c], Dn[a * ns + d]));
+      dn = fmax(dn, fmax(Dn[b * ns + c], Dn[b * ns + d]));
+      const bool pass = !(dn * Qab * P.ket.Q[kl] < P.precision);
+      if (pass && count && P.ket_ent.first[kl] == e) {
+        const int bnp = P.bra.nprim[bra];
+        ++cnt;
+        wb += bnp;
+        wq += (unsigned long long)bnp * P.ket.nprim[kl];
+      }
+      return pass;
+    });
+    // whole rounds of the block's threads; the rest waits for the next stretch
+    const int n = l0 + JK_LIST < end ? got / JK_THREADS * JK_THREADS : got;
+    if (n == 0) {
+      have = got;
+      __syncthreads();
+      continue;
+    }
+    if (!ready) {  // the bra's tables, once there are kets
+      ready = true;
+      load_boys<L>(S.boys, P.boysp);
+      for (int i = tid; i < P.nden * NAB; i += JK_THREADS)
+        S.Dab[i / NAB][i % NAB] =
+            P.Dc[(i / NAB) * P.dstride + (size_t)(a0 + (i % NAB) / NB) * nc + b0 + (i % NAB) % NB];
+      for (int i = 0; i < P.nden * NAB; ++i) s_jab[i * JK_THREADS + tid] = 0.0;
+      load_bra<LA, LB>(S.bra, entry_prims(P.bra_ent, eb), nb, P.sh.x[a], P.sh.y[a], P.sh.z[a], P.sh.x[b],
+                       P.sh.y[b], P.sh.z[b]);
+    }
   for (int t0 = (tid >> 5) * 32; t0 < n; t0 += JK_THREADS) {
     const bool active = t0 + lane < n;
     const int e = S.list[active ? t0 + lane : n - 1];
@@ -254,26 +265,27 @@ __global__ void __launch_bounds__(JK_THREADS) k_jk_direct(const JKParams P) {
       for (int g = 0; g < G; ++g)
 #pragma unroll
         for (int h = 0; h < HAB; ++h) W[g][h] = 0.0;
+      KetPrim next = load_ket<(LCD > 0)>(kp, 0);
       for (int k = 0; k < nkm; ++k) {
-        const int kk = min(k, nk - 1);
-        const double KK = k < nk ? Kb * entry_field(kp, kk, 4) : 0.0;
+        const KetPrim kq = next;  // the next primitive's loads run behind this one's arithmetic
+        next = load_ket<(LCD > 0)>(kp, min(k + 1, nk - 1));
+        const double KK = k < nk ? Kb * kq.K : 0.0;
         if (!__any_sync(0xffffffffu, fabs(KK) > JK_PRIM_EPS)) break;  // largest first: the rest is smaller
-        const double q = entry_field(kp, kk, 0);
-        const double Qx = entry_field(kp, kk, 1), Qy = entry_field(kp, kk, 2), Qz = entry_field(kp, kk, 3);
+        const double Qx = kq.x, Qy = kq.y, Qz = kq.z;
         double R[nherm(L)];
-        quartet_R<L>(p, q, KK, Px - Qx, Py - Qy, Pz - Qz, S.boys, R);
+        quartet_R<L>(p, kq.q, KK, Px - Qx, Py - Qy, Pz - Qz, S.boys, R);
         if constexpr (LCD == 0) {
 #pragma unroll
           for (int h = 0; h < HAB; ++h) W[0][h] += R[h];
         } else if constexpr (MODE == JK_FULL) {  // ps
-          const double h2 = entry_field(kp, kk, 5);
+          const double h2 = kq.h;
           const double QC[3] = {Qx - Cx, Qy - Cy, Qz - Cz};
           static_for<3 * HAB>([&](auto gh) {
             constexpr int g = decltype(gh)::value / HAB, h = decltype(gh)::value % HAB;
             W[g][h] += QC[g] * R[h] - h2 * R[hidx(herm_t(h) + (g == 0), herm_u(h) + (g == 1), herm_v(h) + (g == 2))];
           });
         } else {
-          const double h2 = entry_field(kp, kk, 5);
+          const double h2 = kq.h;
           double e1[3][LCD + 1];
           const double QC[3] = {Qx - Cx, Qy - Cy, Qz - Cz}, QD[3] = {Qx - Ex, Qy - Ey, Qz - Ez};
           const int ce[3] = {cx, cy, cz}, de[3] = {dx, dy, dz};
@@ -309,68 +321,80 @@ __global__ void __launch_bounds__(JK_THREADS) k_jk_direct(const JKParams P) {
       for (int g = 0; g < G; ++g) bra_transform<LA, LB, G>(S.bra.M[LAB > 0 ? ib : 0], W[g], v + g);
     }
     // digestion: 6 updates per integral (src/fockbuild.cpp:121-153)
-    const int c0 = P.sh.coff[c] + ic0, d0 = P.sh.coff[d] + id0;
+    if (active) {
+      const int c0 = P.sh.coff[c] + ic0, d0 = P.sh.coff[d] + id0;
 #pragma unroll 1
-    for (int dd = 0; dd < P.nden; ++dd) {
-      const double* __restrict__ Dc = P.Dc + dd * P.dstride;
-      double* __restrict__ Jd = P.Jc + dd * P.dstride;
-      double* __restrict__ Kd = P.Kc + dd * P.dstride;
-      double* jab = s_jab + (size_t)dd * NAB * JK_THREADS + tid;
-      const double* Dab = S.Dab[dd];
-      double Dcd[G];
+      for (int dd = 0; dd < P.nden; ++dd) {
+        const double* __restrict__ Dc = P.Dc + dd * P.dstride;
+        const double* __restrict__ Dra = Dc + (size_t)a0 * nc;  // the bra's rows
+        const double* __restrict__ Drb = Dc + (size_t)b0 * nc;
+        double* __restrict__ Jd = P.Jc + dd * P.dstride;
+        double* __restrict__ Kra = P.Kc + dd * P.dstride + (size_t)a0 * nc;
+        double* __restrict__ Krb = P.Kc + dd * P.dstride + (size_t)b0 * nc;
+        double* jab = s_jab + (size_t)dd * NAB * JK_THREADS + tid;
+        const double* Dab = S.Dab[dd];
+        double Dcd[G];
 #pragma unroll
-      for (int g = 0; g < G; ++g) Dcd[g] = Dc[(size_t)(c0 + g / GD) * nc + d0 + g % GD];
+        for (int g = 0; g < G; ++g) Dcd[g] = __ldg(Dc + (size_t)(c0 + g / GD) * nc + d0 + g % GD);
 #pragma unroll
-      for (int i = 0; i < NAB; ++i) {
-        double s = 0.0;
+        for (int i = 0; i < NAB; ++i) {
+          double s = 0.0;
 #pragma unroll
-        for (int g = 0; g < G; ++g) s += Dcd[g] * v[i * G + g];
-        jab[i * JK_THREADS] += s;
-      }
+          for (int g = 0; g < G; ++g) s += Dcd[g] * v[i * G + g];
+          jab[i * JK_THREADS] += s;
+        }
 #pragma unroll
-      for (int g = 0; g < G; ++g) {
-        double s = 0.0;
+        for (int g = 0; g < G; ++g) {
+          double s = 0.0;
 #pragma unroll
-        for (int i = 0; i < NAB; ++i) s += Dab[i] * v[i * G + g];
-        atomic_add_f64(Jd + (size_t)(c0 + g / GD) * nc + d0 + g % GD, s);
-      }
-      // K_ac, K_bc from D_bd, D_ad; K_ad, K_bd from D_bc, D_ac
+          for (int i = 0; i < NAB; ++i) s += Dab[i] * v[i * G + g];
+          atomicAdd(Jd + (size_t)(c0 + g / GD) * nc + d0 + g % GD, s);
+        }
+        // K_ac, K_bc from D_bd, D_ad; K_ad, K_bd from D_bc, D_ac
 #pragma unroll
-      for (int side = 0; side < 2; ++side) {
-        const int r0 = side ? d0 : c0, q0 = side ? c0 : d0;
-        constexpr int GX[2] = {GC, GD};
-        const int nr = GX[side], nq = GX[1 - side];
+        for (int side = 0; side < 2; ++side) {
+          const int r0 = side ? d0 : c0, q0 = side ? c0 : d0;
+          constexpr int GX[2] = {GC, GD};
+          const int nr = GX[side], nq = GX[1 - side];
 #pragma unroll
-        for (int r = 0; r < nr; ++r) {
-          double ka[NA], kb[NB];
+          for (int r = 0; r < nr; ++r) {
+            double ka[NA], kb[NB];
 #pragma unroll
-          for (int i = 0; i < NA; ++i) ka[i] = 0.0;
+            for (int i = 0; i < NA; ++i) ka[i] = 0.0;
 #pragma unroll
-          for (int j = 0; j < NB; ++j) kb[j] = 0.0;
+            for (int j = 0; j < NB; ++j) kb[j] = 0.0;
 #pragma unroll
-          for (int q = 0; q < nq; ++q) {
-            const int g = side ? q * GD + r : r * GD + q;
-            double Da[NA], Db[NB];
+            for (int q = 0; q < nq; ++q) {
+              const int g = side ? q * GD + r : r * GD + q;
+              double Da[NA], Db[NB];
 #pragma unroll
-            for (int i = 0; i < NA; ++i) Da[i] = Dc[(size_t)(a0 + i) * nc + q0 + q];
+              for (int i = 0; i < NA; ++i) Da[i] = __ldg(Dra + i * nc + q0 + q);
 #pragma unroll
-            for (int j = 0; j < NB; ++j) Db[j] = Dc[(size_t)(b0 + j) * nc + q0 + q];
+              for (int j = 0; j < NB; ++j) Db[j] = __ldg(Drb + j * nc + q0 + q);
 #pragma unroll
-            for (int i = 0; i < NA; ++i)
+              for (int i = 0; i < NA; ++i)
 #pragma unroll
-              for (int j = 0; j < NB; ++j) {
-                ka[i] += Db[j] * v[(i * NB + j) * G + g];
-                kb[j] += Da[i] * v[(i * NB + j) * G + g];
-              }
+                for (int j = 0; j < NB; ++j) {
+                  ka[i] += Db[j] * v[(i * NB + j) * G + g];
+                  kb[j] += Da[i] * v[(i * NB + j) * G + g];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < NA; ++i) atomicAdd(Kra + i * nc + r0 + r, ka[i]);
+#pragma unroll
+            for (int j = 0; j < NB; ++j) atomicAdd(Krb + j * nc + r0 + r, kb[j]);
           }
-#pragma unroll
-          for (int i = 0; i < NA; ++i) atomic_add_f64(Kd + (size_t)(a0 + i) * nc + r0 + r, ka[i]);
-#pragma unroll
-          for (int j = 0; j < NB; ++j) atomic_add_f64(Kd + (size_t)(b0 + j) * nc + r0 + r, kb[j]);
         }
       }
     }
+    }
+    __syncthreads();  // every warp is through with the list
+    have = got - n;
+    const int keep = tid < have ? S.list[n + tid] : 0;
+    __syncthreads();
+    if (tid < have) S.list[tid] = keep;
   }
+  if (!ready) return;
   __syncthreads();
   // J_ab: one warp per component
   for (int i = tid >> 5; i < P.nden * NAB; i += JK_THREADS / 32) {
@@ -449,7 +473,7 @@ __global__ void __launch_bounds__(SCHWARZ_THREADS, 2) k_schwarz(const SchwarzPar
   const double A[3] = {P.sh.x[a], P.sh.y[a], P.sh.z[a]}, B[3] = {P.sh.x[b], P.sh.y[b], P.sh.z[b]};
   const int pa = P.pure[a], pb = P.pure[b];
   const int ma = pa ? 2 * LA + 1 : NA, mb = pb ? 2 * LB + 1 : NB, nf = ma * mb;
-  for (int i = tid; i < BOYSP_SIZE; i += SCHWARZ_THREADS) S.boys[i] = __ldg(P.boysp + (size_t)L2 * BOYSP_SIZE + i);
+  load_boys<L2>(S.boys, P.boysp);
   for (int i = tid; i < nf; i += SCHWARZ_THREADS) S.diag[i] = 0.0;
 
   auto load = [&](int side, int k0, int n) {

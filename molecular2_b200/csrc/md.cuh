@@ -8,9 +8,7 @@
 //   R^{(n)}_{t+1,u,v} = t R^{(n+1)}_{t-1,u,v} + X_PQ R^{(n+1)}_{t,u,v}
 // (McMurchie & Davidson, J. Comput. Phys. 26, 218 (1978); Helgaker,
 // Jorgensen & Olsen, "Molecular Electronic-Structure Theory" ch. 9).
-// The Boys function is a polynomial per interval at the highest order needed,
-// then downward recursion F_m = (2T F_{m+1} + e^{-T})/(2m+1); for T >= 36 the
-// asymptotic F_0 = sqrt(pi/T)/2 and upward recursion (both in quartet.cuh).
+// (Boys function and R recursion: quartet.cuh.)
 //
 // Index conventions: a Cartesian component (a,b,c) of total l sits at
 // cidx = (l-a)(l-a+1)/2 + c (libint2 order x^l, x^{l-1}y, ...); Hermite
@@ -21,8 +19,6 @@
 #include <cstdint>
 
 namespace m2 {
-
-constexpr double BOYS_TMAX = 36.0;  // the asymptotic form from here on
 
 __host__ __device__ constexpr int ncart(int l) { return (l + 1) * (l + 2) / 2; }
 __host__ __device__ constexpr int nherm(int L) { return (L + 1) * (L + 2) * (L + 3) / 6; }

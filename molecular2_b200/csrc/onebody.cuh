@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(OB_THREADS) k_onebody(const OneBodyParams P) {
   const double* base = entry_prims(P.ent, e);
   const bool with_v = P.V != nullptr;
   if (with_v)
-    for (int i = tid; i < BOYSP_SIZE; i += OB_THREADS) S.boys[i] = __ldg(P.boysp + (size_t)L * BOYSP_SIZE + i);
+    load_boys<L>(S.boys, P.boysp);
   for (int i = tid; i < nb * 3; i += OB_THREADS) {
     const int x = i % 3;
     const double X = entry_field(base, i / 3, 1 + x);
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(OB_THREADS) k_grad1e(const Grad1eParams P) {
   const int tid = threadIdx.x, lane = tid & 31;
   const bool local = P.natom <= G1_ATOMS;
   double* g_atom = local ? s_g : P.grad;
-  for (int i = tid; i < BOYSP_SIZE; i += OB_THREADS) S.boys[i] = __ldg(P.boysp + (size_t)(L + 1) * BOYSP_SIZE + i);
+  load_boys<L + 1>(S.boys, P.boysp);
   if (local)
     for (int i = tid; i < 3 * P.natom; i += OB_THREADS) s_g[i] = 0.0;
   for (int e = blockIdx.x; e < P.ent.nent; e += gridDim.x) {

@@ -59,12 +59,31 @@ __device__ __forceinline__ double entry_field(const double* base, int k, int f) 
   return __ldg(base + (k * ENTRY_FIELDS + f) * 32);
 }
 
-// Ket entries e in [start, end) with pass(e), packed into list; returns their
-// number.  All threads of the block call this (n_shared: a shared counter).
+// One primitive of a ket entry.
+struct KetPrim {
+  double q, x, y, z, K, h;
+};
+template <bool H>
+__device__ __forceinline__ KetPrim load_ket(const double* base, int k) {
+  const double* b = base + k * (ENTRY_FIELDS * 32);
+  KetPrim r;
+  r.K = __ldg(b + 4 * 32);
+  r.q = __ldg(b);
+  r.x = __ldg(b + 32);
+  r.y = __ldg(b + 2 * 32);
+  r.z = __ldg(b + 3 * 32);
+  r.h = H ? __ldg(b + 5 * 32) : 0.0;
+  return r;
+}
+
+// Appends the ket entries e in [start, end) with pass(e) to the `have` entries of
+// list; returns the new number.  All threads of the block call this (n_shared: a
+// shared counter); a barrier must lie between the last use of list or n_shared
+// and the call.
 template <class Pass>
-__device__ __forceinline__ int pack_kets(int start, int end, int* list, int* n_shared, Pass&& pass) {
+__device__ __forceinline__ int pack_kets(int start, int end, int have, int* list, int* n_shared, Pass&& pass) {
   const int lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) *n_shared = 0;
+  if (threadIdx.x == 0) *n_shared = have;
   __syncthreads();
   for (int e0 = start; e0 < end; e0 += blockDim.x) {
     const int e = e0 + threadIdx.x;
@@ -80,40 +99,81 @@ __device__ __forceinline__ int pack_kets(int start, int end, int* list, int* n_s
 }
 
 // ---------------------------------------------------------------- Boys
-// F_M by a degree-8 polynomial on BOYSP_ROWS intervals of [0, 36), table of
-// one order (BOYSP_ROWS x BOYSP_COEF, ascending powers of T - centre) in shared
-// memory: nine conflict-light 8-byte reads against the seven L1 gathers over a
-// 121 KB table of the Taylor form, and small enough (6.9 KB) to stage per
-// block.  Interpolation at Chebyshev nodes: error below 2e-16 of F_M.
-constexpr int BOYSP_ROWS = 96;
+// F_M by a degree-8 polynomial in T - centre on intervals of width 3/8 centred
+// on its multiples, up to T = 36 + 3M; e^{-T} from a table at the centres times
+// a degree-9 polynomial; then downward recursion
+// F_m = (2T F_{m+1} + e^{-T})/(2m+1).  From 36 + 3M on, F_M is its leading
+// asymptotic term (what that drops is below 2e-16 of F_M) and e^{-T} is nothing.
+// The table of one order (9 coefficients a row and e^{-centre}) is staged in
+// shared memory: ten 8-byte reads with few bank conflicts, against seven L1
+// gathers and a call of exp for a Taylor table.  A kernel with exp() in both
+// branches of the asymptotic test and the library's rsqrt ran 280 instructions
+// per (ps|ss) primitive quartet, 85 of them FP64.  Both polynomials interpolate
+// at Chebyshev nodes: errors below 2e-16 of F_M and 4e-17 of e^{-T}.
+constexpr double BOYSP_WIDTH = 0.375;
 constexpr int BOYSP_COEF = 9;
 constexpr int BOYSP_MMAX = 9;   // orders 0..9
-constexpr int BOYSP_SIZE = BOYSP_ROWS * BOYSP_COEF;
+constexpr double boysp_tmax(int m) { return 36.0 + 3.0 * m; }
+constexpr int boysp_rows(int m) { return (int)(boysp_tmax(m) / BOYSP_WIDTH + 0.5) + 1; }
+constexpr int BOYSP_ROWS = boysp_rows(BOYSP_MMAX);
+constexpr int BOYSP_SIZE = BOYSP_ROWS * (BOYSP_COEF + 1);  // polynomials, then e^{-centre}
+
+// The table of order M to shared memory; a barrier must follow.
+template <int M>
+__device__ __forceinline__ void load_boys(double* dst, const double* __restrict__ all) {
+  const double* src = all + (size_t)M * BOYSP_SIZE;
+  for (int i = threadIdx.x; i < boysp_rows(M) * BOYSP_COEF; i += blockDim.x) dst[i] = __ldg(src + i);
+  if constexpr (M > 0)
+    for (int i = threadIdx.x; i < boysp_rows(M); i += blockDim.x)
+      dst[BOYSP_ROWS * BOYSP_COEF + i] = __ldg(src + BOYSP_ROWS * BOYSP_COEF + i);
+}
+
+// x^{-1/2} for x well inside the range of float: the single-precision estimate
+// and one step of third order (relative error e -> 5/16 e^3, e < 2^-21).
+__device__ __forceinline__ double rsqrt_pos(double x) {
+  const double y = (double)rsqrtf((float)x);
+  const double h = 1.0 - x * y * y;
+  return y + y * h * (0.5 + 0.375 * h);
+}
 
 template <int M>
 __device__ __forceinline__ void boys_poly(double T, const double* tab, double* F) {
   static_assert(M <= BOYSP_MMAX, "Boys order too high");
-  if (T < BOYS_TMAX) {
-    const int row = (int)(T * (BOYSP_ROWS / BOYS_TMAX));
-    const double d = T - (row + 0.5) * (BOYS_TMAX / BOYSP_ROWS);
+  double e = 0.0;
+  if (T < boysp_tmax(M)) {
+    // nearest multiple of the width, by the rounding of an addition to 1.5 2^52
+    const double u = T * (1.0 / BOYSP_WIDTH) + 6755399441055744.0;
+    const int row = __double2loint(u);
+    const double d = T - (u - 6755399441055744.0) * BOYSP_WIDTH;
     const double* c = tab + row * BOYSP_COEF;
     double acc = c[BOYSP_COEF - 1];
 #pragma unroll
     for (int j = BOYSP_COEF - 2; j >= 0; --j) acc = acc * d + c[j];
     F[M] = acc;
     if constexpr (M > 0) {
-      const double e = exp(-T), T2 = 2.0 * T;
-#pragma unroll
-      for (int m = M - 1; m >= 0; --m) F[m] = (T2 * F[m + 1] + e) * (1.0 / (2 * m + 1));
+      double x = -2.7579345743837904673e-6;  // e^{-d}, |d| <= 3/16
+      x = x * d + 2.4825818086831339934e-5;
+      x = x * d - 1.9841263064743021626e-4;
+      x = x * d + 1.3888881434054876645e-3;
+      x = x * d - 8.3333333341842252384e-3;
+      x = x * d + 4.1666666676027388464e-2;
+      x = x * d - 1.6666666666666292731e-1;
+      x = x * d + 0.49999999999995886287;
+      x = x * d - 1.0;
+      x = x * d + 1.0;
+      e = x * tab[BOYSP_ROWS * BOYSP_COEF + row];
     }
   } else {
-    const double r = rsqrt(T);
-    F[0] = 0.886226925452758014 * r;  // sqrt(pi)/2 / sqrt(T)
-    if constexpr (M > 0) {
-      const double e = exp(-T), it = 0.5 * r * r;
+    const double r = rsqrt_pos(T), r2 = r * r;
+    double f = 0.886226925452758014 * r;  // Gamma(M + 1/2)/2 T^{-M-1/2}
 #pragma unroll
-      for (int m = 0; m < M; ++m) F[m + 1] = ((2 * m + 1) * F[m] - e) * it;
-    }
+    for (int m = 0; m < M; ++m) f *= (m + 0.5) * r2;
+    F[M] = f;
+  }
+  if constexpr (M > 0) {
+    const double T2 = 2.0 * T;
+#pragma unroll
+    for (int m = M - 1; m >= 0; --m) F[m] = (T2 * F[m + 1] + e) * (1.0 / (2 * m + 1));
   }
 }
 
@@ -157,7 +217,7 @@ __device__ __forceinline__ void hermite_R(double a, double scale, double X, doub
 template <int L>
 __device__ __forceinline__ void quartet_R(double p, double q, double KK, double X, double Y, double Z,
                                           const double* tab, double* R) {
-  const double r = rsqrt(p + q);
+  const double r = rsqrt_pos(p + q);
   hermite_R<L>(p * q * r * r, KK * r, X, Y, Z, tab, R);
 }
 
