@@ -232,6 +232,13 @@ int df_jk_device(jk_engine* e, const double* dC, int nocc, int mode, double* dJ,
 cudaError_t df_syrk_X(jk_engine* e, const double* X, int n, long long len, double* K, cudaStream_t s);
 int one_body_device(jk_engine* e, double* S, double* T, double* V, cudaStream_t s);
 void stage_mark(jk_engine* e, int k, cudaStream_t s);
+// eig.cu, 2 <= n <= SMALL_EIG_MAX: eigenvectors (columns, ascending) and
+// eigenvalues of a symmetric n x n matrix, with scratch of small_eig_scratch(n)
+// bytes; Rayleigh quotients of orthonormal columns
+constexpr int SMALL_EIG_MAX = 160;
+size_t small_eig_scratch(int n);
+cudaError_t small_eig(const double* A, double* vecs, double* vals, int n, void* scratch, cudaStream_t s);
+cudaError_t rayleigh(const double* A, const double* vecs, double* vals, int n, cudaStream_t s);
 // df_mixed.cu
 int df_mixed_device(jk_engine* e, const double* dC, int nocc, double* dJ, double* dK, cudaStream_t s);
 int df_mixed_error(jk_engine* e);

@@ -286,6 +286,12 @@ int scf_rhf(jk_engine* e, const jk_scf_options* o, jk_scf_result* r) {
   } jguard{jinfo};
   if ((st = work.alloc(std::max(std::max(lwork, lwork_j), 1))) != cudaSuccess)
     return check_cuda(e, st, "eigensolver workspace");
+  // one block's shared memory holds the matrix up to SMALL_EIG_MAX, and up to there
+  // eig.cu's solver is the faster one (figures there)
+  const bool small = n >= 2 && n <= SMALL_EIG_MAX;
+  DevBuf<unsigned char> eig_work;
+  if (small && (st = eig_work.alloc(small_eig_scratch(n))) != cudaSuccess)
+    return check_cuda(e, st, "eigensolver scratch");
   auto syev = [&](const double* A, double* vecs, double* vals) -> bool {
     g.copy(A, vecs, nn);
     return cusolverDnDsyevd(e->cusolver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, n, vecs, n, vals, work.p,
@@ -410,6 +416,16 @@ int scf_rhf(jk_engine* e, const jk_scf_options* o, jk_scf_result* r) {
         g.mm(false, false, W.p, Wt.p, t1.p);
         g.copy(t1.p, W.p, nn);
       }
+    } else if (small && ndrop == 0 && have_W) {
+      // In the previous eigenvectors the Fock matrix is nearly diagonal, so the
+      // Jacobi sweeps are few.  (Dropped directions' raised diagonal would set the
+      // scale of Jacobi's stopping rule.)  The vectors are products of products:
+      // one Newton-Schulz step W <- W (3 - W^T W) / 2 keeps them orthonormal to
+      // eps, and Rayleigh quotients take the transform's rounding off eps.
+      ok = g.mm(false, false, Fm.p, W.p, t1.p) && g.mm(true, false, W.p, t1.p, Wt.p) &&
+           small_eig(Wt.p, t1.p, eps.p, n, eig_work.p, s) == cudaSuccess && g.mm(false, false, W.p, t1.p, Wt.p) &&
+           g.mm(true, false, Wt.p, Wt.p, t1.p) && g.copy(Wt.p, W.p, nn) &&
+           g.mm(false, false, Wt.p, t1.p, W.p, -0.5, 1.5) && rayleigh(Fm.p, W.p, eps.p, n, s) == cudaSuccess;
     } else {
       ok = syev(Fm.p, W.p, eps.p);
     }
