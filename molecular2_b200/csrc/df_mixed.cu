@@ -296,7 +296,13 @@ __global__ void __launch_bounds__(G1_THREADS, 1)
 // last row) run N = 128.
 struct G2Params {
   int n;
-  int kblocks;      // (naux*NP)/64
+  // The inner index in 16-wide MMA steps: X holds `steps` per fitted function,
+  // while splits and accumulation groups are counted as if it held `gsteps` (>=
+  // steps, the rest zero), so that a row length without padding sums in the same
+  // groups as one with it (120 orbitals in rows of 160 before, 128 now: 1.86 ->
+  // 1.36 ms at n = 984, the same bits).
+  int steps, gsteps, ksteps;  // ksteps: steps in all
+  int kblocks;      // 64-wide blocks of the counted index
   int ntile_n;      // ceil(n/128)
   int nblocks;      // lower-triangle 128 x 256 blocks
   int splits;
@@ -313,6 +319,12 @@ constexpr int G2_EPI = 2;                            // epilogue warps per TMEM 
 constexpr int G2_THREADS = 64 + 4 * 32 * G2_EPI;     // TMA warp, MMA warp, epilogue warps
 constexpr int G2_COLS = G2_BN / G2_EPI;              // accumulator columns per epilogue warp
 static_assert(G2_SMEM <= SMEM_LIMIT, "GEMM2 ring exceeds shared memory");
+
+// counted step -> held step
+__device__ __forceinline__ int g2_held(int s, const G2Params& P) {
+  if (P.steps != P.gsteps) s = s / P.gsteps * P.steps + min(s % P.gsteps, P.steps);
+  return min(s, P.ksteps);
+}
 
 __host__ __device__ inline int g2_block_count(int nt) {
   int c = 0;
@@ -371,14 +383,17 @@ __global__ void __launch_bounds__(G2_THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const bool have_work = kb1 > kb0;
+  constexpr int SPB = BK / 16;  // steps per 64-wide block
+  const int s0 = SPB * kb0, s1 = SPB * kb1;
+  const int h0 = g2_held(s0, P), h1 = g2_held(s1, P);
+  const bool have_work = h1 > h0;
 
   if (warp == 0) {
     if (lane == 0 && have_work) {
       int last_s = -1;
       uint32_t last_par = 0;
       const uint32_t bytes = wide ? G2_STAGE : 4 * TILE_A_BYTES;
-      for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
+      for (int kb = h0 / SPB, it = 0; kb * SPB < h1; ++kb, ++it) {
         const int s = it % G2_STAGES;
         const uint32_t j = it / G2_STAGES;
         if (!mbar_wait(&empty[s], (j & 1) ^ 1)) {
@@ -406,7 +421,9 @@ __global__ void __launch_bounds__(G2_THREADS, 1)
       const uint32_t idesc = wide ? idesc_bf16_f32(BM, G2_BN) : idesc_bf16_f32(BM, BM);
       bool ok = true;
       int it = 0, gt = 0;
-      for (int kg = kb0; kg < kb1 && ok; kg += ACC_GROUP, ++gt) {
+      for (int sg = s0; sg < s1 && ok; sg += SPB * ACC_GROUP) {
+        const int ha = g2_held(sg, P), hz = g2_held(min(sg + SPB * ACC_GROUP, s1), P);
+        if (ha == hz) continue;  // only padding
         const int b = gt & 1;
         if (!mbar_wait(&tempty[b], ((gt >> 1) & 1) ^ 1)) {
           report(P.err, ERR_WAIT_MMA);
@@ -414,30 +431,32 @@ __global__ void __launch_bounds__(G2_THREADS, 1)
         }
         tc_fence_after();
         const uint32_t d = tmem + b * G2_BN;
-        const int kend = min(kg + ACC_GROUP, kb1);
-        for (int kb = kg; kb < kend; ++kb, ++it) {
-          const int s = it % G2_STAGES;
-          const uint32_t j = it / G2_STAGES;
-          if (!mbar_wait(&full[s], j & 1)) {
-            report(P.err, ERR_WAIT_MMA);
-            ok = false;
-            break;
+        for (int h = ha; h < hz; ++h) {
+          const int s = it % G2_STAGES, k = h % SPB;
+          if (k == 0 || h == h0) {
+            const uint32_t j = it / G2_STAGES;
+            if (!mbar_wait(&full[s], j & 1)) {
+              report(P.err, ERR_WAIT_MMA);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
           }
-          tc_fence_after();
           const uint8_t* st = smem + s * G2_STAGE;
-#pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t ah = sdesc_kmajor_sw128(st + k * 32);
-            const uint64_t al = sdesc_kmajor_sw128(st + TILE_A_BYTES + k * 32);
-            const uint64_t bh = sdesc_kmajor_sw128(st + 2 * TILE_A_BYTES + k * 32);
-            const uint64_t bl = sdesc_kmajor_sw128(st + 4 * TILE_A_BYTES + k * 32);
-            umma_bf16(d, ah, bh, idesc, (kb > kg || k > 0) ? 1u : 0u);
-            umma_bf16(d, ah, bl, idesc, 1u);
-            umma_bf16(d, al, bh, idesc, 1u);
+          const uint64_t ah = sdesc_kmajor_sw128(st + k * 32);
+          const uint64_t al = sdesc_kmajor_sw128(st + TILE_A_BYTES + k * 32);
+          const uint64_t bh = sdesc_kmajor_sw128(st + 2 * TILE_A_BYTES + k * 32);
+          const uint64_t bl = sdesc_kmajor_sw128(st + 4 * TILE_A_BYTES + k * 32);
+          umma_bf16(d, ah, bh, idesc, h > ha ? 1u : 0u);
+          umma_bf16(d, ah, bl, idesc, 1u);
+          umma_bf16(d, al, bh, idesc, 1u);
+          if (k == SPB - 1 || h == h1 - 1) {
+            umma_commit(&empty[s]);
+            ++it;
           }
-          umma_commit(&empty[s]);
         }
         if (ok) umma_commit(&tfull[b]);
+        ++gt;
       }
       umma_commit(drain);
       mbar_wait(drain, 0);
@@ -449,7 +468,9 @@ __global__ void __launch_bounds__(G2_THREADS, 1)
 #pragma unroll
     for (int e = 0; e < G2_COLS; ++e) acc[e] = 0.0f;
     bool ok = true;
-    for (int kg = kb0, gt = 0; kg < kb1; kg += ACC_GROUP, ++gt) {
+    int gt = 0;
+    for (int sg = s0; sg < s1; sg += SPB * ACC_GROUP) {
+      if (g2_held(sg, P) == g2_held(min(sg + SPB * ACC_GROUP, s1), P)) continue;
       const int b = gt & 1;
       if (!mbar_wait(&tfull[b], (gt >> 1) & 1)) {
         report(P.err, ERR_WAIT_EPILOGUE);
@@ -470,6 +491,7 @@ __global__ void __launch_bounds__(G2_THREADS, 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[b]);
+      ++gt;
     }
     const int x = tx * BM + 32 * q + lane;
     if (ok && x < P.n && (part == 0 || wide)) {
@@ -707,7 +729,7 @@ int df_mixed_device(jk_engine* e, const double* dC, int nocc, double* dJ, double
   cudaError_t st = dispatch_g1(NP, m.maps, P1, std::min(nsm, P1.ntiles), s);
   if (st != cudaSuccess) return check_cuda(e, st, "gemm1 launch");
   stage_mark(e, 1, s);
-  st = launch_gemm2(m.maps[4], m.maps[5], n, (naux * NP) / BK, m.Kt.p, m.err.p, nsm, s);
+  st = launch_gemm2(m.maps[4], m.maps[5], n, naux, NP / 16, NP / 16, m.Kt.p, m.err.p, nsm, s);
   if (st != cudaSuccess) return check_cuda(e, st, "gemm2 launch");
   stage_mark(e, 2, s);
   const int kchunk = (naux + 15) / 16;   // 16 K ranges per row x
@@ -771,11 +793,15 @@ cudaError_t launch_split_C(int n, int nocc, int NP, int ld, const double* C, __n
 // Kt (+)= X X^T over the lower-triangle 128 x 256 blocks of the n rows of X
 // (tensor maps tXh, tXl over rows of `kblocks` * 64 BF16, boxes of 64 x 128),
 // split-K over the SMs.
-cudaError_t launch_gemm2(const CUtensorMap& tXh, const CUtensorMap& tXl, int n, int kblocks, double* Kt, int* err,
-                         int nsm, cudaStream_t s) {
+cudaError_t launch_gemm2(const CUtensorMap& tXh, const CUtensorMap& tXl, int n, int w, int steps, int gsteps, double* Kt,
+                         int* err, int nsm, cudaStream_t s) {
+  const int kblocks = (int)(((long long)w * gsteps + BK / 16 - 1) / (BK / 16));
   G2Params P2{};
   P2.n = n;
   P2.kblocks = kblocks;
+  P2.steps = steps;
+  P2.gsteps = gsteps;
+  P2.ksteps = w * steps;
   P2.ntile_n = (n + BM - 1) / BM;
   P2.nblocks = g2_block_count(P2.ntile_n);
   // splits so that the CTA count is close to a whole number of waves

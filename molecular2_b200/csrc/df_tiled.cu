@@ -12,13 +12,13 @@
 // FP64 DMMA GEMM, then the BF16 split; the FP64 B is never stored whole.
 //
 // Mixed build (prec_mode 1), per block of fitted functions:
-//   GEMM1  X_K[x][i] = sum_y B_K[x][y] C[y][i]: one work item = (K, row tile
-//          I, half of the occupied orbitals); its k loop runs over the row
-//          of tiles, reading tile (I, J) as stored (K-major A) for J <= I and
-//          tile (J, I) transposed (MN-major A descriptor, same bytes) for
-//          J > I.  TMA -> 3-stage ring -> tcgen05.mma (M = 128, N = 160) ->
-//          double-buffered TMEM; the epilogue writes X as BF16 hi/lo and adds
-//          gamma_K = sum_{x,i} X C.
+//   GEMM1  X_K[x][i] = sum_y B_K[x][y] C[y][i]: one work item = (two K, or one
+//          above 128 orbitals, row tile I, a share of the occupied orbitals);
+//          its k loop runs over the row of tiles, reading tile (I, J) as stored
+//          (K-major A) for J <= I and tile (J, I) transposed (MN-major A
+//          descriptor, same bytes) for J > I.  TMA ring -> tcgen05.mma (M = 128,
+//          N = the share) -> double-buffered TMEM; the epilogue writes X as
+//          BF16 hi/lo and adds gamma_K = sum_{x,i} X C.
 //   GEMM2  K += X X^T over the block (the tcgen05 kernel of df_mixed.cu).
 // then J = sum_K gamma_K B_K over the stored tiles (HBM stream) and K, J are
 // assembled from their lower triangles.
@@ -79,7 +79,7 @@ __host__ __device__ __forceinline__ void tile_of(int t, int& I, int& J) {
 struct S1Params {
   int nt, npt;       // tile rows, stored tile pairs
   int k0, wstride;   // first fitted function of the block; X row stride in K
-  int nhalf, nitems;
+  int nhalf, nitems, nk;  // nk: fitted functions of the block
   int nocc, n, NPX;
   const float* Cx;   // [x][i] npad x NPX, C in FP32 (zero padded)
   __nv_bfloat16* Xh;  // [x][K_local][NPX]
@@ -103,6 +103,30 @@ __device__ __forceinline__ void s1_item(const S1Params& P, int item, int& Kl, in
 // buffers the MMA warp runs at most two groups ahead of the epilogue, so a
 // group must outlast the epilogue's per-item work (gamma, split, stores).
 constexpr int S1_GROUP = 8;
+
+// One row's 16 NC values as BF16 hi and lo, whole 32-byte sectors per store;
+// returns the sum of the lo parts' squares.
+template <int NC>
+__device__ __forceinline__ float store_split(const float* v, __nv_bfloat16* hi, __nv_bfloat16* lo) {
+  float lsq = 0.0f;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    uint32_t hh[8], ll[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float f0 = v[c * 16 + 2 * e], f1 = v[c * 16 + 2 * e + 1];
+      const __nv_bfloat162 h = __floats2bfloat162_rn(f0, f1);
+      const __nv_bfloat162 l = __floats2bfloat162_rn(f0 - __low2float(h), f1 - __high2float(h));
+      hh[e] = reinterpret_cast<const uint32_t&>(h);
+      ll[e] = reinterpret_cast<const uint32_t&>(l);
+      lsq = fmaf(__low2float(l), __low2float(l), lsq);
+      lsq = fmaf(__high2float(l), __high2float(l), lsq);
+    }
+    st_global_32(hi + c * 16, hh);
+    st_global_32(lo + c * 16, ll);
+  }
+  return lsq;
+}
 
 // One epilogue warp's share of a work item: TMEM columns [16*C0, 16*C1) of its
 // 32 rows summed over the item's accumulation groups (global group counter gt,
@@ -133,37 +157,21 @@ __device__ __forceinline__ bool s1_epilogue_item(uint32_t tbase, int& gt, int ng
     if (lane == 0) mbar_arrive(&tempty[b]);
   }
   const int i0 = h * SN + C0 * 16;
+  double gk = 0.0;
   if (x < P.n) {  // gamma_K += sum_i X[x][K][i] C[x][i], the row of C as 16-byte vectors
     const float4* c4 = reinterpret_cast<const float4*>(P.Cx + (size_t)x * P.NPX + i0);
-    double g4[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
     for (int i = 0; i < NV / 4; ++i) {
       const float4 c = __ldg(c4 + i);
-      g4[0] += (double)v[4 * i] * c.x;
-      g4[1] += (double)v[4 * i + 1] * c.y;
-      g4[2] += (double)v[4 * i + 2] * c.z;
-      g4[3] += (double)v[4 * i + 3] * c.w;
+      gk += ((double)v[4 * i] * c.x + (double)v[4 * i + 1] * c.y) +
+            ((double)v[4 * i + 2] * c.z + (double)v[4 * i + 3] * c.w);
     }
-    atomicAdd(P.gamma + P.k0 + Kl, (g4[0] + g4[1]) + (g4[2] + g4[3]));
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) gk += __shfl_xor_sync(0xffffffffu, gk, o);
+  if (lane == 0) atomicAdd(P.gamma + P.k0 + Kl, gk);  // 32 lanes' adds to one address went one by one
   const size_t row = ((size_t)x * P.wstride + Kl) * P.NPX + i0;
-  uint4* oh = reinterpret_cast<uint4*>(P.Xh + row);
-  uint4* ol = reinterpret_cast<uint4*>(P.Xl + row);
-  float lsq = 0.0f;
-#pragma unroll
-  for (int c = 0; c < NV / 8; ++c) {
-    __align__(16) __nv_bfloat16 hh[8], ll[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float f = v[c * 8 + e];
-      hh[e] = __float2bfloat16_rn(f);
-      ll[e] = __float2bfloat16_rn(f - __bfloat162float(hh[e]));
-      const float lf = __bfloat162float(ll[e]);
-      lsq = fmaf(lf, lf, lsq);
-    }
-    oh[c] = *reinterpret_cast<const uint4*>(hh);
-    ol[c] = *reinterpret_cast<const uint4*>(ll);
-  }
+  const float lsq = store_split<NV / 16>(v, P.Xh + row, P.Xl + row);
   // the lo*lo term GEMM2 drops is sum_k lo_k^2 > 0 on the diagonal of K
   if (x < P.n) atomicAdd(P.Kt + (size_t)x * P.n + x, (double)lsq);
   return true;
@@ -333,6 +341,305 @@ __global__ void __launch_bounds__(S1_THREADS, 1)
     tc_fence_after();
     tmem_dealloc(tmem, 2 * S1_ACC);
   }
+}
+
+// GEMM1 for up to 128 occupied orbitals per work item (N = 16 NCH): an item is
+// TWO fitted functions, (K, K + 1, I, h), whose tiles meet the same columns of C,
+// so each chunk of C is loaded once for both.  Both kernels are bound by what
+// they pull through L2 (8.0 TB/s at n = 656, tensor pipe at 36 to 42 %):
+// k_gemm1_sym 40 KB of C beside each 32 KB of B, this one (32 + 2 NCH) KB per
+// function and chunk.  It also spends no MMA columns on padding to 160, writes X
+// in whole sectors and adds gamma once per warp (32 lanes of one address before:
+// one by one).  n = 984, 120 orbitals, 3600 functions: 4.0 ms -> 3.0 ms (1.3 ms
+// to read B from HBM once); whole build 7.3 -> 5.5 ms, n = 369 with 35 orbitals
+// 0.57 -> 0.30 ms.
+//
+// One ring of 32 KB slots, filled in the order C chunk, B chunk of K, B chunk of
+// K + 1; the C slot is released with the last B chunk.  7 slots: 224 KB.
+// Accumulators: 2 buffers x 2 functions x 128 TMEM columns.
+constexpr int SP_SLOT = 2 * S1_A;
+constexpr int SP_SLOTS = 7;
+constexpr int SP_SMEM = SP_SLOTS * SP_SLOT + 1024 + 1024;
+constexpr int SP_ACC = 128;
+constexpr int SP_EPI = 4;          // epilogue warps per TMEM lane quadrant, a quarter of the columns each
+constexpr int SP_THREADS = 64 + 4 * 32 * SP_EPI;
+constexpr int SP_MAXCH = SP_ACC / 16;
+static_assert(SP_SMEM <= 227 * 1024, "paired GEMM1 ring exceeds shared memory");
+static_assert(SP_MAXCH * 16 * SBK * 2 * 2 <= SP_SLOT, "a C chunk fills one slot at most");
+
+template <int C0, int C1>
+__device__ __forceinline__ bool sp_epilogue_item(uint32_t tbase, int& gt, int ngroups, int nk, int x, int Kl, int i0,
+                                                 const S1Params& P, uint64_t* tfull, uint64_t* tempty, int lane) {
+  constexpr int NC = C1 - C0, NV = NC > 0 ? NC * 16 : 1;
+  float v[2][NV];
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[k][i] = 0.0f;
+  for (int g = 0; g < ngroups; ++g, ++gt) {
+    const int b = gt & 1;
+    if (!mbar_wait(&tfull[b], (gt >> 1) & 1)) return false;
+    tc_fence_after();
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (k < nk) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          float w[16];
+          tmem_ld16(tbase + (2 * b + k) * SP_ACC + (C0 + c) * 16, w);
+          tmem_ld_wait();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) v[k][c * 16 + e] += w[e];
+        }
+      }
+    }
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&tempty[b]);
+  }
+  if (NC <= 0) return true;
+  double g[2] = {0.0, 0.0};
+  if (x < P.n) {  // gamma_K += sum_i X[x][K][i] C[x][i]
+    const float4* c4 = reinterpret_cast<const float4*>(P.Cx + (size_t)x * P.NPX + i0 + C0 * 16);
+#pragma unroll
+    for (int i = 0; i < NC * 4; ++i) {
+      const float4 c = __ldg(c4 + i);
+#pragma unroll
+      for (int k = 0; k < 2; ++k)
+        g[k] += ((double)v[k][4 * i] * c.x + (double)v[k][4 * i + 1] * c.y) +
+                ((double)v[k][4 * i + 2] * c.z + (double)v[k][4 * i + 3] * c.w);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    g[0] += __shfl_xor_sync(0xffffffffu, g[0], o);
+    g[1] += __shfl_xor_sync(0xffffffffu, g[1], o);
+  }
+  if (lane < nk) atomicAdd(P.gamma + P.k0 + Kl + lane, lane == 0 ? g[0] : g[1]);
+  double lsq = 0.0;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    if (k >= nk) break;
+    const size_t row = ((size_t)x * P.wstride + Kl + k) * P.NPX + i0 + C0 * 16;
+    lsq += (double)store_split<NC>(v[k], P.Xh + row, P.Xl + row);
+  }
+  // the lo*lo term GEMM2 drops is sum_k lo_k^2 > 0 on the diagonal of K
+  if (x < P.n) atomicAdd(P.Kt + (size_t)x * P.n + x, lsq);
+  return true;
+}
+
+template <int NCH>
+__global__ void __launch_bounds__(SP_THREADS, 1)
+    k_gemm1_pair(const __grid_constant__ CUtensorMap tBhK, const __grid_constant__ CUtensorMap tBlK,
+                 const __grid_constant__ CUtensorMap tBhM, const __grid_constant__ CUtensorMap tBlM,
+                 const __grid_constant__ CUtensorMap tCh, const __grid_constant__ CUtensorMap tCl, const S1Params P) {
+  constexpr int S = SP_SLOTS, N = 16 * NCH, C_BYTES = N * SBK * 2;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = (uint64_t*)(smem + S * SP_SLOT);
+  uint64_t* empty = full + S;
+  uint64_t* tfull = empty + S;
+  uint64_t* tempty = tfull + 2;
+  uint64_t* drain = tempty + 2;
+  uint32_t* tmem_slot = (uint32_t*)(drain + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kchunks = 2 * P.nt;  // 64-wide k chunks per work item
+  const int npairs = (P.nk + 1) / 2;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tfull[b], 1);
+      mbar_init(&tempty[b], 4 * SP_EPI);
+    }
+    mbar_init(drain, 1);
+    fence_barrier_init();
+    prefetch_tmap(&tBhK);
+    prefetch_tmap(&tBlK);
+    prefetch_tmap(&tBhM);
+    prefetch_tmap(&tBlM);
+    prefetch_tmap(&tCh);
+    prefetch_tmap(&tCl);
+  }
+  if (warp == 0) tmem_alloc(tmem_slot, 4 * SP_ACC);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const int nitems = npairs * P.nt * P.nhalf;
+
+  if (warp == 0) {
+    if (lane == 0) {  // TMA producer
+      int it = 0;
+      bool ok = true;
+      auto slot = [&](uint32_t bytes) -> uint8_t* {
+        const int s = it % S;
+        if (!mbar_wait(&empty[s], ((it / S) & 1) ^ 1)) {
+          report(P.err, ERR_WAIT_PRODUCER);
+          ok = false;
+          return nullptr;
+        }
+        mbar_arrive_expect_tx(&full[s], bytes);
+        return smem + s * SP_SLOT;
+      };
+      for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+        int kp, I, h;
+        s1_item(P, item, kp, I, h);
+        const int nk = min(2, P.nk - 2 * kp);
+        for (int q = 0; q < kchunks && ok; ++q) {
+          const int J = q >> 1, cc = q & 1;
+          uint8_t* st = slot(2 * C_BYTES);
+          if (!ok) break;
+          const int ycol = TB * J + SBK * cc;
+          tma_load_2d(st, &tCh, ycol, h * N, &full[it % S]);
+          tma_load_2d(st + C_BYTES, &tCl, ycol, h * N, &full[it % S]);
+          ++it;
+          for (int k = 0; k < nk; ++k, ++it) {
+            st = slot(SP_SLOT);
+            if (!ok) break;
+            const long long K = P.k0 + 2 * kp + k;
+            uint64_t* bar = &full[it % S];
+            if (J <= I) {  // stored tile (I, J): rows x of I, columns y of J
+              const int row = (int)((K * P.npt + I * (I + 1) / 2 + J) * TB);
+              tma_load_2d(st, &tBhK, SBK * cc, row, bar);
+              tma_load_2d(st + S1_A, &tBlK, SBK * cc, row, bar);
+            } else {       // stored tile (J, I): rows y of J (k), columns x of I (m)
+              const int row = (int)((K * P.npt + J * (J + 1) / 2 + I) * TB) + SBK * cc;
+              tma_load_2d(st, &tBhM, 0, row, bar);
+              tma_load_2d(st + S1_A / 2, &tBhM, SBK, row, bar);
+              tma_load_2d(st + S1_A, &tBlM, 0, row, bar);
+              tma_load_2d(st + S1_A + S1_A / 2, &tBlM, SBK, row, bar);
+            }
+          }
+        }
+      }
+      for (int j = max(0, it - S); j < it; ++j) mbar_wait(&full[j % S], (j / S) & 1);  // no copy in flight at exit
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {  // MMA issuer
+      constexpr uint32_t idk = idesc_bf16_f32(TB, N);
+      constexpr uint32_t idm = idesc_bf16_f32_amn(TB, N);
+      int it = 0, gt = 0;
+      bool ok = true;
+      auto ready = [&](int j) {
+        if (!mbar_wait(&full[j % S], (j / S) & 1)) {
+          report(P.err, ERR_WAIT_MMA);
+          ok = false;
+        }
+        tc_fence_after();
+      };
+      for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
+        int kp, I, h;
+        s1_item(P, item, kp, I, h);
+        const int nk = min(2, P.nk - 2 * kp);
+        for (int qg = 0; qg < kchunks && ok; qg += S1_GROUP, ++gt) {
+          const int b = gt & 1;
+          if (!mbar_wait(&tempty[b], ((gt >> 1) & 1) ^ 1)) {
+            report(P.err, ERR_WAIT_MMA);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const int qend = min(qg + S1_GROUP, kchunks);
+          for (int q = qg; q < qend && ok; ++q) {
+            const bool mn = (q >> 1) > I;
+            const uint32_t id = mn ? idm : idk;
+            const int cslot = it % S;
+            ready(it);
+            if (!ok) break;
+            const uint8_t* sc = smem + cslot * SP_SLOT;
+            ++it;
+            for (int k = 0; k < nk; ++k, ++it) {
+              ready(it);
+              if (!ok) break;
+              const uint8_t* st = smem + (it % S) * SP_SLOT;
+              const uint32_t d = tmem + (2 * b + k) * SP_ACC;
+#pragma unroll
+              for (int kk = 0; kk < SBK / 16; ++kk) {
+                uint64_t ah, al;
+                if (!mn) {
+                  ah = sdesc_kmajor_sw128(st + kk * 32);
+                  al = sdesc_kmajor_sw128(st + S1_A + kk * 32);
+                } else {
+                  ah = sdesc_mnmajor_sw128(st + kk * 2048, S1_A / 2, 1024);
+                  al = sdesc_mnmajor_sw128(st + S1_A + kk * 2048, S1_A / 2, 1024);
+                }
+                const uint64_t bh = sdesc_kmajor_sw128(sc + kk * 32);
+                const uint64_t bl = sdesc_kmajor_sw128(sc + C_BYTES + kk * 32);
+                umma_bf16(d, ah, bh, id, (q > qg || kk > 0) ? 1u : 0u);
+                umma_bf16(d, ah, bl, id, 1u);
+                umma_bf16(d, al, bh, id, 1u);
+              }
+              umma_commit(&empty[it % S]);
+            }
+            if (ok) umma_commit(&empty[cslot]);
+          }
+          if (ok) umma_commit(&tfull[b]);
+        }
+      }
+      umma_commit(drain);  // every issued MMA has finished before TMEM is freed
+      mbar_wait(drain, 0);
+    }
+  } else {  // epilogue: warp w drains TMEM lanes 32*(w%4).. and column chunks of quarter (w-2)/4
+    const int qd = warp & 3, part = (warp - 2) >> 2;
+    const int ngroups = (kchunks + S1_GROUP - 1) / S1_GROUP;
+    const uint32_t tbase = tmem + ((uint32_t)(32 * qd) << 16);
+    int gt = 0;
+    for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
+      int kp, I, h;
+      s1_item(P, item, kp, I, h);
+      const int nk = min(2, P.nk - 2 * kp), x = TB * I + 32 * qd + lane, i0 = h * N, Kl = 2 * kp;
+      bool ok;
+      if (part == 0)
+        ok = sp_epilogue_item<0, NCH / 4>(tbase, gt, ngroups, nk, x, Kl, i0, P, tfull, tempty, lane);
+      else if (part == 1)
+        ok = sp_epilogue_item<NCH / 4, NCH / 2>(tbase, gt, ngroups, nk, x, Kl, i0, P, tfull, tempty, lane);
+      else if (part == 2)
+        ok = sp_epilogue_item<NCH / 2, 3 * NCH / 4>(tbase, gt, ngroups, nk, x, Kl, i0, P, tfull, tempty, lane);
+      else
+        ok = sp_epilogue_item<3 * NCH / 4, NCH>(tbase, gt, ngroups, nk, x, Kl, i0, P, tfull, tempty, lane);
+      if (!ok) {
+        report(P.err, ERR_WAIT_EPILOGUE);
+        break;
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 4 * SP_ACC);
+  }
+}
+
+template <int NCH>
+cudaError_t launch_pair(const CUtensorMap* m, const S1Params& P, int nsm, cudaStream_t s) {
+  cudaError_t st = cudaFuncSetAttribute(k_gemm1_pair<NCH>, cudaFuncAttributeMaxDynamicSharedMemorySize, SP_SMEM);
+  if (st != cudaSuccess) return st;
+  const int items = (P.nk + 1) / 2 * P.nt * P.nhalf;
+  k_gemm1_pair<NCH><<<std::min(nsm, items), SP_THREADS, SP_SMEM, s>>>(m[0], m[1], m[2], m[3], m[4], m[5], P);
+  return cudaGetLastError();
+}
+
+// GEMM1 for sn columns per work item
+cudaError_t launch_gemm1(int sn, const CUtensorMap* m, const S1Params& P, int nsm, cudaStream_t s) {
+  switch (sn / 16) {
+    case 1: return launch_pair<1>(m, P, nsm, s);
+    case 2: return launch_pair<2>(m, P, nsm, s);
+    case 3: return launch_pair<3>(m, P, nsm, s);
+    case 4: return launch_pair<4>(m, P, nsm, s);
+    case 5: return launch_pair<5>(m, P, nsm, s);
+    case 6: return launch_pair<6>(m, P, nsm, s);
+    case 7: return launch_pair<7>(m, P, nsm, s);
+    case 8: return launch_pair<8>(m, P, nsm, s);
+  }
+  cudaError_t st = cudaFuncSetAttribute(k_gemm1_sym, cudaFuncAttributeMaxDynamicSharedMemorySize, S1_SMEM);
+  if (st != cudaSuccess) return st;
+  k_gemm1_sym<<<std::min(nsm, P.nitems), S1_THREADS, S1_SMEM, s>>>(m[0], m[1], m[2], m[3], m[4], m[5], P);
+  return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------- J over the stored tiles
@@ -576,23 +883,38 @@ int df_tiled_setup(jk_engine* e) {
   return JK_OK;
 }
 
+// Occupied orbitals are dealt to GEMM1 work items in the least number of equal
+// parts of at most SN; X rows hold the parts side by side.  A share of up to 128
+// goes to k_gemm1_pair in whole MMA column chunks, a larger one to k_gemm1_sym at
+// SN: two functions' accumulators of it would not fit twice in TMEM, and two
+// parts of k_gemm1_pair read the tiles twice (150 orbitals, whole build: n = 656
+// 2.98 ms against 3.27, n = 820 4.78 against 5.49).
+static int occ_parts(int nocc) { return (nocc + SN - 1) / SN; }
+static int occ_per_item(int nocc) {
+  const int p = occ_parts(nocc), share = ((nocc + p - 1) / p + 15) / 16 * 16;
+  return share <= 16 * SP_MAXCH ? share : SN;
+}
+static int occ_columns(int nocc) { return occ_parts(nocc) * occ_per_item(nocc); }
+
 // Scratch of the mixed build, sized for the largest occupied count seen so far
 // (a smaller count reuses it with tensor maps for its own row length, so the
 // varying column counts of incremental builds allocate nothing).
 static int tiled_mixed_prepare(jk_engine* e, int nocc) {
   TiledDF& T = e->tiled;
   const int naux = e->aux.n_final, n = e->obs.n_final;
-  const int nhalf = (nocc + SN - 1) / SN;
-  const int NPX = nhalf * SN;
+  const int NPX = occ_columns(nocc);
+  // scratch is held for whole parts of SN columns: the varying counts of an
+  // incremental build stay within one allocation
+  const int cap = occ_parts(nocc) * SN;
   cudaError_t st;
-  if (!T.Xh.p || NPX > T.NPX_cap) {
+  if (!T.Xh.p || cap > T.NPX_cap) {
     T.Ch.reset();
     T.Cl.reset();
     T.Xh.reset();
     T.Xl.reset();
-    st = T.Ch.alloc((size_t)NPX * T.npad);
-    if (st == cudaSuccess) st = T.Cx.alloc((size_t)NPX * T.npad);
-    if (st == cudaSuccess) st = T.Cl.alloc((size_t)NPX * T.npad);
+    st = T.Ch.alloc((size_t)cap * T.npad);
+    if (st == cudaSuccess) st = T.Cx.alloc((size_t)cap * T.npad);
+    if (st == cudaSuccess) st = T.Cl.alloc((size_t)cap * T.npad);
     if (st == cudaSuccess) st = T.Kt.alloc((size_t)n * n);
     if (st == cudaSuccess) st = T.err.alloc(1);
     if (st == cudaSuccess) st = e->df.gamma.alloc(naux);
@@ -600,16 +922,14 @@ static int tiled_mixed_prepare(jk_engine* e, int nocc) {
     // X block: as many fitted functions as fit in a quarter of the free memory (at most all)
     size_t fr = 0, tt = 0;
     dev_mem_info(&fr, &tt);
-    const double per_k = 4.0 * T.npad * NPX;  // hi + lo BF16
+    const double per_k = 4.0 * T.npad * cap;  // hi + lo BF16
     int w = (int)std::min<double>(naux, std::max(64.0, 0.25 * fr / per_k));
     if (T.waux_max > 0) w = std::min(w, T.waux_max);
     w = std::max(1, std::min(naux, w));
-    // X rows are padded to an even number of fitted functions, so that a row
-    // is a whole number of 64-wide k blocks (NPX is a multiple of 160)
     for (;; w = w / 2) {
       const int ws = w + (w & 1);
-      st = T.Xh.alloc((size_t)T.npad * ws * NPX);
-      if (st == cudaSuccess) st = T.Xl.alloc((size_t)T.npad * ws * NPX);
+      st = T.Xh.alloc((size_t)T.npad * ws * cap);
+      if (st == cudaSuccess) st = T.Xl.alloc((size_t)T.npad * ws * cap);
       if (st == cudaSuccess) break;
       T.Xh.reset();
       T.Xl.reset();
@@ -618,7 +938,7 @@ static int tiled_mixed_prepare(jk_engine* e, int nocc) {
     }
     T.waux = w;
     T.wstride = w + (w & 1);
-    T.NPX_cap = NPX;
+    T.NPX_cap = cap;
     T.NPX = 0;
     cudaMemsetAsync(T.err.p, 0, sizeof(int), e->stream);
     const uint64_t brows = (uint64_t)naux * T.npt * TB;
@@ -627,7 +947,8 @@ static int tiled_mixed_prepare(jk_engine* e, int nocc) {
     if (!ok) return set_error(e, JK_ERR_CUDA, "cuTensorMapEncodeTiled failed (tiled DF)");
   }
   if (T.NPX != NPX) {
-    const bool ok = make_map(&T.maps[4], T.Ch.p, T.npad, NPX, SBK, SN) && make_map(&T.maps[5], T.Cl.p, T.npad, NPX, SBK, SN) &&
+    const bool ok = make_map(&T.maps[4], T.Ch.p, T.npad, NPX, SBK, occ_per_item(nocc)) &&
+                    make_map(&T.maps[5], T.Cl.p, T.npad, NPX, SBK, occ_per_item(nocc)) &&
                     make_map(&T.maps[6], T.Xh.p, (uint64_t)T.wstride * NPX, T.npad, SBK, TB) &&
                     make_map(&T.maps[7], T.Xl.p, (uint64_t)T.wstride * NPX, T.npad, SBK, TB);
     if (!ok) return set_error(e, JK_ERR_CUDA, "cuTensorMapEncodeTiled failed (tiled DF)");
@@ -652,8 +973,6 @@ static int tiled_mixed(jk_engine* e, const double* dC, int nocc, double* dJ, dou
   cudaMemsetAsync(d.gamma.p, 0, sizeof(double) * naux, s);
   cudaMemsetAsync(T.Kt.p, 0, sizeof(double) * n * n, s);
   cudaMemsetAsync(dJ, 0, sizeof(double) * n * n, s);
-  st = cudaFuncSetAttribute(k_gemm1_sym, cudaFuncAttributeMaxDynamicSharedMemorySize, S1_SMEM);
-  if (st != cudaSuccess) return check_cuda(e, st, "gemm1 attribute");
   const int nblocks = (naux + T.waux - 1) / T.waux;
   e->kev_blocks = 0;
   auto kmark = [&](size_t k) {
@@ -674,7 +993,8 @@ static int tiled_mixed(jk_engine* e, const double* dC, int nocc, double* dJ, dou
     P.npt = T.npt;
     P.k0 = k0;
     P.wstride = T.wstride;
-    P.nhalf = T.NPX / SN;
+    P.nk = w;
+    P.nhalf = occ_parts(nocc);
     P.nitems = w * T.nt * P.nhalf;
     P.nocc = nocc;
     P.n = n;
@@ -685,22 +1005,10 @@ static int tiled_mixed(jk_engine* e, const double* dC, int nocc, double* dJ, dou
     P.gamma = d.gamma.p;
     P.Kt = T.Kt.p;
     P.err = T.err.p;
-    k_gemm1_sym<<<std::min(nsm, P.nitems), S1_THREADS, S1_SMEM, s>>>(T.maps[0], T.maps[1], T.maps[2], T.maps[3],
-                                                                       T.maps[4], T.maps[5], P);
-    st = cudaGetLastError();
+    st = launch_gemm1(occ_per_item(nocc), T.maps, P, nsm, s);
     if (st != cudaSuccess) return check_cuda(e, st, "gemm1 (tiled) launch");
     kmark(3 * blk + 1);
-    // GEMM2 reads whole 64-wide k blocks: when w * NPX is not a multiple of
-    // 64 (odd w with an odd number of 160-orbital halves) the tail of each X
-    // row holds the previous block's values, so clear it
-    const int kbl = (w * T.NPX + SBK - 1) / SBK;
-    if (kbl * SBK != w * T.NPX) {
-      const size_t pitch = (size_t)T.wstride * T.NPX * sizeof(__nv_bfloat16);
-      const size_t off = (size_t)w * T.NPX, width = (size_t)kbl * SBK - off;
-      cudaMemset2DAsync(T.Xh.p + off, pitch, 0, width * sizeof(__nv_bfloat16), T.npad, s);
-      cudaMemset2DAsync(T.Xl.p + off, pitch, 0, width * sizeof(__nv_bfloat16), T.npad, s);
-    }
-    st = launch_gemm2(T.maps[6], T.maps[7], n, kbl, T.Kt.p, T.err.p, nsm, s);
+    st = launch_gemm2(T.maps[6], T.maps[7], n, w, T.NPX / 16, occ_parts(nocc) * SN / 16, T.Kt.p, T.err.p, nsm, s);
     if (st != cudaSuccess) return check_cuda(e, st, "gemm2 (tiled) launch");
     kmark(3 * blk + 2);
   }

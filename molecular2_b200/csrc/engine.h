@@ -133,7 +133,7 @@ struct TiledDF {
   DevBuf<int> plist;                 // pair indices (into the class lists) touching each tile pair
   DevBuf<__nv_bfloat16> Bh, Bl;      // [K][t][r][c]
   // mixed-build scratch
-  int NPX = 0, waux = 0, nocc = 0;   // X row length per K (nhalf * 160), aux block, occupied count
+  int NPX = 0, waux = 0, nocc = 0;   // X row length per K (multiple of 16), aux block, occupied count
   int wstride = 0;                   // X row stride in fitted functions (waux rounded up to even)
   int NPX_cap = 0;                   // NPX the mixed scratch was allocated for
   int waux_max = 0, oc_max = 0;      // caps on the aux block and the FP64 occupied slice (0: memory decides)
@@ -248,8 +248,8 @@ bool make_map(CUtensorMap* m, const void* base, uint64_t cols, uint64_t rows, ui
 cudaError_t launch_rows_C(int n, int nocc, int NP, int nrow, const double* C, float* Cx, cudaStream_t s);
 cudaError_t launch_split_C(int n, int nocc, int NP, int ld, const double* C, __nv_bfloat16* Ch, __nv_bfloat16* Cl,
                            cudaStream_t s);
-cudaError_t launch_gemm2(const CUtensorMap& tXh, const CUtensorMap& tXl, int n, int kblocks, double* Kt, int* err,
-                         int nsm, cudaStream_t s);
+cudaError_t launch_gemm2(const CUtensorMap& tXh, const CUtensorMap& tXl, int n, int w, int steps, int gsteps, double* Kt,
+                         int* err, int nsm, cudaStream_t s);
 cudaError_t launch_finalize_mixed(int n, const double* Kt, double* J, double* K, cudaStream_t s);
 // df_tiled.cu
 int df_tiled_setup(jk_engine* e);

@@ -110,6 +110,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// 32 bytes to a 32-byte aligned address: whole L2 sectors per lane.
+__device__ __forceinline__ void st_global_32(void* p, const uint32_t (&v)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+               "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, rows of 128 B,
 // 8-row core groups 1024 B apart (SBO), sm_100 descriptor version 1.
 __device__ __forceinline__ uint64_t sdesc_kmajor_sw128(const void* smem) {
