@@ -73,6 +73,41 @@ struct G1Layout {
 constexpr int G1_GROUP = 4;
 constexpr int ACC_GROUP = 4;
 
+// gamma, X and the diagonal lo*lo sum of one row's columns [16*C0, 16*C1).
+// GEMM1 is bound by HBM (n = 384, naux = 1856: 1.3 GB in 0.198 ms, 6.6 TB/s), so X
+// leaves in whole 32-byte sectors; 16-byte pieces took 0.218 ms (n = 528 with 150
+// orbitals: the build 1.75 -> 1.59 ms).
+template <int NP, int C0, int C1>
+__device__ __forceinline__ void g1_finish(const float* v, int m, const G1Params& P, int lane) {
+  constexpr int NV = (C1 - C0) * 16;
+  if (m >= P.M) return;
+  const int x = m / P.naux, K = m - x * P.naux;
+  // gamma_K += sum_i X[x][K][i] C[x][i]: the row of C as 16-byte vectors
+  const float4* c4 = reinterpret_cast<const float4*>(P.Cx + (size_t)x * NP + C0 * 16);
+  double g4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int i = 0; i < NV / 4; ++i) {
+    const float4 c = __ldg(c4 + i);
+    g4[0] += (double)v[4 * i] * c.x;
+    g4[1] += (double)v[4 * i + 1] * c.y;
+    g4[2] += (double)v[4 * i + 2] * c.z;
+    g4[3] += (double)v[4 * i + 3] * c.w;
+  }
+  atomicAdd(P.gamma + K, (g4[0] + g4[1]) + (g4[2] + g4[3]));
+  const float lsq = store_split<C1 - C0>(v, P.Xhi + (size_t)m * NP + C0 * 16, P.Xlo + (size_t)m * NP + C0 * 16);
+  // GEMM2 forms hi*hi + hi*lo + lo*hi; the dropped lo*lo term averages out off
+  // the diagonal but is sum_k lo_k^2 > 0 on it, so it is added here (one
+  // atomic per warp when the warp's rows share x, as all but boundary rows do)
+  double lq = (double)lsq;
+  const unsigned mask = __activemask();
+  if (mask == 0xffffffffu && __all_sync(mask, x == __shfl_sync(mask, x, 0))) {
+    for (int o = 16; o > 0; o >>= 1) lq += __shfl_xor_sync(mask, lq, o);
+    if (lane == 0) atomicAdd(P.Kt + (size_t)x * P.n + x, lq);
+  } else {
+    atomicAdd(P.Kt + (size_t)x * P.n + x, lq);
+  }
+}
+
 // One epilogue warp's share of a GEMM1 tile: TMEM columns [16*C0, 16*C1) of
 // its 32 rows, summed over the tile's `ngroups` accumulation groups (global
 // group counter gt, buffer gt & 1).  Each buffer is released as soon as its
@@ -103,48 +138,7 @@ __device__ __forceinline__ bool g1_epilogue_tile(uint32_t tbase, int& gt, int ng
     __syncwarp();
     if (lane == 0) mbar_arrive(&tempty[b]);
   }
-  if (NV == 0 || m >= P.M) return true;
-  const int x = m / P.naux, K = m - x * P.naux;
-  // gamma_K += sum_i X[x][K][i] C[x][i]: the row of C as 16-byte vectors
-  const float4* c4 = reinterpret_cast<const float4*>(P.Cx + (size_t)x * NP + C0 * 16);
-  double g4[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
-  for (int i = 0; i < NV / 4; ++i) {
-    const float4 c = __ldg(c4 + i);
-    g4[0] += (double)v[4 * i] * c.x;
-    g4[1] += (double)v[4 * i + 1] * c.y;
-    g4[2] += (double)v[4 * i + 2] * c.z;
-    g4[3] += (double)v[4 * i + 3] * c.w;
-  }
-  atomicAdd(P.gamma + K, (g4[0] + g4[1]) + (g4[2] + g4[3]));
-  uint4* oh = reinterpret_cast<uint4*>(P.Xhi + (size_t)m * NP + C0 * 16);
-  uint4* ol = reinterpret_cast<uint4*>(P.Xlo + (size_t)m * NP + C0 * 16);
-  float lsq = 0.0f;
-#pragma unroll
-  for (int c = 0; c < NV / 8; ++c) {
-    __align__(16) __nv_bfloat16 h[8], l[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float f = v[c * 8 + e];
-      h[e] = __float2bfloat16_rn(f);
-      l[e] = __float2bfloat16_rn(f - __bfloat162float(h[e]));
-      const float lf = __bfloat162float(l[e]);
-      lsq = fmaf(lf, lf, lsq);
-    }
-    oh[c] = *reinterpret_cast<const uint4*>(h);
-    ol[c] = *reinterpret_cast<const uint4*>(l);
-  }
-  // GEMM2 forms hi*hi + hi*lo + lo*hi; the dropped lo*lo term averages out off
-  // the diagonal but is sum_k lo_k^2 > 0 on it, so it is added here (one
-  // atomic per warp when the warp's rows share x, as all but boundary rows do)
-  double lq = (double)lsq;
-  const unsigned mask = __activemask();
-  if (mask == 0xffffffffu && __all_sync(mask, x == __shfl_sync(mask, x, 0))) {
-    for (int o = 16; o > 0; o >>= 1) lq += __shfl_xor_sync(mask, lq, o);
-    if (lane == 0) atomicAdd(P.Kt + (size_t)x * P.n + x, lq);
-  } else {
-    atomicAdd(P.Kt + (size_t)x * P.n + x, lq);
-  }
+  if constexpr (NV > 0) g1_finish<NP, C0, C1>(v, m, P, lane);
   return true;
 }
 

@@ -104,30 +104,6 @@ __device__ __forceinline__ void s1_item(const S1Params& P, int item, int& Kl, in
 // group must outlast the epilogue's per-item work (gamma, split, stores).
 constexpr int S1_GROUP = 8;
 
-// One row's 16 NC values as BF16 hi and lo, whole 32-byte sectors per store;
-// returns the sum of the lo parts' squares.
-template <int NC>
-__device__ __forceinline__ float store_split(const float* v, __nv_bfloat16* hi, __nv_bfloat16* lo) {
-  float lsq = 0.0f;
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    uint32_t hh[8], ll[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float f0 = v[c * 16 + 2 * e], f1 = v[c * 16 + 2 * e + 1];
-      const __nv_bfloat162 h = __floats2bfloat162_rn(f0, f1);
-      const __nv_bfloat162 l = __floats2bfloat162_rn(f0 - __low2float(h), f1 - __high2float(h));
-      hh[e] = reinterpret_cast<const uint32_t&>(h);
-      ll[e] = reinterpret_cast<const uint32_t&>(l);
-      lsq = fmaf(__low2float(l), __low2float(l), lsq);
-      lsq = fmaf(__high2float(l), __high2float(l), lsq);
-    }
-    st_global_32(hi + c * 16, hh);
-    st_global_32(lo + c * 16, ll);
-  }
-  return lsq;
-}
-
 // One epilogue warp's share of a work item: TMEM columns [16*C0, 16*C1) of its
 // 32 rows summed over the item's accumulation groups (global group counter gt,
 // buffer gt & 1, each released as soon as it is in registers), then added to

@@ -117,6 +117,30 @@ __device__ __forceinline__ void st_global_32(void* p, const uint32_t (&v)[8]) {
                : "memory");
 }
 
+// One row's 16 NC values as BF16 hi and lo, whole 32-byte sectors per store;
+// returns the sum of the lo parts' squares.
+template <int NC>
+__device__ __forceinline__ float store_split(const float* v, __nv_bfloat16* hi, __nv_bfloat16* lo) {
+  float lsq = 0.0f;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    uint32_t hh[8], ll[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float f0 = v[c * 16 + 2 * e], f1 = v[c * 16 + 2 * e + 1];
+      const __nv_bfloat162 h = __floats2bfloat162_rn(f0, f1);
+      const __nv_bfloat162 l = __floats2bfloat162_rn(f0 - __low2float(h), f1 - __high2float(h));
+      hh[e] = reinterpret_cast<const uint32_t&>(h);
+      ll[e] = reinterpret_cast<const uint32_t&>(l);
+      lsq = fmaf(__low2float(l), __low2float(l), lsq);
+      lsq = fmaf(__high2float(l), __high2float(l), lsq);
+    }
+    st_global_32(hi + c * 16, hh);
+    st_global_32(lo + c * 16, ll);
+  }
+  return lsq;
+}
+
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, rows of 128 B,
 // 8-row core groups 1024 B apart (SBO), sm_100 descriptor version 1.
 __device__ __forceinline__ uint64_t sdesc_kmajor_sw128(const void* smem) {
