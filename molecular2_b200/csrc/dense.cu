@@ -222,53 +222,64 @@ constexpr int CNB = 64;  // panel width
 // (CNB x CNB, column-major, ld CNB).  A non-positive pivot sets *info to 1 +
 // its index (first one wins) and the block continues with a unit pivot so
 // that every later value stays finite.
-__global__ void __launch_bounds__(256) k_potrf_diag(double* A, int n, int j, double* Dinv, int* info) {
-  extern __shared__ double psm[];
-  double(*S)[CNB + 1] = reinterpret_cast<double(*)[CNB + 1]>(psm);
-  double(*I)[CNB + 1] = reinterpret_cast<double(*)[CNB + 1]>(psm + CNB * (CNB + 1));
-  const int b = min(CNB, n - j);
-  const int t = threadIdx.x;
-  for (int idx = t; idx < b * b; idx += blockDim.x) {
-    const int r = idx % b, c = idx / b;
-    S[r][c] = A[(size_t)(j + c) * n + j + r];
+//
+// A chain of 64 steps on one SM, so what counts is a step's latency.  Thread (r, q)
+// keeps row r, columns q, q + 4, .. of the block and of the inverse in registers;
+// step c publishes column c of the block and row c of the inverse, both still
+// unscaled, and every later row subtracts (a_rc / a_cc) times them: one barrier and
+// one division a step.  The square roots are taken once, at the end.  41 us a
+// block; 98 us with the block in shared memory, three barriers a step and the
+// inverse by columns after it.
+__global__ void __launch_bounds__(4 * CNB) k_potrf_diag(double* A, int n, int j, double* Dinv, int* info) {
+  __shared__ double col[2][CNB], row[2][CNB], piv[CNB];
+  const int b = min(CNB, n - j), t = threadIdx.x, r = t % CNB, q = t / CNB;
+  double a[CNB / 4], x[CNB / 4];
+#pragma unroll
+  for (int k = 0; k < CNB / 4; ++k) {
+    const int c = 4 * k + q;
+    // rows past b: the unit matrix
+    a[k] = r < b && c < b ? (r >= c ? A[(size_t)(j + c) * n + j + r] : 0.0) : (r == c ? 1.0 : 0.0);
+    x[k] = r == c ? 1.0 : 0.0;
   }
-  __syncthreads();
-  for (int c = 0; c < b; ++c) {
-    if (t == 0) {
-      double d = S[c][c];
+#pragma unroll
+  for (int k = 0; k < CNB / 4; ++k) {
+    for (int cq = 0; cq < 4; ++cq) {
+      const int c = 4 * k + cq, s = c & 1;
+      if (q == cq) col[s][r] = a[k];
+      if (r == c) {
+#pragma unroll
+        for (int l = 0; l <= k; ++l) row[s][4 * l + q] = x[l];
+      }
+      __syncthreads();
+      double d = col[s][c];
       if (!(d > 0.0)) {
-        atomicCAS(info, 0, 1 + j + c);
+        if (t == 0) atomicCAS(info, 0, 1 + j + c);
         d = 1.0;
       }
-      S[c][c] = sqrt(d);
-    }
-    __syncthreads();
-    const double inv = 1.0 / S[c][c];
-    for (int r = c + 1 + t; r < b; r += blockDim.x) S[r][c] *= inv;
-    __syncthreads();
-    const int rem = b - c - 1;
-    for (int idx = t; idx < rem * rem; idx += blockDim.x) {
-      const int r = c + 1 + idx % rem, cc = c + 1 + idx / rem;
-      if (cc <= r) S[r][cc] -= S[r][c] * S[cc][c];
-    }
-    __syncthreads();
-  }
-  // inverse of the lower-triangular block, one column per thread
-  if (t < b) {
-    const int col = t;
-    for (int r = 0; r < col; ++r) I[r][col] = 0.0;
-    I[col][col] = 1.0 / S[col][col];
-    for (int r = col + 1; r < b; ++r) {
-      double acc = 0.0;
-      for (int k = col; k < r; ++k) acc += S[r][k] * I[k][col];
-      I[r][col] = -acc / S[r][r];
+      if (t == 0) piv[c] = d;
+      if (r > c) {
+        const double f = -col[s][r] / d;
+#pragma unroll
+        for (int l = k; l < CNB / 4; ++l) {
+          // a column up to c has its final value; the rest of the upper triangle is not used
+          if (4 * l + q > c) a[l] = fma(f, col[s][4 * l + q], a[l]);
+        }
+#pragma unroll
+        for (int l = 0; l <= k; ++l)
+          if (4 * l + q <= c) x[l] = fma(f, row[s][4 * l + q], x[l]);
+      }
     }
   }
   __syncthreads();
-  for (int idx = t; idx < b * b; idx += blockDim.x) {
-    const int r = idx % b, c = idx / b;
-    A[(size_t)(j + c) * n + j + r] = r >= c ? S[r][c] : 0.0;
-    Dinv[(size_t)c * CNB + r] = r >= c ? I[r][c] : 0.0;
+  const double dr = sqrt(piv[r]);
+#pragma unroll
+  for (int k = 0; k < CNB / 4; ++k) {
+    const int c = 4 * k + q;
+    if (r < b && c < b) {
+      const double dc = sqrt(piv[c]);
+      A[(size_t)(j + c) * n + j + r] = r > c ? a[k] / dc : (r == c ? dc : 0.0);
+      Dinv[(size_t)c * CNB + r] = r >= c ? x[k] / dr : 0.0;
+    }
   }
 }
 
@@ -402,12 +413,9 @@ void mirror_lower(double* C, int n, cudaStream_t s) {
 
 int cholesky(jk_engine* e, double* A, int n, double* work, int* info, cudaStream_t s) {
   cudaMemsetAsync(info, 0, sizeof(int), s);
-  constexpr int PSMEM = 2 * CNB * (CNB + 1) * (int)sizeof(double);
-  cudaError_t sa = cudaFuncSetAttribute(k_potrf_diag, cudaFuncAttributeMaxDynamicSharedMemorySize, PSMEM);
-  if (sa != cudaSuccess) return check_cuda(e, sa, "cholesky attribute");
   for (int j = 0; j < n; j += CNB) {
     const int b = std::min(CNB, n - j);
-    k_potrf_diag<<<1, 256, PSMEM, s>>>(A, n, j, work, info);
+    k_potrf_diag<<<1, 4 * CNB, 0, s>>>(A, n, j, work, info);
     const int R = n - j - b;
     if (R <= 0) break;
     // L21 = A21 L11^-T, in place: at most 64 columns are one tile wide
