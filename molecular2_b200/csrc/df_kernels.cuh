@@ -96,7 +96,7 @@ __device__ __forceinline__ void pure_d(const double* in, double* out, const doub
 // primitive has only Hermite terms of its top degree (solid harmonics are
 // harmonic), (1/2q)^l of its Cartesian coefficients.  Measured through the FP64
 // build on tiled storage, (H2O)16/aug-cc-pVDZ (n 656, naux 2400), which takes
-// one pass of T and one of J: 340 -> 79 ms (a thread per contracted (pair,
+// one pass of T and one of J: 340 -> 79 ms, 43 ms with the later GEMM (a thread per contracted (pair,
 // shell) before, T re-made for J).
 template <int LA, int LB, int LP, bool PURE>
 __global__ void __launch_bounds__(E3_THREADS, 2) k_eri3(const Eri3Params P) {

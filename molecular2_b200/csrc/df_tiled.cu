@@ -8,7 +8,7 @@
 // t = I(I+1)/2 + J (I >= J) holds B_K[128I + r][128J + c] for r, c < 128, as
 // split BF16 (hi + lo) in [K][t][r][c] order (145 GB at the size above).
 // Set-up builds it one tile pair at a time: the three-index integrals
-// T[r][P][c] = (P | x y) of the tile pair (k_eri3_tile), B = L^-1 T on the
+// T[r][c][P] = (P | x y) of the tile pair (k_eri3), B = L^-1 T on the
 // FP64 DMMA GEMM, then the BF16 split; the FP64 B is never stored whole.
 //
 // Mixed build (prec_mode 1), per block of fitted functions:

@@ -139,7 +139,7 @@ constexpr size_t jk_smem(int nden) {
 // src/fockbuild.cpp:266-362) are digested from the same integrals; the screen
 // uses the norms of their sum.
 // Measured (one thread per contracted quartet with its 6 to 81 integrals in
-// local memory -> this kernel): H2O/cc-pVDZ 18.0 -> 0.26 ms, (H2O)8/cc-pVDZ
+// local memory -> this kernel): H2O/cc-pVDZ 18.0 -> 0.24 ms, (H2O)8/cc-pVDZ
 // 44.3 -> 4.4 ms, C20H42/6-311G** 262 -> 44 ms.  Of that, 52 -> 44 ms came from
 // fewer instructions per primitive (Boys function, reciprocal square root), the
 // next primitive's loads issued ahead, and rounds of whole warps over the packed

@@ -3,15 +3,17 @@ numerator).
 
     python molecular2_b200/data/make_flop_table.py
 
-Counts the floating-point operations (an FMA counts 2) that the
-McMurchie-Davidson quartet evaluation of csrc/jk_kernels.cuh (quartet_cart,
-with md_E1, boys and md_R of csrc/md.cuh) performs for one shell quartet of
-angular class (LA LB | LC LD), split into
+Counts the floating-point operations (an FMA counts 2) that a plain
+McMurchie-Davidson quartet evaluation (E tables of both pairs, Boys function,
+Hermite R table, two contraction stages per primitive quartet) performs for one
+shell quartet of angular class (LA LB | LC LD).  The kernels do less (bra tables
+once per block, ket expansions per entry), so a rate from this table counts the
+plain work, not the executed one.  It is split into
   * bra: work done once per bra primitive pair (its three E tables),
   * quartet: work done once per primitive quartet (ket E tables, Boys
     function, Hermite R table, the two contraction stages),
 and the J/K digestion, 6 FMAs (12 flops) per Cartesian integral and density.
-The counts follow the loop structure of the kernel source term by term
+The counts follow the loop structure of that evaluation term by term
 (exp, sqrt and divisions count 1 each).  The work model of one build is
   sum over classes  bra * (bra primitive pairs) + quartet * (primitive quartets)
                     + digest * (quartets)
