@@ -445,10 +445,14 @@ struct SchwarzParams {
 };
 
 // One block per pair.  The Hermite expansions of the final functions' products
-// are formed for SCHWARZ_PRIMS primitives at a time, a thread takes one
-// (primitive, primitive, function pair) item, and the diagonals are summed in
-// shared memory: one thread per pair walked up to 6,561 primitive quartets and
-// the whole (ab|ab) block (creating the engine of (H2O)8: 32 ms, now 6.3 ms).
+// are formed for SCHWARZ_PRIMS primitives at a time, a thread takes primitive
+// quartets of one function pair: one thread per pair walked up to 6,561 of them
+// and the whole (ab|ab) block (creating the engine of (H2O)8: 32 ms, now 6.3 ms).
+// A thread keeps its function pair over the whole block and the partial sums are
+// added in a fixed order, so that the bounds are the same to the last bit in
+// every run: the ranks of a partitioned build (jk_direct_set_partition) each sort
+// their class lists by them and must get the same order, also where pairs have
+// equal bounds by symmetry.
 constexpr int SCHWARZ_THREADS = 128;
 constexpr int SCHWARZ_PRIMS = 8;
 
@@ -459,7 +463,7 @@ struct SchwarzShared {
   double prim[2][SCHWARZ_PRIMS][5];      // p, P, K'
   double E[SCHWARZ_PRIMS][3][e1_size(LA, LB)];
   double M[2][SCHWARZ_PRIMS][NF * H];    // [function pair][h]
-  double diag[NF];
+  double part[SCHWARZ_THREADS];
 };
 
 template <int LA, int LB>
@@ -474,7 +478,9 @@ __global__ void __launch_bounds__(SCHWARZ_THREADS, 2) k_schwarz(const SchwarzPar
   const int pa = P.pure[a], pb = P.pure[b];
   const int ma = pa ? 2 * LA + 1 : NA, mb = pb ? 2 * LB + 1 : NB, nf = ma * mb;
   load_boys<L2>(S.boys, P.boysp);
-  for (int i = tid; i < nf; i += SCHWARZ_THREADS) S.diag[i] = 0.0;
+  // threads of a function pair, and this thread's
+  const int ng = SCHWARZ_THREADS / nf, f = tid % nf, group = tid / nf;
+  double diag = 0.0;
 
   auto load = [&](int side, int k0, int n) {
     __syncthreads();
@@ -528,8 +534,8 @@ __global__ void __launch_bounds__(SCHWARZ_THREADS, 2) k_schwarz(const SchwarzPar
       if (k1 != k0) load(1, k1, nk);
       const int ks = k1 != k0 ? 1 : 0;
       const double w = k1 != k0 ? 2.0 : 1.0;  // both orders of two primitive ranges
-      for (int it = tid; it < nb * nk * nf; it += SCHWARZ_THREADS) {
-        const int f = it % nf, ib = (it / nf) % nb, ik = it / (nf * nb);
+      for (int it = group < ng ? group : nb * nk; it < nb * nk; it += ng) {
+        const int ib = it % nb, ik = it / nb;
         const double* pb_ = S.prim[0][ib];
         const double* pk_ = S.prim[ks][ik];
         double R[nherm(L2)];
@@ -547,14 +553,19 @@ __global__ void __launch_bounds__(SCHWARZ_THREADS, 2) k_schwarz(const SchwarzPar
           });
           acc += ((herm_t(g) + herm_u(g) + herm_v(g)) & 1) ? -Mk[g] * s : Mk[g] * s;
         });
-        atomicAdd(&S.diag[f], acc);
+        diag += acc;
       }
     }
   }
+  S.part[tid] = diag;
   __syncthreads();
   if (tid == 0) {
     double m = 0.0;
-    for (int f = 0; f < nf; ++f) m = fmax(m, fabs(S.diag[f]));
+    for (int k = 0; k < nf; ++k) {
+      double d = 0.0;
+      for (int g = 0; g < ng; ++g) d += S.part[g * nf + k];
+      m = fmax(m, fabs(d));
+    }
     P.Qout[ip] = sqrt(m);
   }
 }
