@@ -115,9 +115,10 @@ int eri3_all(jk_engine* e, bool j, cudaStream_t s, const std::function<bool(Eri3
   static decltype(&launch_eri3_s) const launch[jk_engine::NAUXGROUP] = {
       launch_eri3_s, launch_eri3_p, launch_eri3_d_pure, launch_eri3_d_cart, launch_eri3_f_pure, launch_eri3_f_cart};
   ClassStreams cs(e, s);
-  for (const Item& it : items) launch[it.g](it.pc, it.P, j, cs.next(it.cost));
+  LaunchStatus status;
+  for (const Item& it : items) status(launch[it.g](it.pc, it.P, j, cs.next(it.cost)));
   cs.join();
-  return check_cuda(e, cudaGetLastError(), "three-index launch");
+  return check_cuda(e, status.st, "three-index launch");
 }
 
 // T3[x][y][P] = (P|xy), full n x n x naux.
@@ -162,6 +163,7 @@ int eri3_J(jk_engine* e, const double* c, double* cc, double* J, cudaStream_t s)
 
 int compute_V(jk_engine* e, double* V, cudaStream_t s) {
   ClassStreams cs(e, s);
+  LaunchStatus status;
   for (int gP = jk_engine::NAUXGROUP - 1; gP >= 0; --gP)
     for (int gQ = gP; gQ >= 0; --gQ) {
       if (!e->aux_group_count[gP] || !e->aux_group_count[gQ]) continue;
@@ -173,10 +175,10 @@ int compute_V(jk_engine* e, double* V, cudaStream_t s) {
       P.naux = e->aux.n_final;
       P.same = gP == gQ;
       P.V = V;
-      launch_eri2(gP, gQ, P, cs.next((double)P.P.count * P.Q.count));
+      status(launch_eri2(gP, gQ, P, cs.next((double)P.P.count * P.Q.count)));
     }
   cs.join();
-  return check_cuda(e, cudaGetLastError(), "eri2 launch");
+  return check_cuda(e, status.st, "eri2 launch");
 }
 
 // packed reference layout: Tp[(x(x+1)/2 + y) + P*npair], x >= y, from T3[x][y][P]:
@@ -455,9 +457,8 @@ int one_body_device(jk_engine* e, double* S, double* T, double* V, cudaStream_t 
     P.S = S;
     P.T = T;
     P.V = V;
-    launch_onebody(pc, P, s);
+    if ((st = launch_onebody(pc, P, s)) != cudaSuccess) break;
   }
-  st = cudaGetLastError();
   if (st == cudaSuccess) st = cudaStreamSynchronize(s);  // Z, C die on return
   return check_cuda(e, st, "one_body");
 }

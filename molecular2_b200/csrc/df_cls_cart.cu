@@ -4,7 +4,7 @@
 
 namespace m2 {
 
-void launch_eri3_d_cart(int pc, const Eri3Params& P, bool j, cudaStream_t s) { launch_eri3_l<2, false>(pc, P, j, s); }
-void launch_eri3_f_cart(int pc, const Eri3Params& P, bool j, cudaStream_t s) { launch_eri3_l<3, false>(pc, P, j, s); }
+cudaError_t launch_eri3_d_cart(int pc, const Eri3Params& P, bool j, cudaStream_t s) { return launch_eri3_l<2, false>(pc, P, j, s); }
+cudaError_t launch_eri3_f_cart(int pc, const Eri3Params& P, bool j, cudaStream_t s) { return launch_eri3_l<3, false>(pc, P, j, s); }
 
 }  // namespace m2

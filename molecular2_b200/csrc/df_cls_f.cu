@@ -4,6 +4,6 @@
 
 namespace m2 {
 
-void launch_eri3_f_pure(int pc, const Eri3Params& P, bool j, cudaStream_t s) { launch_eri3_l<3, true>(pc, P, j, s); }
+cudaError_t launch_eri3_f_pure(int pc, const Eri3Params& P, bool j, cudaStream_t s) { return launch_eri3_l<3, true>(pc, P, j, s); }
 
 }  // namespace m2

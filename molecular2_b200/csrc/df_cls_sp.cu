@@ -4,7 +4,7 @@
 
 namespace m2 {
 
-void launch_eri3_s(int pc, const Eri3Params& P, bool j, cudaStream_t s) { launch_eri3_l<0, true>(pc, P, j, s); }
-void launch_eri3_p(int pc, const Eri3Params& P, bool j, cudaStream_t s) { launch_eri3_l<1, true>(pc, P, j, s); }
+cudaError_t launch_eri3_s(int pc, const Eri3Params& P, bool j, cudaStream_t s) { return launch_eri3_l<0, true>(pc, P, j, s); }
+cudaError_t launch_eri3_p(int pc, const Eri3Params& P, bool j, cudaStream_t s) { return launch_eri3_l<1, true>(pc, P, j, s); }
 
 }  // namespace m2

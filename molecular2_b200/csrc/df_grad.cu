@@ -81,8 +81,8 @@ static void launch_cart_rows(const jk_engine* e, int o, const double* C, double*
 // group, with W3 (Cartesian orbital functions) holding fitting functions from
 // w3_f0 on; the launches add to the gradient and run on the side streams,
 // longest first.
-static void launch_grad3_all(jk_engine* e, const int* const* shells, const int* counts, const double* W3, int w3_f0,
-                             double* g2e, cudaStream_t s) {
+static cudaError_t launch_grad3_all(jk_engine* e, const int* const* shells, const int* counts, const double* W3,
+                                    int w3_f0, double* g2e, cudaStream_t s) {
   static decltype(&launch_grad3_s) const launch[jk_engine::NAUXGROUP] = {
       launch_grad3_s, launch_grad3_p, launch_grad3_d_pure, launch_grad3_d_cart, launch_grad3_f_pure, launch_grad3_f_cart};
   static const double ncp[NPAIRCLASS] = {1, 3, 9, 6, 18, 36};
@@ -98,6 +98,7 @@ static void launch_grad3_all(jk_engine* e, const int* const* shells, const int* 
         items.push_back({g, pc, (double)e->pcls[pc].nent * counts[g] * ncp[pc] * (gl[g] + 1) * (gl[g] + 2)});
   std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.cost > b.cost; });
   ClassStreams cs(e, s);
+  LaunchStatus status;
   for (const Item& it : items) {
     Grad3Params P{};
     P.aux = aux_group_view(e, shells[it.g], counts[it.g]);
@@ -116,14 +117,16 @@ static void launch_grad3_all(jk_engine* e, const int* const* shells, const int* 
     P.w3_f0 = w3_f0;
     P.natom = e->natom;
     P.grad = g2e;
-    launch[it.g](it.pc, P, cs.next(it.cost));
+    status(launch[it.g](it.pc, P, cs.next(it.cost)));
   }
   cs.join();
+  return status.st;
 }
 
 // k_grad2 over every ordered pair of fitting groups with the weights W2.
-static void launch_grad2_all(jk_engine* e, const double* W2, double* g2e, cudaStream_t s) {
+static cudaError_t launch_grad2_all(jk_engine* e, const double* W2, double* g2e, cudaStream_t s) {
   ClassStreams cs(e, s);
+  LaunchStatus status;
   for (int gP = jk_engine::NAUXGROUP - 1; gP >= 0; --gP)
     for (int gQ = jk_engine::NAUXGROUP - 1; gQ >= 0; --gQ) {
       if (!e->aux_group_count[gP] || !e->aux_group_count[gQ]) continue;
@@ -136,9 +139,10 @@ static void launch_grad2_all(jk_engine* e, const double* W2, double* g2e, cudaSt
       P.naux = e->aux.n_final;
       P.W2 = W2;
       P.grad = g2e;
-      launch_grad2(gP, gQ, P, cs.next((double)P.P.count * P.Q.count));
+      status(launch_grad2(gP, gQ, P, cs.next((double)P.P.count * P.Q.count)));
     }
   cs.join();
+  return status.st;
 }
 
 // dC: n x nocc column-major occupied orbitals; dD = 2 C C^T; g2e receives
@@ -247,11 +251,10 @@ int grad_df_2e_device(jk_engine* e, const double* dC, int nocc, const double* dD
   {
     const int* shells[jk_engine::NAUXGROUP];
     for (int g = 0; g < jk_engine::NAUXGROUP; ++g) shells[g] = e->aux_group[g].p;
-    launch_grad3_all(e, shells, e->aux_group_count, Z.p, 0, g2e, s);
+    st = launch_grad3_all(e, shells, e->aux_group_count, Z.p, 0, g2e, s);
   }
   // metric derivatives
-  launch_grad2_all(e, W2.p, g2e, s);
-  st = cudaGetLastError();
+  if (st == cudaSuccess) st = launch_grad2_all(e, W2.p, g2e, s);
   if (st == cudaSuccess) st = cudaStreamSynchronize(s);  // scratch dies on return
   return check_cuda(e, st, "DF gradient kernels");
 }
@@ -453,14 +456,13 @@ int grad_df_2e_tiled(jk_engine* e, const double* dC, int nocc, const double* dD,
         shells[g] = lists[g].p;
         counts[g] = (int)sh[g].size();
       }
-      launch_grad3_all(e, shells, counts, Z.p, f0, g2e, s);
-      st = cudaStreamSynchronize(s);  // Y, Z and the shell lists are reused by the next block
+      st = launch_grad3_all(e, shells, counts, Z.p, f0, g2e, s);
+      if (st == cudaSuccess) st = cudaStreamSynchronize(s);  // Y, Z and the shell lists are reused by the next block
       if (st != cudaSuccess) return check_cuda(e, st, "tiled DF gradient block");
       s0 = s1;
     }
   }
-  launch_grad2_all(e, W2.p, g2e, s);
-  st = cudaGetLastError();
+  st = launch_grad2_all(e, W2.p, g2e, s);
   if (st == cudaSuccess) st = cudaStreamSynchronize(s);
   return check_cuda(e, st, "tiled DF gradient kernels");
 }

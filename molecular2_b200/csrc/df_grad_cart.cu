@@ -5,7 +5,7 @@
 
 namespace m2 {
 
-void launch_grad3_d_cart(int pc, const Grad3Params& P, cudaStream_t s) { launch_grad3_l<2, false>(pc, P, s); }
-void launch_grad3_f_cart(int pc, const Grad3Params& P, cudaStream_t s) { launch_grad3_l<3, false>(pc, P, s); }
+cudaError_t launch_grad3_d_cart(int pc, const Grad3Params& P, cudaStream_t s) { return launch_grad3_l<2, false>(pc, P, s); }
+cudaError_t launch_grad3_f_cart(int pc, const Grad3Params& P, cudaStream_t s) { return launch_grad3_l<3, false>(pc, P, s); }
 
 }  // namespace m2

@@ -5,6 +5,6 @@
 
 namespace m2 {
 
-void launch_grad3_d_pure(int pc, const Grad3Params& P, cudaStream_t s) { launch_grad3_l<2, true>(pc, P, s); }
+cudaError_t launch_grad3_d_pure(int pc, const Grad3Params& P, cudaStream_t s) { return launch_grad3_l<2, true>(pc, P, s); }
 
 }  // namespace m2

@@ -174,23 +174,23 @@ __global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad3(const Grad3Params P) 
 }
 
 template <int LP, bool PURE, int LC, int LD>
-inline void launch_grad3_class(const Grad3Params& P, cudaStream_t s) {
+inline cudaError_t launch_grad3_class(const Grad3Params& P, cudaStream_t s) {
   const size_t sm = sizeof(Grad3Shared<LP>) + 16 + (P.natom <= GRAD_ATOMS ? 24 * (size_t)P.natom : 0);
-  cudaFuncSetAttribute(k_grad3<LP, PURE, LC, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   const int layers = ncart(LC) * ncart(LD), chunks = (P.ent.nent + GRAD_THREADS - 1) / GRAD_THREADS;
   // blocks walk over several ket chunks where there are enough of them to fill the GPU
   int y = 1;
   while (y < chunks && (long long)P.aux.count * layers * y < 16 * 148) ++y;
-  k_grad3<LP, PURE, LC, LD><<<dim3(P.aux.count, y, layers), GRAD_THREADS, sm, s>>>(P);
+  return launch_smem(k_grad3<LP, PURE, LC, LD>, dim3(P.aux.count, y, layers), GRAD_THREADS, sm, s, P);
 }
 template <int LP, bool PURE>
-inline void launch_grad3_l(int pc, const Grad3Params& P, cudaStream_t s) {
-  if (pc == 0) launch_grad3_class<LP, PURE, 0, 0>(P, s);
-  if (pc == 1) launch_grad3_class<LP, PURE, 1, 0>(P, s);
-  if (pc == 2) launch_grad3_class<LP, PURE, 1, 1>(P, s);
-  if (pc == 3) launch_grad3_class<LP, PURE, 2, 0>(P, s);
-  if (pc == 4) launch_grad3_class<LP, PURE, 2, 1>(P, s);
-  if (pc == 5) launch_grad3_class<LP, PURE, 2, 2>(P, s);
+inline cudaError_t launch_grad3_l(int pc, const Grad3Params& P, cudaStream_t s) {
+  if (pc == 0) return launch_grad3_class<LP, PURE, 0, 0>(P, s);
+  if (pc == 1) return launch_grad3_class<LP, PURE, 1, 0>(P, s);
+  if (pc == 2) return launch_grad3_class<LP, PURE, 1, 1>(P, s);
+  if (pc == 3) return launch_grad3_class<LP, PURE, 2, 0>(P, s);
+  if (pc == 4) return launch_grad3_class<LP, PURE, 2, 1>(P, s);
+  if (pc == 5) return launch_grad3_class<LP, PURE, 2, 2>(P, s);
+  return cudaErrorInvalidValue;
 }
 
 struct Grad2Params {
@@ -327,12 +327,12 @@ __global__ void __launch_bounds__(G2_THREADS) k_grad2(const Grad2Params P) {
 }
 
 // launchers (df_grad_*.cu): orbital pair class id; fitting groups gP, gQ
-void launch_grad3_s(int pair_class_id, const Grad3Params& P, cudaStream_t s);
-void launch_grad3_p(int pair_class_id, const Grad3Params& P, cudaStream_t s);
-void launch_grad3_d_pure(int pair_class_id, const Grad3Params& P, cudaStream_t s);
-void launch_grad3_d_cart(int pair_class_id, const Grad3Params& P, cudaStream_t s);
-void launch_grad3_f_pure(int pair_class_id, const Grad3Params& P, cudaStream_t s);
-void launch_grad3_f_cart(int pair_class_id, const Grad3Params& P, cudaStream_t s);
-void launch_grad2(int gP, int gQ, const Grad2Params& P, cudaStream_t s);
+cudaError_t launch_grad3_s(int pair_class_id, const Grad3Params& P, cudaStream_t s);
+cudaError_t launch_grad3_p(int pair_class_id, const Grad3Params& P, cudaStream_t s);
+cudaError_t launch_grad3_d_pure(int pair_class_id, const Grad3Params& P, cudaStream_t s);
+cudaError_t launch_grad3_d_cart(int pair_class_id, const Grad3Params& P, cudaStream_t s);
+cudaError_t launch_grad3_f_pure(int pair_class_id, const Grad3Params& P, cudaStream_t s);
+cudaError_t launch_grad3_f_cart(int pair_class_id, const Grad3Params& P, cudaStream_t s);
+cudaError_t launch_grad2(int gP, int gQ, const Grad2Params& P, cudaStream_t s);
 
 }  // namespace m2

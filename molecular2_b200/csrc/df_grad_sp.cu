@@ -5,7 +5,7 @@
 
 namespace m2 {
 
-void launch_grad3_s(int pc, const Grad3Params& P, cudaStream_t s) { launch_grad3_l<0, true>(pc, P, s); }
-void launch_grad3_p(int pc, const Grad3Params& P, cudaStream_t s) { launch_grad3_l<1, true>(pc, P, s); }
+cudaError_t launch_grad3_s(int pc, const Grad3Params& P, cudaStream_t s) { return launch_grad3_l<0, true>(pc, P, s); }
+cudaError_t launch_grad3_p(int pc, const Grad3Params& P, cudaStream_t s) { return launch_grad3_l<1, true>(pc, P, s); }
 
 }  // namespace m2

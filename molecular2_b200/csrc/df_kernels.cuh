@@ -319,30 +319,26 @@ __global__ void __launch_bounds__(E3_THREADS, 2) k_eri3_J(const Eri3Params P) {
 }
 
 template <int LA, int LB, int LP, bool PURE>
-inline void launch_eri3_class(const Eri3Params& P, bool j, cudaStream_t s) {
+inline cudaError_t launch_eri3_class(const Eri3Params& P, bool j, cudaStream_t s) {
   const size_t sm = sizeof(Eri3Shared<LA, LB, LP>);
   const int iters = (P.aux.count + E3_THREADS - 1) / E3_THREADS;
   const int threads = ((P.aux.count + iters - 1) / iters + 31) / 32 * 32;
-  if (j) {
-    cudaFuncSetAttribute(k_eri3_J<LA, LB, LP, PURE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_eri3_J<LA, LB, LP, PURE><<<P.pairs.npair, threads, sm, s>>>(P);
-    return;
-  }
-  cudaFuncSetAttribute(k_eri3<LA, LB, LP, PURE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (j) return launch_smem(k_eri3_J<LA, LB, LP, PURE>, P.pairs.npair, threads, sm, s, P);
   const int layers = e3_full(LA, LB, LP, PURE) ? 1 : e3_nfun(LP, PURE);
   // one block walks over all fitting shells of a pair unless that leaves the GPU short of blocks
   int z = 1;
   while (z < iters && (long long)P.nlist * layers * z < 8 * 148) ++z;
-  k_eri3<LA, LB, LP, PURE><<<dim3(P.nlist, layers, z), threads, sm, s>>>(P);
+  return launch_smem(k_eri3<LA, LB, LP, PURE>, dim3(P.nlist, layers, z), threads, sm, s, P);
 }
 template <int LP, bool PURE>
-inline void launch_eri3_l(int pc, const Eri3Params& P, bool j, cudaStream_t s) {
-  if (pc == 0) launch_eri3_class<0, 0, LP, PURE>(P, j, s);
-  if (pc == 1) launch_eri3_class<1, 0, LP, PURE>(P, j, s);
-  if (pc == 2) launch_eri3_class<1, 1, LP, PURE>(P, j, s);
-  if (pc == 3) launch_eri3_class<2, 0, LP, PURE>(P, j, s);
-  if (pc == 4) launch_eri3_class<2, 1, LP, PURE>(P, j, s);
-  if (pc == 5) launch_eri3_class<2, 2, LP, PURE>(P, j, s);
+inline cudaError_t launch_eri3_l(int pc, const Eri3Params& P, bool j, cudaStream_t s) {
+  if (pc == 0) return launch_eri3_class<0, 0, LP, PURE>(P, j, s);
+  if (pc == 1) return launch_eri3_class<1, 0, LP, PURE>(P, j, s);
+  if (pc == 2) return launch_eri3_class<1, 1, LP, PURE>(P, j, s);
+  if (pc == 3) return launch_eri3_class<2, 0, LP, PURE>(P, j, s);
+  if (pc == 4) return launch_eri3_class<2, 1, LP, PURE>(P, j, s);
+  if (pc == 5) return launch_eri3_class<2, 2, LP, PURE>(P, j, s);
+  return cudaErrorInvalidValue;
 }
 
 // Group number of a fitting shell: s, p, pure d, Cartesian d, pure f, Cartesian f.
@@ -452,12 +448,12 @@ __global__ void __launch_bounds__(E2_THREADS) k_eri2(const Eri2Params P) {
 }
 
 // launchers in df_cls_*.cu: pair class id, T (j false) or J (j true)
-void launch_eri3_s(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
-void launch_eri3_p(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
-void launch_eri3_d_pure(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
-void launch_eri3_d_cart(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
-void launch_eri3_f_pure(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
-void launch_eri3_f_cart(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
-void launch_eri2(int gP, int gQ, const Eri2Params& P, cudaStream_t s);  // groups gP >= gQ
+cudaError_t launch_eri3_s(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
+cudaError_t launch_eri3_p(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
+cudaError_t launch_eri3_d_pure(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
+cudaError_t launch_eri3_d_cart(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
+cudaError_t launch_eri3_f_pure(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
+cudaError_t launch_eri3_f_cart(int pair_class_id, const Eri3Params& P, bool j, cudaStream_t s);
+cudaError_t launch_eri2(int gP, int gQ, const Eri2Params& P, cudaStream_t s);  // groups gP >= gQ
 
 }  // namespace m2

@@ -34,12 +34,12 @@ __global__ void k_pair_sig(PairView pairs, const int* __restrict__ foff, const d
   sig[i] = (same || sqrt(s2) >= 1e-12) ? 1 : 0;
 }
 
-static void launch_grad2e(const jk_engine* e, int A, int B, const Grad2eParams& Pin, cudaStream_t s) {
+static cudaError_t launch_grad2e(const jk_engine* e, int A, int B, const Grad2eParams& Pin, cudaStream_t s) {
   Grad2eParams P = Pin;
   const PairClassDev &ca = e->pcls[A], &cb = e->pcls[B];
   int nb = 0;
   bra_share(e, ca.npair, P.bra0, P.bra_step, nb);
-  if (nb == 0) return;
+  if (nb == 0) return cudaSuccess;
   P.bra = view(ca);
   P.ket = view(cb);
   P.bra_ent = entry_view(ca);
@@ -53,16 +53,10 @@ static void launch_grad2e(const jk_engine* e, int A, int B, const Grad2eParams& 
          nbra * ((nket + P.kchunk - 1) / P.kchunk) * layers < (P.kchunk > GRAD_THREADS ? 32 : 8) * 148)
     P.kchunk /= 2;
   dim3 grid(ca.nent, (unsigned)((nket + P.kchunk - 1) / P.kchunk), (unsigned)layers);
-  if (A <= 2)
-    launch_grad2e_bra_s(A, B, P, grid, s);
-  else if (A == 3)
-    launch_grad2e_bra_ds(B, P, grid, s);
-  else if (A == 4)
-    launch_grad2e_bra_dp(B, P, grid, s);
-  else if (B < 4)
-    launch_grad2e_bra_dd(B, P, grid, s);
-  else
-    launch_grad2e_bra_dd_hi(B, P, grid, s);
+  if (A <= 2) return launch_grad2e_bra_s(A, B, P, grid, s);
+  if (A == 3) return launch_grad2e_bra_ds(B, P, grid, s);
+  if (A == 4) return launch_grad2e_bra_dp(B, P, grid, s);
+  return B < 4 ? launch_grad2e_bra_dd(B, P, grid, s) : launch_grad2e_bra_dd_hi(B, P, grid, s);
 }
 
 // dE_nuc/dx, natom x 3 (src/rhfgrad.cpp:59-86)
@@ -145,11 +139,12 @@ int grad_rhf_device(jk_engine* e, const double* dD, const double* dW, double pre
         items.push_back({A, B, (double)e->pcls[A].npair * e->pcls[B].npair * ncp[A] * ncp[B] * (A == B ? 0.5 : 1.0)});
   std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.cost > b.cost; });
   ClassStreams cs(e, s);
+  LaunchStatus status;
   for (const Item& it : items) {
     Grad2eParams Q = P;
     Q.bra_sig = sig[it.A].p;
     Q.ket_sig = sig[it.B].p;
-    launch_grad2e(e, it.A, it.B, Q, cs.next(it.cost));
+    status(launch_grad2e(e, it.A, it.B, Q, cs.next(it.cost)));
   }
   cs.join();
   // one-body terms: whole on the first rank of a partition, none on the others
@@ -173,9 +168,9 @@ int grad_rhf_device(jk_engine* e, const double* dD, const double* dW, double pre
     Q.Z = Z.p;
     Q.cxyz = C.p;
     Q.grad = g1e;
-    launch_grad1e(k, Q, s);
+    status(launch_grad1e(k, Q, s));
   }
-  st = cudaGetLastError();
+  st = status.st;
   if (st == cudaSuccess) st = cudaStreamSynchronize(s);  // scratch dies on return
   return check_cuda(e, st, "gradient kernels");
 }

@@ -235,17 +235,16 @@ __global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad2e(const Grad2eParams P
 }
 
 template <int LA, int LB, int LC, int LD>
-inline void launch_grad2e_class(const Grad2eParams& P, dim3 grid, cudaStream_t s) {
+inline cudaError_t launch_grad2e_class(const Grad2eParams& P, dim3 grid, cudaStream_t s) {
   const size_t sm = sizeof(GradShared<LA, LB>) + 16 + (P.natom <= GRAD_ATOMS ? 24 * (size_t)P.natom : 0);
-  cudaFuncSetAttribute(k_grad2e<LA, LB, LC, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_grad2e<LA, LB, LC, LD><<<grid, GRAD_THREADS, sm, s>>>(P);
+  return launch_smem(k_grad2e<LA, LB, LC, LD>, grid, GRAD_THREADS, sm, s, P);
 }
 
 // launchers (grad_cls_*.cu)
-void launch_grad2e_bra_s(int A, int B, const Grad2eParams& P, dim3 grid, cudaStream_t s);
-void launch_grad2e_bra_ds(int B, const Grad2eParams& P, dim3 grid, cudaStream_t s);
-void launch_grad2e_bra_dp(int B, const Grad2eParams& P, dim3 grid, cudaStream_t s);
-void launch_grad2e_bra_dd(int B, const Grad2eParams& P, dim3 grid, cudaStream_t s);
-void launch_grad2e_bra_dd_hi(int B, const Grad2eParams& P, dim3 grid, cudaStream_t s);
+cudaError_t launch_grad2e_bra_s(int A, int B, const Grad2eParams& P, dim3 grid, cudaStream_t s);
+cudaError_t launch_grad2e_bra_ds(int B, const Grad2eParams& P, dim3 grid, cudaStream_t s);
+cudaError_t launch_grad2e_bra_dp(int B, const Grad2eParams& P, dim3 grid, cudaStream_t s);
+cudaError_t launch_grad2e_bra_dd(int B, const Grad2eParams& P, dim3 grid, cudaStream_t s);
+cudaError_t launch_grad2e_bra_dd_hi(int B, const Grad2eParams& P, dim3 grid, cudaStream_t s);
 
 }  // namespace m2

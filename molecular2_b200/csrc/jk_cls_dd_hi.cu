@@ -3,9 +3,10 @@
 #include "jk_kernels.cuh"
 
 namespace m2 {
-void launch_jk_bra_dd_hi(int B, const JKParams& P, dim3 grid, cudaStream_t s) {
-  if (B == 4) launch_jk_class<2, 2, 2, 1>(P, grid, s);
-  if (B == 5) launch_jk_class<2, 2, 2, 2>(P, grid, s);
+cudaError_t launch_jk_bra_dd_hi(int B, const JKParams& P, dim3 grid, cudaStream_t s) {
+  if (B == 4) return launch_jk_class<2, 2, 2, 1>(P, grid, s);
+  if (B == 5) return launch_jk_class<2, 2, 2, 2>(P, grid, s);
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace m2

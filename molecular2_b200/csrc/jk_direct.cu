@@ -181,7 +181,8 @@ int build_pairs(jk_engine* e) {
       const PairView v{di.p + io[k][0], di.p + io[k][1], di.p + io[k][2], di.p + io[k][3], nullptr, e->pcls[k].npair};
       SchwarzParams P{v, prim_view(e), shell_view(e), e->dobs.l.p, e->dobs.pure.p, e->dobs.sph.p, e->boysp.p,
                       dq.p + qo[k]};
-      launch_schwarz(cls[k].la, cls[k].lb, P, s);
+      if ((st = launch_schwarz(cls[k].la, cls[k].lb, P, s)) != cudaSuccess)
+        return check_cuda(e, st, "schwarz launch");
     }
     st = cudaMemcpyAsync(Q.data(), dq.p, ntot * sizeof(double), cudaMemcpyDeviceToHost, s);
     if (st == cudaSuccess) st = cudaStreamSynchronize(s);
@@ -276,7 +277,7 @@ static double class_cost(int A, int B, int nbra, int nket) {
 // ones instead of one after another; J, K and the counters are accumulated
 // with atomics, so the launches commute.
 template <class Launch>
-static void launch_classes(jk_engine* e, cudaStream_t s, Launch&& launch) {
+static cudaError_t launch_classes(jk_engine* e, cudaStream_t s, Launch&& launch) {
   struct Item {
     int A, B;
     double cost;
@@ -288,16 +289,18 @@ static void launch_classes(jk_engine* e, cudaStream_t s, Launch&& launch) {
         items.push_back({A, B, class_cost(A, B, e->pcls[A].npair, e->pcls[B].npair)});
   std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.cost > b.cost; });
   ClassStreams cs(e, s);
-  for (const Item& it : items) launch(it.A, it.B, cs.next(it.cost));
+  LaunchStatus status;
+  for (const Item& it : items) status(launch(it.A, it.B, cs.next(it.cost)));
   cs.join();
+  return status.st;
 }
 
-static void launch_jk(const jk_engine* e, int A, int B, const JKParams& Pin, cudaStream_t s) {
+static cudaError_t launch_jk(const jk_engine* e, int A, int B, const JKParams& Pin, cudaStream_t s) {
   JKParams P = Pin;
   const PairClassDev &ca = e->pcls[A], &cb = e->pcls[B];
   int nb = 0;
   bra_share(e, ca.npair, P.bra0, P.bra_step, nb);
-  if (nb == 0) return;
+  if (nb == 0) return cudaSuccess;
   P.bra = view(ca);
   P.ket = view(cb);
   P.bra_ent = entry_view(ca);
@@ -305,16 +308,10 @@ static void launch_jk(const jk_engine* e, int A, int B, const JKParams& Pin, cud
   P.same_class = (A == B);
   P.kchunk = ket_chunk((long long)ca.nent / P.bra_step, cb.nent, jk_layers(ca.la, ca.lb, cb.la, cb.lb));
   dim3 grid(ca.nent, (cb.nent + P.kchunk - 1) / P.kchunk);
-  if (A <= 2)
-    launch_jk_bra_s(A, B, P, grid, s);
-  else if (A == 3)
-    launch_jk_bra_ds(B, P, grid, s);
-  else if (A == 4)
-    launch_jk_bra_dp(B, P, grid, s);
-  else if (B < 4)
-    launch_jk_bra_dd_lo(B, P, grid, s);
-  else
-    launch_jk_bra_dd_hi(B, P, grid, s);
+  if (A <= 2) return launch_jk_bra_s(A, B, P, grid, s);
+  if (A == 3) return launch_jk_bra_ds(B, P, grid, s);
+  if (A == 4) return launch_jk_bra_dp(B, P, grid, s);
+  return B < 4 ? launch_jk_bra_dd_lo(B, P, grid, s) : launch_jk_bra_dd_hi(B, P, grid, s);
 }
 
 int direct_jk_device(jk_engine* e, const double* dD, double precision, double mult, double* dJ, double* dK,
@@ -352,15 +349,15 @@ int direct_jk_device(jk_engine* e, const double* dD, double precision, double mu
   P.precision = precision;
   P.boysp = e->boysp.p;
   P.counter = counter;
-  launch_classes(e, s, [&](int A, int B, cudaStream_t cs) {
+  const cudaError_t launched = launch_classes(e, s, [&](int A, int B, cudaStream_t cs) {
     JKParams Q = P;
     Q.work = e->class_work.p + 3 * (A * NPAIRCLASS + B);
-    launch_jk(e, A, B, Q, cs);
+    return launch_jk(e, A, B, Q, cs);
   });
   // J = 1/4 (J + J^T) mult, K = 1/2 * 1/4 (K + K^T) mult  (src/fockbuild.cpp:146-149, 161-162)
   launch_cart_to_final_sym(e, e->Jcart.p, 0.25 * mult, dJ, s);
   launch_cart_to_final_sym(e, e->Kcart.p, 0.125 * mult, dK, s);
-  return check_cuda(e, cudaGetLastError(), "jk_direct launch");
+  return check_cuda(e, launched != cudaSuccess ? launched : cudaGetLastError(), "jk_direct launch");
 }
 
 // J and K of two densities (UHF alpha and beta) from one pass over the shell
@@ -406,16 +403,16 @@ int direct_jk_uhf_device(jk_engine* e, const double* dDa, const double* dDb, dou
     return check_cuda(e, st, "jk_direct_uhf work counters");
   cudaMemsetAsync(e->class_work.p, 0, sizeof(unsigned long long) * 3 * NPAIRCLASS * NPAIRCLASS, s);
   e->class_work_valid = true;
-  launch_classes(e, s, [&](int A, int B, cudaStream_t cs) {
+  const cudaError_t launched = launch_classes(e, s, [&](int A, int B, cudaStream_t cs) {
     JKParams Q = P;
     Q.work = e->class_work.p + 3 * (A * NPAIRCLASS + B);
-    launch_jk(e, A, B, Q, cs);
+    return launch_jk(e, A, B, Q, cs);
   });
   launch_cart_to_final_sym(e, Jc2.p, 0.25 * mult, dJa, s);
   launch_cart_to_final_sym(e, Jc2.p + ncc, 0.25 * mult, dJb, s);
   launch_cart_to_final_sym(e, Kc2.p, 0.125 * mult, dKa, s);
   launch_cart_to_final_sym(e, Kc2.p + ncc, 0.125 * mult, dKb, s);
-  st = cudaGetLastError();
+  st = launched != cudaSuccess ? launched : cudaGetLastError();
   if (st == cudaSuccess) st = cudaStreamSynchronize(s);  // the scratch dies on return
   return check_cuda(e, st, "jk_direct_uhf");
 }
@@ -502,12 +499,12 @@ int direct_jk_noalloc(jk_engine* e, const double* dD, double precision, double m
   P.boysp = e->boysp.p;
   P.counter = counter;
   P.dstride = NOALLOC_CC;
-  launch_classes(e, s, [&](int A, int B, cudaStream_t cs) {
-    launch_jk(e, A, B, P, cs);
+  const cudaError_t launched = launch_classes(e, s, [&](int A, int B, cudaStream_t cs) {
+    return launch_jk(e, A, B, P, cs);
   });
   launch_cart_to_final_sym(e, Jc, 0.25 * mult, dJ, s);
   launch_cart_to_final_sym(e, Kc, 0.125 * mult, dK, s);
-  return check_cuda(e, cudaGetLastError(), "jk_direct_noalloc launch");
+  return check_cuda(e, launched != cudaSuccess ? launched : cudaGetLastError(), "jk_direct_noalloc launch");
 }
 
 }  // namespace m2

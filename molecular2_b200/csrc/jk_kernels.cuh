@@ -1,6 +1,7 @@
 // Device side of the integral-direct J/K build and the Schwarz bounds (FP64).
 // Included by the per-class translation units jk_cls_*.cu and jk_direct.cu.
 #pragma once
+#include "launch.cuh"
 #include "md.cuh"
 #include "quartet.cuh"
 
@@ -424,11 +425,10 @@ __global__ void __launch_bounds__(JK_THREADS) k_jk_direct(const JKParams P) {
 }
 
 template <int LA, int LB, int LC, int LD>
-inline void launch_jk_class(const JKParams& P, dim3 grid, cudaStream_t s) {
+inline cudaError_t launch_jk_class(const JKParams& P, dim3 grid, cudaStream_t s) {
   const size_t sm = jk_smem<LA, LB>(P.nden);
-  cudaFuncSetAttribute(k_jk_direct<LA, LB, LC, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   grid.z = jk_layers(LA, LB, LC, LD);
-  k_jk_direct<LA, LB, LC, LD><<<grid, JK_THREADS, sm, s>>>(P);
+  return launch_smem(k_jk_direct<LA, LB, LC, LD>, grid, JK_THREADS, sm, s, P);
 }
 
 // Schwarz bound of each pair of one class: sqrt(max diag (ab|ab)) over the
@@ -571,10 +571,9 @@ __global__ void __launch_bounds__(SCHWARZ_THREADS, 2) k_schwarz(const SchwarzPar
 }
 
 template <int LA, int LB>
-inline void launch_schwarz_class(const SchwarzParams& P, cudaStream_t s) {
+inline cudaError_t launch_schwarz_class(const SchwarzParams& P, cudaStream_t s) {
   const size_t sm = sizeof(SchwarzShared<LA, LB>);
-  cudaFuncSetAttribute(k_schwarz<LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  k_schwarz<LA, LB><<<P.pairs.npair, SCHWARZ_THREADS, sm, s>>>(P);
+  return launch_smem(k_schwarz<LA, LB>, P.pairs.npair, SCHWARZ_THREADS, sm, s, P);
 }
 
 struct PairClassDev;
@@ -583,11 +582,11 @@ PairView view(const PairClassDev& c);
 EntryView entry_view(const PairClassDev& c);
 
 // per-translation-unit launchers (jk_cls_*.cu); A, B are pair-class ids
-void launch_jk_bra_s(int A, int B, const JKParams& P, dim3 grid, cudaStream_t s);   // A in {0,1,2}
-void launch_jk_bra_ds(int B, const JKParams& P, dim3 grid, cudaStream_t s);         // A = 3
-void launch_jk_bra_dp(int B, const JKParams& P, dim3 grid, cudaStream_t s);         // A = 4
-void launch_jk_bra_dd_lo(int B, const JKParams& P, dim3 grid, cudaStream_t s);      // A = 5, B < 4
-void launch_jk_bra_dd_hi(int B, const JKParams& P, dim3 grid, cudaStream_t s);      // A = 5, B >= 4
-void launch_schwarz(int la, int lb, const SchwarzParams& P, cudaStream_t s);  // schwarz.cu
+cudaError_t launch_jk_bra_s(int A, int B, const JKParams& P, dim3 grid, cudaStream_t s);   // A in {0,1,2}
+cudaError_t launch_jk_bra_ds(int B, const JKParams& P, dim3 grid, cudaStream_t s);         // A = 3
+cudaError_t launch_jk_bra_dp(int B, const JKParams& P, dim3 grid, cudaStream_t s);         // A = 4
+cudaError_t launch_jk_bra_dd_lo(int B, const JKParams& P, dim3 grid, cudaStream_t s);      // A = 5, B < 4
+cudaError_t launch_jk_bra_dd_hi(int B, const JKParams& P, dim3 grid, cudaStream_t s);      // A = 5, B >= 4
+cudaError_t launch_schwarz(int la, int lb, const SchwarzParams& P, cudaStream_t s);  // schwarz.cu
 
 }  // namespace m2

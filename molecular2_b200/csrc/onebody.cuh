@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(OB_THREADS) k_grad1e(const Grad1eParams P) {
       if (s_g[i] != 0.0) atomicAdd(P.grad + i, s_g[i]);
 }
 
-void launch_onebody(int pc, const OneBodyParams& P, cudaStream_t s);  // onebody.cu
-void launch_grad1e(int pc, const Grad1eParams& P, cudaStream_t s);
+cudaError_t launch_onebody(int pc, const OneBodyParams& P, cudaStream_t s);  // onebody.cu
+cudaError_t launch_grad1e(int pc, const Grad1eParams& P, cudaStream_t s);
 
 }  // namespace m2

@@ -10,7 +10,7 @@ import pytest
 
 from molecular2_b200 import geometry
 from molecular2_b200.basis import BasisSet, Molecule
-from molecular2_b200.engine import IntegralEngine
+from molecular2_b200.engine import IntegralEngine, JKError
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +52,29 @@ def test_partial_builds_of_separate_engines_sum_to_the_whole():
         assert sq == quartets
         assert max(np.abs(sJ - J).max(), np.abs(sK - K).max()) < 1e-11 * scale
         assert np.abs(sg - g).max() < 1e-10 * max(1.0, np.abs(g).max())
+
+
+def many_kets():
+    """Diffuse s shells, 2.2 million pairs, around one tight d shell: with the
+    density on the d shell alone and this threshold only the (dd|ss) integrals
+    pass the screen (bounds: dd about 5, ss 0.07, products 0.3 and 0.004)."""
+    mol = Molecule(["he"], [[0.0, 0.0, 0.0]])
+    shells = [(0, [float(x)], [1.0], 0) for x in np.linspace(1e-5, 2e-5, 2100)] + [(2, [1e3], [1.0], 0)]
+    obs = BasisSet.from_shells(shells, mol)
+    D = np.zeros((obs.nbf, obs.nbf))
+    D[2100:, 2100:] = np.eye(5)
+    return obs, D, 0.05
+
+
+def test_no_class_is_left_out_of_a_build_without_an_error():
+    """One bra pair and eight ranks: a launch that cannot be made is reported."""
+    obs, D, precision = many_kets()
+    eng = IntegralEngine(obs)
+    J, _ = eng.jk_direct(D, precision)
+    assert np.abs(J[:2100, :2100]).min() > 1e-3
+    eng.set_direct_partition(0, 8)
+    try:
+        part, _ = eng.jk_direct(D, precision)
+    except JKError:
+        return
+    assert np.abs(part - J)[:2100, :2100].max() < 1e-14
