@@ -47,7 +47,7 @@ static cudaError_t launch_grad2e(const jk_engine* e, int A, int B, const Grad2eP
   P.same_class = (A == B);
   // ket entries per block: many share the bra set-up, fewer where the blocks
   // would not fill the GPU
-  const long long layers = ncart(cb.la) * ncart(cb.lb), nbra = ca.nent / P.bra_step, nket = cb.nent;
+  const long long layers = ncart(cb.la) * ncart(cb.lb), nbra = std::max(1, ca.nent / P.bra_step), nket = cb.nent;
   P.kchunk = GRAD_LIST;
   while (P.kchunk > 32 &&
          nbra * ((nket + P.kchunk - 1) / P.kchunk) * layers < (P.kchunk > GRAD_THREADS ? 32 : 8) * 148)

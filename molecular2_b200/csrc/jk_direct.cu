@@ -260,6 +260,7 @@ int build_pairs(jk_engine* e) {
 // GPU otherwise.
 static int ket_chunk(long long nbra, long long nket, int layers) {
   int k = 4 * JK_LIST;
+  nbra = std::max(nbra, 1LL);  // a rank's share of few entries; the grid's y limit is 65,535
   while (k > 32 && nbra * ((nket + k - 1) / k) * layers < (k > JK_THREADS ? 32 : 8) * 148) k /= 2;
   return k;
 }

@@ -78,3 +78,15 @@ def test_no_class_is_left_out_of_a_build_without_an_error():
     except JKError:
         return
     assert np.abs(part - J)[:2100, :2100].max() < 1e-14
+
+
+def test_fewer_bra_entries_than_ranks_with_many_kets():
+    """The ket range of the (dd|ss) launch stays within the grid's limits."""
+    obs, D, precision = many_kets()
+    eng = IntegralEngine(obs)
+    J, K = eng.jk_direct(D, precision)
+    eng.set_direct_partition(0, 8)
+    pJ, _ = eng.jk_direct(D, precision)
+    assert np.abs(pJ - J)[:2100, :2100].max() < 1e-14
+    uhf = eng.jk_direct_uhf(D, D, precision)
+    assert np.abs(uhf[0] - J)[:2100, :2100].max() < 1e-14
