@@ -175,12 +175,14 @@ __global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad3(const Grad3Params P) 
 
 template <int LP, bool PURE, int LC, int LD>
 inline cudaError_t launch_grad3_class(const Grad3Params& P, cudaStream_t s) {
-  const size_t sm = sizeof(Grad3Shared<LP>) + 16 + (P.natom <= GRAD_ATOMS ? 24 * (size_t)P.natom : 0);
+  constexpr size_t base = sizeof(Grad3Shared<LP>) + 16, most = base + 24 * GRAD_ATOMS;
+  static_assert(most <= SMEM_BLOCK_MAX, "shared memory of GRAD_ATOMS atoms");
+  const size_t sm = base + (P.natom <= GRAD_ATOMS ? 24 * (size_t)P.natom : 0);
   const int layers = ncart(LC) * ncart(LD), chunks = (P.ent.nent + GRAD_THREADS - 1) / GRAD_THREADS;
   // blocks walk over several ket chunks where there are enough of them to fill the GPU
   int y = 1;
   while (y < chunks && (long long)P.aux.count * layers * y < 16 * 148) ++y;
-  return launch_smem(k_grad3<LP, PURE, LC, LD>, dim3(P.aux.count, y, layers), GRAD_THREADS, sm, s, P);
+  return launch_smem(k_grad3<LP, PURE, LC, LD>, dim3(P.aux.count, y, layers), GRAD_THREADS, sm, most, s, P);
 }
 template <int LP, bool PURE>
 inline cudaError_t launch_grad3_l(int pc, const Grad3Params& P, cudaStream_t s) {

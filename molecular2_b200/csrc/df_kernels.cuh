@@ -323,12 +323,12 @@ inline cudaError_t launch_eri3_class(const Eri3Params& P, bool j, cudaStream_t s
   const size_t sm = sizeof(Eri3Shared<LA, LB, LP>);
   const int iters = (P.aux.count + E3_THREADS - 1) / E3_THREADS;
   const int threads = ((P.aux.count + iters - 1) / iters + 31) / 32 * 32;
-  if (j) return launch_smem(k_eri3_J<LA, LB, LP, PURE>, P.pairs.npair, threads, sm, s, P);
+  if (j) return launch_smem(k_eri3_J<LA, LB, LP, PURE>, P.pairs.npair, threads, sm, sm, s, P);
   const int layers = e3_full(LA, LB, LP, PURE) ? 1 : e3_nfun(LP, PURE);
   // one block walks over all fitting shells of a pair unless that leaves the GPU short of blocks
   int z = 1;
   while (z < iters && (long long)P.nlist * layers * z < 8 * 148) ++z;
-  return launch_smem(k_eri3<LA, LB, LP, PURE>, dim3(P.nlist, layers, z), threads, sm, s, P);
+  return launch_smem(k_eri3<LA, LB, LP, PURE>, dim3(P.nlist, layers, z), threads, sm, sm, s, P);
 }
 template <int LP, bool PURE>
 inline cudaError_t launch_eri3_l(int pc, const Eri3Params& P, bool j, cudaStream_t s) {

@@ -23,6 +23,7 @@
 #include <cmath>
 
 #include "engine.h"
+#include "launch.cuh"
 
 namespace m2 {
 namespace {
@@ -224,7 +225,7 @@ __global__ void __launch_bounds__(32 * VEC_WARPS) k_jacobi_vectors(int n, const 
     for (int k = lane; k < n; k += 32) vecs[(size_t)meta[1 + k] * n + row] = v[k];
 }
 
-size_t jacobi_smem(int n) {
+constexpr size_t jacobi_smem(int n) {
   const size_t np = (n + 1) & ~1;
   return sizeof(double) * np * (np + 1) + np / 2 * (sizeof(double2) + sizeof(double) + sizeof(int2));
 }
@@ -264,10 +265,10 @@ cudaError_t small_eig(const double* A, double* vecs, double* vals, int n, void* 
   const int np = (n + 1) & ~1;
   double2* rot = static_cast<double2*>(scratch);
   int* meta = reinterpret_cast<int*>(rot + (size_t)JAC_SWEEPS * (np - 1) * (np / 2));
-  cudaError_t st =
-      cudaFuncSetAttribute(k_jacobi, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jacobi_smem(n));
+  static_assert(jacobi_smem(SMALL_EIG_MAX) <= SMEM_BLOCK_MAX, "one block holds the matrix");
+  const cudaError_t st =
+      launch_smem(k_jacobi, 1, JAC_THREADS, jacobi_smem(n), jacobi_smem(SMALL_EIG_MAX), s, n, A, vals, rot, meta);
   if (st != cudaSuccess) return st;
-  k_jacobi<<<1, JAC_THREADS, jacobi_smem(n), s>>>(n, A, vals, rot, meta);
   const size_t vs = sizeof(double2) * (size_t)VEC_ROUNDS * (np / 2) + sizeof(double) * (size_t)VEC_WARPS * np;
   k_jacobi_vectors<<<(n + VEC_WARPS - 1) / VEC_WARPS, 32 * VEC_WARPS, vs, s>>>(n, rot, meta, vecs);
   return cudaGetLastError();

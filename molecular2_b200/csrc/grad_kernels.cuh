@@ -236,8 +236,10 @@ __global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad2e(const Grad2eParams P
 
 template <int LA, int LB, int LC, int LD>
 inline cudaError_t launch_grad2e_class(const Grad2eParams& P, dim3 grid, cudaStream_t s) {
-  const size_t sm = sizeof(GradShared<LA, LB>) + 16 + (P.natom <= GRAD_ATOMS ? 24 * (size_t)P.natom : 0);
-  return launch_smem(k_grad2e<LA, LB, LC, LD>, grid, GRAD_THREADS, sm, s, P);
+  constexpr size_t base = sizeof(GradShared<LA, LB>) + 16, most = base + 24 * GRAD_ATOMS;
+  static_assert(most <= SMEM_BLOCK_MAX, "shared memory of GRAD_ATOMS atoms");
+  const size_t sm = base + (P.natom <= GRAD_ATOMS ? 24 * (size_t)P.natom : 0);
+  return launch_smem(k_grad2e<LA, LB, LC, LD>, grid, GRAD_THREADS, sm, most, s, P);
 }
 
 // launchers (grad_cls_*.cu)

@@ -125,7 +125,7 @@ struct JKShared {
   int n;
 };
 template <int LA, int LB>
-constexpr size_t jk_smem(int nden) {
+__host__ __device__ constexpr size_t jk_smem(int nden) {
   return sizeof(JKShared<LA, LB>) + sizeof(double) * (size_t)nden * ncart(LA) * ncart(LB) * JK_THREADS + 16;
 }
 
@@ -426,9 +426,9 @@ __global__ void __launch_bounds__(JK_THREADS) k_jk_direct(const JKParams P) {
 
 template <int LA, int LB, int LC, int LD>
 inline cudaError_t launch_jk_class(const JKParams& P, dim3 grid, cudaStream_t s) {
-  const size_t sm = jk_smem<LA, LB>(P.nden);
+  static_assert(jk_smem<LA, LB>(2) <= SMEM_BLOCK_MAX, "shared memory of two densities");
   grid.z = jk_layers(LA, LB, LC, LD);
-  return launch_smem(k_jk_direct<LA, LB, LC, LD>, grid, JK_THREADS, sm, s, P);
+  return launch_smem(k_jk_direct<LA, LB, LC, LD>, grid, JK_THREADS, jk_smem<LA, LB>(P.nden), jk_smem<LA, LB>(2), s, P);
 }
 
 // Schwarz bound of each pair of one class: sqrt(max diag (ab|ab)) over the
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(SCHWARZ_THREADS, 2) k_schwarz(const SchwarzPar
 template <int LA, int LB>
 inline cudaError_t launch_schwarz_class(const SchwarzParams& P, cudaStream_t s) {
   const size_t sm = sizeof(SchwarzShared<LA, LB>);
-  return launch_smem(k_schwarz<LA, LB>, P.pairs.npair, SCHWARZ_THREADS, sm, s, P);
+  return launch_smem(k_schwarz<LA, LB>, P.pairs.npair, SCHWARZ_THREADS, sm, sm, s, P);
 }
 
 struct PairClassDev;

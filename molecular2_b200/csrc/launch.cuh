@@ -9,11 +9,16 @@
 
 namespace m2 {
 
-// Launch with `smem` bytes of dynamic shared memory.
+constexpr size_t SMEM_BLOCK_MAX = 227 * 1024;
+
+// Launch with `smem` bytes of dynamic shared memory, of the `most` that any launch
+// of this kernel asks for.  The limit belongs to the function in the whole process:
+// one that followed the call would be lowered by another thread between its setting
+// and the launch.
 template <class... A, class... B>
-inline cudaError_t launch_smem(void (*kernel)(A...), dim3 grid, int threads, size_t smem, cudaStream_t s,
+inline cudaError_t launch_smem(void (*kernel)(A...), dim3 grid, int threads, size_t smem, size_t most, cudaStream_t s,
                                const B&... args) {
-  const cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t st = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
   if (st != cudaSuccess) return st;
   kernel<<<grid, threads, smem, s>>>(args...);
   return cudaGetLastError();
