@@ -42,10 +42,12 @@ Pool& pool() {
 }
 
 // Sizes are rounded to an eighth of their power of two (at least 512 bytes), so
-// that nearly equal requests share blocks.
+// that nearly equal requests share blocks, but to no more than the 2 MB pages that
+// cudaMalloc takes by itself: the callers that size their scratch by the free
+// memory (0.94 of it for one array) get what they ask for.
 size_t round_size(size_t n) {
   size_t step = 512;
-  while (step * 16 < n) step *= 2;
+  while (step * 16 < n && step < (size_t(2) << 20)) step *= 2;
   return (n + step - 1) / step * step;
 }
 size_t cached_bytes(int device) {
