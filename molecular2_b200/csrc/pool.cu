@@ -10,7 +10,8 @@
 //   * the cache is bounded (POOL_BYTES per device, oldest blocks returned to the
 //     driver first; larger blocks are never kept), is emptied when an allocation
 //     fails, and can be emptied by jk_release_cached;
-//   * one mutex guards the lists, so engines may live on several threads.
+//   * one mutex guards the lists, so engines may live on several threads; no call
+//     that may wait for the device is made under it.
 #include <cuda_runtime.h>
 
 #include <iterator>
@@ -32,6 +33,7 @@ struct Block {
 };
 struct Pool {
   std::mutex mu;
+  std::mutex full;         // held while the cache is emptied for an allocation that failed
   std::list<Block> cache;  // oldest first
   std::unordered_map<void*, Block> in_use;
 };
@@ -56,19 +58,22 @@ size_t cached_bytes(int device) {
     if (k.device == device) b += k.bytes;
   return b;
 }
-// Returns cached blocks of the device to the driver until at most `keep` bytes stay.
-void trim(int device, size_t keep) {
+// Takes the oldest cached blocks of the device out of the list until at most
+// `keep` bytes stay; the caller returns them to the driver without the lock.
+std::list<Block> take(int device, size_t keep) {
   std::list<Block>& cache = pool().cache;
+  std::list<Block> out;
   size_t have = cached_bytes(device);
   for (auto it = cache.begin(); it != cache.end() && have > keep;) {
-    if (it->device != device) {
-      ++it;
-      continue;
-    }
-    have -= it->bytes;
-    cudaFree(it->p);
-    it = cache.erase(it);
+    const auto b = it++;
+    if (b->device != device) continue;
+    have -= b->bytes;
+    out.splice(out.end(), cache, b);
   }
+  return out;
+}
+void give_back(const std::list<Block>& blocks) {
+  for (const Block& b : blocks) cudaFree(b.p);
 }
 
 }  // namespace
@@ -79,7 +84,7 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
   if (st != cudaSuccess) return st;
   const size_t n = round_size(bytes);
   Pool& P = pool();
-  std::lock_guard<std::mutex> lock(P.mu);
+  std::unique_lock<std::mutex> lock(P.mu);
   for (auto it = P.cache.rbegin(); it != P.cache.rend(); ++it)
     if (it->device == device && it->bytes == n) {
       *p = it->p;
@@ -87,35 +92,50 @@ cudaError_t dev_alloc(void** p, size_t bytes) {
       P.cache.erase(std::next(it).base());
       return cudaSuccess;
     }
+  lock.unlock();
   st = cudaMalloc(p, n);
-  if (st == cudaErrorMemoryAllocation && cached_bytes(device) > 0) {
-    cudaGetLastError();  // clears the failure
-    trim(device, 0);
+  if (st == cudaErrorMemoryAllocation) {
+    std::lock_guard<std::mutex> one(P.full);
+    lock.lock();
+    const std::list<Block> old = take(device, 0);
+    lock.unlock();
+    give_back(old);
+    cudaGetLastError();  // or a later query finds the failure
     st = cudaMalloc(p, n);
   }
-  if (st == cudaSuccess) P.in_use[*p] = Block{*p, n, device};
+  if (st != cudaSuccess) {
+    cudaGetLastError();
+    return st;
+  }
+  lock.lock();
+  P.in_use[*p] = Block{*p, n, device};
   return st;
 }
 
 void dev_free(void* p) {
   if (!p) return;
   Pool& P = pool();
-  std::lock_guard<std::mutex> lock(P.mu);
+  std::unique_lock<std::mutex> lock(P.mu);
   auto it = P.in_use.find(p);
   if (it == P.in_use.end()) {
+    lock.unlock();
     cudaFree(p);
     return;
   }
   const Block b = it->second;
   P.in_use.erase(it);
+  lock.unlock();  // other threads allocate while this one waits for the device
   int device = -1;
   const bool here = cudaGetDevice(&device) == cudaSuccess && device == b.device;
   if (!here || b.bytes > POOL_BYTES / 2 || cudaDeviceSynchronize() != cudaSuccess) {
     cudaFree(p);
     return;
   }
-  trim(device, POOL_BYTES - b.bytes);
+  lock.lock();
+  const std::list<Block> old = take(device, POOL_BYTES - b.bytes);
   P.cache.push_back(b);
+  lock.unlock();
+  give_back(old);
 }
 
 cudaError_t dev_mem_info(size_t* free_bytes, size_t* total) {
@@ -134,10 +154,12 @@ extern "C" int jk_release_cached(int device) {
   int cur = -1;
   if (cudaGetDevice(&cur) != cudaSuccess) return JK_ERR_CUDA;
   if (cur != device && cudaSetDevice(device) != cudaSuccess) return JK_ERR_ARG;
+  std::list<m2::Block> old;
   {
     std::lock_guard<std::mutex> lock(m2::pool().mu);
-    m2::trim(device, 0);
+    old = m2::take(device, 0);
   }
+  m2::give_back(old);
   if (cur != device) cudaSetDevice(cur);
   return JK_OK;
 }

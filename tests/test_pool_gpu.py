@@ -5,6 +5,7 @@ The thread test compares builds of the same inputs: only the order of FP64
 atomic additions differs, 24 x 24 sums of size <= 10: 1e-12.
 """
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -64,3 +65,30 @@ def test_threads_share_the_cache():
     for s, ref in enumerate(refs):
         for a, b in zip(got[s], ref):
             assert np.abs(a - b).max() < 1e-12
+
+
+def test_allocations_do_not_wait_for_a_free_on_another_thread():
+    """A free waits for the device; meanwhile another thread's call that needs
+    memory and only queues work comes back."""
+    import torch
+    mol = geometry.water_cluster(1, 3.5, 1)
+    obs = BasisSet(mol, "cc-pvdz")
+    D = torch.eye(obs.nbf, dtype=torch.float64, device="cuda")
+    J, K = torch.empty_like(D), torch.empty_like(D)
+    warm = IntegralEngine(obs)
+    warm.jk_direct_device(D.data_ptr(), J.data_ptr(), K.data_ptr())  # the kernels' code
+    warm.close()
+    going, fresh = IntegralEngine(obs), IntegralEngine(obs)
+    side, done = torch.cuda.Stream(), torch.cuda.Event()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(2_000_000_000)  # about a second
+        done.record()
+    t = threading.Thread(target=going.close)
+    t.start()
+    time.sleep(0.2)  # close() is in its first free
+    assert t.is_alive()
+    fresh.jk_direct_device(D.data_ptr(), J.data_ptr(), K.data_ptr())
+    assert not done.query()
+    t.join()
+    torch.cuda.synchronize()
