@@ -145,6 +145,70 @@ static cudaError_t launch_grad2_all(jk_engine* e, const double* W2, double* g2e,
   return status.st;
 }
 
+// Z[P] = W3^P = c_P D - 2 C d^P C^T over Cartesian orbital functions (Cc: nc x o,
+// Dc: nc x nc) for w fitting functions with coefficients c and d^P in dd; Y is
+// scratch of w nc o elements.
+static int w3_block(jk_engine* e, int o, int w, const double* Cc, const double* Dc, const double* dd, const double* c,
+                    double* Y, double* Z, cudaStream_t s) {
+  const int nc = e->obs.n_cart;
+  const size_t ncc = (size_t)nc * nc;
+  DGemm y;  // Y[P] = Cc d^P (nc x o)
+  y.M = nc; y.N = o; y.K = o; y.batch = w;
+  y.A = Cc; y.sam = 1; y.sak = nc;
+  y.B = dd; y.sbk = 1; y.sbn = o; y.bsb = (long long)o * o;
+  y.C = Y; y.scm = 1; y.scn = nc; y.bsc = (long long)nc * o;
+  cudaError_t st = dgemm(y, s);
+  if (st != cudaSuccess) return check_cuda(e, st, "DF gradient: Y = C d");
+  DGemm z;  // Z[P] = Y[P] Cc^T (nc x nc)
+  z.M = nc; z.N = nc; z.K = o; z.batch = w;
+  z.A = Y; z.sam = 1; z.sak = nc; z.bsa = (long long)nc * o;
+  z.B = Cc; z.sbk = nc; z.sbn = 1;
+  z.C = Z; z.scm = 1; z.scn = nc; z.bsc = (long long)ncc;
+  if ((st = dgemm(z, s)) != cudaSuccess) return check_cuda(e, st, "DF gradient: Z = Y C^T");
+  k_w3<<<(unsigned)((ncc * w + 255) / 256), 256, 0, s>>>(ncc, w, c, Dc, Z);
+  return check_cuda(e, cudaGetLastError(), "DF gradient: W3");
+}
+
+// W3 and its contraction with the derivative integrals, as many fitting shells
+// at a time as the free memory holds (at least 16 functions).
+static int grad3_blocks(jk_engine* e, int o, const double* Cc, const double* Dc, const double* dd, const double* c,
+                        double* g2e, cudaStream_t s) {
+  const int nc = e->obs.n_cart;
+  const size_t ncc = (size_t)nc * nc, oo = (size_t)o * o;
+  size_t fr = 0, tot = 0;
+  dev_mem_info(&fr, &tot);
+  const double per_f = 8.0 * ((double)ncc + (double)nc * o);
+  const int wmax = (int)std::max(16.0, std::min<double>(e->aux.n_final, 0.6 * (double)fr / per_f));
+  DevBuf<double> Y, Z;
+  cudaError_t st = Y.alloc((size_t)nc * o * wmax);
+  if (st == cudaSuccess) st = Z.alloc(ncc * wmax);
+  if (st != cudaSuccess) return check_cuda(e, st, "DF gradient W3 block");
+  const HostBasis& ab = e->aux;
+  DevBuf<int> lists[jk_engine::NAUXGROUP];
+  for (int s0 = 0; s0 < ab.nshell;) {
+    int s1 = s0;
+    while (s1 < ab.nshell && ab.off_final[s1 + 1] - ab.off_final[s0] <= wmax) ++s1;
+    if (s1 == s0) return set_error(e, JK_ERR_ARG, "DF gradient: fitting shell wider than the block");
+    const int f0 = ab.off_final[s0], w = ab.off_final[s1] - f0;
+    int rc = w3_block(e, o, w, Cc, Dc, dd + (size_t)f0 * oo, c + f0, Y.p, Z.p, s);
+    if (rc) return rc;
+    std::vector<int> sh[jk_engine::NAUXGROUP];
+    for (int k = s0; k < s1; ++k) sh[aux_group_of(ab.l[k], ab.pure[k])].push_back(k);
+    const int* shells[jk_engine::NAUXGROUP];
+    int counts[jk_engine::NAUXGROUP];
+    for (int g = 0; g < jk_engine::NAUXGROUP; ++g) {
+      if ((st = lists[g].upload(sh[g], s)) != cudaSuccess) return check_cuda(e, st, "DF gradient shells");
+      shells[g] = lists[g].p;
+      counts[g] = (int)sh[g].size();
+    }
+    st = launch_grad3_all(e, shells, counts, Z.p, f0, g2e, s);
+    if (st == cudaSuccess) st = cudaStreamSynchronize(s);  // Y, Z and the shell lists are reused by the next block
+    if (st != cudaSuccess) return check_cuda(e, st, "DF gradient block");
+    s0 = s1;
+  }
+  return JK_OK;
+}
+
 // dC: n x nocc column-major occupied orbitals; dD = 2 C C^T; g2e receives
 // the two-electron DF gradient (zeroed here).  Synchronises the stream.
 int grad_df_2e_device(jk_engine* e, const double* dC, int nocc, const double* dD, double* g2e, cudaStream_t s) {
@@ -156,19 +220,21 @@ int grad_df_2e_device(jk_engine* e, const double* dC, int nocc, const double* dD
       return set_error(e, JK_ERR_ARG, "DF gradient: every fitting shell needs an owning atom (jk_basis.atom)");
   const int nc = e->obs.n_cart;
   const size_t ncc = (size_t)nc * nc;
-  DevBuf<double> X, bt, c, W2, Z, Cc, Dc;
-  cudaError_t st = X.alloc((size_t)nc * naux * o);
-  if (st == cudaSuccess) st = bt.alloc((size_t)o * o * naux);
+  if (!d.Linv.p) return set_error(e, JK_ERR_STATE, "DF gradient: L^-1 missing (run jk_df_setup)");
+  DevBuf<double> X, bt, c, W2, Z, Cc, Dc, dd, gt;
+  cudaError_t st = bt.alloc((size_t)o * o * naux);
   if (st == cudaSuccess) st = c.alloc(naux);
   if (st == cudaSuccess) st = W2.alloc((size_t)naux * naux);
-  if (st == cudaSuccess) st = Z.alloc(ncc * naux);
   if (st == cudaSuccess) st = Cc.alloc((size_t)nc * o);
   if (st == cudaSuccess) st = Dc.alloc(ncc);
-  if (st != cudaSuccess) return check_cuda(e, st, "DF gradient allocation");
-  if (!d.Linv.p) return set_error(e, JK_ERR_STATE, "DF gradient: L^-1 missing (run jk_df_setup)");
-  DevBuf<double> dd, gt;
-  st = dd.alloc((size_t)o * o * naux);
+  if (st == cudaSuccess) st = dd.alloc((size_t)o * o * naux);
   if (st == cudaSuccess) st = gt.alloc(naux);
+  // X, later Y, and the whole of W3; where W3 does not fit, it is made in blocks
+  // in the place of X
+  if (st == cudaSuccess) st = X.alloc((size_t)nc * naux * o);
+  if (st == cudaSuccess) st = Z.alloc(ncc * naux);
+  const bool whole = st == cudaSuccess;
+  if (st == cudaErrorMemoryAllocation) st = X.alloc((size_t)n * naux * o);
   if (st != cudaSuccess) return check_cuda(e, st, "DF gradient allocation");
   auto gemm = [&](const DGemm& g, const char* what) {
     const cudaError_t r = dgemm(g, s);
@@ -228,30 +294,19 @@ int grad_df_2e_device(jk_engine* e, const double* dC, int nocc, const double* dD
     r.alpha = -0.5; r.beta = 1.0;
     if ((rc = gemm(r, "DF gradient: W2"))) return rc;
   }
-  // W3 over Cartesian orbital functions: Y[P] = Cc d^P (nc x o, reusing X), Z[P] = Y[P] Cc^T
   launch_cart_rows(e, o, dC, Cc.p, s);
   launch_final_to_cart(e, dD, Dc.p, s);
-  {
-    DGemm g;
-    g.M = nc; g.N = o; g.K = o; g.batch = naux;
-    g.A = Cc.p; g.sam = 1; g.sak = nc;
-    g.B = dd.p; g.sbk = 1; g.sbn = o; g.bsb = (long long)o * o;
-    g.C = X.p; g.scm = 1; g.scn = nc; g.bsc = (long long)nc * o;
-    if ((rc = gemm(g, "DF gradient: Y = C d"))) return rc;
-    DGemm z;
-    z.M = nc; z.N = nc; z.K = o; z.batch = naux;
-    z.A = X.p; z.sam = 1; z.sak = nc; z.bsa = (long long)nc * o;
-    z.B = Cc.p; z.sbk = nc; z.sbn = 1;
-    z.C = Z.p; z.scm = 1; z.scn = nc; z.bsc = (long long)ncc;
-    if ((rc = gemm(z, "DF gradient: Z = Y C^T"))) return rc;
-  }
-  k_w3<<<(unsigned)((ncc * naux + 255) / 256), 256, 0, s>>>(ncc, naux, c.p, Dc.p, Z.p);
   cudaMemsetAsync(g2e, 0, sizeof(double) * 3 * na, s);
   // three-index derivatives
-  {
+  if (whole) {
+    if ((rc = w3_block(e, o, naux, Cc.p, Dc.p, dd.p, c.p, X.p, Z.p, s))) return rc;
     const int* shells[jk_engine::NAUXGROUP];
     for (int g = 0; g < jk_engine::NAUXGROUP; ++g) shells[g] = e->aux_group[g].p;
     st = launch_grad3_all(e, shells, e->aux_group_count, Z.p, 0, g2e, s);
+  } else {
+    X.reset();
+    bt.reset();
+    if ((rc = grad3_blocks(e, o, Cc.p, Dc.p, dd.p, c.p, g2e, s))) return rc;
   }
   // metric derivatives
   if (st == cudaSuccess) st = launch_grad2_all(e, W2.p, g2e, s);
@@ -418,50 +473,7 @@ int grad_df_2e_tiled(jk_engine* e, const double* dC, int nocc, const double* dD,
   launch_cart_rows(e, o, dC, Cc.p, s);
   launch_final_to_cart(e, dD, Dc.p, s);
   cudaMemsetAsync(g2e, 0, sizeof(double) * 3 * na, s);
-  // W3 = c_P D - 2 C d^P C^T and its contraction, one block of fitting shells at a time
-  {
-    size_t fr = 0, tot = 0;
-    dev_mem_info(&fr, &tot);
-    const double per_f = 8.0 * ((double)ncc + (double)nc * o);
-    const int wmax = (int)std::max(16.0, std::min<double>(naux, 0.6 * (double)fr / per_f));
-    DevBuf<double> Y, Z;
-    if ((st = Y.alloc((size_t)nc * o * wmax)) == cudaSuccess) st = Z.alloc(ncc * wmax);
-    if (st != cudaSuccess) return check_cuda(e, st, "tiled DF gradient W3 block");
-    const HostBasis& ab = e->aux;
-    DevBuf<int> lists[jk_engine::NAUXGROUP];
-    for (int s0 = 0; s0 < ab.nshell;) {
-      int s1 = s0;
-      while (s1 < ab.nshell && ab.off_final[s1 + 1] - ab.off_final[s0] <= wmax) ++s1;
-      if (s1 == s0) return set_error(e, JK_ERR_ARG, "tiled DF gradient: fitting shell wider than the block");
-      const int f0 = ab.off_final[s0], w = ab.off_final[s1] - f0;
-      DGemm y;  // Y[P] = Cc d^P (nc x o)
-      y.M = nc; y.N = o; y.K = o; y.batch = w;
-      y.A = Cc.p; y.sam = 1; y.sak = nc;
-      y.B = dd.p + (size_t)f0 * oo; y.sbk = 1; y.sbn = o; y.bsb = (long long)oo;
-      y.C = Y.p; y.scm = 1; y.scn = nc; y.bsc = (long long)nc * o;
-      if ((rc = gemm(y, "tiled DF gradient: Y = C d"))) return rc;
-      DGemm z;  // Z[P] = Y[P] Cc^T (nc x nc)
-      z.M = nc; z.N = nc; z.K = o; z.batch = w;
-      z.A = Y.p; z.sam = 1; z.sak = nc; z.bsa = (long long)nc * o;
-      z.B = Cc.p; z.sbk = nc; z.sbn = 1;
-      z.C = Z.p; z.scm = 1; z.scn = nc; z.bsc = (long long)ncc;
-      if ((rc = gemm(z, "tiled DF gradient: Z = Y C^T"))) return rc;
-      k_w3<<<(unsigned)((ncc * w + 255) / 256), 256, 0, s>>>(ncc, w, c.p + f0, Dc.p, Z.p);
-      std::vector<int> sh[jk_engine::NAUXGROUP];
-      for (int k = s0; k < s1; ++k) sh[aux_group_of(ab.l[k], ab.pure[k])].push_back(k);
-      const int* shells[jk_engine::NAUXGROUP];
-      int counts[jk_engine::NAUXGROUP];
-      for (int g = 0; g < jk_engine::NAUXGROUP; ++g) {
-        if ((st = lists[g].upload(sh[g], s)) != cudaSuccess) return check_cuda(e, st, "tiled DF gradient shells");
-        shells[g] = lists[g].p;
-        counts[g] = (int)sh[g].size();
-      }
-      st = launch_grad3_all(e, shells, counts, Z.p, f0, g2e, s);
-      if (st == cudaSuccess) st = cudaStreamSynchronize(s);  // Y, Z and the shell lists are reused by the next block
-      if (st != cudaSuccess) return check_cuda(e, st, "tiled DF gradient block");
-      s0 = s1;
-    }
-  }
+  if ((rc = grad3_blocks(e, o, Cc.p, Dc.p, dd.p, c.p, g2e, s))) return rc;
   st = launch_grad2_all(e, W2.p, g2e, s);
   if (st == cudaSuccess) st = cudaStreamSynchronize(s);
   return check_cuda(e, st, "tiled DF gradient kernels");

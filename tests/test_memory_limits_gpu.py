@@ -64,3 +64,28 @@ def test_large_blocks_take_what_they_hold():
     held = before - free_bytes()
     assert eng.df_tensor_bytes > 1 << 30
     assert held - eng.df_tensor_bytes - 2 * 8 * eng.naux ** 2 < 32 * MB
+
+
+def test_df_gradient_in_the_memory_of_the_final_functions():
+    """DF gradient on unpacked storage with room for X and W3 over the final
+    functions (n = 160 against 180 Cartesian ones) and 16 MB: W3 over Cartesian
+    functions does not fit and is made in blocks.  Sums in another order: 1e-10."""
+    mol = geometry.water_cluster(4, 6.0, 5)
+    shells = [(l, [x], [1.0], a) for a in range(0, 12, 3) for l, xs in ((2, (0.3, 0.6, 1.1, 2.5, 5.0)), (1, (0.4, 1.5)),
+                                                                        (0, (0.2, 0.5, 1.2, 4.0, 12.0, 40.0, 150.0, 600.0, 3000.0)))
+              for x in xs]
+    obs = BasisSet.from_shells(shells, mol)
+    fit = BasisSet(mol, "vdz-jkfit")
+    n, o, naux = obs.nbf, 12, fit.nbf
+    assert n == 160
+    C = np.linalg.qr(np.random.default_rng(7).normal(size=(n, o)))[0]
+    eps = np.linspace(-1.0, -0.5, o)
+    eng = IntegralEngine(obs, fit)
+    eng.set_df_storage("unpacked")
+    eng.df_setup()
+    ref = eng.compute_forces_df(C, eps)
+    need = 8 * (n * naux * o + n * n * naux + 2 * o * o * naux + naux * naux)
+    with leave(need + 16 * MB):
+        got = eng.compute_forces_df(C, eps)
+    for a, b in zip(got, ref):
+        assert np.abs(a - b).max() < 1e-10 * max(1.0, np.abs(b).max())
