@@ -213,6 +213,14 @@ static std::vector<double> boys_poly_tables() {
   constexpr int NC = BOYSP_COEF, M = BOYSP_MMAX;
   const long double width = BOYSP_WIDTH, pi = acosl(-1.0L);
   std::vector<double> t((size_t)(M + 1) * BOYSP_SIZE);
+  // the same for every row and order: cosines of the Chebyshev sums and the powers
+  // of u = (T - mid) / (width / 2) in each Chebyshev polynomial
+  long double cs[NC][NC], tk[NC][NC] = {};
+  for (int k = 0; k < NC; ++k)
+    for (int j = 0; j < NC; ++j) cs[k][j] = (k == 0 ? 1.0L : 2.0L) / NC * cosl(pi * k * (j + 0.5L) / NC);
+  tk[0][0] = tk[1][1] = 1.0L;
+  for (int k = 2; k < NC; ++k)
+    for (int i = 0; i <= k; ++i) tk[k][i] = (i > 0 ? 2.0L * tk[k - 1][i - 1] : 0.0L) - tk[k - 2][i];
   for (int row = 0; row < BOYSP_ROWS; ++row) {
     const long double mid = row * width;
     long double f[M + 1][NC];  // F_m at the nodes (the first interval reaches below T = 0, where the series still holds)
@@ -227,21 +235,11 @@ static std::vector<double> boys_poly_tables() {
       for (int m = M - 1; m >= 0; --m) f[m][j] = (2.0L * T * f[m + 1][j] + ex) / (2 * m + 1);
     }
     for (int m = 0; m <= M; ++m) {
-      // Chebyshev coefficients, then powers of u = (T - mid) / (width / 2)
-      long double mono[NC] = {0}, t0[NC] = {0}, t1[NC] = {0};
-      t0[0] = 1.0L;
-      t1[1] = 1.0L;
+      long double mono[NC] = {};
       for (int k = 0; k < NC; ++k) {
         long double c = 0.0L;
-        for (int j = 0; j < NC; ++j) c += f[m][j] * cosl(pi * k * (j + 0.5L) / NC);
-        c *= (k == 0 ? 1.0L : 2.0L) / NC;
-        for (int i = 0; i < NC; ++i) mono[i] += c * t0[i];
-        long double t2[NC];  // T_{k+2} = 2 u T_{k+1} - T_k
-        for (int i = 0; i < NC; ++i) t2[i] = (i > 0 ? 2.0L * t1[i - 1] : 0.0L) - t0[i];
-        for (int i = 0; i < NC; ++i) {
-          t0[i] = t1[i];
-          t1[i] = t2[i];
-        }
+        for (int j = 0; j < NC; ++j) c += f[m][j] * cs[k][j];
+        for (int i = 0; i <= k; ++i) mono[i] += c * tk[k][i];
       }
       long double sc = 1.0L;
       for (int i = 0; i < NC; ++i, sc *= 2.0L / width)
