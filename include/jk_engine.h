@@ -187,6 +187,11 @@ int jk_df_mp2(jk_engine* e, const double* C, const double* eps, int nmo, int noc
  * counterpart; the engine's device must be current. */
 int jk_wait_selftest(jk_engine* e, unsigned polls, int* timed_out, int* completed_timed_out);
 
+/* Accuracy check of the Boys function every integral uses: F_0 .. F_m at the n
+ * arguments T >= 0 as a kernel of top order m (0 .. 9) evaluates them, at
+ * F[k * n + i].  No molecular2 counterpart (libint2 has its own). */
+int jk_boys_selftest(jk_engine* e, int m, const double* T, int n, double* F);
+
 /* Layout of the fitted tensor, chosen before jk_df_setup (molecular2 keeps one
  * packed FP64 (n(n+1)/2) x naux matrix, src/fockbuild.cpp:598-619, which
  * stops fitting in device memory near n = 2600, naux = 9600):

@@ -37,7 +37,7 @@ struct Grad3Params {
 
 template <int LP>
 struct Grad3Shared {
-  double boys[BOYSP_SIZE];
+  double boys[boysp_size(LP + 5)];  // orbital pairs up to dd
   double sphP[(2 * LP + 1) * ncart(LP)];
   double red[GRAD_THREADS / 32][3];
 };
@@ -52,6 +52,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad3(const Grad3Params P) 
   constexpr int NP = ncart(LP), NF = e3_nfun(LP, PURE), ND = ncart(LD), LCD = LC + LD, L = LP + LCD;
   constexpr bool TOP = LP <= 1 || PURE;
   constexpr int NG = TOP ? NP : nherm(LP);
+  static_assert(LCD <= 4, "the Boys table covers the ket");
   extern __shared__ __align__(16) unsigned char g3_sm[];
   Grad3Shared<LP>& S = *reinterpret_cast<Grad3Shared<LP>*>(g3_sm);
   double* s_g = reinterpret_cast<double*>(g3_sm + ((sizeof(Grad3Shared<LP>) + 15) & ~(size_t)15));
@@ -229,7 +230,7 @@ template <int LP, bool PP, int LQ, bool PQ>
 __global__ void __launch_bounds__(G2_THREADS) k_grad2(const Grad2Params P) {
   constexpr int NP = ncart(LP), NQ = ncart(LQ), FP = e3_nfun(LP, PP), FQ = e3_nfun(LQ, PQ), L = LP + LQ + 1;
   constexpr bool TOP = (LP <= 1 || PP) && (LQ <= 1 || PQ);
-  __shared__ double boys[BOYSP_SIZE];
+  __shared__ double boys[boysp_size(L)];
   __shared__ double sphP[FP * NP], sphQ[FQ * NQ];
   const int tid = threadIdx.x, lane = tid & 31;
   load_boys<L>(boys, P.boysp);

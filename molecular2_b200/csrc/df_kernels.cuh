@@ -60,7 +60,7 @@ __host__ __device__ constexpr bool e3_full(int la, int lb, int lp, bool pure) {
 
 template <int LA, int LB, int LP>
 struct Eri3Shared {
-  double boys[BOYSP_SIZE];
+  double boys[boysp_size(LA + LB + LP)];
   BraShared<LA, LB> bra;
   double sphP[(2 * LP + 1) * ncart(LP)];
   double red[E3_THREADS / 32][nherm(LA + LB)];
@@ -369,7 +369,7 @@ template <int LP, bool PP, int LQ, bool PQ>
 __global__ void __launch_bounds__(E2_THREADS) k_eri2(const Eri2Params P) {
   constexpr int NP = ncart(LP), NQ = ncart(LQ), FP = e3_nfun(LP, PP), FQ = e3_nfun(LQ, PQ), L = LP + LQ;
   constexpr bool TOP = (LP <= 1 || PP) && (LQ <= 1 || PQ);
-  __shared__ double boys[BOYSP_SIZE];
+  __shared__ double boys[boysp_size(L)];
   __shared__ double sphP[FP * NP], sphQ[FQ * NQ];
   const int tid = threadIdx.x;
   load_boys<L>(boys, P.boysp);

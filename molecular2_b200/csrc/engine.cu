@@ -243,11 +243,25 @@ static std::vector<double> boys_poly_tables() {
       }
       long double sc = 1.0L;
       for (int i = 0; i < NC; ++i, sc *= 2.0L / width)
-        t[(size_t)m * BOYSP_SIZE + row * NC + i] = (double)(mono[i] * sc);
-      t[(size_t)m * BOYSP_SIZE + BOYSP_ROWS * NC + row] = (double)expl(-mid);
+        t[(size_t)m * BOYSP_SIZE + row * BOYSP_ROW + i] = (double)(mono[i] * sc);
+      t[(size_t)m * BOYSP_SIZE + row * BOYSP_ROW + NC] = (double)expl(-mid);
     }
   }
   return t;
+}
+
+// F_0 .. F_M at T[i] from the table of order M, at F[m n + i].
+template <int M>
+__global__ void k_boys(int n, const double* __restrict__ T, const double* __restrict__ boysp, double* __restrict__ F) {
+  __shared__ double tab[boysp_size(M)];
+  load_boys<M>(tab, boysp);
+  __syncthreads();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double f[M + 1];
+  boys_poly<M>(T[i], tab, f);
+#pragma unroll
+  for (int m = 0; m <= M; ++m) F[(size_t)m * n + i] = f[m];
 }
 
 // ---------------------------------------------------------------- transforms
@@ -469,6 +483,24 @@ long long jk_last_quartets(const jk_engine* e) {
   if (cudaMemcpyAsync(&c, e->last_counter, sizeof(c), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess) return -1;
   if (cudaStreamSynchronize(e->stream) != cudaSuccess) return -1;
   return (long long)c;
+}
+
+int jk_boys_selftest(jk_engine* e, int m, const double* T, int n, double* F) {
+  if (!e || !T || !F) return JK_ERR_ARG;
+  if (m < 0 || m > BOYSP_MMAX || n < 1) return set_error(e, JK_ERR_ARG, "jk_boys_selftest: order or count out of range");
+  DevBuf<double> dT, dF;
+  cudaError_t st = dT.alloc(n);
+  if (st == cudaSuccess) st = dF.alloc((size_t)(m + 1) * n);
+  if (st == cudaSuccess) st = cudaMemcpyAsync(dT.p, T, sizeof(double) * n, cudaMemcpyHostToDevice, e->stream);
+  if (st != cudaSuccess) return check_cuda(e, st, "jk_boys_selftest");
+  static decltype(&k_boys<0>) const k[BOYSP_MMAX + 1] = {k_boys<0>, k_boys<1>, k_boys<2>, k_boys<3>, k_boys<4>,
+                                                        k_boys<5>, k_boys<6>, k_boys<7>, k_boys<8>, k_boys<9>};
+  k[m]<<<(n + 127) / 128, 128, 0, e->stream>>>(n, dT.p, e->boysp.p, dF.p);
+  st = cudaGetLastError();
+  if (st == cudaSuccess)
+    st = cudaMemcpyAsync(F, dF.p, sizeof(double) * (m + 1) * (size_t)n, cudaMemcpyDeviceToHost, e->stream);
+  if (st == cudaSuccess) st = cudaStreamSynchronize(e->stream);
+  return check_cuda(e, st, "jk_boys_selftest");
 }
 
 }  // extern "C"

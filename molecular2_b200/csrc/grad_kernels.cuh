@@ -41,7 +41,7 @@ constexpr int GRAD_ATOMS = 512;  // atoms whose gradient a block sums in shared 
 
 template <int LA, int LB>
 struct GradShared {
-  double boys[BOYSP_SIZE];
+  double boys[boysp_size(2 * (LA + LB) + 1)];
   BraGradShared<LA, LB> bra;
   double Dab[ncart(LA) * ncart(LB)];
   double red[GRAD_THREADS / 32][6];
@@ -65,6 +65,7 @@ template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad2e(const Grad2eParams P) {
   constexpr int NA = ncart(LA), NB = ncart(LB), ND = ncart(LD), NAB = NA * NB;
   constexpr int LAB = LA + LB, LCD = LC + LD, L = LAB + LCD, HAB = nherm(LAB);
+  static_assert(LCD <= LAB, "the bra's Boys table covers the ket");
   extern __shared__ __align__(16) unsigned char grad_sm[];
   GradShared<LA, LB>& S = *reinterpret_cast<GradShared<LA, LB>*>(grad_sm);
   double* s_g = reinterpret_cast<double*>(grad_sm + ((sizeof(GradShared<LA, LB>) + 15) & ~(size_t)15));

@@ -118,7 +118,7 @@ constexpr double JK_PRIM_EPS = 1e-21;
 
 template <int LA, int LB>
 struct JKShared {
-  double boys[BOYSP_SIZE];
+  double boys[boysp_size(2 * (LA + LB))];  // no ket class is above the bra's
   BraShared<LA, LB> bra;
   double Dab[2][ncart(LA) * ncart(LB)];
   int list[JK_LIST + JK_THREADS];
@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(JK_THREADS) k_jk_direct(const JKParams P) {
   constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD), NAB = NA * NB;
   constexpr int LAB = LA + LB, LCD = LC + LD, L = LAB + LCD, HAB = nherm(LAB);
   constexpr int MODE = jk_mode(LA, LB, LC, LD);
+  static_assert(LCD <= LAB, "the bra's Boys table covers the ket");
   constexpr int GC = MODE == JK_FULL ? NC : 1, GD = MODE == JK_ONE ? 1 : ND, G = GC * GD;
   extern __shared__ __align__(16) unsigned char jk_sm[];
   JKShared<LA, LB>& S = *reinterpret_cast<JKShared<LA, LB>*>(jk_sm);
@@ -459,7 +460,7 @@ constexpr int SCHWARZ_PRIMS = 8;
 template <int LA, int LB>
 struct SchwarzShared {
   static constexpr int NF = ncart(LA) * ncart(LB), H = nherm(LA + LB);
-  double boys[BOYSP_SIZE];
+  double boys[boysp_size(2 * (LA + LB))];
   double prim[2][SCHWARZ_PRIMS][5];      // p, P, K'
   double E[SCHWARZ_PRIMS][3][e1_size(LA, LB)];
   double M[2][SCHWARZ_PRIMS][NF * H];    // [function pair][h]

@@ -67,7 +67,7 @@ __device__ __forceinline__ void cart_exps(int i, int* e) {
 
 template <int LA, int LB>
 struct OneBodyShared {
-  double boys[BOYSP_SIZE];
+  double boys[boysp_size(LA + LB)];
   BraShared<LA, LB> bra;
   double E0[ENTRY_PRIMS][3][(LA + 1) * (LB + 3)];
   double Rs[ENTRY_PRIMS][nherm(LA + LB)];  // sum over nuclei of -Z R
@@ -177,7 +177,7 @@ constexpr int G1_ATOMS = 2048;  // atoms whose gradient a block sums in shared m
 
 template <int LA, int LB>
 struct Grad1eShared {
-  double boys[BOYSP_SIZE];
+  double boys[boysp_size(LA + LB + 1)];
   BraGradShared<LA, LB> bra;
   double E0[ENTRY_PRIMS][3][(LA + 2) * (LB + 3)];
   double G[ENTRY_PRIMS][4][nherm(LA + LB)];  // sum over ab of D_ab M, and of the d/dR tables

@@ -99,37 +99,51 @@ __device__ __forceinline__ int pack_kets(int start, int end, int have, int* list
 }
 
 // ---------------------------------------------------------------- Boys
-// F_M by a degree-8 polynomial in T - centre on intervals of width 3/8 centred
+// F_M by a degree-9 polynomial in T - centre on intervals of width 3/8 centred
 // on its multiples, up to T = 36 + 3M; e^{-T} from a table at the centres times
 // a degree-9 polynomial; then downward recursion
-// F_m = (2T F_{m+1} + e^{-T})/(2m+1).  From 36 + 3M on, F_M is its leading
-// asymptotic term (what that drops is below 2e-16 of F_M) and e^{-T} is nothing.
-// The table of one order (9 coefficients a row and e^{-centre}) is staged in
-// shared memory: ten 8-byte reads with few bank conflicts, against seven L1
-// gathers and a call of exp for a Taylor table.  A kernel with exp() in both
-// branches of the asymptotic test and the library's rsqrt ran 280 instructions
-// per (ps|ss) primitive quartet, 85 of them FP64.  Both polynomials interpolate
-// at Chebyshev nodes: errors below 2e-16 of F_M and 4e-17 of e^{-T}.
+// F_m = (2T F_{m+1} + e^{-T})/(2m+1).  From 36 + 3M on, F_m is its leading
+// asymptotic term (what that drops is below 3e-17 of F_m).
+// The table of one order (a row: 10 coefficients, e^{-centre}; 11 words, so that
+// rows start in different banks) is staged in shared memory: eleven 8-byte reads,
+// against seven L1 gathers and a call of exp for a Taylor table.  A kernel with
+// exp() in both branches of the asymptotic test and the library's rsqrt ran 280
+// instructions per (ps|ss) primitive quartet, 85 of them FP64.  Both polynomials
+// interpolate at Chebyshev nodes; what they leave is below 2e-17 of F_M and 4e-17
+// of e^{-T}.  Largest relative error in double arithmetic, of F_M below 36 + 3M:
+// 2.2e-16 for every M (a Taylor table of 7 terms and step 1/20: 2.4e-16 at M = 0,
+// 7.7e-16 at 4, 1.6e-15 at 9; nine coefficients: 6e-16 at 1, 2e-15 at 9); of all
+// F_m from there: 3.8e-16 at M = 1, 8.5e-16 at 4, 1.6e-15 at 9.  There the orders
+// are products of their own: downward recursion for both ranges gave 1.0e-15 at
+// M = 4 (the direct build of C20H42 44.4 ms with it, 44.65 so, 44.4 with nine
+// coefficients).
 constexpr double BOYSP_WIDTH = 0.375;
-constexpr int BOYSP_COEF = 9;
+constexpr int BOYSP_COEF = 10;
+constexpr int BOYSP_ROW = BOYSP_COEF + 1;
 constexpr int BOYSP_MMAX = 9;   // orders 0..9
 constexpr double boysp_tmax(int m) { return 36.0 + 3.0 * m; }
 constexpr int boysp_rows(int m) { return (int)(boysp_tmax(m) / BOYSP_WIDTH + 0.5) + 1; }
+constexpr int boysp_size(int m) { return boysp_rows(m) * BOYSP_ROW; }  // table of order m
 constexpr int BOYSP_ROWS = boysp_rows(BOYSP_MMAX);
-constexpr int BOYSP_SIZE = BOYSP_ROWS * (BOYSP_COEF + 1);  // polynomials, then e^{-centre}
+constexpr int BOYSP_SIZE = boysp_size(BOYSP_MMAX);                     // distance of the orders' tables
+// Gamma(m + 1/2) / 2
+__host__ __device__ constexpr double boys_gamma(int m) {
+  constexpr double g[BOYSP_MMAX + 1] = {0.886226925452758,  0.443113462726379,  0.6646701940895685, 1.6616754852239213,
+                                        5.815864198283724,  26.17138889227676,  143.94263890752217, 935.6271528988942,
+                                        7017.2036467417065, 59646.230997304505};
+  return g[m];
+}
 
 // The table of order M to shared memory; a barrier must follow.
 template <int M>
 __device__ __forceinline__ void load_boys(double* dst, const double* __restrict__ all) {
   const double* src = all + (size_t)M * BOYSP_SIZE;
-  for (int i = threadIdx.x; i < boysp_rows(M) * BOYSP_COEF; i += blockDim.x) dst[i] = __ldg(src + i);
-  if constexpr (M > 0)
-    for (int i = threadIdx.x; i < boysp_rows(M); i += blockDim.x)
-      dst[BOYSP_ROWS * BOYSP_COEF + i] = __ldg(src + BOYSP_ROWS * BOYSP_COEF + i);
+  for (int i = threadIdx.x; i < boysp_size(M); i += blockDim.x) dst[i] = __ldg(src + i);
 }
 
-// x^{-1/2} for x well inside the range of float: the single-precision estimate
-// and one step of third order (relative error e -> 5/16 e^3, e < 2^-21).
+// x^{-1/2} for x well inside the range of float: the single-precision estimate y
+// times the binomial series of (1 - h)^{-1/2}, h = 1 - x y^2, to its second order
+// (relative error e -> 5/2 e^3, e < 2^-21).
 __device__ __forceinline__ double rsqrt_pos(double x) {
   const double y = (double)rsqrtf((float)x);
   const double h = 1.0 - x * y * y;
@@ -139,13 +153,12 @@ __device__ __forceinline__ double rsqrt_pos(double x) {
 template <int M>
 __device__ __forceinline__ void boys_poly(double T, const double* tab, double* F) {
   static_assert(M <= BOYSP_MMAX, "Boys order too high");
-  double e = 0.0;
   if (T < boysp_tmax(M)) {
     // nearest multiple of the width, by the rounding of an addition to 1.5 2^52
     const double u = T * (1.0 / BOYSP_WIDTH) + 6755399441055744.0;
     const int row = __double2loint(u);
     const double d = T - (u - 6755399441055744.0) * BOYSP_WIDTH;
-    const double* c = tab + row * BOYSP_COEF;
+    const double* c = tab + row * BOYSP_ROW;
     double acc = c[BOYSP_COEF - 1];
 #pragma unroll
     for (int j = BOYSP_COEF - 2; j >= 0; --j) acc = acc * d + c[j];
@@ -161,19 +174,19 @@ __device__ __forceinline__ void boys_poly(double T, const double* tab, double* F
       x = x * d + 0.49999999999995886287;
       x = x * d - 1.0;
       x = x * d + 1.0;
-      e = x * tab[BOYSP_ROWS * BOYSP_COEF + row];
+      const double e = x * c[BOYSP_COEF], T2 = 2.0 * T;
+#pragma unroll
+      for (int m = M - 1; m >= 0; --m) F[m] = (T2 * F[m + 1] + e) * (1.0 / (2 * m + 1));
     }
-  } else {
-    const double r = rsqrt_pos(T), r2 = r * r;
-    double f = 0.886226925452758014 * r;  // Gamma(M + 1/2)/2 T^{-M-1/2}
+  } else {  // Gamma(m + 1/2)/2 T^{-m-1/2}
+    const double r = rsqrt_pos(T);
+    double f = r, r2 = r * r;
+    r2 = r2 + r2 * (1.0 - T * r2);  // r's rounding would be in every factor
 #pragma unroll
-    for (int m = 0; m < M; ++m) f *= (m + 0.5) * r2;
-    F[M] = f;
-  }
-  if constexpr (M > 0) {
-    const double T2 = 2.0 * T;
-#pragma unroll
-    for (int m = M - 1; m >= 0; --m) F[m] = (T2 * F[m + 1] + e) * (1.0 / (2 * m + 1));
+    for (int m = 0; m <= M; ++m) {
+      F[m] = boys_gamma(m) * f;
+      f *= r2;
+    }
   }
 }
 

@@ -52,6 +52,7 @@ SIGNATURES = {
     "jk_df_mp2": (_I, [_P, _P, _P, _I, _I, _I, _P]),
     "jk_wait_selftest": (_I, [_P, ctypes.c_uint, ctypes.POINTER(_I), ctypes.POINTER(_I)]),
     "jk_release_cached": (_I, [_I]),
+    "jk_boys_selftest": (_I, [_P, _I, _P, _I, _P]),
     "jk_df_storage": (_I, [_P]),
     "jk_df_tensor_bytes": (ctypes.c_longlong, [_P]),
     "jk_df_set_tiled_blocks": (_I, [_P, _I, _I]),
@@ -261,6 +262,13 @@ class IntegralEngine:
         a, b = _I(-1), _I(-1)
         self._check(self.lib.jk_wait_selftest(self.h, polls, ctypes.byref(a), ctypes.byref(b)))
         return bool(a.value), bool(b.value)
+
+    def boys_selftest(self, m, T):
+        """F_0 .. F_m at the arguments T, (m + 1) x len(T), as a kernel of top order m evaluates them."""
+        T = np.ascontiguousarray(T, dtype=np.float64)
+        F = np.zeros((m + 1, T.size))
+        self._check(self.lib.jk_boys_selftest(self.h, m, _p(T), T.size, _p(F)))
+        return F
 
     DF_STORAGE = {"auto": 0, "unpacked": 1, "tiled": 2}
 
