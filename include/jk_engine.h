@@ -77,7 +77,12 @@ int jk_schwarz(const jk_engine* e, double* Q);
 /* Integral-direct J[D] and K[D] (both w.r.t. the full D passed in, scaled by
  * `multiplier`), FP64, Schwarz x density screening at `precision`:
  * Fock::formJKdirect(Schwarz, D, multiplier) (src/fockbuild.cpp:64-164);
- * the caller forms jkints = J - 0.5 K as :163 does. Host pointers. */
+ * the caller forms jkints = J - 0.5 K as :163 does. Host pointers.
+ * `precision` also bounds the primitive quartets inside a shell quartet: those
+ * with a prefactor below min(1e-21, 1e-9 precision) may be skipped;
+ * 0 means every shell quartet and every listed primitive pair (primitive pairs
+ * with |K| < 1e-18 are never listed).  The same holds for every call with a
+ * `precision` below. */
 int jk_direct(jk_engine* e, const double* D, double precision, double multiplier, double* J, double* K);
 int jk_direct_device(jk_engine* e, const double* dD, double precision, double multiplier, double* dJ,
                      double* dK, void* stream);

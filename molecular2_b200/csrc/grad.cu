@@ -122,6 +122,7 @@ int grad_rhf_device(jk_engine* e, const double* dD, const double* dW, double pre
   P.Dc = Dc.p;
   P.nc = nc;
   P.precision = precision;
+  P.eps = prim_eps(precision);
   P.boysp = e->boysp.p;
   P.grad = g2e;
   P.natom = na;

@@ -27,7 +27,7 @@ struct Grad2eParams {
   const double* Dmax;
   const double* Dc;    // Cartesian density, nc x nc
   int nc;
-  double precision;
+  double precision, eps;  // eps: prim_eps(precision)
   const double* boysp;
   double* grad;        // 3 * natom
   int natom;
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad2e(const Grad2eParams P
         const double ga = entry_field(kp, min(k, nk - 1), 6);
         next = load_ket<true>(kp, min(k + 1, nk - 1));
         const double KK = k < nk && active ? Kb * kq.K : 0.0;
-        if (!__any_sync(0xffffffffu, fabs(KK) > JK_PRIM_EPS)) break;  // largest first: the rest is smaller
+        if (!__any_sync(0xffffffffu, fabs(KK) > P.eps)) break;  // largest first: the rest is smaller
         const double q = kq.q, h2 = kq.h;
         const double Q[3] = {kq.x, kq.y, kq.z};
         double R[nherm(L + 1)];

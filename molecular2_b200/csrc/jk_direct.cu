@@ -348,6 +348,7 @@ int direct_jk_device(jk_engine* e, const double* dD, double precision, double mu
   P.Kc = e->Kcart.p;
   P.dstride = (size_t)nc * nc;
   P.precision = precision;
+  P.eps = prim_eps(precision);
   P.boysp = e->boysp.p;
   P.counter = counter;
   const cudaError_t launched = launch_classes(e, s, [&](int A, int B, cudaStream_t cs) {
@@ -398,6 +399,7 @@ int direct_jk_uhf_device(jk_engine* e, const double* dDa, const double* dDb, dou
   P.Kc = Kc2.p;
   P.dstride = ncc;
   P.precision = precision;
+  P.eps = prim_eps(precision);
   P.boysp = e->boysp.p;
   P.counter = counter;
   if ((st = e->class_work.alloc(3 * NPAIRCLASS * NPAIRCLASS)) != cudaSuccess)
@@ -497,6 +499,7 @@ int direct_jk_noalloc(jk_engine* e, const double* dD, double precision, double m
   P.Jc = Jc;
   P.Kc = Kc;
   P.precision = precision;
+  P.eps = prim_eps(precision);
   P.boysp = e->boysp.p;
   P.counter = counter;
   P.dstride = NOALLOC_CC;

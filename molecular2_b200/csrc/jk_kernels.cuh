@@ -55,7 +55,7 @@ struct JKParams {
   double* Jc;           // raw accumulators (nden of each, dstride apart)
   double* Kc;
   size_t dstride;       // elements between consecutive densities / accumulators
-  double precision;
+  double precision, eps;  // eps: prim_eps(precision)
   const double* boysp;  // polynomial Boys tables, BOYSP_SIZE doubles per order
   unsigned long long* counter;
   unsigned long long* work;  // NULL or this class pair's [quartets, sum bra primitive pairs, sum primitive quartets]
@@ -112,9 +112,12 @@ __host__ __device__ constexpr int jk_layers(int la, int lb, int lc, int ld) {
 }
 constexpr int JK_THREADS = 128;
 constexpr int JK_LIST = 1024;      // ket entries screened and packed at a time
-// primitive quartets whose prefactor is below this in every lane are skipped
-// (their integrals are below 1e-18, like the primitive pairs never listed)
-constexpr double JK_PRIM_EPS = 1e-21;
+// Primitive quartets whose prefactor is below this in every lane of a warp are
+// skipped.  The line follows the caller's threshold: an integral is its prefactor
+// times the density and the expansions' |P - A|, 1/(2p), ... (up to four factors a
+// side, above 1e3 in all for diffuse distant pairs), and nine decades below the
+// threshold leave room for both.  precision = 0 skips nothing but exact zeros.
+inline double prim_eps(double precision) { return precision < 1e-12 ? 1e-9 * precision : 1e-21; }
 
 template <int LA, int LB>
 struct JKShared {
@@ -272,7 +275,7 @@ __global__ void __launch_bounds__(JK_THREADS) k_jk_direct(const JKParams P) {
         const KetPrim kq = next;  // the next primitive's loads run behind this one's arithmetic
         next = load_ket<(LCD > 0)>(kp, min(k + 1, nk - 1));
         const double KK = k < nk ? Kb * kq.K : 0.0;
-        if (!__any_sync(0xffffffffu, fabs(KK) > JK_PRIM_EPS)) break;  // largest first: the rest is smaller
+        if (!__any_sync(0xffffffffu, fabs(KK) > P.eps)) break;  // largest first: the rest is smaller
         const double Qx = kq.x, Qy = kq.y, Qz = kq.z;
         double R[nherm(L)];
         quartet_R<L>(p, kq.q, KK, Px - Qx, Py - Qy, Pz - Qz, S.boys, R);
