@@ -438,6 +438,8 @@ int one_body_device(jk_engine* e, double* S, double* T, double* V, cudaStream_t 
   // lists; their blocks are zero, not whatever the buffers held before
   for (double* M : {S, T, V})
     if (M) cudaMemsetAsync(M, 0, sizeof(double) * (size_t)n * n, s);
+  ClassStreams cs(e, s);  // the classes write disjoint blocks
+  LaunchStatus status;
   for (int pc = 0; pc < NPAIRCLASS; ++pc) {
     if (!e->pcls[pc].npair) continue;
     OneBodyParams P{};
@@ -457,8 +459,10 @@ int one_body_device(jk_engine* e, double* S, double* T, double* V, cudaStream_t 
     P.S = S;
     P.T = T;
     P.V = V;
-    if ((st = launch_onebody(pc, P, s)) != cudaSuccess) break;
+    status(launch_onebody(pc, P, cs.next(1.0)));
   }
+  cs.join();
+  st = status.st;
   if (st == cudaSuccess) st = cudaStreamSynchronize(s);  // Z, C die on return
   return check_cuda(e, st, "one_body");
 }

@@ -6,7 +6,7 @@ namespace m2 {
 template <int LA, int LB>
 static cudaError_t launch_onebody_class(const OneBodyParams& P, cudaStream_t s) {
   const size_t sm = sizeof(OneBodyShared<LA, LB>);
-  return launch_smem(k_onebody<LA, LB>, P.ent.nent, OB_THREADS, sm, sm, s, P);
+  return launch_smem(k_onebody<LA, LB>, P.pairs.npair, OB_THREADS, sm, sm, s, P);
 }
 
 cudaError_t launch_onebody(int pc, const OneBodyParams& P, cudaStream_t s) {
@@ -27,7 +27,7 @@ static cudaError_t launch_grad1e_class(const Grad1eParams& P, cudaStream_t s) {
   // a few blocks per SM walk over the entries, so that the per-atom sums leave
   // a block once
   const int blocks = P.ent.nent < 8 * 148 ? P.ent.nent : 8 * 148;
-  return launch_smem(k_grad1e<LA, LB>, blocks, OB_THREADS, sm, most, s, P);
+  return launch_smem(k_grad1e<LA, LB>, blocks, G1_THREADS, sm, most, s, P);
 }
 
 cudaError_t launch_grad1e(int pc, const Grad1eParams& P, cudaStream_t s) {

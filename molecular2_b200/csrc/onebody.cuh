@@ -8,7 +8,8 @@
 
 namespace m2 {
 
-constexpr int OB_THREADS = 64;
+constexpr int OB_THREADS = 128;  // of k_onebody
+constexpr int G1_THREADS = 64;   // of k_grad1e
 
 struct OneBodyParams {
   PairView pairs;
@@ -22,7 +23,7 @@ struct OneBodyParams {
   const double* Z;
   const double* cxyz;  // 3*natom
   int n;
-  double *S, *T, *V;   // n x n final basis, zeroed by the caller; T and V may both be NULL
+  double *S, *T, *V;   // n x n final basis, pairs that are not listed set to zero by the caller; T and V may both be NULL
 };
 
 // E^{ij}_0 of one direction for i <= LI, j <= LJ (all that overlap and kinetic
@@ -74,86 +75,100 @@ struct OneBodyShared {
   double blk[3][ncart(LA) * ncart(LB)];
 };
 
-// One block per pair entry.  A warp sums the Hermite integrals of one primitive
-// over the nuclei (lanes), a thread then forms one Cartesian element of S, T
-// and V; entries of one pair add up through atomics on the zeroed matrices.
+// One block per pair, entry by entry.  A warp sums the Hermite integrals of one
+// primitive over the nuclei (lanes), a thread then adds to its Cartesian element
+// of S, T and V.  Every element is summed by one thread in a fixed order and
+// written to both triangles, so that the matrices are the same in every run and
+// exactly symmetric.  Bound by the chain of a contracted pair's entries (11 of a
+// 9 x 9 contraction, 50 us for (H2O)8's ss class), which the classes' side streams
+// overlap: jk_one_body of (H2O)8/cc-pVDZ 0.34 ms, of H2O 0.14 (a block per entry
+// with atomics, the classes one after another: 0.39 and 0.17).
 template <int LA, int LB>
 __global__ void __launch_bounds__(OB_THREADS) k_onebody(const OneBodyParams P) {
   constexpr int NA = ncart(LA), NB = ncart(LB), NAB = NA * NB, L = LA + LB, H = nherm(L);
+  static_assert(NAB <= OB_THREADS, "a thread per Cartesian element");
   extern __shared__ __align__(16) unsigned char ob_sm[];
   OneBodyShared<LA, LB>& S = *reinterpret_cast<OneBodyShared<LA, LB>*>(ob_sm);
-  const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
-  const int ip = P.ent.pair[e], a = P.pairs.sa[ip], b = P.pairs.sb[ip], nb = P.ent.np[e];
+  const int ip = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+  const int a = P.pairs.sa[ip], b = P.pairs.sb[ip];
   const double A[3] = {P.ox[a], P.oy[a], P.oz[a]}, B[3] = {P.ox[b], P.oy[b], P.oz[b]};
-  const double* base = entry_prims(P.ent, e);
   const bool with_v = P.V != nullptr;
-  if (with_v)
-    load_boys<L>(S.boys, P.boysp);
-  for (int i = tid; i < nb * 3; i += OB_THREADS) {
-    const int x = i % 3;
-    const double X = entry_field(base, i / 3, 1 + x);
-    e0_table<LA, LB + 2>(X - A[x], X - B[x], entry_field(base, i / 3, 5), S.E0[i / 3][x]);
+  if (with_v) load_boys<L>(S.boys, P.boysp);
+  int ea[3] = {0, 0, 0}, eb[3] = {0, 0, 0};
+  if (tid < NAB) {
+    cart_exps<LA>(tid / NB, ea);
+    cart_exps<LB>(tid % NB, eb);
   }
-  load_bra<LA, LB>(S.bra, base, nb, A[0], A[1], A[2], B[0], B[1], B[2]);
-  if (with_v) {
-    for (int ib = tid >> 5; ib < nb; ib += OB_THREADS / 32) {
-      const double* q = S.bra.prim[ib];
-      double acc[H];
+  double s = 0.0, t = 0.0, v = 0.0;
+  for (int e = P.ent.first[ip]; e < P.ent.first[ip + 1]; ++e) {
+    const int nb = P.ent.np[e];
+    const double* base = entry_prims(P.ent, e);
+    __syncthreads();  // the entry before is done with
+    for (int i = tid; i < nb * 3; i += OB_THREADS) {
+      const int x = i % 3;
+      const double X = entry_field(base, i / 3, 1 + x);
+      e0_table<LA, LB + 2>(X - A[x], X - B[x], entry_field(base, i / 3, 5), S.E0[i / 3][x]);
+    }
+    load_bra<LA, LB>(S.bra, base, nb, A[0], A[1], A[2], B[0], B[1], B[2]);
+    if (with_v) {
+      for (int ib = tid >> 5; ib < nb; ib += OB_THREADS / 32) {
+        const double* q = S.bra.prim[ib];
+        double acc[H];
 #pragma unroll
-      for (int h = 0; h < H; ++h) acc[h] = 0.0;
-      for (int c = lane; c < P.natom; c += 32) {
-        double R[H];
-        hermite_R<L>(q[0], -P.Z[c], q[1] - P.cxyz[3 * c], q[2] - P.cxyz[3 * c + 1], q[3] - P.cxyz[3 * c + 2], S.boys,
-                     R);
+        for (int h = 0; h < H; ++h) acc[h] = 0.0;
+        for (int c = lane; c < P.natom; c += 32) {
+          double R[H];
+          hermite_R<L>(q[0], -P.Z[c], q[1] - P.cxyz[3 * c], q[2] - P.cxyz[3 * c + 1], q[3] - P.cxyz[3 * c + 2],
+                       S.boys, R);
 #pragma unroll
-        for (int h = 0; h < H; ++h) acc[h] += R[h];
+          for (int h = 0; h < H; ++h) acc[h] += R[h];
+        }
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) acc[h] += __shfl_down_sync(0xffffffffu, acc[h], o);
+          if (lane == 0) S.Rs[ib][h] = acc[h];
+        }
       }
-#pragma unroll
-      for (int h = 0; h < H; ++h) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc[h] += __shfl_down_sync(0xffffffffu, acc[h], o);
-        if (lane == 0) S.Rs[ib][h] = acc[h];
+      __syncthreads();
+    }
+    if (tid < NAB) {
+      for (int ib = 0; ib < nb; ++ib) {
+        const double p = S.bra.prim[ib][0], K = S.bra.prim[ib][4] * p / SQRT_PI25X2();
+        const double be = p - entry_field(base, ib, 6), pip = M_PI / p, ov = K * pip * sqrt(pip);
+        double o[3], k[3];
+        for (int x = 0; x < 3; ++x) {
+          o[x] = S.E0[ib][x][ea[x] * (LB + 3) + eb[x]];
+          k[x] = kin1(S.E0[ib][x], LB + 3, ea[x], eb[x], be);
+        }
+        s += ov * o[0] * o[1] * o[2];
+        t += ov * (k[0] * o[1] * o[2] + o[0] * k[1] * o[2] + o[0] * o[1] * k[2]);
+        if (with_v) v += 2.0 * M_PI / p * K * bra_component<LA, LB>(S.bra.M[L > 0 ? ib : 0], S.Rs[ib], tid);
       }
     }
-    __syncthreads();
   }
-  for (int i = tid; i < NAB; i += OB_THREADS) {
-    int ea[3], eb[3];
-    cart_exps<LA>(i / NB, ea);
-    cart_exps<LB>(i % NB, eb);
-    double s = 0.0, t = 0.0, v = 0.0;
-    for (int ib = 0; ib < nb; ++ib) {
-      const double p = S.bra.prim[ib][0], K = S.bra.prim[ib][4] * p / SQRT_PI25X2();
-      const double be = p - entry_field(base, ib, 6), pip = M_PI / p, ov = K * pip * sqrt(pip);
-      double o[3], k[3];
-      for (int x = 0; x < 3; ++x) {
-        o[x] = S.E0[ib][x][ea[x] * (LB + 3) + eb[x]];
-        k[x] = kin1(S.E0[ib][x], LB + 3, ea[x], eb[x], be);
-      }
-      s += ov * o[0] * o[1] * o[2];
-      t += ov * (k[0] * o[1] * o[2] + o[0] * k[1] * o[2] + o[0] * o[1] * k[2]);
-      if (with_v) v += 2.0 * M_PI / p * K * bra_component<LA, LB>(S.bra.M[L > 0 ? ib : 0], S.Rs[ib], i);
-    }
-    S.blk[0][i] = s;
-    S.blk[1][i] = t;
-    S.blk[2][i] = v;
+  if (tid < NAB) {
+    S.blk[0][tid] = s;
+    S.blk[1][tid] = t;
+    S.blk[2][tid] = v;
   }
   __syncthreads();
-  // final basis, both orientations
+  // final basis, both triangles
   const int pa = P.pure[a], pb = P.pure[b];
   const int fa = pa ? 2 * LA + 1 : NA, fb = pb ? 2 * LB + 1 : NB;
   const int a0 = P.foff[a], b0 = P.foff[b];
   double* outs[3] = {P.S, P.T, P.V};
   for (int i = tid; i < (with_v ? 3 : 1) * fa * fb; i += OB_THREADS) {
     const int k = i / (fa * fb), m = (i / fb) % fa, q = i % fb;
+    if (a == b && m < q) continue;  // (q, m) writes it
     double val = 0.0;
     for (int i1 = pa ? 0 : m; i1 < (pa ? NA : m + 1); ++i1) {
       const double ta = pa ? P.sph[sph_off(LA) + m * NA + i1] : 1.0;
       for (int j1 = pb ? 0 : q; j1 < (pb ? NB : q + 1); ++j1)
         val += ta * (pb ? P.sph[sph_off(LB) + q * NB + j1] : 1.0) * S.blk[k][i1 * NB + j1];
     }
-    atomicAdd(outs[k] + (size_t)(b0 + q) * P.n + a0 + m, val);
-    if (a != b) atomicAdd(outs[k] + (size_t)(a0 + m) * P.n + b0 + q, val);
+    outs[k][(size_t)(b0 + q) * P.n + a0 + m] = val;
+    outs[k][(size_t)(a0 + m) * P.n + b0 + q] = val;
   }
 }
 
@@ -181,7 +196,7 @@ struct Grad1eShared {
   BraGradShared<LA, LB> bra;
   double E0[ENTRY_PRIMS][3][(LA + 2) * (LB + 3)];
   double G[ENTRY_PRIMS][4][nherm(LA + LB)];  // sum over ab of D_ab M, and of the d/dR tables
-  double red[OB_THREADS / 32][6];
+  double red[G1_THREADS / 32][6];
 };
 
 // T'.D - 2 S'.W + V'.D.  Blocks walk over the pair entries; the density is
@@ -191,7 +206,7 @@ struct Grad1eShared {
 // with a Hermite sum per component and nucleus took 29 ms for (H2O)8, the six
 // launches now take under 1 ms.
 template <int LA, int LB>
-__global__ void __launch_bounds__(OB_THREADS) k_grad1e(const Grad1eParams P) {
+__global__ void __launch_bounds__(G1_THREADS) k_grad1e(const Grad1eParams P) {
   constexpr int NA = ncart(LA), NB = ncart(LB), NAB = NA * NB, L = LA + LB, H = nherm(L), LD = LB + 3;
   extern __shared__ __align__(16) unsigned char g1_sm[];
   Grad1eShared<LA, LB>& S = *reinterpret_cast<Grad1eShared<LA, LB>*>(g1_sm);
@@ -201,7 +216,7 @@ __global__ void __launch_bounds__(OB_THREADS) k_grad1e(const Grad1eParams P) {
   double* g_atom = local ? s_g : P.grad;
   load_boys<L + 1>(S.boys, P.boysp);
   if (local)
-    for (int i = tid; i < 3 * P.natom; i += OB_THREADS) s_g[i] = 0.0;
+    for (int i = tid; i < 3 * P.natom; i += G1_THREADS) s_g[i] = 0.0;
   for (int e = blockIdx.x; e < P.ent.nent; e += gridDim.x) {
     const int ip = P.ent.pair[e];
     if (!P.sig[ip]) continue;
@@ -211,13 +226,13 @@ __global__ void __launch_bounds__(OB_THREADS) k_grad1e(const Grad1eParams P) {
     const double A[3] = {P.ox[a], P.oy[a], P.oz[a]}, B[3] = {P.ox[b], P.oy[b], P.oz[b]};
     const double* base = entry_prims(P.ent, e);
     const int a0 = P.coff[a], b0 = P.coff[b];
-    for (int i = tid; i < nb * 3; i += OB_THREADS) {
+    for (int i = tid; i < nb * 3; i += G1_THREADS) {
       const int x = i % 3;
       const double X = entry_field(base, i / 3, 1 + x);
       e0_table<LA + 1, LB + 2>(X - A[x], X - B[x], entry_field(base, i / 3, 5), S.E0[i / 3][x]);
     }
     load_bra_grad<LA, LB>(S.bra, base, nb, A[0], A[1], A[2], B[0], B[1], B[2]);
-    for (int i = tid; i < nb * 4; i += OB_THREADS) {
+    for (int i = tid; i < nb * 4; i += G1_THREADS) {
       const double* M = S.bra.M[i / 4][i % 4];
       double g[H];
 #pragma unroll
@@ -234,7 +249,7 @@ __global__ void __launch_bounds__(OB_THREADS) k_grad1e(const Grad1eParams P) {
     __syncthreads();
     double gA[3] = {0, 0, 0}, gB[3] = {0, 0, 0};
     // nuclear attraction
-    for (int i = tid; i < nb * P.natom; i += OB_THREADS) {
+    for (int i = tid; i < nb * P.natom; i += G1_THREADS) {
       const int c = i % P.natom, ib = i / P.natom;
       const double* q = S.bra.prim[ib];
       double R[nherm(L + 1)];
@@ -260,7 +275,7 @@ __global__ void __launch_bounds__(OB_THREADS) k_grad1e(const Grad1eParams P) {
       }
     }
     // overlap and kinetic: d/dB = -d/dA
-    for (int i = tid; i < nb * NAB; i += OB_THREADS) {
+    for (int i = tid; i < nb * NAB; i += G1_THREADS) {
       const int ib = i / NAB, ia = (i % NAB) / NB, jb = i % NB;
       int ea[3], eb[3];
       cart_exps<LA>(ia, ea);
@@ -303,13 +318,13 @@ __global__ void __launch_bounds__(OB_THREADS) k_grad1e(const Grad1eParams P) {
     __syncthreads();
     if (tid < 6) {
       double v = 0.0;
-      for (int w = 0; w < OB_THREADS / 32; ++w) v += S.red[w][tid];
+      for (int w = 0; w < G1_THREADS / 32; ++w) v += S.red[w][tid];
       atomicAdd(g_atom + 3 * P.atom[tid < 3 ? a : b] + tid % 3, v);
     }
   }
   __syncthreads();
   if (local)
-    for (int i = tid; i < 3 * P.natom; i += OB_THREADS)
+    for (int i = tid; i < 3 * P.natom; i += G1_THREADS)
       if (s_g[i] != 0.0) atomicAdd(P.grad + i, s_g[i]);
 }
 

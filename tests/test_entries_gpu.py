@@ -82,3 +82,16 @@ def test_gradient_contraction_lengths(lens, spherical):
         [np.sum((T1[i] + V1[i]) * D) - 2.0 * np.sum(S1[i] * W) for i in range(3 * na)]).reshape(na, 3)
     assert max(np.abs(ref).max(), np.abs(ref2).max()) < 100.0
     assert max(np.abs(g - ref).max(), np.abs(g2 - ref2).max()) < 2e-11
+
+
+@pytest.mark.parametrize("spherical", [True, False])
+def test_one_body_is_symmetric_and_repeatable(spherical):
+    """To the last bit, also for pairs of up to 37 entries and within a shell."""
+    obs = basis([(0, 17), (1, 9), (2, 9), (0, 9), (2, 1)], spherical)
+    eng = IntegralEngine(obs)
+    ref = eng.one_body()
+    for M in ref:
+        assert np.array_equal(M, M.T)
+    for _ in range(5):
+        for M, R in zip(eng.one_body(), ref):
+            assert np.array_equal(M, R)
