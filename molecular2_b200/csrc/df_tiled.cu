@@ -1099,8 +1099,9 @@ static int tiled_fp64(jk_engine* e, const double* dC, int nocc, double* dJ, doub
   const int nch = (nocc + oc - 1) / oc;
   oc = (nocc + nch - 1) / nch;
   // where a second array of X's size fits easily, Y is formed at once and K reads
-  // it there; otherwise XB rows at a time, copied back over X'
-  const bool whole = 8.0 * (double)(npad + n) * naux * oc < 0.5 * (double)fr;
+  // it there; otherwise, and where the caller caps the slice, XB rows at a time,
+  // copied back over X'
+  const bool whole = T.oc_max == 0 && 8.0 * (double)(npad + n) * naux * oc < 0.5 * (double)fr;
   const int yrows = whole ? n : XB;
   DevBuf<double> X, Yb;
   st = X.alloc((size_t)npad * naux * oc);

@@ -281,7 +281,8 @@ class IntegralEngine:
 
     def set_tiled_blocks(self, waux_max=0, oc_max=0):
         """Caps on the mixed build's fitted-function block and the FP64 build's
-        occupied slice for tiled storage (0: sized from free device memory)."""
+        occupied slice for tiled storage (0: sized from free device memory).  A
+        capped slice is also transformed a few rows at a time."""
         self._check(self.lib.jk_df_set_tiled_blocks(self.h, waux_max, oc_max))
 
     @property
