@@ -26,7 +26,14 @@ int check_cuda(jk_engine* e, cudaError_t st, const char* what) {
 
 // Only the SCF driver needs the libraries; making and destroying the two handles
 // costs 5 ms, as much as everything else of a small engine.
+// They allocate device memory of their own, here and in their first calls, which
+// must not fail on what the block cache holds.
 int library_handles(jk_engine* e) {
+  constexpr size_t LIBRARY_BYTES = size_t(512) << 20;
+  if (!e->cublas || !e->cusolver) {
+    size_t fr = 0, tot = 0;
+    if (cudaMemGetInfo(&fr, &tot) == cudaSuccess && fr < LIBRARY_BYTES) jk_release_cached(e->device);
+  }
   if (!e->cublas && (cublasCreate(&e->cublas) != CUBLAS_STATUS_SUCCESS ||
                      cublasSetStream(e->cublas, e->stream) != CUBLAS_STATUS_SUCCESS))
     return set_error(e, JK_ERR_CUDA, "cublasCreate failed");

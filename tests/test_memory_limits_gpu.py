@@ -89,3 +89,22 @@ def test_df_gradient_in_the_memory_of_the_final_functions():
         got = eng.compute_forces_df(C, eps)
     for a, b in zip(got, ref):
         assert np.abs(a - b).max() < 1e-10 * max(1.0, np.abs(b).max())
+
+
+def test_scf_when_the_free_memory_is_in_the_cache():
+    """The first SCF of an engine makes the libraries' handles, which take device
+    memory of their own: with 8 MB free and the rest in the library's cache it runs."""
+    import torch
+    mol, obs, _, _ = system(2)
+    ref = IntegralEngine(obs).scf_rhf(mol.nocc, mol.enuc())[0].energy  # the libraries' code
+    eng = IntegralEngine(obs)
+    _, big, fit, C = system(8)
+    other = IntegralEngine(big, fit)
+    other.compute_forces_df(C, np.linspace(-1.0, -0.5, 40))
+    other.close()
+    torch.cuda.empty_cache()
+    t = torch.empty(free_bytes() - 8 * MB, dtype=torch.uint8, device="cuda")
+    r = eng.scf_rhf(mol.nocc, mol.enuc())[0]
+    del t
+    torch.cuda.empty_cache()
+    assert r.converged and abs(r.energy - ref) < 1e-6
