@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(E3_THREADS, 2) k_eri3(const Eri3Params P) {
   const int a = P.pairs.sa[ip], b = P.pairs.sb[ip];
   const int e0 = P.ent.first[ip], e1 = P.ent.first[ip + 1];
   const int f0 = blockIdx.y;  // the layer's function
-  load_boys<L>(S.boys, P.boysp);
+  load_boys<L, BOYSP_COEF_DF>(S.boys, P.boysp);
   if constexpr (PURE && LP > 1)
     for (int i = tid; i < NF * NP; i += blockDim.x) S.sphP[i] = P.sph[sph_off(LP) + i];
   const double A[3] = {P.ox[a], P.oy[a], P.oz[a]}, B[3] = {P.ox[b], P.oy[b], P.oz[b]};
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(E3_THREADS, 2) k_eri3(const Eri3Params P) {
           const int k = j0 + min(j, nj - 1);
           const double KK = j < nj ? q[4] * __ldg(P.aux.Kp + k) : 0.0;
           double R[nherm(L)];
-          quartet_R<L>(q[0], __ldg(P.aux.p + k), KK, q[1] - __ldg(P.aux.x + k), q[2] - __ldg(P.aux.y + k),
+          quartet_R<L, BOYSP_COEF_DF>(q[0], __ldg(P.aux.p + k), KK, q[1] - __ldg(P.aux.x + k), q[2] - __ldg(P.aux.y + k),
                        q[3] - __ldg(P.aux.z + k), S.boys, R);
           if constexpr (LP == 0) {
 #pragma unroll
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(E2_THREADS) k_eri2(const Eri2Params P) {
   __shared__ double boys[boysp_size(L)];
   __shared__ double sphP[FP * NP], sphQ[FQ * NQ];
   const int tid = threadIdx.x;
-  load_boys<L>(boys, P.boysp);
+  load_boys<L, BOYSP_COEF_DF>(boys, P.boysp);
   for (int i = tid; i < FP * NP; i += E2_THREADS)
     sphP[i] = PP && LP > 1 ? P.sph[sph_off(LP) + i] : (i / NP == i % NP ? 1.0 : 0.0);
   for (int i = tid; i < FQ * NQ; i += E2_THREADS)
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(E2_THREADS) k_eri2(const Eri2Params P) {
     for (int k = P.Q.prim_off[sQ]; k < P.Q.prim_off[sQ] + P.Q.nprim[sQ]; ++k) {
       const double hp = __ldg(P.P.h + j), hq = __ldg(P.Q.h + k);
       double R[nherm(L)];
-      quartet_R<L>(__ldg(P.P.p + j), __ldg(P.Q.p + k), __ldg(P.P.Kp + j) * __ldg(P.Q.Kp + k),
+      quartet_R<L, BOYSP_COEF_DF>(__ldg(P.P.p + j), __ldg(P.Q.p + k), __ldg(P.P.Kp + j) * __ldg(P.Q.Kp + k),
                    __ldg(P.P.x + j) - __ldg(P.Q.x + k), __ldg(P.P.y + j) - __ldg(P.Q.y + k),
                    __ldg(P.P.z + j) - __ldg(P.Q.z + k), boys, R);
       if constexpr (TOP) {

@@ -214,17 +214,17 @@ int upload_basis(jk_engine* e, const HostBasis& hb, DevBasis& db) {
 }
 
 // Polynomial Boys tables (quartet.cuh): per order and interval the polynomial of
-// degree BOYSP_COEF - 1 in (T - centre) that interpolates F_m at the interval's
-// Chebyshev nodes, in extended precision; then e^{-centre}.
-static std::vector<double> boys_poly_tables() {
-  constexpr int NC = BOYSP_COEF, M = BOYSP_MMAX;
+// degree NC - 1 in (T - centre) that interpolates F_m at the interval's Chebyshev
+// nodes, in extended precision, and e^{-centre}.
+template <int NC>
+static void boys_poly_tables(double* t) {
+  constexpr int M = BOYSP_MMAX;
   const long double width = BOYSP_WIDTH, pi = acosl(-1.0L);
-  std::vector<double> t((size_t)(M + 1) * BOYSP_SIZE);
   // the same for every row and order: cosines of the Chebyshev sums and the powers
   // of u = (T - mid) / (width / 2) in each Chebyshev polynomial
   long double cs[NC][NC], tk[NC][NC] = {};
   for (int k = 0; k < NC; ++k)
-    for (int j = 0; j < NC; ++j) cs[k][j] = (k == 0 ? 1.0L : 2.0L) / NC * cosl(pi * k * (j + 0.5L) / NC);
+    for (int j = 0; j < NC; ++j) cs[k][j] = cosl(pi * k * (j + 0.5L) / NC);
   tk[0][0] = tk[1][1] = 1.0L;
   for (int k = 2; k < NC; ++k)
     for (int i = 0; i <= k; ++i) tk[k][i] = (i > 0 ? 2.0L * tk[k - 1][i - 1] : 0.0L) - tk[k - 2][i];
@@ -246,14 +246,20 @@ static std::vector<double> boys_poly_tables() {
       for (int k = 0; k < NC; ++k) {
         long double c = 0.0L;
         for (int j = 0; j < NC; ++j) c += f[m][j] * cs[k][j];
+        c *= (k == 0 ? 1.0L : 2.0L) / NC;
         for (int i = 0; i <= k; ++i) mono[i] += c * tk[k][i];
       }
+      double* out = t + (size_t)m * BOYSP_SIZE + row * BOYSP_ROW;
       long double sc = 1.0L;
-      for (int i = 0; i < NC; ++i, sc *= 2.0L / width)
-        t[(size_t)m * BOYSP_SIZE + row * BOYSP_ROW + i] = (double)(mono[i] * sc);
-      t[(size_t)m * BOYSP_SIZE + row * BOYSP_ROW + NC] = (double)expl(-mid);
+      for (int i = 0; i < NC; ++i, sc *= 2.0L / width) out[i] = (double)(mono[i] * sc);
+      out[NC] = (double)expl(-mid);
     }
   }
+}
+static std::vector<double> boys_tables() {
+  std::vector<double> t(2 * (size_t)BOYSP_SET, 0.0);
+  boys_poly_tables<BOYSP_COEF>(t.data());
+  boys_poly_tables<BOYSP_COEF_DF>(t.data() + BOYSP_SET);
   return t;
 }
 
@@ -419,7 +425,7 @@ int jk_create(const jk_basis* obs, const jk_basis* aux, int natom, const double*
   rc = upload_basis(e, e->obs, e->dobs);
   if (rc == JK_OK && e->has_aux) rc = upload_basis(e, e->aux, e->daux);
   if (rc == JK_OK) {
-    static const std::vector<double> poly = boys_poly_tables();
+    static const std::vector<double> poly = boys_tables();
     rc = check_cuda(e, e->boysp.upload(poly, e->stream), "boys polynomials");
   }
   if (rc == JK_OK) rc = check_cuda(e, cudaStreamSynchronize(e->stream), "boys polynomials");

@@ -117,8 +117,16 @@ __device__ __forceinline__ int pack_kets(int start, int end, int have, int* list
 // are products of their own: downward recursion for both ranges gave 1.0e-15 at
 // M = 4 (the direct build of C20H42 44.4 ms with it, 44.65 so, 44.4 with nine
 // coefficients).
+//
+// The three- and two-index integrals (k_eri3, k_eri2) keep nine coefficients and
+// the asymptotic value of F_M carried down: the fitted tensor made of them is split
+// into BF16, and a last bit of B that rounds the other way is a step of 2^-17 of
+// its element there.  With ten coefficients J and K of a split-BF16 build move by
+// 1e-9 to 3e-9, at the same error against 64 bits (4.1e-6), and stored results of
+// such builds would no longer be met; FP64 results of the fitted builds carry the
+// metric's condition number times eps, some 1e-12, either way.
 constexpr double BOYSP_WIDTH = 0.375;
-constexpr int BOYSP_COEF = 10;
+constexpr int BOYSP_COEF = 10, BOYSP_COEF_DF = 9;
 constexpr int BOYSP_ROW = BOYSP_COEF + 1;
 constexpr int BOYSP_MMAX = 9;   // orders 0..9
 constexpr double boysp_tmax(int m) { return 36.0 + 3.0 * m; }
@@ -126,6 +134,7 @@ constexpr int boysp_rows(int m) { return (int)(boysp_tmax(m) / BOYSP_WIDTH + 0.5
 constexpr int boysp_size(int m) { return boysp_rows(m) * BOYSP_ROW; }  // table of order m
 constexpr int BOYSP_ROWS = boysp_rows(BOYSP_MMAX);
 constexpr int BOYSP_SIZE = boysp_size(BOYSP_MMAX);                     // distance of the orders' tables
+constexpr int BOYSP_SET = (BOYSP_MMAX + 1) * BOYSP_SIZE;               // ten coefficients, then nine
 // Gamma(m + 1/2) / 2
 __host__ __device__ constexpr double boys_gamma(int m) {
   constexpr double g[BOYSP_MMAX + 1] = {0.886226925452758,  0.443113462726379,  0.6646701940895685, 1.6616754852239213,
@@ -135,9 +144,9 @@ __host__ __device__ constexpr double boys_gamma(int m) {
 }
 
 // The table of order M to shared memory; a barrier must follow.
-template <int M>
+template <int M, int NC = BOYSP_COEF>
 __device__ __forceinline__ void load_boys(double* dst, const double* __restrict__ all) {
-  const double* src = all + (size_t)M * BOYSP_SIZE;
+  const double* src = all + (NC == BOYSP_COEF ? 0 : BOYSP_SET) + (size_t)M * BOYSP_SIZE;
   for (int i = threadIdx.x; i < boysp_size(M); i += blockDim.x) dst[i] = __ldg(src + i);
 }
 
@@ -150,18 +159,20 @@ __device__ __forceinline__ double rsqrt_pos(double x) {
   return y + y * h * (0.5 + 0.375 * h);
 }
 
-template <int M>
+template <int M, int NC = BOYSP_COEF>
 __device__ __forceinline__ void boys_poly(double T, const double* tab, double* F) {
   static_assert(M <= BOYSP_MMAX, "Boys order too high");
+  static_assert(NC == BOYSP_COEF || NC == BOYSP_COEF_DF, "no such table");
+  double e = 0.0;
   if (T < boysp_tmax(M)) {
     // nearest multiple of the width, by the rounding of an addition to 1.5 2^52
     const double u = T * (1.0 / BOYSP_WIDTH) + 6755399441055744.0;
     const int row = __double2loint(u);
     const double d = T - (u - 6755399441055744.0) * BOYSP_WIDTH;
     const double* c = tab + row * BOYSP_ROW;
-    double acc = c[BOYSP_COEF - 1];
+    double acc = c[NC - 1];
 #pragma unroll
-    for (int j = BOYSP_COEF - 2; j >= 0; --j) acc = acc * d + c[j];
+    for (int j = NC - 2; j >= 0; --j) acc = acc * d + c[j];
     F[M] = acc;
     if constexpr (M > 0) {
       double x = -2.7579345743837904673e-6;  // e^{-d}, |d| <= 3/16
@@ -174,11 +185,9 @@ __device__ __forceinline__ void boys_poly(double T, const double* tab, double* F
       x = x * d + 0.49999999999995886287;
       x = x * d - 1.0;
       x = x * d + 1.0;
-      const double e = x * c[BOYSP_COEF], T2 = 2.0 * T;
-#pragma unroll
-      for (int m = M - 1; m >= 0; --m) F[m] = (T2 * F[m + 1] + e) * (1.0 / (2 * m + 1));
+      e = x * c[NC];
     }
-  } else {  // Gamma(m + 1/2)/2 T^{-m-1/2}
+  } else if constexpr (NC == BOYSP_COEF) {  // Gamma(m + 1/2)/2 T^{-m-1/2}
     const double r = rsqrt_pos(T);
     double f = r, r2 = r * r;
     r2 = r2 + r2 * (1.0 - T * r2);  // r's rounding would be in every factor
@@ -187,15 +196,27 @@ __device__ __forceinline__ void boys_poly(double T, const double* tab, double* F
       F[m] = boys_gamma(m) * f;
       f *= r2;
     }
+    return;
+  } else {
+    const double r = rsqrt_pos(T), r2 = r * r;
+    double f = 0.886226925452758014 * r;
+#pragma unroll
+    for (int m = 0; m < M; ++m) f *= (m + 0.5) * r2;
+    F[M] = f;
+  }
+  if constexpr (M > 0) {
+    const double T2 = 2.0 * T;
+#pragma unroll
+    for (int m = M - 1; m >= 0; --m) F[m] = (T2 * F[m + 1] + e) * (1.0 / (2 * m + 1));
   }
 }
 
 // scale R_tuv (t + u + v <= L) for the reduced exponent a and distance (X, Y, Z).
-template <int L>
+template <int L, int NC = BOYSP_COEF>
 __device__ __forceinline__ void hermite_R(double a, double scale, double X, double Y, double Z, const double* tab,
                                           double* R) {
   double F[L + 1];
-  boys_poly<L>(a * (X * X + Y * Y + Z * Z), tab, F);
+  boys_poly<L, NC>(a * (X * X + Y * Y + Z * Z), tab, F);
   const double m2a = -2.0 * a;
   double pw = scale;
 #pragma unroll
@@ -227,11 +248,11 @@ __device__ __forceinline__ void hermite_R(double a, double scale, double X, doub
 }
 // The same for a primitive quartet with exponents p, q and prefactors KK =
 // K'_ab K'_cd: prefactor and reduced exponent from one reciprocal square root.
-template <int L>
+template <int L, int NC = BOYSP_COEF>
 __device__ __forceinline__ void quartet_R(double p, double q, double KK, double X, double Y, double Z,
                                           const double* tab, double* R) {
   const double r = rsqrt_pos(p + q);
-  hermite_R<L>(p * q * r * r, KK * r, X, Y, Z, tab, R);
+  hermite_R<L, NC>(p * q * r * r, KK * r, X, Y, Z, tab, R);
 }
 
 // ---------------------------------------------------------------- bra tables
