@@ -74,6 +74,7 @@ AuxView aux_group_view(const jk_engine* e, const int* shells, int count) {
 // pair class pc.
 static Eri3Params eri3_params(const jk_engine* e, int g, int pc) {
   Eri3Params P{};
+  P.nsm = e->nsm;
   P.aux = aux_group_view(e, e->aux_group[g].p, e->aux_group_count[g]);
   P.ent = entry_view(e->pcls[pc]);
   P.pairs = view(e->pcls[pc]);

@@ -101,6 +101,7 @@ static cudaError_t launch_grad3_all(jk_engine* e, const int* const* shells, cons
   LaunchStatus status;
   for (const Item& it : items) {
     Grad3Params P{};
+    P.nsm = e->nsm;
     P.aux = aux_group_view(e, shells[it.g], counts[it.g]);
     P.aux_atom = e->daux.atom.p;
     P.atom = e->dobs.atom.p;

@@ -19,6 +19,7 @@
 namespace m2 {
 
 struct Grad3Params {
+  int nsm;
   AuxView aux;            // fitting shells of one group
   const int* aux_atom;
   const int* atom;        // orbital shell -> atom
@@ -182,7 +183,7 @@ inline cudaError_t launch_grad3_class(const Grad3Params& P, cudaStream_t s) {
   const int layers = ncart(LC) * ncart(LD), chunks = (P.ent.nent + GRAD_THREADS - 1) / GRAD_THREADS;
   // blocks walk over several ket chunks where there are enough of them to fill the GPU
   int y = 1;
-  while (y < chunks && (long long)P.aux.count * layers * y < 16 * 148) ++y;
+  while (y < chunks && (long long)P.aux.count * layers * y < 16 * P.nsm) ++y;
   return launch_smem(k_grad3<LP, PURE, LC, LD>, dim3(P.aux.count, y, layers), GRAD_THREADS, sm, most, s, P);
 }
 template <int LP, bool PURE>

@@ -24,6 +24,7 @@ struct AuxView {
 AuxView aux_group_view(const jk_engine* e, const int* shells, int count);  // df.cu
 
 struct Eri3Params {
+  int nsm;
   AuxView aux;
   EntryView ent;          // orbital pairs of one class
   PairView pairs;
@@ -327,7 +328,7 @@ inline cudaError_t launch_eri3_class(const Eri3Params& P, bool j, cudaStream_t s
   const int layers = e3_full(LA, LB, LP, PURE) ? 1 : e3_nfun(LP, PURE);
   // one block walks over all fitting shells of a pair unless that leaves the GPU short of blocks
   int z = 1;
-  while (z < iters && (long long)P.nlist * layers * z < 8 * 148) ++z;
+  while (z < iters && (long long)P.nlist * layers * z < 8 * P.nsm) ++z;
   return launch_smem(k_eri3<LA, LB, LP, PURE>, dim3(P.nlist, layers, z), threads, sm, sm, s, P);
 }
 template <int LP, bool PURE>

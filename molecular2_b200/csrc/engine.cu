@@ -411,6 +411,7 @@ int jk_create(const jk_basis* obs, const jk_basis* aux, int natom, const double*
   e->Z.assign(Z, Z + natom);
   e->device = device;
   cudaError_t st = cudaSetDevice(device);
+  if (st == cudaSuccess) st = cudaDeviceGetAttribute(&e->nsm, cudaDevAttrMultiProcessorCount, device);
   if (st == cudaSuccess) st = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
   for (int i = 0; i < jk_engine::NCLS_STREAMS && st == cudaSuccess; ++i) {
     st = cudaStreamCreateWithFlags(&e->cls_stream[i], cudaStreamNonBlocking);

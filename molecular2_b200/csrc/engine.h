@@ -89,7 +89,7 @@ struct PairClassDev {
   DevSpan<int> sa, sb, prim_off, nprim;
   DevSpan<double> Q;
   // entries: slices of a pair's primitives (quartet.cuh)
-  int nent = 0, max_np = 0;
+  int nent = 0;
   DevSpan<int> ent_pair, ent_np, ent_first;
   DevSpan<long long> ent_goff;
   DevSpan<double> ent_prim;
@@ -149,6 +149,7 @@ struct TiledDF {
 
 struct jk_engine {
   int device = 0;
+  int nsm = 0;  // its multiprocessors: launch rules count blocks per SM
   cudaStream_t stream = nullptr;
   // side streams of the per-class kernel launches (direct J/K, gradient):
   // forked from and joined back to the call's stream with events

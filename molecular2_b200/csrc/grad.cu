@@ -50,7 +50,7 @@ static cudaError_t launch_grad2e(const jk_engine* e, int A, int B, const Grad2eP
   const long long layers = ncart(cb.la) * ncart(cb.lb), nbra = std::max(1, ca.nent / P.bra_step), nket = cb.nent;
   P.kchunk = GRAD_LIST;
   while (P.kchunk > 32 &&
-         nbra * ((nket + P.kchunk - 1) / P.kchunk) * layers < (P.kchunk > GRAD_THREADS ? 32 : 8) * 148)
+         nbra * ((nket + P.kchunk - 1) / P.kchunk) * layers < (P.kchunk > GRAD_THREADS ? 32 : 8) * e->nsm)
     P.kchunk /= 2;
   dim3 grid(ca.nent, (unsigned)((nket + P.kchunk - 1) / P.kchunk), (unsigned)layers);
   if (A <= 2) return launch_grad2e_bra_s(A, B, P, grid, s);
@@ -153,6 +153,7 @@ int grad_rhf_device(jk_engine* e, const double* dD, const double* dW, double pre
   for (int k = 0; k < NPAIRCLASS && with_1e; ++k) {
     if (!e->pcls[k].npair) continue;
     Grad1eParams Q{};
+    Q.nsm = e->nsm;
     Q.pairs = view(e->pcls[k]);
     Q.ent = entry_view(e->pcls[k]);
     Q.ox = e->dobs.x.p;

@@ -225,7 +225,6 @@ int build_pairs(jk_engine* e) {
     HostEntries E;
     build_entries(sorted, pp, E);
     d.nent = (int)E.pair.size();
-    d.max_np = E.np.empty() ? 0 : *std::max_element(E.np.begin(), E.np.end());
     pos[k] = Pos{append(ints, sorted.sa), append(ints, sorted.sb), append(ints, sorted.prim_off),
                  append(ints, sorted.nprim), append(dbls, sorted.Q), append(ints, E.pair), append(ints, E.np),
                  append(ints, E.first), append(offs, E.goff), 0};
@@ -258,10 +257,10 @@ int build_pairs(jk_engine* e) {
 // Ket entries per block: many, so that the bra set-up (Boys table, term
 // products) is shared, but fewer for classes whose blocks would not fill the
 // GPU otherwise.
-static int ket_chunk(long long nbra, long long nket, int layers) {
+static int ket_chunk(long long nbra, long long nket, int layers, int nsm) {
   int k = 4 * JK_LIST;
   nbra = std::max(nbra, 1LL);  // a rank's share of few entries; the grid's y limit is 65,535
-  while (k > 32 && nbra * ((nket + k - 1) / k) * layers < (k > JK_THREADS ? 32 : 8) * 148) k /= 2;
+  while (k > 32 && nbra * ((nket + k - 1) / k) * layers < (k > JK_THREADS ? 32 : 8) * nsm) k /= 2;
   return k;
 }
 
@@ -307,7 +306,7 @@ static cudaError_t launch_jk(const jk_engine* e, int A, int B, const JKParams& P
   P.bra_ent = entry_view(ca);
   P.ket_ent = entry_view(cb);
   P.same_class = (A == B);
-  P.kchunk = ket_chunk((long long)ca.nent / P.bra_step, cb.nent, jk_layers(ca.la, ca.lb, cb.la, cb.lb));
+  P.kchunk = ket_chunk((long long)ca.nent / P.bra_step, cb.nent, jk_layers(ca.la, ca.lb, cb.la, cb.lb), e->nsm);
   dim3 grid(ca.nent, (cb.nent + P.kchunk - 1) / P.kchunk);
   if (A <= 2) return launch_jk_bra_s(A, B, P, grid, s);
   if (A == 3) return launch_jk_bra_ds(B, P, grid, s);

@@ -26,7 +26,7 @@ static cudaError_t launch_grad1e_class(const Grad1eParams& P, cudaStream_t s) {
   const size_t sm = base + (P.natom <= G1_ATOMS ? 24 * (size_t)P.natom : 0);
   // a few blocks per SM walk over the entries, so that the per-atom sums leave
   // a block once
-  const int blocks = P.ent.nent < 8 * 148 ? P.ent.nent : 8 * 148;
+  const int blocks = P.ent.nent < 8 * P.nsm ? P.ent.nent : 8 * P.nsm;
   return launch_smem(k_grad1e<LA, LB>, blocks, G1_THREADS, sm, most, s, P);
 }
 

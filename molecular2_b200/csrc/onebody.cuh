@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(OB_THREADS) k_onebody(const OneBodyParams P) {
 }
 
 struct Grad1eParams {
+  int nsm;
   PairView pairs;
   EntryView ent;
   const double *ox, *oy, *oz;
