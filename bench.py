@@ -336,8 +336,9 @@ def measure_direct(local):
     q = eng.last_quartets()
     work = eng.last_class_work()
     eng.close()
-    # FP64 work of the build from the frozen per-class table (flops per bra
-    # primitive pair, per primitive quartet, per quartet of digestion)
+    # FP64 work of a plain evaluation of the build's quartets from the frozen
+    # per-class table (flops per bra primitive pair, per primitive quartet, per
+    # quartet of digestion); the kernels share tables and execute less
     table = json.load(open(os.path.join(ROOT, "molecular2_b200", "data", "flop_table.json")))["table"]
     flops = 0.0
     for A in range(6):
@@ -346,7 +347,10 @@ def measure_direct(local):
             nq, wb, wq = (float(x) for x in work[A, B])
             flops += t["bra"] * wb + t["quartet"] * wq + t["digest"] * nq
     fp64_peak = 40.0   # TFLOP/s, nominal B200 FP64 (no measured FP64 figure is available)
-    roof = {"kernel": "k_jk_direct (all classes)", "bound": "fp64", "flops_per_build": flops,
+    roof = {"kernel": "k_jk_direct (all classes)",
+            "bound": "l1 data path, half of it scattered fp64 atomics (profiles/direct_jk_c20h42.md); the rate below "
+                     "counts plain-evaluation flops, which the kernels do not all execute",
+            "flops_per_build": flops,
             "achieved_tflops": flops / (ms * 1e-3) / 1e12, "peak_tflops": fp64_peak, "peak_source": "nominal",
             "frac": flops / (ms * 1e-3) / 1e12 / fp64_peak,
             "work_model": "molecular2_b200/data/flop_table.json x jk_last_class_work counts"}

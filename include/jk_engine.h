@@ -274,7 +274,9 @@ typedef struct jk_scf_options {
   int mixed_refresh;       /* 0 (default): FP64 builds after the switch.  k > 0: mixed builds
                               plus the correction G64 - Gmixed refreshed every k iterations,
                               energy from a final FP64 build */
-  int eig_mode;            /* 0 = cuSOLVER syevd every iteration; 1 = Jacobi (syevj) on the
+  int eig_mode;            /* 0 = an own Jacobi solver in the previous eigenvectors from the second
+                              iteration on for up to 160 functions with none dropped, cuSOLVER
+                              syevd otherwise; 1 = Jacobi (syevj) on the
                               Fock matrix in the previous eigenvectors after the first */
   int maxiter;             /* molecular2 default 40 */
   int maxdiis;             /* default 8 */

@@ -59,7 +59,8 @@ struct GradShared {
 // same addresses would serialise).  Measured, the 21 class launches of
 // (H2O)8/cc-pVDZ: 340 -> 14 ms against six shifted quartet evaluations per
 // quartet with the integral block and its weights in local memory; the whole
-// call 372 -> 18 ms, 12.8 ms with the Boys table and cached device blocks.  Two blocks per SM are asked for because ptxas otherwise
+// call 372 -> 18 ms, 13.5 ms with the Boys table and cached device blocks.  Two
+// blocks per SM are asked for because ptxas otherwise
 // gives the dd classes 32 registers and 50 to 120 KB of spills.
 template <int LA, int LB, int LC, int LD>
 __global__ void __launch_bounds__(GRAD_THREADS, 2) k_grad2e(const Grad2eParams P) {

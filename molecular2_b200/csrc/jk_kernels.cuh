@@ -143,8 +143,8 @@ __host__ __device__ constexpr size_t jk_smem(int nden) {
 // src/fockbuild.cpp:266-362) are digested from the same integrals; the screen
 // uses the norms of their sum.
 // Measured (one thread per contracted quartet with its 6 to 81 integrals in
-// local memory -> this kernel): H2O/cc-pVDZ 18.0 -> 0.24 ms, (H2O)8/cc-pVDZ
-// 44.3 -> 4.4 ms, C20H42/6-311G** 262 -> 44 ms.  Of that, 52 -> 44 ms came from
+// local memory -> this kernel): H2O/cc-pVDZ 18.0 -> 0.25 ms, (H2O)8/cc-pVDZ
+// 44.3 -> 4.6 ms, C20H42/6-311G** 262 -> 45 ms.  Of that, 52 -> 44 ms came from
 // fewer instructions per primitive (Boys function, reciprocal square root), the
 // next primitive's loads issued ahead, and rounds of whole warps over the packed
 // list.  Tried and slower on C20H42: entries of 16 primitives (56 for 52 ms),
@@ -451,7 +451,7 @@ struct SchwarzParams {
 // One block per pair.  The Hermite expansions of the final functions' products
 // are formed for SCHWARZ_PRIMS primitives at a time, a thread takes primitive
 // quartets of one function pair: one thread per pair walked up to 6,561 of them
-// and the whole (ab|ab) block (creating the engine of (H2O)8: 32 ms, now 6.3 ms).
+// and the whole (ab|ab) block (creating the engine of (H2O)8: 32 ms, now 3.5 ms).
 // A thread keeps its function pair over the whole block and the partial sums are
 // added in a fixed order, so that the bounds are the same to the last bit in
 // every run: the ranks of a partitioned build (jk_direct_set_partition) each sort
