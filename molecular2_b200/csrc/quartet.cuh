@@ -115,8 +115,10 @@ __device__ __forceinline__ int pack_kets(int start, int end, int have, int* list
 // 7.7e-16 at 4, 1.6e-15 at 9; nine coefficients: 6e-16 at 1, 2e-15 at 9); of all
 // F_m from there: 3.8e-16 at M = 1, 8.5e-16 at 4, 1.6e-15 at 9.  There the orders
 // are products of their own: downward recursion for both ranges gave 1.0e-15 at
-// M = 4 (the direct build of C20H42 44.4 ms with it, 44.65 so, 44.4 with nine
-// coefficients).
+// M = 4 (direct builds of C20H42 and H2O 44.6 and 0.250 ms with it, 44.9 and 0.252
+// so, 44.4 and 0.247 with nine coefficients).  Even and odd coefficients side by side,
+// a shorter chain of more operations, took 45.3 ms and 14.05 for the (H2O)8 gradient's
+// 13.5.
 //
 // The three- and two-index integrals (k_eri3, k_eri2) keep nine coefficients and
 // the asymptotic value of F_M carried down: the fitted tensor made of them is split
@@ -159,55 +161,73 @@ __device__ __forceinline__ double rsqrt_pos(double x) {
   return y + y * h * (0.5 + 0.375 * h);
 }
 
+// Row of the interval that holds T and T's distance d from its centre.
+__device__ __forceinline__ const double* boys_row(double T, const double* tab, double& d) {
+  // nearest multiple of the width, by the rounding of an addition to 1.5 2^52
+  const double u = T * (1.0 / BOYSP_WIDTH) + 6755399441055744.0;
+  d = T - (u - 6755399441055744.0) * BOYSP_WIDTH;
+  return tab + __double2loint(u) * BOYSP_ROW;
+}
+template <int NC>
+__device__ __forceinline__ double boys_horner(const double* c, double d) {
+  double acc = c[NC - 1];
+#pragma unroll
+  for (int j = NC - 2; j >= 0; --j) acc = acc * d + c[j];
+  return acc;
+}
+__device__ __forceinline__ double exp_minus(double d) {  // e^{-d}, |d| <= 3/16
+  double x = -2.7579345743837904673e-6;
+  x = x * d + 2.4825818086831339934e-5;
+  x = x * d - 1.9841263064743021626e-4;
+  x = x * d + 1.3888881434054876645e-3;
+  x = x * d - 8.3333333341842252384e-3;
+  x = x * d + 4.1666666676027388464e-2;
+  x = x * d - 1.6666666666666292731e-1;
+  x = x * d + 0.49999999999995886287;
+  x = x * d - 1.0;
+  return x * d + 1.0;
+}
+template <int M>
+__device__ __forceinline__ void boys_down(double T, double e, double* F) {
+  const double T2 = 2.0 * T;
+#pragma unroll
+  for (int m = M - 1; m >= 0; --m) F[m] = (T2 * F[m + 1] + e) * (1.0 / (2 * m + 1));
+}
+
 template <int M, int NC = BOYSP_COEF>
 __device__ __forceinline__ void boys_poly(double T, const double* tab, double* F) {
   static_assert(M <= BOYSP_MMAX, "Boys order too high");
   static_assert(NC == BOYSP_COEF || NC == BOYSP_COEF_DF, "no such table");
-  double e = 0.0;
-  if (T < boysp_tmax(M)) {
-    // nearest multiple of the width, by the rounding of an addition to 1.5 2^52
-    const double u = T * (1.0 / BOYSP_WIDTH) + 6755399441055744.0;
-    const int row = __double2loint(u);
-    const double d = T - (u - 6755399441055744.0) * BOYSP_WIDTH;
-    const double* c = tab + row * BOYSP_ROW;
-    double acc = c[NC - 1];
+  double d;
+  if constexpr (NC == BOYSP_COEF) {
+    if (T < boysp_tmax(M)) {
+      const double* c = boys_row(T, tab, d);
+      F[M] = boys_horner<NC>(c, d);
+      if constexpr (M > 0) boys_down<M>(T, exp_minus(d) * c[NC], F);
+    } else {  // Gamma(m + 1/2)/2 T^{-m-1/2}
+      const double r = rsqrt_pos(T);
+      double f = r, r2 = r * r;
+      r2 = r2 + r2 * (1.0 - T * r2);  // r's rounding would be in every factor
 #pragma unroll
-    for (int j = NC - 2; j >= 0; --j) acc = acc * d + c[j];
-    F[M] = acc;
-    if constexpr (M > 0) {
-      double x = -2.7579345743837904673e-6;  // e^{-d}, |d| <= 3/16
-      x = x * d + 2.4825818086831339934e-5;
-      x = x * d - 1.9841263064743021626e-4;
-      x = x * d + 1.3888881434054876645e-3;
-      x = x * d - 8.3333333341842252384e-3;
-      x = x * d + 4.1666666676027388464e-2;
-      x = x * d - 1.6666666666666292731e-1;
-      x = x * d + 0.49999999999995886287;
-      x = x * d - 1.0;
-      x = x * d + 1.0;
-      e = x * c[NC];
+      for (int m = 0; m <= M; ++m) {
+        F[m] = boys_gamma(m) * f;
+        f *= r2;
+      }
     }
-  } else if constexpr (NC == BOYSP_COEF) {  // Gamma(m + 1/2)/2 T^{-m-1/2}
-    const double r = rsqrt_pos(T);
-    double f = r, r2 = r * r;
-    r2 = r2 + r2 * (1.0 - T * r2);  // r's rounding would be in every factor
-#pragma unroll
-    for (int m = 0; m <= M; ++m) {
-      F[m] = boys_gamma(m) * f;
-      f *= r2;
-    }
-    return;
   } else {
-    const double r = rsqrt_pos(T), r2 = r * r;
-    double f = 0.886226925452758014 * r;
+    double e = 0.0;
+    if (T < boysp_tmax(M)) {
+      const double* c = boys_row(T, tab, d);
+      F[M] = boys_horner<NC>(c, d);
+      if constexpr (M > 0) e = exp_minus(d) * c[NC];
+    } else {
+      const double r = rsqrt_pos(T), r2 = r * r;
+      double f = 0.886226925452758014 * r;
 #pragma unroll
-    for (int m = 0; m < M; ++m) f *= (m + 0.5) * r2;
-    F[M] = f;
-  }
-  if constexpr (M > 0) {
-    const double T2 = 2.0 * T;
-#pragma unroll
-    for (int m = M - 1; m >= 0; --m) F[m] = (T2 * F[m + 1] + e) * (1.0 / (2 * m + 1));
+      for (int m = 0; m < M; ++m) f *= (m + 0.5) * r2;
+      F[M] = f;
+    }
+    if constexpr (M > 0) boys_down<M>(T, e, F);
   }
 }
 
